@@ -31,9 +31,8 @@ namespace bl {
 
 constexpr int QBM = 128;                  // weight rows per tile (MMA M)
 constexpr int QBK = 128;                  // depth per stage: two swizzle atoms of 64 values
-constexpr int QATOM_A = QBM * 128;        // 16 KiB: 128 rows of 128 bytes
-constexpr int QPRODUCERS = 256;           // threads that expand weights: (row, half of the stage's depth)
-constexpr int QTHREADS = 192 + QPRODUCERS;
+constexpr int QPRODUCERS = 512;           // threads that expand weights: four per weight row
+constexpr int QTHREADS = 256 + QPRODUCERS;
 
 struct QTile { int group, row0, row_end, pad; };   // token tile: rows row0 .. of X use weight matrix `group`
 
@@ -54,6 +53,10 @@ struct QGemmArgs {
   const float* resid;         // optional addend, indexed like the output
   long ldr;
   unsigned* status;
+  int fixed_tiles;            // the table holds max_tiles tiles and was written before the launches in flight
+  int splits;                 // CTAs that share a tile's depth (1 with w2)
+  float* partial;             // splits > 1: [tiles][splits][tile rows][128] sums
+  int* tickets;               // splits > 1: four per tile, zero between launches
 };
 
 __device__ __forceinline__ uint4 q_pack8(const float* v) {
@@ -65,30 +68,11 @@ __device__ __forceinline__ uint4 q_pack8(const float* v) {
   return o;
 }
 
-// Unit u (64 values of row `row`) of stage kb into the swizzled A stage at `sa`: value position p of the stage lives in
-// atom p / 64, row `row`, 16-byte chunk ((p % 64) / 8) ^ (row % 8).
-template <class T>
-__device__ __forceinline__ void expand_unit(const typename Unit<T>::Regs& regs, int u, int kb, int row, uint8_t* sa) {
-  float v[64];
-  Unit<T>::decodeu(regs, u, v);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int p = Unit<T>::pos(u, 8 * j) - QBK * kb;
-    const int atom = p >> 6, ch = (p & 63) >> 3;
-    *reinterpret_cast<uint4*>(sa + atom * QATOM_A + row * 128 + ((ch ^ (row & 7)) << 4)) = q_pack8(v + 8 * j);
-  }
-}
-
 // ---- fast expanders ---------------------------------------------------------------------
 // Integer-to-float conversions run at a quarter of the FMA rate, so the K-quant expanders avoid them.
-//   exact form (token tiles of 128, i.e. prompts): a code byte q (< 128) dropped into mantissa bits 16..22 of 1.0f
-//   reads as X = 1 + q / 128, and the block's affine map v = s * q + o becomes one FMA
-//   v = (128 s) * X + (o - 128 s) on a packed pair (fma.rn.f32x2), rounded to bf16 once.  The result equals the fp32
-//   decode to within an fp32 rounding of the offset.
-//   short form (token tiles of 32 / 64, i.e. decode batches, where the expanders are the bottleneck): two code bytes
-//   become the bf16 pair (128 + q0, 128 + q1) with one byte permute, a packed bf16 subtract gives (q0, q1) exactly and
-//   a packed bf16 FMA gives s * q + o with s and o rounded to bf16: 1.5 instructions per value, at most about one
-//   more bf16 ulp of error per weight than the exact form.
+//   A code byte q (< 128) dropped into mantissa bits 16..22 of 1.0f reads as X = 1 + q / 128, and the block's affine map
+//   v = s * q + o becomes one FMA v = (128 s) * X + (o - 128 s) on a packed pair (fma.rn.f32x2), rounded to bf16 once.
+//   The result equals the fp32 decode to within an fp32 rounding of the offset.
 // FastUnit<T>::codes yields the unit's 64 code bytes in value order (16 words; word w belongs to group w / 4) and the
 // (scale, offset) pair of each of the four groups of 16 values.
 template <class T> struct FastUnit { static constexpr bool kHas = false; };
@@ -159,50 +143,17 @@ __device__ __forceinline__ uint4 fast8(uint32_t w0, uint32_t w1, float a, float 
   return out;
 }
 
-// bf16x2 FMA / subtract on raw register pairs
+// bf16x2 FMA on raw register pairs
 __device__ __forceinline__ uint32_t bf2_fma(uint32_t a, uint32_t b, uint32_t c) {
   uint32_t d;
   asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-  return d;
-}
-__device__ __forceinline__ uint32_t bf2_sub(uint32_t a, uint32_t b) {
-  uint32_t d;
-  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
 }
 __device__ __forceinline__ uint32_t bf2_dup(float v) {
   __nv_bfloat162 p = __float2bfloat162_rn(v);
   return *reinterpret_cast<uint32_t*>(&p);
 }
-__device__ __forceinline__ uint4 short8(uint32_t w0, uint32_t w1, uint32_t s2, uint32_t o2) {
-  constexpr uint32_t k128 = 0x43004300u;                       // (128, 128) in bf16
-  uint4 out;
-  out.x = bf2_fma(bf2_sub(__byte_perm(w0, k128, 0x5150), k128), s2, o2);   // bytes (low to high): q0, 0x43, q1, 0x43
-  out.y = bf2_fma(bf2_sub(__byte_perm(w0, k128, 0x5352), k128), s2, o2);
-  out.z = bf2_fma(bf2_sub(__byte_perm(w1, k128, 0x5150), k128), s2, o2);
-  out.w = bf2_fma(bf2_sub(__byte_perm(w1, k128, 0x5352), k128), s2, o2);
-  return out;
-}
 
-template <class T, bool SHORT>
-__device__ __forceinline__ void expand_unit_fast(const typename Unit<T>::Regs& regs, int u, int kb, int row, uint8_t* sa) {
-  uint32_t cw[16];
-  float s[4], o[4];
-  FastUnit<T>::codes(regs, u, cw, s, o);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int g = j >> 1;
-    const int p = Unit<T>::pos(u, 8 * j) - QBK * kb;
-    const int atom = p >> 6, ch = (p & 63) >> 3;
-    uint4* dst = reinterpret_cast<uint4*>(sa + atom * QATOM_A + row * 128 + ((ch ^ (row & 7)) << 4));
-    if (SHORT) {
-      *dst = short8(cw[2 * j], cw[2 * j + 1], bf2_dup(s[g]), bf2_dup(o[g]));
-    } else {
-      const float a = 128.0f * s[g], c = o[g] - a;
-      *dst = fast8(cw[2 * j], cw[2 * j + 1], a, c);
-    }
-  }
-}
 // ---- float-coded types ---------------------------------------------------------------------
 // ChunkUnit<T>::chunk(regs, j) yields values 8j .. 8j+7 of the unit as eight bf16, never holding the unit's 64 floats.
 //   FP8 (E4M3 codes, one f32 scale per 128 values): the hardware converter takes two codes to an f16 pair; the pair
@@ -260,124 +211,119 @@ template <> struct ChunkUnit<NvFp4> {
   }
 };
 
+// Unit u (64 values of this thread's weight row) of stage kb into the A operand in tensor memory: lane = weight row,
+// 32-bit column c of the stage holds values 2c and 2c + 1.  A unit's groups of 16 values are contiguous in the row, so
+// each is one 8-column store.  Warp-collective.
 template <class T>
-__device__ __forceinline__ void expand_unit_chunks(const typename Unit<T>::Regs& regs, int u, int kb, int row, uint8_t* sa) {
-  const typename ChunkUnit<T>::Pre pr = ChunkUnit<T>::pre(regs);
+__device__ __forceinline__ void expand_unit(const typename Unit<T>::Regs& regs, int u, int kb, uint32_t ta) {
+  auto put = [&](int g, const uint4& x, const uint4& y) {
+    tmem_st8(ta + (uint32_t)((Unit<T>::pos(u, 16 * g) - QBK * kb) >> 1), x, y);
+  };
+  if constexpr (FastUnit<T>::kHas) {
+    uint32_t cw[16];
+    float s[4], o[4];
+    FastUnit<T>::codes(regs, u, cw, s, o);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int p = Unit<T>::pos(u, 8 * j) - QBK * kb;
-    const int atom = p >> 6, ch = (p & 63) >> 3;
-    *reinterpret_cast<uint4*>(sa + atom * QATOM_A + row * 128 + ((ch ^ (row & 7)) << 4)) = ChunkUnit<T>::chunk(regs, pr, j);
+    for (int g = 0; g < 4; ++g) {
+      const float a = 128.0f * s[g], c = o[g] - a;
+      put(g, fast8(cw[4 * g], cw[4 * g + 1], a, c), fast8(cw[4 * g + 2], cw[4 * g + 3], a, c));
+    }
+  } else if constexpr (ChunkUnit<T>::kHas) {
+    const typename ChunkUnit<T>::Pre pr = ChunkUnit<T>::pre(regs);
+#pragma unroll
+    for (int g = 0; g < 4; ++g) put(g, ChunkUnit<T>::chunk(regs, pr, 2 * g), ChunkUnit<T>::chunk(regs, pr, 2 * g + 1));
+  } else {
+    float v[64];
+    Unit<T>::decodeu(regs, u, v);
+#pragma unroll
+    for (int g = 0; g < 4; ++g) put(g, q_pack8(v + 16 * g), q_pack8(v + 16 * g + 8));
   }
 }
 
-template <class T, bool SHORT>
-__device__ __forceinline__ void expand_any(const typename Unit<T>::Regs& regs, int u, int kb, int row, uint8_t* sa) {
-  if constexpr (FastUnit<T>::kHas) expand_unit_fast<T, SHORT>(regs, u, kb, row, sa);
-  else if constexpr (ChunkUnit<T>::kHas) expand_unit_chunks<T>(regs, u, kb, row, sa);
-  else expand_unit<T>(regs, u, kb, row, sa);
-}
-
-__host__ __device__ constexpr int q_stages(bool dual, int bn) {
-  const int stage = (dual ? 2 : 1) * 2 * QATOM_A + 2 * bn * 128;
-  const int n = (220 * 1024) / stage;
-  return n > 4 ? 4 : n;
-}
 // Raw ring: slots of [matrices][128 rows][super-block bytes]; 0 slots = the register-load path.
 template <class T> struct SbBytes { static constexpr int v = 0; };
 template <> struct SbBytes<Q4K> { static constexpr int v = Q4K::kSbBytes; };
 template <> struct SbBytes<Q5K> { static constexpr int v = Q5K::kSbBytes; };
 template <> struct SbBytes<Q6K> { static constexpr int v = Q6K::kSbBytes; };
+// Tensor memory (512 columns): accumulators of all tokens first (two sets; one for gate+up at 128 tokens, where two
+// would leave nothing), the A stages behind them.
+__host__ __device__ constexpr int q_accs(bool dual, int bn) { return (dual ? 2 : 1) * bn > 128 ? 1 : 2; }
+__host__ __device__ constexpr int q_stages(bool dual, int bn) {
+  const int n = (512 - q_accs(dual, bn) * (dual ? 2 : 1) * bn) / ((dual ? 2 : 1) * (QBK / 2));
+  return n > 6 ? 6 : n;
+}
 __host__ __device__ constexpr int q_raw_slots(int sb_bytes, bool dual, int bn) {
   if (sb_bytes == 0) return 0;
-  const int stage = (dual ? 2 : 1) * 2 * QATOM_A + 2 * bn * 128;
-  const int raw = (dual ? 2 : 1) * QBM * sb_bytes;
-  const int n = (220 * 1024 - 2 * stage) / raw;
-  const int cap = dual ? 2 : 4;                                    // super-blocks in flight per SM; the rest goes to stages
-  return n > cap ? cap : (n < 0 ? 0 : n);
-}
-__host__ __device__ constexpr int q_stages_raw(int sb_bytes, bool dual, int bn) {
-  const int stage = (dual ? 2 : 1) * 2 * QATOM_A + 2 * bn * 128;
-  const int raw = (dual ? 2 : 1) * QBM * sb_bytes;
-  const int n = (220 * 1024 - q_raw_slots(sb_bytes, dual, bn) * raw) / stage;
-  return n > 4 ? 4 : n;
-}
-__host__ __device__ constexpr int q_tmem_cols(bool dual, int bn) {
-  const int need = 2 * (dual ? 2 : 1) * bn;
-  return need <= 32 ? 32 : need <= 64 ? 64 : need <= 128 ? 128 : need <= 256 ? 256 : 512;
+  const int n = (220 * 1024 - q_stages(dual, bn) * 2 * bn * 128) / ((dual ? 2 : 1) * QBM * sb_bytes);
+  return n > 6 ? 6 : n;
 }
 
-// 448 threads: warp 0 = TMA producer of the token tiles, warp 1 = MMA issuer and TMEM owner, warps 2..5 = epilogue
-// (warp id modulo 4 = TMEM lane quarter), warps 6..13 = weight expanders.
+// 768 threads: warp 0 = TMA of the token tiles, warp 1 = MMA issuer and TMEM owner, warps 2..5 = epilogue, warp 6 = TMA
+// of the raw weight super-blocks, warp 7 idle, warps 8..23 = weight expanders (warp id modulo 4 = TMEM lane quarter).
 template <class T, bool DUAL, int BN>
 __global__ void __launch_bounds__(QTHREADS, 1)
 qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUtensorMap tma_w,
              const __grid_constant__ CUtensorMap tma_w2, const QGemmArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   constexpr int SB = SbBytes<T>::v;
+  constexpr int STAGES = q_stages(DUAL, BN);
   constexpr int RS = q_raw_slots(SB, DUAL, BN);                      // raw ring slots (0: register loads)
   constexpr int RAW_MAT = QBM * SB;                                  // one matrix's 128 super-blocks
   constexpr int RAW_SLOT = (DUAL ? 2 : 1) * RAW_MAT;
-  constexpr int STAGES = RS > 0 ? q_stages_raw(SB, DUAL, BN) : q_stages(DUAL, BN);
-  constexpr int A_BYTES = 2 * QATOM_A;
   constexpr int B_ATOM = BN * 128;
-  constexpr int STAGE_BYTES = (DUAL ? 2 : 1) * A_BYTES + 2 * B_ATOM;
-  constexpr int B_OFF = (DUAL ? 2 : 1) * A_BYTES;
+  constexpr int B_STAGE = 2 * B_ATOM;
+  constexpr int NACC = q_accs(DUAL, BN);
   constexpr int ACC_COLS = (DUAL ? 2 : 1) * BN;
-  constexpr int TMEM_COLS = q_tmem_cols(DUAL, BN);
+  constexpr int A_MAT = QBK / 2;                                     // columns of one matrix's stage
+  constexpr int A_COLS = (DUAL ? 2 : 1) * A_MAT;
+  constexpr int FILLERS = DUAL ? QPRODUCERS / 32 : QPRODUCERS / 64;  // warps that write one stage
   __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
   __shared__ __align__(8) uint64_t raw_full[RS > 0 ? RS : 1], raw_empty[RS > 0 ? RS : 1];
-  uint8_t* const raw_ring = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023) + (size_t)STAGES * STAGE_BYTES;
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t* const raw_ring = smem + (size_t)STAGES * B_STAGE;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1 + QPRODUCERS / 32); mbar_init(&empty_bar[s], 1); }
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1 + FILLERS); mbar_init(&empty_bar[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4); }
     for (int r = 0; r < RS; ++r) { mbar_init(&raw_full[r], 1); mbar_init(&raw_empty[r], QPRODUCERS / 32); }
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)), "r"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  pdl_wait();
-  pdl_launch();
+  // Weights never change, and neither does the tile table of a dense product: its weight stream starts while the launch
+  // that writes the activations still runs.  Every other role waits for that launch.
+  if (!(a.fixed_tiles && warp >= 6)) {
+    pdl_wait();
+    pdl_launch();
+  }
   const uint32_t tmem_base = s_tmem_base;
+  const uint32_t tmem_a = tmem_base + NACC * ACC_COLS;
   volatile int* abort_flag = &s_abort;
 
-  const int n_tt = min(*a.n_tiles, a.max_tiles);
-  const int total_tiles = n_tt * a.tiles_w;
-  const int kblocks = a.K / QBK;
+  const int n_tt = a.fixed_tiles ? a.max_tiles : min(*a.n_tiles, a.max_tiles);
+  const int total_tiles = n_tt * a.tiles_w * a.splits;
+  const int kblocks = a.K / QBK / a.splits;                          // stages of one tile: an even number
 
   if (warp == 0) {
     if (lane == 0) {
       int stage = 0; uint32_t phase = 0;
-      int rslot = 0; uint32_t rphase = 0;
       int issued = 0;
       for (int t = blockIdx.x; t < total_tiles && !*abort_flag; t += gridDim.x) {
-        const QTile mt = a.tiles[t / a.tiles_w];
-        const int n0 = (t % a.tiles_w) * QBM;
-        for (int kb = 0; kb < kblocks; ++kb) {
-          if (RS > 0 && (kb & 1) == 0) {
-            // the super-block of stages kb and kb + 1: rows n0 .. n0 + 127 of the group's matrix (rows past the
-            // matrix arrive as zeros and are never stored)
-            if (!mbar_wait(&raw_empty[rslot], rphase ^ 1, abort_flag)) break;
-            uint8_t* dst = raw_ring + (size_t)rslot * RAW_SLOT;
-            mbar_expect_tx(&raw_full[rslot], RAW_SLOT);
-            tma_load_3d(dst, &tma_w, (kb >> 1) * SB, n0, mt.group, &raw_full[rslot]);
-            if (DUAL) tma_load_3d(dst + RAW_MAT, &tma_w2, (kb >> 1) * SB, n0, mt.group, &raw_full[rslot]);
-            if (++rslot == RS) { rslot = 0; rphase ^= 1; }
-          }
+        const QTile mt = a.tiles[t / a.splits / a.tiles_w];
+        const int kb0 = (t % a.splits) * kblocks;
+        for (int kb = kb0; kb < kb0 + kblocks; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) break;
-          uint8_t* sb = smem + (size_t)stage * STAGE_BYTES + B_OFF;
-          mbar_expect_tx(&full_bar[stage], 2 * B_ATOM);
+          uint8_t* sb = smem + (size_t)stage * B_STAGE;
+          mbar_expect_tx(&full_bar[stage], B_STAGE);
           tma_load_2d(sb, &tma_x, kb * QBK, mt.row0, &full_bar[stage]);
           tma_load_2d(sb + B_ATOM, &tma_x, kb * QBK + 64, mt.row0, &full_bar[stage]);
           ++issued;
@@ -396,8 +342,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
       int stage = 0; uint32_t phase = 0;
       int it = 0;
       for (int t = blockIdx.x; t < total_tiles && !*abort_flag; t += gridDim.x) {
-        const int ab = it & 1;
-        const uint32_t acc_phase = (it >> 1) & 1;
+        const int ab = it % NACC;
+        const uint32_t acc_phase = (it / NACC) & 1;
         ++it;
         if (!mbar_wait(&acc_empty[ab], acc_phase ^ 1, abort_flag)) break;
         tc_fence_after();
@@ -406,17 +352,14 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + (size_t)stage * STAGE_BYTES);
+          const uint32_t sb = smem_u32(smem + (size_t)stage * B_STAGE);
+          const uint32_t ta = tmem_a + stage * A_COLS;
 #pragma unroll
-          for (int atom = 0; atom < 2; ++atom) {
-            const uint64_t da = umma_desc(sa + atom * QATOM_A), db = umma_desc(sa + B_OFF + atom * B_ATOM);
-#pragma unroll
-            for (int k = 0; k < 64 / UMMA_K; ++k) {
-              const uint32_t acc = (kb > 0 || atom > 0 || k > 0) ? 1u : 0u;
-              const uint64_t step = (uint64_t)(k * UMMA_K * 2 / 16);
-              umma_bf16(d0, da + step, db + step, idesc, acc);
-              if (DUAL) umma_bf16(d0 + BN, umma_desc(sa + A_BYTES + atom * QATOM_A) + step, db + step, idesc, acc);
-            }
+          for (int k = 0; k < QBK / UMMA_K; ++k) {
+            const uint64_t db = umma_desc(sb + (k >> 2) * B_ATOM) + (uint64_t)((k & 3) * UMMA_K * 2 / 16);
+            const uint32_t acc = (kb > 0 || k > 0) ? 1u : 0u;
+            umma_bf16_ta(d0, ta + k * (UMMA_K / 2), db, idesc, acc);
+            if (DUAL) umma_bf16_ta(d0 + BN, ta + A_MAT + k * (UMMA_K / 2), db, idesc, acc);
           }
           umma_commit(&empty_bar[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -428,107 +371,173 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
   } else if (warp < 6) {
     const int q = warp & 3;
     int it = 0;
-    for (int t = blockIdx.x; t < total_tiles && !*abort_flag; t += gridDim.x) {
-      const QTile mt = a.tiles[t / a.tiles_w];
-      const int n = (t % a.tiles_w) * QBM + q * 32 + lane;         // weight row = output column of this thread
+    for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
+      const int tile = t / a.splits;
+      const QTile mt = a.tiles[tile / a.tiles_w];
+      const int n = (tile % a.tiles_w) * QBM + q * 32 + lane;      // weight row = output column of this thread
       const bool n_ok = n < a.N;
-      const int ab = it & 1;
-      const uint32_t acc_phase = (it >> 1) & 1;
+      const int ab = it % NACC;
+      const uint32_t acc_phase = (it / NACC) & 1;
       ++it;
-      if (!mbar_wait(&acc_full[ab], acc_phase, abort_flag)) break;
+      if (!__all_sync(0xFFFFFFFFu, mbar_wait(&acc_full[ab], acc_phase, abort_flag))) break;
       tc_fence_after();
       const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + ab * ACC_COLS;
+      const int n_rows = min(BN, mt.row_end - mt.row0);            // token rows of this tile
+      // partial sums of a split tile: [tile][split][token][128 weight rows]
+      float* const part = a.partial + (long)tile * a.splits * (BN * QBM) + q * 32 + lane;
+      bool mine = true;                                            // this warp finishes its quarter of the tile
+      if (!DUAL && a.splits > 1) {
+        float* const own = part + (long)(t % a.splits) * (BN * QBM);
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        if (mt.row0 + c * 32 >= mt.row_end) break;
-        uint32_t v[32], u[32];
-        tmem_ld32(tbase + c * 32, v);
-        if (DUAL) tmem_ld32(tbase + BN + c * 32, u);
-        tmem_ld_wait();
-        // lane i fetches the routing of token row i of this chunk; the store loop broadcasts it
-        const int r_l = mt.row0 + c * 32 + lane;
-        int orow_l = -1;
-        float sc_l = 1.0f;
-        if (r_l < mt.row_end) {
-          orow_l = a.dst_row ? a.dst_row[r_l] : r_l;
-          if (a.row_scale) sc_l = a.row_scale[r_l];
-        }
+        for (int c = 0; c < n_rows; c += 16) {
+          uint32_t v[16];
+          tmem_ld16(tbase + c, v);
+          tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int orow = __shfl_sync(0xFFFFFFFFu, orow_l, i);
-          const float sc = __shfl_sync(0xFFFFFFFFu, sc_l, i);
-          if (orow < 0 || !n_ok) continue;
-          float f = __uint_as_float(v[i]);
-          if (DUAL) f = (f / (1.0f + __expf(-f))) * __uint_as_float(u[i]);
-          f *= sc;
-          if (a.resid) f += a.resid[(long)orow * a.ldr + n];
-          if (a.c_f32) a.c_f32[(long)orow * a.ldc + n] = f;
-          else a.c_bf16[(long)orow * a.ldc + n] = __float2bfloat16_rn(f);
+          for (int i = 0; i < 16; ++i) __stcg(own + (c + i) * QBM, __uint_as_float(v[i]));
+        }
+        __threadfence();
+        __syncwarp();
+        int last = 0;
+        if (lane == 0) {
+          last = atomicAdd(&a.tickets[tile * 4 + q], 1) == a.splits - 1;
+          if (last) a.tickets[tile * 4 + q] = 0;                   // ready for the next launch
+        }
+        mine = __shfl_sync(0xFFFFFFFFu, last, 0) != 0;
+        if (mine) __threadfence();
+      }
+      if (mine) {
+#pragma unroll 1
+        for (int c = 0; c < n_rows; c += 16) {
+          uint32_t v[16], u[DUAL ? 16 : 1];
+          if (!DUAL && a.splits > 1) {
+            // the splits' sums are added in ascending order whichever warp arrived last: same bits on every run
+            float f[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) f[i] = 0.f;
+            for (int sp = 0; sp < a.splits; ++sp)
+#pragma unroll
+              for (int i = 0; i < 16; ++i) f[i] += __ldcg(part + (long)sp * (BN * QBM) + (c + i) * QBM);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(f[i]);
+          } else {
+            tmem_ld16(tbase + c, v);
+            if constexpr (DUAL) tmem_ld16(tbase + BN + c, u);
+            tmem_ld_wait();
+          }
+          // lane i fetches the routing of token row i of this chunk; the store loop broadcasts it
+          const int r_l = mt.row0 + c + (lane & 15);
+          int orow_l = -1;
+          float sc_l = 1.0f;
+          if (r_l < mt.row_end) {
+            orow_l = a.dst_row ? a.dst_row[r_l] : r_l;
+            if (a.row_scale) sc_l = a.row_scale[r_l];
+          }
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const int orow = __shfl_sync(0xFFFFFFFFu, orow_l, i);
+            const float sc = __shfl_sync(0xFFFFFFFFu, sc_l, i);
+            if (orow < 0 || !n_ok) continue;
+            float f = __uint_as_float(v[i]);
+            if constexpr (DUAL) f = (f / (1.0f + __expf(-f))) * __uint_as_float(u[i]);
+            f *= sc;
+            if (a.resid) f += a.resid[(long)orow * a.ldr + n];
+            if (a.c_f32) a.c_f32[(long)orow * a.ldc + n] = f;
+            else a.c_bf16[(long)orow * a.ldc + n] = __float2bfloat16_rn(f);
+          }
         }
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[ab]);
     }
-  } else {
-    // Producer thread = (weight row, part): in dual mode the part is the matrix (gate / up) and the thread expands both
-    // units of the stage; otherwise the part is the unit.  The blocks of stage kb + 1 are fetched into a second register
-    // set before stage kb is decoded, so a load has a whole decode (and the wait for the ring) to land.
+  } else if (warp == 6) {
+    if (RS > 0 && lane == 0) {
+      int rslot = 0; uint32_t rphase = 0;
+      int issued = 0;
+      for (int t = blockIdx.x; t < total_tiles && !*abort_flag; t += gridDim.x) {
+        const int tile = t / a.splits;
+        const int group = a.tiles[tile / a.tiles_w].group;
+        const int n0 = (tile % a.tiles_w) * QBM;
+        const int sb0 = (t % a.splits) * (kblocks / 2);
+        for (int sbi = sb0; sbi < sb0 + kblocks / 2; ++sbi) {
+          // rows n0 .. n0 + 127 of the group's matrix (rows past the matrix arrive as zeros and are never stored)
+          if (!mbar_wait(&raw_empty[rslot], rphase ^ 1, abort_flag)) break;
+          uint8_t* dst = raw_ring + (size_t)rslot * RAW_SLOT;
+          mbar_expect_tx(&raw_full[rslot], RAW_SLOT);
+          tma_load_3d(dst, &tma_w, sbi * SB, n0, group, &raw_full[rslot]);
+          if (DUAL) tma_load_3d(dst + RAW_MAT, &tma_w2, sbi * SB, n0, group, &raw_full[rslot]);
+          ++issued;
+          if (++rslot == RS) { rslot = 0; rphase ^= 1; }
+        }
+      }
+      if (*abort_flag) {
+        unsigned long long t0 = globaltimer();
+        while (issued > 0 && globaltimer() - t0 < 2000000ull) {}
+      }
+    }
+  } else if (warp >= 8) {
+    // Four groups of four warps, one per TMEM lane quarter: thread = weight row.  Gate+up: every group expands one unit
+    // (matrix grp / 2, unit grp % 2) of every stage; one matrix: groups 0 and 1 the even stages, 2 and 3 the odd ones.
     using U = Unit<T>;
-    constexpr int NU = DUAL ? 2 : 1;
-    const int pt = threadIdx.x - 192;
-    const int row = pt & 127, part = pt >> 7;
-    int stage = 0; uint32_t phase = 0;
+    constexpr int STEP = DUAL ? 1 : 2;                               // stages from one item of a group to its next
+    const int grp = (warp - 8) >> 2, q = warp & 3;
+    const int row = q * 32 + lane, mat = DUAL ? grp >> 1 : 0, half = grp & 1;
+    const int kb_first = DUAL ? 0 : grp >> 1;
+    const uint32_t ta0 = tmem_a + ((uint32_t)(q * 32) << 16) + mat * A_MAT;
+    unsigned lin = (unsigned)kb_first;                               // stages of this CTA so far, over all its tiles
     bool ok = true;
-    auto fetch = [&](const uint8_t* wrow, int kb, typename U::Regs (&r)[NU]) {
-#pragma unroll
-      for (int i = 0; i < NU; ++i) U::loadu(wrow, 2 * kb + (DUAL ? i : part), a.K, r[i]);
-    };
-    auto emit = [&](int kb, const typename U::Regs (&r)[NU]) {
-      if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) { ok = false; return; }
+    auto emit = [&](int kb, const typename U::Regs& r) {
+      const unsigned stage = lin % STAGES, phase = (lin / STAGES) & 1;
+      lin += STEP;
+      ok = __all_sync(0xFFFFFFFFu, mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag));
+      if (!ok) return;
       tc_fence_after();
-      uint8_t* sa = smem + (size_t)stage * STAGE_BYTES + (DUAL ? part * A_BYTES : 0);
-#pragma unroll
-      for (int i = 0; i < NU; ++i) expand_any<T, (BN < 128)>(r[i], 2 * kb + (DUAL ? i : part), kb, row, sa);
-      fence_async_smem();
+      expand_unit<T>(r, 2 * kb + half, kb, ta0 + stage * A_COLS);
+      tmem_st_wait();
+      tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&full_bar[stage]);
-      if (++stage == STAGES) { stage = 0; phase ^= 1; }
     };
     if constexpr (RS > 0) {
       // raw ring: the tile's super-blocks arrive by TMA; a thread reads its row's units out of shared memory
       int rslot = 0; uint32_t rphase = 0;
-      for (int t = blockIdx.x; t < total_tiles && ok && !*abort_flag; t += gridDim.x) {
-        for (int sbi = 0; sbi < kblocks / 2 && ok; ++sbi) {
-          if (!mbar_wait(&raw_full[rslot], rphase, abort_flag)) { ok = false; break; }
-          const uint8_t* rawrow = raw_ring + (size_t)rslot * RAW_SLOT + (DUAL ? part * RAW_MAT : 0) + row * SB - (long)sbi * SB;
+      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+        const int sb0 = (t % a.splits) * (kblocks / 2);
+        for (int sbi = sb0; sbi < sb0 + kblocks / 2 && ok; ++sbi) {
+          ok = __all_sync(0xFFFFFFFFu, mbar_wait(&raw_full[rslot], rphase, abort_flag));
+          if (!ok) break;
+          const uint8_t* rawrow = raw_ring + (size_t)rslot * RAW_SLOT + mat * RAW_MAT + row * SB - (long)sbi * SB;
+          typename U::Regs r[DUAL ? 2 : 1];
 #pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            const int kb = 2 * sbi + half;
-            typename U::Regs r[NU];
-            fetch(rawrow, kb, r);
-            emit(kb, r);
-            if (!ok) break;
-          }
+          for (int h = 0; h < (DUAL ? 2 : 1); ++h) U::loadu(rawrow, 2 * (2 * sbi + h + kb_first) + half, a.K, r[h]);
           __syncwarp();
           if (lane == 0) mbar_arrive(&raw_empty[rslot]);
           if (++rslot == RS) { rslot = 0; rphase ^= 1; }
+#pragma unroll
+          for (int h = 0; h < (DUAL ? 2 : 1); ++h)
+            if (ok) emit(2 * sbi + h + kb_first, r[h]);
         }
       }
-    } else
-    for (int t = blockIdx.x; t < total_tiles && ok && !*abort_flag; t += gridDim.x) {
-      const QTile mt = a.tiles[t / a.tiles_w];
-      int n = (t % a.tiles_w) * QBM + row;
-      n = n < a.N ? n : a.N - 1;                                   // rows past the matrix repeat the last one (never stored)
-      const uint8_t* wrow = (DUAL && part ? a.w2 : a.w) + (long)mt.group * a.group_bytes + (long)n * a.row_bytes;
-      typename U::Regs ra[NU], rb[NU];
-      fetch(wrow, 0, ra);
-      for (int kb = 0; kb < kblocks && ok; kb += 2) {
-        if (kb + 1 < kblocks) fetch(wrow, kb + 1, rb);
-        emit(kb, ra);
-        if (!ok) break;
-        if (kb + 2 < kblocks) fetch(wrow, kb + 2, ra);
-        if (kb + 1 < kblocks) emit(kb + 1, rb);
+    } else {
+      // the blocks of a group's next item are fetched before the present one is decoded
+      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+        const int tile = t / a.splits;
+        const int group = a.tiles[tile / a.tiles_w].group;
+        int n = (tile % a.tiles_w) * QBM + row;
+        n = n < a.N ? n : a.N - 1;                                   // rows past the matrix repeat the last one (never stored)
+        const uint8_t* wrow = (mat ? a.w2 : a.w) + (long)group * a.group_bytes + (long)n * a.row_bytes;
+        const int kb0 = (t % a.splits) * kblocks, kend = kb0 + kblocks;
+        typename U::Regs ra, rb;
+        int kb = kb0 + kb_first;
+        U::loadu(wrow, 2 * kb + half, a.K, ra);
+        for (; kb < kend && ok; kb += 2 * STEP) {
+          if (kb + STEP < kend) U::loadu(wrow, 2 * (kb + STEP) + half, a.K, rb);
+          emit(kb, ra);
+          if (!ok) break;
+          if (kb + 2 * STEP < kend) U::loadu(wrow, 2 * (kb + 2 * STEP) + half, a.K, ra);
+          if (kb + STEP < kend) emit(kb + STEP, rb);
+        }
       }
     }
   }
@@ -537,7 +546,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
   }
   if (threadIdx.x == 0 && s_abort && a.status) atomicMax(a.status, 1u);
 }
@@ -546,8 +555,8 @@ template <class T, bool DUAL, int BN>
 static int qgemm_go(const CUtensorMap& mx, const QGemmArgs& a, int n_groups, int grid, cudaStream_t st) {
   constexpr int SB = SbBytes<T>::v;
   constexpr int RS = q_raw_slots(SB, DUAL, BN);
-  constexpr int STAGES = RS > 0 ? q_stages_raw(SB, DUAL, BN) : q_stages(DUAL, BN);
-  constexpr size_t smem = (size_t)STAGES * ((DUAL ? 2 : 1) * 2 * QATOM_A + 2 * BN * 128) + (size_t)RS * (DUAL ? 2 : 1) * QBM * SB + 1024;
+  constexpr size_t smem = (size_t)q_stages(DUAL, BN) * 2 * BN * 128 + (size_t)RS * (DUAL ? 2 : 1) * QBM * SB + 1024;
+  static_assert(q_stages(DUAL, BN) >= 2 && (SB == 0 || RS >= 2), "operand rings");
   CUtensorMap mw = mx, mw2 = mx;
   if (RS > 0) {
     cuuint64_t dims[3] = {(cuuint64_t)a.row_bytes, (cuuint64_t)a.N, (cuuint64_t)n_groups};
@@ -595,14 +604,18 @@ int bl_qgemm_supports(int wtype) {
 //   X [rows_x, K] bf16 (ldx elements); W, W2 [n_groups, N, row_bytes] resident blocks of type wtype;
 //   tiles: {group, row0, row_end, -} token tiles of at most tile_rows (32, 64 or 128) rows; exactly one of c_f32 / c_bf16;
 //   W2 != null: output = silu(X W^T) * (X W2^T).  status: device word, set to 1 when a wait ran out.
-int bl_qgemm(const void* X, long ldx, long rows_x, const void* W, const void* W2, int wtype, int n_groups, int N, int K,
+//   fixed_tiles: the table has exactly max_tiles tiles and no launch in flight writes it.  splits > 1 (fixed tiles, one
+//   matrix, K / 256 divisible): that many CTAs share a tile's depth; partial: max_tiles * ceil(N / 128) * splits *
+//   tile_rows * 128 floats, tickets: max_tiles * ceil(N / 128) * 4 zeroed words, both of one stream at a time.
+int bl_qgemm_split(const void* X, long ldx, long rows_x, const void* W, const void* W2, int wtype, int n_groups, int N, int K,
              const void* tiles, const int* n_tiles, int max_tiles, int tile_rows, float* c_f32, void* c_bf16, long ldc,
              const int* dst_row, const float* row_scale, const float* resid, long ldr, unsigned* status, int sm_count,
-             cudaStream_t st) {
+             int fixed_tiles, int splits, float* partial, int* tickets, cudaStream_t st) {
   BL_REQUIRE(K >= 256 && K % 256 == 0 && N >= 1 && rows_x >= 1 && n_groups >= 1 && max_tiles >= 1, BL_ERR_SHAPE);
   BL_REQUIRE(tile_rows == 32 || tile_rows == 64 || tile_rows == 128, BL_ERR_SHAPE);
   BL_REQUIRE(ldx % 8 == 0 && ((uintptr_t)X & 15) == 0 && ((uintptr_t)W & 15) == 0 && ((uintptr_t)W2 & 15) == 0, BL_ERR_ALIGN);
   BL_REQUIRE((c_f32 != nullptr) != (c_bf16 != nullptr), BL_ERR_SHAPE);
+  BL_REQUIRE(splits == 1 || (splits > 1 && fixed_tiles && !W2 && partial && tickets && (K / 256) % splits == 0), BL_ERR_SHAPE);
   const long rb = resident_row_bytes(wtype, K);
   BL_REQUIRE(rb > 0 && bl_qgemm_supports(wtype), BL_ERR_TYPE);
   CUtensorMap mx;
@@ -620,7 +633,8 @@ int bl_qgemm(const void* X, long ldx, long rows_x, const void* W, const void* W2
   a.tiles = (const QTile*)tiles; a.n_tiles = n_tiles; a.max_tiles = max_tiles;
   a.c_f32 = c_f32; a.c_bf16 = (__nv_bfloat16*)c_bf16; a.ldc = ldc;
   a.dst_row = dst_row; a.row_scale = row_scale; a.resid = resid; a.ldr = ldr; a.status = status;
-  const long tiles_total = (long)max_tiles * a.tiles_w;
+  a.fixed_tiles = fixed_tiles; a.splits = splits; a.partial = partial; a.tickets = tickets;
+  const long tiles_total = (long)max_tiles * a.tiles_w * splits;
   const int grid = (int)(tiles_total < sm_count ? tiles_total : sm_count);
   const bool dual = W2 != nullptr;
   switch (wtype) {
@@ -633,6 +647,14 @@ int bl_qgemm(const void* X, long ldx, long rows_x, const void* W, const void* W2
     case WT_Q8_F32: return qgemm_pick<Q8F>(dual, tile_rows, mx, a, n_groups, grid, st);
   }
   return BL_ERR_TYPE;
+}
+
+int bl_qgemm(const void* X, long ldx, long rows_x, const void* W, const void* W2, int wtype, int n_groups, int N, int K,
+             const void* tiles, const int* n_tiles, int max_tiles, int tile_rows, float* c_f32, void* c_bf16, long ldc,
+             const int* dst_row, const float* row_scale, const float* resid, long ldr, unsigned* status, int sm_count,
+             cudaStream_t st) {
+  return bl_qgemm_split(X, ldx, rows_x, W, W2, wtype, n_groups, N, K, tiles, n_tiles, max_tiles, tile_rows, c_f32, c_bf16, ldc,
+                        dst_row, row_scale, resid, ldr, status, sm_count, 0, 1, nullptr, nullptr, st);
 }
 
 }  // extern "C"

@@ -23,6 +23,7 @@ class TileTable:
         self.mtiles = torch.zeros(self.max_mtiles, 4, dtype=torch.int32, device=device)
         self.n_mtiles = torch.zeros(1, dtype=torch.int32, device=device)
         self.offsets = torch.zeros(n_groups + 1, dtype=torch.int32, device=device)
+        self.fixed = 0                          # number of tiles when the host wrote the table once and for all
 
     def build(self, group_rows: torch.Tensor, group_div: int = 1, group_stride: int = 0, base: int = 0,
               causal_pos0: int = -1, causal_kind: int = 0) -> None:
@@ -59,6 +60,7 @@ class TileTable:
             rows0 = list(range(0, rows, tile_rows))
             t.mtiles[:len(rows0)] = torch.tensor([[0, r, rows, 0] for r in rows0], dtype=torch.int32).to(device)
             t.n_mtiles.fill_(len(rows0))
+            t.fixed = len(rows0)
             t.offsets.copy_(torch.tensor([0, rows], dtype=torch.int32))
         return t
 
@@ -219,23 +221,50 @@ def qgemm_supports(w: QWeight) -> bool:
     return bool(cuda().bl_qgemm_supports(I(w.wt))) and w.k % 256 == 0
 
 
+class QgemmWork:
+    """Partial sums and tickets of split products: one per stream that runs them."""
+
+    def __init__(self, device, tile_rows: int = 64):
+        self.tile_rows = tile_rows
+        sm = sm_count(device)
+        self.partial = torch.empty(sm * tile_rows * 128, dtype=torch.float32, device=device)
+        self.tickets = torch.zeros(sm * 4, dtype=torch.int32, device=device)
+
+
+def qgemm_splits(n_tiles: int, depth_blocks: int, sm: int) -> int:
+    """CTAs that share the depth (in 256-value blocks) of each of ``n_tiles`` output tiles: as many as leave one CTA a
+    processor, in equal shares.  A projection of a decode round has 4 to 32 tiles on 148 processors, and each tile walks
+    its whole depth in one serial pipeline (2,048 deep: about 12 us; an eighth of 4,096: about 5)."""
+    best = 1
+    for s in range(2, min(16, depth_blocks) + 1):
+        if depth_blocks % s == 0 and n_tiles * s <= sm:
+            best = s
+    return best
+
+
 def qgemm(X: torch.Tensor, W: QWeight, tiles: TileTable, *, out_f32: Optional[torch.Tensor] = None,
           out_bf16: Optional[torch.Tensor] = None, W2: Optional[QWeight] = None, dst_row=None, row_scale=None,
-          resid=None, status: Optional[torch.Tensor] = None) -> None:
+          resid=None, status: Optional[torch.Tensor] = None, work: Optional[QgemmWork] = None) -> None:
     """C = X @ W[g].T per token tile with W left block-quantised (``csrc/qgemm_tcgen05.cu``): X [rows, K] bf16, W (and
     W2) resident Q4_K / Q5_K / Q6_K / Q8_0 / FP8_B128 / NVFP4 / Q8_F32 matrices [N, bytes] or stacks [G, N, bytes]; tiles of
     32, 64 or 128 token rows.
-    With W2 the output is silu(X W^T) * (X W2^T)."""
+    With W2 the output is silu(X W^T) * (X W2^T).  With ``work`` a product of few tiles splits its depth over CTAs."""
     assert X.dtype == torch.bfloat16 and X.stride(-1) == 1 and W.data.is_contiguous() and tiles.tile_rows in (32, 64, 128)
     assert W2 is None or (W2.wt == W.wt and W2.data.shape == W.data.shape and W2.data.is_contiguous())
     G = W.data.shape[0] if W.data.dim() == 3 else 1
     N = W.data.shape[-2]
     out = out_f32 if out_f32 is not None else out_bf16
-    rc = cuda().bl_qgemm(p(X), L(X.stride(0)), L(X.shape[0]), p(W.data), p(W2.data if W2 is not None else None), I(W.wt),
-                         I(G), I(N), I(W.k), p(tiles.mtiles), p(tiles.n_mtiles), I(tiles.max_mtiles), I(tiles.tile_rows),
-                         p(out_f32), p(out_bf16), L(out.stride(0)), p(dst_row), p(row_scale), p(resid),
-                         L(resid.stride(0) if resid is not None else 0), p(status), I(sm_count()), stream())
-    check(rc, "bl_qgemm")
+    sm = sm_count()
+    splits = 1
+    if work is not None and tiles.fixed and W2 is None and tiles.tile_rows <= work.tile_rows:
+        splits = qgemm_splits(tiles.fixed * ((N + 127) // 128), W.k // 256, sm)
+    rc = cuda().bl_qgemm_split(p(X), L(X.stride(0)), L(X.shape[0]), p(W.data), p(W2.data if W2 is not None else None), I(W.wt),
+                               I(G), I(N), I(W.k), p(tiles.mtiles), p(tiles.n_mtiles), I(tiles.fixed or tiles.max_mtiles),
+                               I(tiles.tile_rows), p(out_f32), p(out_bf16), L(out.stride(0)), p(dst_row), p(row_scale),
+                               p(resid), L(resid.stride(0) if resid is not None else 0), p(status), I(sm),
+                               I(1 if tiles.fixed else 0), I(splits), p(work.partial if splits > 1 else None),
+                               p(work.tickets if splits > 1 else None), stream())
+    check(rc, "bl_qgemm_split")
 
 
 def fp8_rows(x: torch.Tensor, codes: torch.Tensor, scales: torch.Tensor, gain: Optional[torch.Tensor] = None,

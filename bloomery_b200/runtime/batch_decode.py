@@ -121,6 +121,8 @@ class BatchDecode:
         self.graphs: Dict[Tuple[int, bool], torch.cuda.CUDAGraph] = {}
         self.launches_per_step = 0
         self._scratch_w: Dict[str, torch.Tensor] = {}
+        # split products: one workspace for each branch of the pass (the main one and the two side streams)
+        self._work = [G.QgemmWork(dev) for _ in range(3)]
         from ..utils import levers
         self.fp8_native = bool(levers.get("BLOOMERY_FP8_NATIVE"))
         # the engine's own stream: its 8-row passes and prompts and these passes touch the same KV pages in order
@@ -144,10 +146,11 @@ class BatchDecode:
     def _native_fp8(self, Wq) -> bool:
         return self.fp8_native and Wq.qtype == "FP8_B128" and Wq.k % 128 == 0
 
-    def _mm(self, X, Wq, tiles, M, x8=None, W2=None, **kw):
+    def _mm(self, X, Wq, tiles, M, x8=None, W2=None, branch=0, **kw):
         """X [rows, K] bf16 times a resident matrix (or, with W2, the SwiGLU pair): FP8 weights against E4M3 rows on the
         tensor cores, other quantised types expanded in flight, the rest through a bf16 expansion launch.  ``x8``: the
-        rows' E4M3 form when the caller already made it (several products of one input).  Returns the launch count."""
+        rows' E4M3 form when the caller already made it (several products of one input).  ``branch``: 0 on the pass's own stream, 1 / 2 on its side streams.  Returns the
+        launch count."""
         if self._native_fp8(Wq):
             n = 0
             if x8 is None:
@@ -157,7 +160,7 @@ class BatchDecode:
             G.fp8_gemm(x8[0], x8[1], Wq, tiles, W2=W2, status=self.status, **kw)
             return n + 1
         if G.qgemm_supports(Wq):
-            G.qgemm(X, Wq, tiles, W2=W2, status=self.status, **kw)
+            G.qgemm(X, Wq, tiles, W2=W2, status=self.status, work=self._work[branch], **kw)
             return 1
         if Wq.qtype == "BF16":
             # bf16 rows need no expansion: the bf16 GEMM reads them in place (token tiles of 128 rows)
@@ -271,11 +274,12 @@ class BatchDecode:
         fork = torch.cuda.Event()
         fork.record(main)
         joins = []
-        for side, name, lo, hi in ((self._side[0], "attn_k.weight", s.q_rows, s.q_rows + s.kv_rows),
-                                   (self._side[1], "attn_v.weight", s.q_rows + s.kv_rows, s.q_rows + 2 * s.kv_rows)):
+        for branch, name, lo, hi in ((1, "attn_k.weight", s.q_rows, s.q_rows + s.kv_rows),
+                                     (2, "attn_v.weight", s.q_rows + s.kv_rows, s.q_rows + 2 * s.kv_rows)):
+            side = self._side[branch - 1]
             side.wait_event(fork)
             with torch.cuda.stream(side):
-                n += self._mm(xn, w.q[b + name], tiles, M, x8=x8, out_f32=self.qkv[:M, lo:hi])
+                n += self._mm(xn, w.q[b + name], tiles, M, x8=x8, branch=branch, out_f32=self.qkv[:M, lo:hi])
                 ev = torch.cuda.Event()
                 ev.record(side)
                 joins.append(ev)
@@ -310,7 +314,7 @@ class BatchDecode:
         side = self._side[0]
         side.wait_event(fork)
         with torch.cuda.stream(side):
-            n += self._mm(xn, w.q[b + "attn_kv_a_mqa.weight"], tiles, M, x8=x8, out_f32=self.qkv[:M, self.qa_w:])
+            n += self._mm(xn, w.q[b + "attn_kv_a_mqa.weight"], tiles, M, x8=x8, branch=1, out_f32=self.qkv[:M, self.qa_w:])
             K.mla_kv_append(self.qkv[:, self.qa_w:], w.f[b + "attn_kv_a_norm.weight"], e.inv_freq, s.rms_eps, M, self.row_pos,
                             self.row_seq, kvp.table, kvp.n_pages, kvp.k[il], e.fault, il); n += 1
             join = torch.cuda.Event()

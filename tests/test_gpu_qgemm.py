@@ -195,3 +195,36 @@ def test_fp8_block_scaled_grouped_dual_and_scatter():
             ref[t_] += wts[t_, j] * (a @ ref_d[e].T)
     # activations rounded to E4M3 twice (in front of gate / up and in front of down): a few percent of the expert sum
     assert float((y - ref).abs().max()) < 0.06 * float((ref - resid).abs().max()) + 1e-3, (y - ref).abs().max()
+
+
+@pytest.mark.parametrize("t", ["Q4_K", "Q6_K", "NVFP4"])
+@pytest.mark.parametrize("rows,tile,N,K", [(5, 32, 512, 1024), (33, 32, 128, 4096), (64, 64, 2048, 4096), (17, 64, 200, 768)])
+def test_dense_qgemm_with_its_depth_split(t, rows, tile, N, K):
+    """A product of few tiles shares each tile's depth among CTAs: the same sums to fp32 rounding, the same bits on every
+    run, and tickets that are ready for the next launch."""
+    from bloomery_b200.ops import gemm as G
+    from bloomery_b200.ops.decode import sm_count
+    qw, _ = _weight(t, (N,), K, 1)
+    torch.manual_seed(2)
+    X = (torch.randn(rows, K, device=DEV) * 0.5).bfloat16()
+    R = torch.randn(rows, N, device=DEV)
+    tiles = G.TileTable.dense(rows, DEV, tile)
+    assert G.qgemm_splits(tiles.fixed * ((N + 127) // 128), K // 256, sm_count()) > 1
+    st, work = _status(), G.QgemmWork(DEV)
+    C = [torch.full((rows, N), float("nan"), device=DEV) for _ in range(3)]
+    G.qgemm(X, qw, tiles, out_f32=C[0], resid=R, status=st)
+    for c in C[1:]:
+        G.qgemm(X, qw, tiles, out_f32=c, resid=R, status=st, work=work)
+    torch.cuda.synchronize()
+    assert int(st) == 0 and int(work.tickets.abs().max()) == 0
+    assert torch.equal(C[1], C[2])
+    # K products of order 0.5 x 0.05, their fp32 sums regrouped once: sqrt(K) * 0.025 * 2^-24 * a few, far below 1e-4
+    assert torch.allclose(C[0], C[1], rtol=1e-5, atol=1e-4), (C[0] - C[1]).abs().max()
+
+
+def test_the_split_takes_equal_shares_and_no_more_ctas_than_processors():
+    from bloomery_b200.ops import gemm as G
+    for tiles in (1, 4, 16, 32, 147, 148, 1187):
+        for blocks in (1, 2, 3, 8, 16, 30):
+            s = G.qgemm_splits(tiles, blocks, 148)
+            assert blocks % s == 0 and (s == 1 or tiles * s <= 148)
