@@ -14,6 +14,7 @@
 // KV layout per layer: [n_pages][n_kv][PAGE][HEAD] f16 for K and the same for V,
 // PAGE = 64 positions.  block_table[seq][i] names the page of positions 64i..64i+63.
 #include "common.cuh"
+#include "flash_mma.cuh"
 
 namespace bl {
 
@@ -470,6 +471,85 @@ __global__ void __launch_bounds__(256, 2) flash_decode_seg_mma_kernel(const Flas
   }
 }
 
+// ------------------------------------------------------------------------------------
+// The segment pass for f16 caches and groups of up to eight query heads: four warps, each with its own keys and its own
+// ring (flash_mma.cuh); they meet once, at the end.  grid (n_seg, n_kv, M).
+// Segment pass + merge, 64 rows of about 2,000 positions on the 30 B shape (32 query heads, 4 KV heads): 179 -> 79 us
+// (42 us of keys and values at the copy rate); 24 rows of 1,000: 52 -> 32 us.
+// ------------------------------------------------------------------------------------
+constexpr int kWfWarps = 4, kWfStages = 2;
+
+template <int HEAD>
+__global__ void __launch_bounds__(kWfWarps * 32, 3) flash_decode_seg_wf_kernel(const FlashArgs a) {
+  using W = WarpFlash<HEAD>;
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ float s_ml[kWfWarps][16];
+  float* sq = reinterpret_cast<float*>(smem);                              // [G][HEAD]
+  const int G = a.n_q / a.n_kv;
+  const int seg = blockIdx.x, kvh = blockIdx.y, m = blockIdx.z;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint8_t* const rings = smem + 8 * HEAD * 4;
+  __half* const ring = reinterpret_cast<__half*>(rings + (size_t)warp * kWfStages * W::kStageBytes);
+  pdl_wait();
+  pdl_launch();
+  const int seq = a.row_seq[m];
+  if (seq < 0) return;
+  const int n_keys = a.row_pos[m] + 1;
+  const bool bad = n_keys <= 0 || n_keys > a.ctx_limit;
+  if (bad && tid == 0 && seg == 0 && kvh == 0) raise_fault(a.fault, a.layer, FS_KEY_COUNT);
+  const int n_tiles = bad ? 0 : (n_keys + kKeyTile - 1) / kKeyTile;
+  const int tps = (n_tiles + a.n_seg - 1) / a.n_seg;
+  const int t0 = seg * tps, t1 = min(n_tiles, t0 + tps);
+  if (!bad && t0 >= t1) return;                  // past the row's last key tile: the merge does not read this segment
+  const int key_lo = t0 * kKeyTile, key_hi = bad ? key_lo : min(n_keys, t1 * kKeyTile);
+  const int n_steps = (key_hi - key_lo + W::kKeys - 1) / W::kKeys;         // of the block; warp w takes w, w + 4, ...
+
+  const int* bt = a.block_table + (long)seq * a.max_pages;
+  auto page_of = [&](int j) { return j < n_steps ? bt[(key_lo + j * W::kKeys) / kPage] : 0; };
+  auto issue = [&](int j, int page, int st) {
+    if (j < n_steps) {
+      const int key0 = key_lo + j * W::kKeys;
+      page = (page < 0 || page >= a.n_pages) ? 0 : page;                   // fault is raised by the append kernel; stay in bounds
+      const long base = (((long)page * a.n_kv + kvh) * kPage + (key0 % kPage)) * HEAD;
+      W::issue(ring + (size_t)st * (W::kStageBytes / 2), a.k_cache + base, a.v_cache + base, n_keys - key0, lane);
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int st = 0; st < kWfStages; ++st) issue(warp + st * kWfWarps, page_of(warp + st * kWfWarps), st);
+  for (int i = tid; i < G * HEAD; i += kWfWarps * 32) sq[i] = a.q[((long)m * a.n_q + (long)kvh * G) * HEAD + i];
+  __syncthreads();
+  W w;
+  w.init(sq, G, lane);
+  int st = 0;
+  for (int j = warp; j < n_steps; j += kWfWarps) {
+    const int ahead = j + kWfStages * kWfWarps;
+    const int page = page_of(ahead);                                       // looked up a step before it is needed
+    cp_async_wait<kWfStages - 1>();
+    __syncwarp();
+    w.step(ring + (size_t)st * (W::kStageBytes / 2), n_keys - (key_lo + j * W::kKeys), lane);
+    __syncwarp();
+    issue(ahead, page, st);
+    st = st + 1 == kWfStages ? 0 : st + 1;
+  }
+  cp_async_wait<0>();
+  __syncwarp();
+  w.store(s_ml[warp], reinterpret_cast<float*>(ring), lane);
+  __syncthreads();
+  const int n_w = min(kWfWarps, n_steps);
+  for (int hg = warp; hg < G; hg += kWfWarps) {
+    float acc[HEAD / 32], mx, l;
+    wf_merge<HEAD>(&s_ml[0][0], reinterpret_cast<const float*>(rings), kWfStages * W::kStageBytes / 4, n_w, hg, lane, acc, mx, l);
+    const long pidx = ((long)m * a.n_q + (long)kvh * G + hg) * a.n_seg + seg;
+    if (lane == 0) {
+      a.part_ml[pidx * 2] = bad ? __int_as_float(0x7fc00000) : mx;
+      a.part_ml[pidx * 2 + 1] = l;
+    }
+#pragma unroll
+    for (int d = 0; d < HEAD / 32; ++d) a.part_acc[pidx * HEAD + lane * (HEAD / 32) + d] = acc[d];
+  }
+}
+
 int g_flash_mma = 0;
 
 struct MergeArgs {
@@ -482,6 +562,7 @@ struct MergeArgs {
   float* out;        // optional fp32 [M, n_q*HEAD]
   int8_t* outq;      // q8 codes [M, n_q*HEAD]
   float2* outds;     // [M, n_q*HEAD/32]
+  __nv_bfloat16* out_bf16;  // optional [M, n_q*HEAD]: then outq / outds may be null
 };
 
 // grid (n_q, M), HEAD threads
@@ -522,6 +603,8 @@ __global__ void __launch_bounds__(HEAD) flash_decode_merge_kernel(const MergeArg
   const long col = (long)qh * HEAD + d;
   const long width = (long)a.n_q * HEAD;
   if (a.out) a.out[(long)m * width + col] = o;
+  if (a.out_bf16) a.out_bf16[(long)m * width + col] = __float2bfloat16_rn(o);
+  if (!a.outq) return;
   float ds_d, ds_s;
   int8_t q = q8_lane(o, ds_d, ds_s);
   a.outq[(long)m * width + col] = q;
@@ -574,7 +657,7 @@ void bl_set_flash_mma(int on) { bl::g_flash_mma = on ? 1 : 0; }
 static int flash_decode_go(const float* q, const void* k_cache, const void* v_cache, const int* row_pos, const int* row_seq,
                            const int* block_table, int max_pages, int n_pages, int head, int n_q, int n_kv, int M, int n_seg,
                            int ctx_limit, float* part_ml, float* part_acc, float* out, int8_t* outq, float* outds,
-                           unsigned* fault, int layer, int kv_q8, cudaStream_t st) {
+                           unsigned* fault, int layer, int kv_q8, void* out_bf16, cudaStream_t st) {
   BL_REQUIRE(head == 128 || head == 64, BL_ERR_SHAPE);
   BL_REQUIRE(n_kv >= 1 && n_q >= 1 && n_q % n_kv == 0 && n_q / n_kv <= 16, BL_ERR_SHAPE);
   BL_REQUIRE(n_seg >= 1 && M >= 1, BL_ERR_SHAPE);
@@ -608,18 +691,26 @@ static int flash_decode_go(const float* q, const void* k_cache, const void* v_ca
       if (!set64) { cudaFuncSetAttribute(flash_decode_seg_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2); set64 = true; }
       e = launch(flash_decode_seg_mma_kernel<64>, grid, dim3(256), sm2, st, a);
     }
-  } else if (head == 128) {
-    if (G <= 8) e = launch(flash_decode_seg_kernel<128, 1>, grid, dim3(256), smem, st, a);
-    else {
-      cudaFuncSetAttribute(flash_decode_seg_kernel<128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-      e = launch(flash_decode_seg_kernel<128, 2>, grid, dim3(256), smem, st, a);
+  } else if (G <= 8) {
+    // up to eight heads a group: both halves of the split operands fit one tile
+    static bool wf128 = false, wf64 = false;
+    if (head == 128) {
+      constexpr int sm3 = 8 * 128 * 4 + kWfWarps * kWfStages * WarpFlash<128>::kStageBytes;
+      if (!wf128) { cudaFuncSetAttribute(flash_decode_seg_wf_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm3); wf128 = true; }
+      e = launch(flash_decode_seg_wf_kernel<128>, grid, dim3(kWfWarps * 32), sm3, st, a);
+    } else {
+      constexpr int sm3 = 8 * 64 * 4 + kWfWarps * kWfStages * WarpFlash<64>::kStageBytes;
+      if (!wf64) { cudaFuncSetAttribute(flash_decode_seg_wf_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm3); wf64 = true; }
+      e = launch(flash_decode_seg_wf_kernel<64>, grid, dim3(kWfWarps * 32), sm3, st, a);
     }
+  } else if (head == 128) {
+    cudaFuncSetAttribute(flash_decode_seg_kernel<128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+    e = launch(flash_decode_seg_kernel<128, 2>, grid, dim3(256), smem, st, a);
   } else {
-    if (G <= 8) e = launch(flash_decode_seg_kernel<64, 1>, grid, dim3(256), smem, st, a);
-    else e = launch(flash_decode_seg_kernel<64, 2>, grid, dim3(256), smem, st, a);
+    e = launch(flash_decode_seg_kernel<64, 2>, grid, dim3(256), smem, st, a);
   }
   if (e != cudaSuccess) return (int)e;
-  MergeArgs mg{part_ml, part_acc, n_q, n_seg, M, row_seq, row_pos, ctx_limit, out, outq, (float2*)outds};
+  MergeArgs mg{part_ml, part_acc, n_q, n_seg, M, row_seq, row_pos, ctx_limit, out, outq, (float2*)outds, (__nv_bfloat16*)out_bf16};
   if (head == 128) return (int)launch(flash_decode_merge_kernel<128>, dim3(n_q, M), dim3(128), 0, st, mg);
   return (int)launch(flash_decode_merge_kernel<64>, dim3(n_q, M), dim3(64), 0, st, mg);
 }
@@ -632,7 +723,18 @@ int bl_flash_decode(const float* q, const void* k_cache, const void* v_cache, co
                     int ctx_limit, float* part_ml, float* part_acc, float* out, int8_t* outq, float* outds,
                     unsigned* fault, int layer, cudaStream_t st) {
   return flash_decode_go(q, k_cache, v_cache, row_pos, row_seq, block_table, max_pages, n_pages, head, n_q, n_kv, M, n_seg,
-                         ctx_limit, part_ml, part_acc, out, outq, outds, fault, layer, 0, st);
+                         ctx_limit, part_ml, part_acc, out, outq, outds, fault, layer, 0, nullptr, st);
+}
+
+// The same over either kind of cache with the rows as bf16 [M, n_q * head] alone, which is what the o product of a batched
+// pass takes.
+int bl_flash_decode_bf16(const float* q, const void* k_cache, const void* v_cache, const int* row_pos, const int* row_seq,
+                         const int* block_table, int max_pages, int n_pages, int head, int n_q, int n_kv, int M, int n_seg,
+                         int ctx_limit, float* part_ml, float* part_acc, void* out_bf16, int kv_q8, unsigned* fault, int layer,
+                         cudaStream_t st) {
+  BL_REQUIRE(out_bf16 != nullptr, BL_ERR_SHAPE);
+  return flash_decode_go(q, k_cache, v_cache, row_pos, row_seq, block_table, max_pages, n_pages, head, n_q, n_kv, M, n_seg,
+                         ctx_limit, part_ml, part_acc, nullptr, nullptr, nullptr, fault, layer, kv_q8 ? 1 : 0, out_bf16, st);
 }
 
 // The same over q8_0 caches (see bl_qk_norm_rope_append_q8).
@@ -641,7 +743,7 @@ int bl_flash_decode_q8(const float* q, const void* k_cache, const void* v_cache,
                        int ctx_limit, float* part_ml, float* part_acc, float* out, int8_t* outq, float* outds,
                        unsigned* fault, int layer, cudaStream_t st) {
   return flash_decode_go(q, k_cache, v_cache, row_pos, row_seq, block_table, max_pages, n_pages, head, n_q, n_kv, M, n_seg,
-                         ctx_limit, part_ml, part_acc, out, outq, outds, fault, layer, 1, st);
+                         ctx_limit, part_ml, part_acc, out, outq, outds, fault, layer, 1, nullptr, st);
 }
 
 }  // extern "C"

@@ -23,6 +23,7 @@
 // crates/gpu/src/rope_neox.rs, crates/gpu/src/flash_gqa.rs; the completion ticket is the reference's own
 // device-side idiom (crates/gpu/src/route_softmax.rs:33-36).
 #include "staged.cuh"
+#include "flash_mma.cuh"
 
 namespace bl {
 
@@ -152,6 +153,7 @@ __global__ void __launch_bounds__(256, 2) gemv_staged_kernel(const GemvArgs a) {
 constexpr int kPage = 64;
 constexpr int kKeyTile = 32;
 constexpr int kStages = 4;        // key / value tiles in flight per block
+constexpr int kWfStages = 2;      // the same for a warp that walks keys on its own
 constexpr int kMaxPatch = 64;     // rows of one pass whose keys a block may have to take from the pass itself
 
 struct AttnArgs {
@@ -208,18 +210,23 @@ __device__ __forceinline__ void head_out_q8(const float (&o)[HEAD / 32], int lan
   if ((lane % LPB) == 0) a.outds[((long)m * width + col) / 32] = make_float2(dd, dd * (float)sum);
 }
 
-// grid (n_seg, n_kv, M); 256 threads = 8 warps; warp w serves q heads w, w + 8 of the KV head's group
+// grid (n_seg, n_kv, M); 256 threads = 8 warps.  Groups of up to eight query heads (HPW 1): every warp takes 16 keys a step
+// for all heads on tensor-core tiles (flash_mma.cuh) and the warps meet at the segment's end; larger groups: warp w serves
+// heads w and w + 8 over tiles that the block stages together.
 template <int HEAD, int HPW>
-__global__ void __launch_bounds__(256, 2) attn_fused_kernel(const AttnArgs a) {
+__global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const AttnArgs a) {
   constexpr int KSTR = HEAD + 8, DPL = HEAD / 32;
   extern __shared__ __align__(128) uint8_t smem[];
   const int G = a.n_q / a.n_kv;
   float* sq = reinterpret_cast<float*>(smem);                              // [G][HEAD]
   __half* sk = reinterpret_cast<__half*>(smem + (size_t)G * HEAD * 4);     // [kStages][32][KSTR]
   __half* sv = sk + kStages * kKeyTile * KSTR;                             // [kStages][32][HEAD]
-  __half* snew = sv + kStages * kKeyTile * HEAD;                           // [patch rows][2][HEAD]: keys and values of this pass
+  using W = WarpFlash<HEAD>;
+  uint8_t* const rings = smem + (size_t)G * HEAD * 4;                      // HPW 1: [8 warps][kWfStages] in their place
+  __half* snew = HPW == 1 ? reinterpret_cast<__half*>(rings + (size_t)8 * kWfStages * W::kStageBytes) : sv + kStages * kKeyTile * HEAD;                           // [patch rows][2][HEAD]: keys and values of this pass
   __shared__ int s_last, s_np;
   __shared__ int s_pm[kMaxPatch], s_ppos[kMaxPatch];
+  __shared__ float s_ml[HPW == 1 ? 8 : 1][16];
   const int seg = blockIdx.x, kvh = blockIdx.y, m = blockIdx.z;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
@@ -267,10 +274,28 @@ __global__ void __launch_bounds__(256, 2) attn_fused_kernel(const AttnArgs a) {
   // keys of earlier positions are already in the cache: the first kStages tiles stream in while the predecessor
   // still runs (one copy group per stage, empty past the last tile, so the group count stays uniform)
   probe_mark(a.probe, 0);
+  const int key_lo = t0 * kKeyTile, key_hi = min(n_keys, t1 * kKeyTile);
+  const int n_steps = (key_hi - key_lo + W::kKeys - 1) / W::kKeys;         // HPW 1: warp w takes steps w, w + 8, ...
+  __half* const ring = reinterpret_cast<__half*>(rings + (size_t)warp * kWfStages * W::kStageBytes);
+  auto page_of = [&](int j) { return j < n_steps ? bt[(key_lo + j * W::kKeys) / kPage] : 0; };
+  auto issue_step = [&](int j, int page, int st) {
+    if (j < n_steps) {
+      const int key0 = key_lo + j * W::kKeys;
+      page = (page < 0 || page >= a.n_pages) ? 0 : page;
+      const long base = (((long)page * a.n_kv + kvh) * kPage + (key0 % kPage)) * HEAD;
+      W::issue(ring + (size_t)st * (W::kStageBytes / 2), a.k_cache + base, a.v_cache + base, n_keys - key0, lane);
+    }
+    cp_async_commit();
+  };
+  if constexpr (HPW == 1) {
 #pragma unroll
-  for (int st = 0; st < kStages; ++st) {
-    if (t0 + st < t1) issue_tile(t0 + st, st);
-    else cp_async_commit();
+    for (int st = 0; st < kWfStages; ++st) issue_step(warp + 8 * st, page_of(warp + 8 * st), st);
+  } else {
+#pragma unroll
+    for (int st = 0; st < kStages; ++st) {
+      if (t0 + st < t1) issue_tile(t0 + st, st);
+      else cp_async_commit();
+    }
   }
   pdl_wait();
   pdl_launch();
@@ -365,6 +390,41 @@ __global__ void __launch_bounds__(256, 2) attn_fused_kernel(const AttnArgs a) {
 #pragma unroll
     for (int d = 0; d < DPL; ++d) acc[h][d] = 0.f;
   }
+  if constexpr (HPW == 1) {
+    __syncthreads();                                 // queries and this pass's keys and values are in shared memory
+    if (warp < n_steps) {
+      W w;
+      w.init(sq, G, lane);
+      int st = 0;
+      for (int j = warp; j < n_steps; j += 8) {
+        const int page = page_of(j + 8 * kWfStages);
+        cp_async_wait<kWfStages - 1>();
+        __syncwarp();
+        __half* tile = ring + (size_t)st * (W::kStageBytes / 2);
+        const int key0 = key_lo + j * W::kKeys;
+        for (int idx = 0; idx < np; ++idx) {
+          const int r = s_ppos[idx] - key0;
+          if (r >= 0 && r < W::kKeys)                            // a row of this pass: the copy raced its store
+            for (int i = lane; i < HEAD; i += 32) {
+              tile[r * W::kStr + i] = snew[(size_t)idx * 2 * HEAD + i];
+              tile[W::kTile + r * W::kStr + i] = snew[((size_t)idx * 2 + 1) * HEAD + i];
+            }
+        }
+        __syncwarp();
+        w.step(tile, n_keys - key0, lane);
+        __syncwarp();
+        issue_step(j + 8 * kWfStages, page, st);
+        st = st + 1 == kWfStages ? 0 : st + 1;
+      }
+      cp_async_wait<0>();
+      __syncwarp();
+      w.store(s_ml[warp], reinterpret_cast<float*>(ring), lane);
+    }
+    __syncthreads();
+    if (warp < G)
+      wf_merge<HEAD>(&s_ml[0][0], reinterpret_cast<const float*>(rings), kWfStages * W::kStageBytes / 4, min(8, n_steps), warp,
+                     lane, acc[0], mx[0], l[0]);
+  } else
   for (int t = t0; t < t1; ++t) {
     const int stage = (t - t0) % kStages;
     cp_async_wait<kStages - 1>();                    // the oldest group in flight (tile t) has landed
@@ -1249,10 +1309,12 @@ int bl_attn_fused(const float* qkv, long qkv_stride, const float* q_gain, const 
              (float2*)outds, fault, layer, g_stage_probe, 0};
   dim3 grid(n_seg, n_kv, M);
   const int n_patch = M < kMaxPatch ? M : kMaxPatch;
-  const size_t smem = (size_t)G * head * 4 + kStages * kKeyTile * (head + 8) * 2 + kStages * kKeyTile * head * 2 + (size_t)n_patch * 2 * head * 2;
+  const size_t rings = G <= 8 ? (size_t)8 * kWfStages * (head == 128 ? WarpFlash<128>::kStageBytes : WarpFlash<64>::kStageBytes)
+                              : (size_t)kStages * kKeyTile * (head + 8) * 2 + kStages * kKeyTile * head * 2;
+  const size_t smem = (size_t)G * head * 4 + rings + (size_t)n_patch * 2 * head * 2;
   static bool attr_set = false;
   if (!attr_set) {
-    cudaFuncSetAttribute(attn_fused_kernel<128, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
+    cudaFuncSetAttribute(attn_fused_kernel<128, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 180 * 1024);
     cudaFuncSetAttribute(attn_fused_kernel<128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
     cudaFuncSetAttribute(attn_fused_kernel<64, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
     cudaFuncSetAttribute(attn_fused_kernel<64, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);

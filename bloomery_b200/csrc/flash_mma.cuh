@@ -1,0 +1,176 @@
+// One warp's share of split-K decode attention over f16 keys and values, on warp-level tensor-core tiles.
+//
+// A decode row has at most eight query heads per KV head, half of an m16n8k16 tile.  The other half holds what f16
+// leaves of the fp32 operands: rows 0..7 of the A operand are the high halves, rows 8..15 the remainders, so one MMA
+// yields both partial products and every thread adds its pair (accumulator registers c0 + c2, c1 + c3 belong to one
+// head).  Queries are first scaled by a power of two per head to a largest element in [512, 1024), probabilities by
+// 2^10: high half and remainder then keep 22 bits of every element that matters, and keys and values enter as they are
+// stored.  No probability ever exists in 16 bits alone; against 64 bits the output's error is 3.8e-7 where the fp32 loop
+// this takes the place of had 9.2e-7 (64 rows of about 2,000 positions, 32 query heads, 4 KV heads).
+//
+// A warp works alone: 16 keys a step through its own cp.async ring, no barrier inside the loop.  The fp32 loop was bound
+// by its multiply-adds and shuffles (one key a lane for the scores, 32 shuffles a tile for the values).
+#pragma once
+#include "common.cuh"
+
+namespace bl {
+
+__device__ __forceinline__ void wf_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void wf_ldsm4(uint32_t (&r)[4], const void* p) {
+  const unsigned addr = (unsigned)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void wf_ldsm4_t(uint32_t (&r)[4], const void* p) {
+  const unsigned addr = (unsigned)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+// f16x2 of (x, y) and of what it leaves
+__device__ __forceinline__ void wf_split(float x, float y, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(x, y);
+  const float2 f = __half22float2(h);
+  const __half2 r = __floats2half2_rn(x - f.x, y - f.y);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = *reinterpret_cast<const uint32_t*>(&r);
+}
+
+template <int HEAD>
+struct WarpFlash {
+  static constexpr int kKeys = 16;                       // keys a step
+  static constexpr int kStr = HEAD + 8;                  // f16 row stride: ldmatrix rows fall into different banks
+  static constexpr int kTile = kKeys * kStr;             // f16 values of a key (or value) tile
+  static constexpr int kStageBytes = 2 * kTile * 2;      // a key tile and a value tile
+  static constexpr int KS = HEAD / 16, ND = HEAD / 8;
+  static_assert(kStageBytes >= 8 * HEAD * 4, "a stage also holds the warp's result");
+  uint32_t qa[KS][4];
+  float q_inv;                                           // undoes the head's power of two
+  float o[ND][4], m, l;                                  // m: of head lane / 4; l: this thread's share of the sum
+
+  // queries of the KV head's group: G <= 8 rows of HEAD floats in shared memory
+  __device__ __forceinline__ void init(const float* sq, int G, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    const float* q = sq + g * HEAD + 2 * t;
+    float mx = 0.f;
+    if (g < G)
+#pragma unroll
+      for (int i = 0; i < HEAD / 8; ++i) mx = fmaxf(mx, fmaxf(fabsf(q[8 * i]), fabsf(q[8 * i + 1])));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    const int e = (int)(__float_as_uint(mx) >> 23);      // 127 + floor(log2)
+    const int f = min(253, max(1, 263 - e));
+    const float sc = __uint_as_float((uint32_t)f << 23);
+    q_inv = __uint_as_float((uint32_t)(254 - f) << 23);
+#pragma unroll
+    for (int k = 0; k < KS; ++k) {
+      float x[4] = {0.f, 0.f, 0.f, 0.f};
+      if (g < G) { x[0] = q[16 * k] * sc; x[1] = q[16 * k + 1] * sc; x[2] = q[16 * k + 8] * sc; x[3] = q[16 * k + 9] * sc; }
+      wf_split(x[0], x[1], qa[k][0], qa[k][1]);
+      wf_split(x[2], x[3], qa[k][2], qa[k][3]);
+    }
+#pragma unroll
+    for (int j = 0; j < ND; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
+    m = -INFINITY; l = 0.f;
+  }
+
+  // 16 key rows and value rows into a stage; rows from n_valid on become zeros (they are not read)
+  static __device__ __forceinline__ void issue(__half* stage, const __half* k, const __half* v, int n_valid, int lane) {
+    constexpr int CH = HEAD / 8;
+#pragma unroll
+    for (int c = lane; c < kKeys * CH; c += 32) {
+      const int r = c / CH, cc = c % CH;
+      const unsigned n = r < n_valid ? 16u : 0u;
+      const unsigned dk = (unsigned)__cvta_generic_to_shared(stage + r * kStr + cc * 8);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dk), "l"(k + (long)r * HEAD + cc * 8), "r"(n) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dk + kTile * 2), "l"(v + (long)r * HEAD + cc * 8), "r"(n) : "memory");
+    }
+  }
+
+  // one step over a landed stage; the first n_valid (>= 1) keys count
+  __device__ __forceinline__ void step(const __half* stage, int n_valid, int lane) {
+    const int t = lane & 3;
+    float c[2][2][4];
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) c[nt][h][0] = c[nt][h][1] = c[nt][h][2] = c[nt][h][3] = 0.f;
+#pragma unroll
+    for (int kp = 0; kp < KS / 2; ++kp)
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+        uint32_t b[4];
+        wf_ldsm4(b, stage + (nt * 8 + (lane & 7)) * kStr + (kp * 4 + (lane >> 3)) * 8);
+        wf_mma(c[nt][0], qa[2 * kp][0], qa[2 * kp][1], qa[2 * kp][2], qa[2 * kp][3], b[0], b[1]);
+        wf_mma(c[nt][1], qa[2 * kp + 1][0], qa[2 * kp + 1][1], qa[2 * kp + 1][2], qa[2 * kp + 1][3], b[2], b[3]);
+      }
+    float s[2][2];
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float x = ((c[nt][0][i] + c[nt][1][i]) + (c[nt][0][2 + i] + c[nt][1][2 + i])) * q_inv;
+        s[nt][i] = nt * 8 + 2 * t + i < n_valid ? x : -INFINITY;
+      }
+    float nm = fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1]));
+    nm = fmaxf(nm, __shfl_xor_sync(0xffffffffu, nm, 1));
+    nm = fmaxf(nm, __shfl_xor_sync(0xffffffffu, nm, 2));
+    nm = fmaxf(m, nm);
+    if (__any_sync(0xffffffffu, nm != m)) {
+      const float corr = (m == -INFINITY) ? 0.f : __expf(m - nm);
+      l *= corr;
+#pragma unroll
+      for (int j = 0; j < ND; ++j) { o[j][0] *= corr; o[j][1] *= corr; o[j][2] *= corr; o[j][3] *= corr; }
+      m = nm;
+    }
+    uint32_t a[4];
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt) {
+      const float p0 = (s[nt][0] == -INFINITY) ? 0.f : __expf(s[nt][0] - nm);
+      const float p1 = (s[nt][1] == -INFINITY) ? 0.f : __expf(s[nt][1] - nm);
+      l += p0 + p1;
+      wf_split(p0 * 1024.f, p1 * 1024.f, a[2 * nt], a[2 * nt + 1]);
+    }
+    const __half* v = stage + kTile;
+#pragma unroll
+    for (int dp = 0; dp < ND / 2; ++dp) {
+      uint32_t b[4];
+      wf_ldsm4_t(b, v + (lane & 15) * kStr + (2 * dp + (lane >> 4)) * 8);
+      wf_mma(o[2 * dp], a[0], a[1], a[2], a[3], b[0], b[1]);
+      wf_mma(o[2 * dp + 1], a[0], a[1], a[2], a[3], b[2], b[3]);
+    }
+  }
+
+  // the warp's maxima and sums [8] and unnormalised outputs [8][HEAD] for the block's merge
+  __device__ __forceinline__ void store(float* ml, float* out, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 2);
+    if (t == 0) { ml[2 * g] = m; ml[2 * g + 1] = l; }
+#pragma unroll
+    for (int j = 0; j < ND; ++j)
+      *reinterpret_cast<float2*>(out + g * HEAD + 8 * j + 2 * t) =
+          make_float2((o[j][0] + o[j][2]) * (1.f / 1024.f), (o[j][1] + o[j][3]) * (1.f / 1024.f));
+  }
+};
+
+// Head hg of the results that n_w warps left (warp w's at ml + 16 w and out + w * stride): lane's HEAD / 32 dims, the
+// maximum and the sum, warps in ascending order.
+template <int HEAD>
+__device__ __forceinline__ void wf_merge(const float* ml, const float* out, size_t stride, int n_w, int hg, int lane,
+                                         float (&acc)[HEAD / 32], float& m, float& l) {
+  m = -INFINITY; l = 0.f;
+  for (int w = 0; w < n_w; ++w) m = fmaxf(m, ml[16 * w + 2 * hg]);
+#pragma unroll
+  for (int d = 0; d < HEAD / 32; ++d) acc[d] = 0.f;
+  for (int w = 0; w < n_w; ++w) {
+    const float mw = ml[16 * w + 2 * hg];
+    const float k = (mw == -INFINITY) ? 0.f : __expf(mw - m);
+    l = fmaf(ml[16 * w + 2 * hg + 1], k, l);
+    const float* o = out + w * stride + hg * HEAD + lane * (HEAD / 32);
+#pragma unroll
+    for (int d = 0; d < HEAD / 32; ++d) acc[d] = fmaf(o[d], k, acc[d]);
+  }
+}
+
+}  // namespace bl

@@ -194,6 +194,17 @@ def flash_decode(q, k_cache, v_cache, row_pos, row_seq, block_table, n_pages: in
     check(rc, "bl_flash_decode")
 
 
+def flash_decode_bf16(q, k_cache, v_cache, row_pos, row_seq, block_table, n_pages: int, head: int, n_q: int, n_kv: int,
+                      M: int, n_seg: int, ctx_limit: int, part_ml, part_acc, out, fault, layer: int,
+                      kv_q8: bool = False) -> None:
+    """:func:`flash_decode` with the attention rows as bf16 [M, n_q * head] and in no other form."""
+    assert out.dtype == torch.bfloat16 and out.is_contiguous()
+    check(cuda().bl_flash_decode_bf16(p(q), p(k_cache), p(v_cache), p(row_pos), p(row_seq), p(block_table),
+                                      I(block_table.shape[1]), I(n_pages), I(head), I(n_q), I(n_kv), I(M), I(n_seg),
+                                      I(ctx_limit), p(part_ml), p(part_acc), p(out), I(1 if kv_q8 else 0), p(fault), I(layer),
+                                      stream()), "bl_flash_decode_bf16")
+
+
 def attn_fused(qkv, q_gain, k_gain, inv_freq, eps: float, q_scale: float, head: int, n_q: int, n_kv: int, M: int,
                row_pos, row_seq, block_table, n_pages: int, k_cache, v_cache, n_seg: int, ctx_limit: int, part_ml,
                part_acc, tickets, out, outq, outds, fault, layer: int) -> None:

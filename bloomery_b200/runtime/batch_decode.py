@@ -70,10 +70,12 @@ class BatchDecode:
         else:
             self.qkv = torch.zeros(R, s.q_rows + 2 * s.kv_rows, **f32)
             self.q_out = torch.zeros(R, s.n_q, s.head_dim, **f32)
-            # key segments: enough blocks to fill the card at the smallest bucket, no more
-            self.n_seg = max(1, min(e.n_seg, (2 * sm) // (s.n_kv * BUCKETS[0]) + 1))
-            self.part_ml = torch.zeros(R * s.n_q * self.n_seg * 2, **f32)
-            self.part_acc = torch.zeros(R * s.n_q * self.n_seg * s.head_dim, **f32)
+            # key segments: about eight blocks a processor at every bucket (three are resident), so that rows of unequal
+            # length leave no long last wave
+            self.n_segs = {m: max(1, min(e.n_seg, (8 * sm) // (s.n_kv * m))) for m in BUCKETS}
+            cells = max(m * n for m, n in self.n_segs.items() if m <= R) * s.n_q
+            self.part_ml = torch.zeros(cells * 2, **f32)
+            self.part_acc = torch.zeros(cells * s.head_dim, **f32)
             aw = s.q_rows
         self.attn = torch.zeros(R, aw, **f32)
         self.attn_bf = torch.zeros(R, aw, **bf)
@@ -259,7 +261,7 @@ class BatchDecode:
         yield n
 
     def _attn_gqa(self, il: int, M: int, xn: torch.Tensor, tiles) -> int:
-        """Grouped-query attention of layer il up to the attention rows (fp32, before the o product)."""
+        """Grouped-query attention of layer il up to the bf16 rows of the o product."""
         e = self.e
         s, w = e.spec, e.w
         b = f"blk.{il}."
@@ -291,9 +293,9 @@ class BatchDecode:
         K.qk_norm_rope_append(self.qkv, w.f.get(b + "attn_q_norm.weight"), w.f.get(b + "attn_k_norm.weight"), e.inv_freq,
                               s.rms_eps, q_scale, s.head_dim, s.n_q, s.n_kv, M, self.row_pos, self.row_seq, kvp.table,
                               kvp.n_pages, kvp.k[il], kvp.v[il], self.q_out, e.fault, il, kv_q8=e.kv_q8); n += 1
-        K.flash_decode(self.q_out, kvp.k[il], kvp.v[il], self.row_pos, self.row_seq, kvp.table, kvp.n_pages, s.head_dim,
-                       s.n_q, s.n_kv, M, self.n_seg, e.slot_ctx, self.part_ml, self.part_acc, self.attn, self.attn_q,
-                       self.attn_ds, e.fault, il, kv_q8=e.kv_q8); n += 2
+        K.flash_decode_bf16(self.q_out, kvp.k[il], kvp.v[il], self.row_pos, self.row_seq, kvp.table, kvp.n_pages, s.head_dim,
+                            s.n_q, s.n_kv, M, self.n_segs[M], e.slot_ctx, self.part_ml, self.part_acc, self.attn_bf, e.fault,
+                            il, kv_q8=e.kv_q8); n += 2
         return n
 
     def _attn_mla(self, il: int, M: int, xn: torch.Tensor, tiles) -> int:
@@ -333,6 +335,7 @@ class BatchDecode:
         K.mla_flash_decode(self.q_out, kvp.k[il], self.row_pos, self.row_seq, kvp.table, kvp.n_pages, s.n_q, M, self.n_seg,
                            e.slot_ctx, self.part_ml, self.part_acc, w.f[b + "attn_v_b.weight"], s.v_dim, self.attn,
                            self.attn_q, self.attn_ds, e.fault, il); n += 2
+        G.rmsnorm_bf16(self.attn[:M], None, s.rms_eps, self.attn_bf[:M]); n += 1
         return n
 
     def enqueue_steps(self, M: int, advance: bool = False):
@@ -354,7 +357,6 @@ class BatchDecode:
                 n += self._attn_mla(il, M, xn, tiles)
             else:
                 n += self._attn_gqa(il, M, xn, tiles)
-            G.rmsnorm_bf16(self.attn[:M], None, s.rms_eps, self.attn_bf[:M]); n += 1
             mark(il, "attention")
             n += self._mm(self.attn_bf[:M], w.q[b + "attn_output.weight"], tiles, M, out_f32=x, resid=x)
             mark(il, "o_proj")
