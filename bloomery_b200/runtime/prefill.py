@@ -19,6 +19,7 @@ band test covers it, as the reference does (``ubatch.rs:19-30``).
 from __future__ import annotations
 
 import math
+import weakref
 from typing import List, Optional, Sequence
 
 import os
@@ -42,7 +43,9 @@ def _poison() -> bool:
 
 class GemmPrefill:
     def __init__(self, engine, ubatch: int = 2048, score_bytes: int = 1 << 30):
-        self.e = engine
+        # the engine owns this object: no cycle, so an engine goes with its last reference and not in some later garbage
+        # collection, which could release its CUDA graphs inside another engine's capture
+        self.e = weakref.proxy(engine)
         self.ubatch = ubatch
         self.score_bytes = score_bytes
         self._buf = {}
@@ -63,6 +66,13 @@ class GemmPrefill:
         self._resident_ok = None
         from .timing import PromptTiming
         self.timing = PromptTiming()            # arm() it to get per-unit milliseconds of the next micro-batch
+        # Micro-batches of at most this many tokens multiply the block-quantised weights as they are (csrc/qgemm_tcgen05.cu)
+        # instead of their bf16 copies: a layer's copies are 1.2 GB on the 30 B shape, its blocks 0.35 GB, and with few rows
+        # an expert nothing but those bytes counts (64 rows: gate+up and down 182 us a layer, 185 us just to read the copies;
+        # 512 rows: 231 us, 200 us over the copies).
+        self.direct_rows = 128
+        self._direct_ok = None
+        self._work = None
 
     def _get(self, name: str, shape, dtype) -> torch.Tensor:
         n = 1
@@ -108,14 +118,20 @@ class GemmPrefill:
         qkv = self._get("qkv", (T, qkv_w), f32)
         # Quantised weights are expanded to bf16 one layer AHEAD of their use, on a side stream: the expansion is bound
         # by HBM traffic, the products by the tensor cores, so the two overlap.  Two sets of bf16 buffers alternate.
-        resident = self._use_resident()
-        ahead = self.expert_source is None and self.expand_ahead and not resident
+        direct = self._direct(T)
+        resident = not direct and self._use_resident()
+        ahead = self.expert_source is None and self.expand_ahead and not resident and not direct
         nset = 2 if ahead else 1
-        wqkv_s = [self._get(f"wqkv{i}", (qkv_w, H), bf) for i in range(nset)]
-        wo_s = [self._get(f"wo{i}", (H, s.q_rows), bf) for i in range(nset)]
+        wqkv_s = [None if direct else self._get(f"wqkv{i}", (qkv_w, H), bf) for i in range(nset)]
+        wo_s = [None if direct else self._get(f"wo{i}", (H, s.q_rows), bf) for i in range(nset)]
         q_bf = self._get("q_bf", (s.n_q, T, s.head_dim), bf)
         attn = self._get("attn", (T, s.q_rows), bf)
-        dense_tiles = G.TileTable.dense(T, dev)
+        if direct:
+            dense_tiles = G.TileTable.dense(T, dev, 32 if T <= 32 else 64 if T <= 64 else 128, host=True)
+            if self._work is None:
+                self._work = G.QgemmWork(dev, 128)
+        else:
+            dense_tiles = G.TileTable.dense(T, dev)
         n_keys = p0 + T
         T_pad = (n_keys + 127) // 128 * 128
         Kb = self._get("Kb", (s.n_kv, T_pad, s.head_dim), bf)
@@ -126,9 +142,9 @@ class GemmPrefill:
             E, I_, k = s.n_expert, s.moe_inter, s.n_used
             nslot = T * k
             cap = nslot + 128
-            wg_s = [self._get(f"wg{i}", (E, I_, H), bf) for i in range(nset)]
-            wu_s = [self._get(f"wu{i}", (E, I_, H), bf) for i in range(nset)]
-            wd_s = [self._get(f"wd{i}", (E, H, I_), bf) for i in range(nset)]
+            wg_s = [None if direct else self._get(f"wg{i}", (E, I_, H), bf) for i in range(nset)]
+            wu_s = [None if direct else self._get(f"wu{i}", (E, I_, H), bf) for i in range(nset)]
+            wd_s = [None if direct else self._get(f"wd{i}", (E, H, I_), bf) for i in range(nset)]
             logits = self._get("rl", (T, E), f32)
             xn3 = self._get("xn3", (T, 3 * H), bf)
             ids = self._get("ids", (T, k), i32)
@@ -141,7 +157,7 @@ class GemmPrefill:
             Ap = self._get("Ap", (cap, H), bf)
             act = self._get("act", (cap, I_), bf)
             slot_out = self._get("slot_out", (nslot, H), f32)
-            moe_tiles = G.TileTable(nslot, E, dev)
+            moe_tiles = G.TileTable(nslot, E, dev, 32) if direct else G.TileTable(nslot, E, dev)
         if s.dense_inter and (s.first_dense > 0 or not s.is_moe):
             Id = s.dense_inter
             dg_s = [self._get(f"dg{i}", (Id, H), bf) for i in range(nset)]
@@ -221,9 +237,16 @@ class GemmPrefill:
                         ready[il + 1].record(side)
                 main.wait_event(ready[il])
             G.rmsnorm_bf16(x, w.f[b + "attn_norm.weight"], s.rms_eps, xn)
-            if not ahead and not resident:
-                expand(il, "attn")
-            G.gemm_bf16(xn, wqkv, dense_tiles, out_f32=qkv, status=st)
+            if direct:
+                lo = 0
+                for nm in ("attn_q", "attn_k", "attn_v"):
+                    wq = w.q[b + nm + ".weight"]
+                    G.qgemm(xn, wq, dense_tiles, out_f32=qkv[:, lo:lo + wq.rows], status=st, work=self._work, exact=True)
+                    lo += wq.rows
+            else:
+                if not ahead and not resident:
+                    expand(il, "attn")
+                G.gemm_bf16(xn, wqkv, dense_tiles, out_f32=qkv, status=st)
             self.timing.mark(il, "qkv_gemm")
             G.qk_norm_rope_append_prefill(qkv, w.f.get(b + "attn_q_norm.weight"), w.f.get(b + "attn_k_norm.weight"),
                                           e.inv_freq, s.rms_eps, 1.0 / math.sqrt(s.head_dim), s.head_dim, s.n_q, s.n_kv,
@@ -250,7 +273,11 @@ class GemmPrefill:
                 G.gemm_bf16(P, Vt, pv_tiles, out_bf16=attn.view(T * s.n_q, s.head_dim), dst_row=map_o, status=st)
                 self.timing.mark(il, "values")
             self.timing.mark(il, "attention")
-            G.gemm_bf16(attn, wo, dense_tiles, out_f32=x, resid=x, status=st)
+            if direct:
+                G.qgemm(attn, w.q[b + "attn_output.weight"], dense_tiles, out_f32=x, resid=x, status=st, work=self._work,
+                        exact=True)
+            else:
+                G.gemm_bf16(attn, wo, dense_tiles, out_f32=x, resid=x, status=st)
             self.timing.mark(il, "o_proj")
             if s.layer_is_moe(il):
                 rw = w.q[b + "ffn_gate_inp.weight"]
@@ -272,15 +299,21 @@ class GemmPrefill:
                 self.timing.mark(il, "count_scatter")
                 G.gather_rows_bf16(xn, dst_row, moe_tiles.offsets[E:E + 1], cap, k, Ap)
                 self.timing.mark(il, "dispatch")
-                if not ahead and not resident:
-                    expand(il, "gate_up")
-                self.timing.mark(il, "expand_gate_up")
-                G.gemm_bf16(Ap, wg, moe_tiles, out_bf16=act, B2=wu, status=st)
-                self.timing.mark(il, "gemm_gate_up")
-                if not ahead and not resident:
-                    expand(il, "down")
-                self.timing.mark(il, "expand_down")
-                G.gemm_bf16(act, wd, moe_tiles, out_f32=slot_out, dst_row=dst_row, row_scale=row_scale, status=st)
+                if direct:
+                    qg, qu, qd = (w.q[b + f"ffn_{n}_exps.weight"] for n in ("gate", "up", "down"))
+                    G.qgemm(Ap, qg, moe_tiles, out_bf16=act, W2=qu, status=st, exact=True)
+                    self.timing.mark(il, "gemm_gate_up")
+                    G.qgemm(act, qd, moe_tiles, out_f32=slot_out, dst_row=dst_row, row_scale=row_scale, status=st, exact=True)
+                else:
+                    if not ahead and not resident:
+                        expand(il, "gate_up")
+                    self.timing.mark(il, "expand_gate_up")
+                    G.gemm_bf16(Ap, wg, moe_tiles, out_bf16=act, B2=wu, status=st)
+                    self.timing.mark(il, "gemm_gate_up")
+                    if not ahead and not resident:
+                        expand(il, "down")
+                    self.timing.mark(il, "expand_down")
+                    G.gemm_bf16(act, wd, moe_tiles, out_f32=slot_out, dst_row=dst_row, row_scale=row_scale, status=st)
                 self.timing.mark(il, "gemm_down")
                 G.moe_combine(slot_out, pos_of, T, k, x, x)
                 self.timing.mark(il, "combine")
@@ -299,6 +332,20 @@ class GemmPrefill:
         e.x[0].copy_(x[T - 1])
         if int(st.item()) != 0:
             raise RuntimeError("a bounded wait inside the GEMM kernel ran out (status word set)")
+
+    def _direct(self, T: int) -> bool:
+        """Whether a micro-batch of T tokens multiplies the quantised blocks themselves: short ones of a model whose layers
+        are all routed and whose matrices all have a kernel for that (and whose experts are on the card)."""
+        if T > self.direct_rows or self.expert_source is not None:
+            return False
+        if self._direct_ok is None:
+            s, w = self.e.spec, self.e.w
+            names = ("attn_q", "attn_k", "attn_v", "attn_output", "ffn_gate_exps", "ffn_up_exps", "ffn_down_exps")
+            self._direct_ok = all(
+                s.layer_is_moe(il) and all(G.qgemm_supports(w.q[f"blk.{il}.{n}.weight"]) for n in names)
+                and w.q[f"blk.{il}.ffn_gate_exps.weight"].qtype == w.q[f"blk.{il}.ffn_up_exps.weight"].qtype
+                for il in range(s.n_layer))
+        return self._direct_ok
 
     def _use_resident(self) -> bool:
         """Whether the layers' bf16 copies stay in HBM between prompts (decided once, before the first copy exists)."""
