@@ -183,6 +183,99 @@ __global__ void __launch_bounds__(256) router_kernel(const RouterArgs a0) {
   }
 }
 
+// The router of many rows (a decode round past the chain, a short prompt): logits alone, and the normed rows as bf16 for
+// the expert products.  A block takes eight rows and four experts: with one expert a block every row was read from L2 once
+// an expert, 64 MB a layer at 64 rows.  The sums are router_kernel's, in its order.
+constexpr int kRouteE = 4;
+__global__ void __launch_bounds__(256) router_rows_kernel(const float* x, long x_stride, const float* gain, float eps, const uint8_t* w,
+                                                          int wtype, int K, int E, int M, float* logits, __nv_bfloat16* xn, long xn_stride) {
+  __shared__ float s_dot[8][8][kRouteE];
+  __shared__ double s_ss[8][8];
+  __shared__ float s_scale[8];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int e0 = blockIdx.x * kRouteE, m0 = blockIdx.y * 8;
+  const int rows = min(8, M - m0);
+  const long rb = resident_row_bytes(wtype, K);
+  float dot[8][kRouteE], ss[8];
+#pragma unroll
+  for (int m = 0; m < 8; ++m) {
+    ss[m] = 0.f;
+#pragma unroll
+    for (int j = 0; j < kRouteE; ++j) dot[m][j] = 0.f;
+  }
+  bool waited = false;
+  for (int i0 = tid * 8; i0 < K; i0 += 2048) {
+    float wv[kRouteE][8];
+#pragma unroll
+    for (int j = 0; j < kRouteE; ++j) {
+      const uint8_t* row = w + (long)min(e0 + j, E - 1) * rb;
+      if (wtype == WT_F32) {
+        const float4 p = __ldg(reinterpret_cast<const float4*>(row) + i0 / 4), q = __ldg(reinterpret_cast<const float4*>(row) + i0 / 4 + 1);
+        wv[j][0] = p.x; wv[j][1] = p.y; wv[j][2] = p.z; wv[j][3] = p.w; wv[j][4] = q.x; wv[j][5] = q.y; wv[j][6] = q.z; wv[j][7] = q.w;
+      } else {
+        const uint4 p = __ldg(reinterpret_cast<const uint4*>(row) + i0 / 8);
+        const uint32_t ws[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float2 f = (wtype == WT_F16) ? __half22float2(*reinterpret_cast<const __half2*>(&ws[c]))
+                                             : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ws[c]));
+          wv[j][2 * c] = f.x; wv[j][2 * c + 1] = f.y;
+        }
+      }
+    }
+    const float4 g0 = __ldg(reinterpret_cast<const float4*>(gain + i0)), g1 = __ldg(reinterpret_cast<const float4*>(gain + i0 + 4));
+    if (!waited) { pdl_wait(); waited = true; }
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      const float* xr = x + (long)(m0 + min(m, rows - 1)) * x_stride;
+      const float4 x0 = *reinterpret_cast<const float4*>(xr + i0), x1 = *reinterpret_cast<const float4*>(xr + i0 + 4);
+      ss[m] += x0.x * x0.x + x0.y * x0.y + x0.z * x0.z + x0.w * x0.w + x1.x * x1.x + x1.y * x1.y + x1.z * x1.z + x1.w * x1.w;
+      const float xg[8] = {x0.x * g0.x, x0.y * g0.y, x0.z * g0.z, x0.w * g0.w, x1.x * g1.x, x1.y * g1.y, x1.z * g1.z, x1.w * g1.w};
+#pragma unroll
+      for (int j = 0; j < kRouteE; ++j)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) dot[m][j] = fmaf(wv[j][c], xg[c], dot[m][j]);
+    }
+  }
+  if (!waited) pdl_wait();
+  pdl_launch();
+#pragma unroll
+  for (int m = 0; m < 8; ++m) {
+    const double q = warp_sum_d((double)ss[m]);
+    if (lane == 0) s_ss[warp][m] = q;
+#pragma unroll
+    for (int j = 0; j < kRouteE; ++j) {
+      const float d = warp_sum(dot[m][j]);
+      if (lane == 0) s_dot[warp][m][j] = d;
+    }
+  }
+  __syncthreads();
+  if (tid < 8) {
+    double q = 0.0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q += s_ss[i][tid];
+    s_scale[tid] = (float)(1.0 / sqrt(q / (double)K + (double)eps));
+  }
+  __syncthreads();
+  if (tid < 8 * kRouteE) {
+    const int m = tid / kRouteE, j = tid % kRouteE;
+    float d = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) d += s_dot[i][m][j];
+    if (m < rows && e0 + j < E) logits[(long)(m0 + m) * E + e0 + j] = d * s_scale[m];
+  }
+  // every block of a row group knows the scales: they share its normed rows
+  if (xn)
+    for (int i = (blockIdx.x * 256 + tid) * 4; i < rows * K; i += gridDim.x * 1024) {
+      const int m = i / K, c = i - m * K;
+      const float4 v = *reinterpret_cast<const float4*>(x + (long)(m0 + m) * x_stride + c);
+      const float4 g = __ldg(reinterpret_cast<const float4*>(gain + c));
+      const float sc = s_scale[m];
+      __nv_bfloat162 o[2] = {__floats2bfloat162_rn(v.x * sc * g.x, v.y * sc * g.y), __floats2bfloat162_rn(v.z * sc * g.z, v.w * sc * g.w)};
+      *reinterpret_cast<uint2*>(xn + (long)(m0 + m) * xn_stride + c) = *reinterpret_cast<const uint2*>(o);
+    }
+}
+
 // ------------------------------------------------------------------------------------
 // gate·up·SwiGLU over device-side expert ids
 // grid (I/32, n_used, M), 256 threads: warp w computes activation rows 4w..4w+3 of the chunk
@@ -200,6 +293,9 @@ struct GateUpArgs {
   float* act_f32;                        // optional fp32 copy
   unsigned* fault; int layer;
   const uint8_t* down; long down_expert_bytes;   // optional: the down stack, whose chosen matrices L2 is asked to prefetch
+  // optional [M] (with route.logits): rows with a negative entry only fill the bucket.  They route nowhere, so neither this
+  // launch nor the one behind it reads a weight for them (five rows in the bucket of eight were charged for eight).
+  const int* row_seq;
 };
 
 // two activation outputs (2 gate rows + 2 up rows) of one warp
@@ -238,6 +334,13 @@ __global__ void __launch_bounds__(256, 2) gate_up_sel_kernel(const GateUpArgs a)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   pdl_wait();
   pdl_launch();
+  if (a.row_seq && a.row_seq[m] < 0) {
+    if (chunk == 0 && j == 0 && tid < a.n_used) {
+      a.ids[(long)m * a.n_used + tid] = kExpertElsewhere;
+      a.wts[(long)m * a.n_used + tid] = 0.f;
+    }
+    return;
+  }
   if (a.route.logits) {
     // block-wide rank counting: measured faster here than top_k rounds of a single warp's arg-max
     __shared__ RouteShared rs;
@@ -491,6 +594,18 @@ int bl_router(const float* x, long x_stride, const float* gain, float eps, const
   }
 }
 
+// Router logits of M rows and, with xn, the normed rows as bf16 (row stride xn_stride).  x and gain 16-byte aligned rows.
+int bl_router_rows(const float* x, long x_stride, const float* gain, float eps, const void* w, int wtype, int K, int E, int M,
+                   float* logits, void* xn, long xn_stride, cudaStream_t st) {
+  BL_REQUIRE(E >= 1 && E <= kMaxExperts, BL_ERR_LIMIT);
+  BL_REQUIRE(K % 256 == 0 && K >= 256 && M >= 1 && M <= 8 * 65535, BL_ERR_SHAPE);
+  BL_REQUIRE(wtype == WT_F32 || wtype == WT_F16 || wtype == WT_BF16, BL_ERR_TYPE);
+  BL_REQUIRE((((uintptr_t)x | (uintptr_t)gain | (uintptr_t)w) & 15) == 0 && x_stride % 4 == 0 && ((uintptr_t)xn & 7) == 0 &&
+             xn_stride % 4 == 0, BL_ERR_ALIGN);
+  return (int)launch(router_rows_kernel, dim3((E + kRouteE - 1) / kRouteE, (M + 7) / 8), dim3(256), 0, st, x, x_stride, gain, eps,
+                     (const uint8_t*)w, wtype, K, E, M, logits, (__nv_bfloat16*)xn, xn_stride);
+}
+
 // Asks L2 to prefetch the gate / up (and optionally down) matrices of the experts named in ids[n] (negative = skip),
 // 32 KB pieces dealt round-robin over the blocks; lane 0 of every warp issues.
 __global__ void __launch_bounds__(256) prefetch_experts_kernel(const int* ids, int n, const uint8_t* gate, const uint8_t* up,
@@ -514,12 +629,20 @@ __global__ void __launch_bounds__(256) prefetch_experts_kernel(const int* ids, i
 }
 
 // Standalone routing of M rows from logits (tests, prefill, host paths): one warp per row.
+// row_seq (optional): rows with a negative entry fill a bucket and nothing else; they route nowhere and count nowhere.
 __global__ void __launch_bounds__(256) route_rows_kernel(RouteParams p, int M, int* ids, float* wts, unsigned* heat,
-                                                         unsigned* fault, int layer) {
+                                                         unsigned* fault, int layer, const int* row_seq) {
   __shared__ RouteShared rs;
   pdl_wait();
   pdl_launch();
   const int m = blockIdx.x, lane = threadIdx.x & 31;
+  if (row_seq && row_seq[m] < 0) {
+    if (threadIdx.x < p.top_k) {
+      ids[(long)m * p.top_k + threadIdx.x] = kExpertElsewhere;
+      wts[(long)m * p.top_k + threadIdx.x] = 0.f;
+    }
+    return;
+  }
   int id; float w;
   const bool ok = route_block(p, m, rs, id, w);
   if (threadIdx.x >= 32) return;
@@ -541,11 +664,11 @@ int bl_prefetch_experts(const int* ids, int n, const void* gate, const void* up,
 
 int bl_route_rows(const float* logits, const float* bias, int E, int M, int top_k, int mode, int renorm, float scale,
                   int n_group, int topk_group, int* ids, float* wts, unsigned* heat, unsigned* fault, int layer,
-                  cudaStream_t st) {
+                  const int* row_seq, cudaStream_t st) {
   BL_REQUIRE(E >= 4 && E % 4 == 0 && E <= kMaxExperts && top_k >= 1 && top_k <= kMaxTopK && top_k <= E, BL_ERR_LIMIT);
   BL_REQUIRE(n_group >= 1 && n_group <= 16 && E % n_group == 0 && topk_group >= 1 && topk_group <= n_group, BL_ERR_SHAPE);
   RouteParams p{logits, bias, E, top_k, mode, renorm, scale, n_group, topk_group};
-  return (int)launch(route_rows_kernel, dim3(M), dim3(256), 0, st, p, M, ids, wts, heat, fault, layer);
+  return (int)launch(route_rows_kernel, dim3(M), dim3(256), 0, st, p, M, ids, wts, heat, fault, layer, row_seq);
 }
 
 // route_logits != null: every block routes its row from the logits (and block 0 writes
@@ -554,7 +677,8 @@ int bl_gate_up_sel(const int8_t* xq, const float* xds, const float* route_logits
                    int renorm, float scale, int n_group, int topk_group, int* ids, float* wts, unsigned* heat,
                    const int* slot_map, const void* gate, const void* up, int gtype, int utype, int K, int I, int E,
                    int n_used, int M, int8_t* actq, float* actds, float* act_f32, unsigned* fault, int layer,
-                   const void* down, long down_expert_bytes, cudaStream_t st) {
+                   const void* down, long down_expert_bytes, const int* row_seq, cudaStream_t st) {
+  BL_REQUIRE(!row_seq || route_logits, BL_ERR_SHAPE);
   BL_REQUIRE(K % 256 == 0 && I % 32 == 0 && M >= 1 && n_used >= 1 && n_used <= kMaxTopK, BL_ERR_SHAPE);
   BL_REQUIRE(gtype == utype, BL_ERR_TYPE);
   BL_REQUIRE(gtype == WT_Q4_K || gtype == WT_Q5_K || gtype == WT_Q6_K || gtype == WT_Q8_0 || gtype == WT_Q8_F32 || is_plane_family(gtype), BL_ERR_TYPE);
@@ -568,6 +692,7 @@ int bl_gate_up_sel(const int8_t* xq, const float* xds, const float* route_logits
   a.actq = actq; a.actds = (float2*)actds; a.act_f32 = act_f32; a.fault = fault; a.layer = layer;
   BL_REQUIRE(((uintptr_t)down & 15) == 0 && down_expert_bytes % 16 == 0, BL_ERR_ALIGN);
   a.down = (const uint8_t*)down; a.down_expert_bytes = down_expert_bytes;
+  a.row_seq = row_seq;
   if (is_plane_family(gtype)) return (int)launch(gate_up_sel_kernel<2>, dim3(I / 32, n_used, M), dim3(256), 0, st, a);
   return (int)launch(gate_up_sel_kernel<0>, dim3(I / 32, n_used, M), dim3(256), 0, st, a);
 }

@@ -261,6 +261,12 @@ def router(x, gain, eps: float, w: QWeight, M: int, logits, xq_out, xds_out, xn_
     check(rc, "bl_router")
 
 
+def router_rows(x, gain, eps: float, w: QWeight, M: int, logits, xn=None) -> None:
+    """Router logits of many rows (RMSNorm folded in) and, with ``xn``, the normed rows as bf16."""
+    check(cuda().bl_router_rows(p(x), L(x.stride(0)), p(gain), F(eps), p(w.data), I(w.wt), I(w.k), I(w.rows), I(M), p(logits),
+                                p(xn), L(xn.stride(0) if xn is not None else 0), stream()), "bl_router_rows")
+
+
 @dataclass
 class RouteRule:
     """How logits become (ids, weights): softmax or sigmoid scores, optional selection bias,
@@ -275,19 +281,21 @@ class RouteRule:
     bias: Optional[torch.Tensor] = None
 
 
-def route_rows(logits, rule: RouteRule, M: int, ids, wts, heat, fault, layer: int) -> None:
+def route_rows(logits, rule: RouteRule, M: int, ids, wts, heat, fault, layer: int, row_seq=None) -> None:
+    """``row_seq``: rows with a negative entry only fill a bucket; their ids become -1, their weights 0."""
     rc = cuda().bl_route_rows(p(logits), p(rule.bias), I(logits.shape[-1]), I(M), I(rule.top_k), I(rule.mode),
                               I(1 if rule.renorm else 0), F(rule.scale), I(rule.n_group), I(rule.topk_group), p(ids),
-                              p(wts), p(heat), p(fault), I(layer), stream())
+                              p(wts), p(heat), p(fault), I(layer), p(row_seq), stream())
     check(rc, "bl_route_rows")
 
 
 def gate_up_sel(xq, xds, ids, slot_map, gate: QWeight, up: QWeight, n_expert: int, n_used: int, M: int, actq, actds,
                 act_f32, fault, layer: int, *, route_logits=None, rule: Optional[RouteRule] = None, wts=None,
-                heat=None, down: Optional[QWeight] = None) -> None:
+                heat=None, down: Optional[QWeight] = None, row_seq=None) -> None:
     """gate·up·SwiGLU of the chosen experts.  With ``route_logits`` every block routes its own
     row (and ids / wts / heat are written for the launches that follow); else ``ids`` is read.  ``down``: the
-    layer's down stack; the launch asks L2 to prefetch the chosen experts' matrices for the launch that follows."""
+    layer's down stack; the launch asks L2 to prefetch the chosen experts' matrices for the launch that follows.
+    ``row_seq`` (with ``route_logits``): rows with a negative entry are left out of this launch and the next."""
     r = rule or RouteRule(n_used)
     if "prefetch" not in _PARTS:
         down = None
@@ -296,7 +304,7 @@ def gate_up_sel(xq, xds, ids, slot_map, gate: QWeight, up: QWeight, n_expert: in
                                p(gate.data), p(up.data), I(gate.wt), I(up.wt), I(gate.k), I(gate.rows), I(n_expert),
                                I(n_used), I(M), p(actq), p(actds), p(act_f32), p(fault), I(layer),
                                p(down.data if down is not None else None), L(down.data.stride(0) if down is not None else 0),
-                               stream())
+                               p(row_seq), stream())
     check(rc, "bl_gate_up_sel")
 
 

@@ -181,6 +181,12 @@ def gather_rows_bf16(src, dst_row, n_rows, max_rows: int, k: int, out) -> None:
                                      I(src.shape[1]), p(out), stream()), "bl_gather_rows_bf16")
 
 
+def moe_combine_norm(slot_out, pos_of, T: int, k: int, resid, out, gain, eps: float, xn) -> None:
+    """:func:`moe_combine` and, of its rows, ``xn`` = bf16 RMSNorm with ``gain`` (rows of at most 8,192 values)."""
+    check(cuda().bl_moe_combine_norm(p(slot_out), p(pos_of), I(T), I(k), I(out.shape[1]), p(resid), L(resid.stride(0)), p(out),
+                                     L(out.stride(0)), p(gain), F(eps), p(xn), L(xn.stride(0)), stream()), "bl_moe_combine_norm")
+
+
 def moe_combine(slot_out, pos_of, T: int, k: int, resid, out) -> None:
     check(cuda().bl_moe_combine(p(slot_out), p(pos_of), I(T), I(k), I(out.shape[1]), p(resid),
                                 L(resid.stride(0) if resid is not None else 0), p(out), L(out.stride(0)), stream()),

@@ -254,7 +254,13 @@ class BatchDecode:
         mark(il, "gate_up")
         n += self._mm(self.act, qd, self.moe_tiles, M, out_f32=self.slot_out, dst_row=self.dst_row, row_scale=self.row_scale)
         mark(il, "down")
-        G.moe_combine(self.slot_out, self.pos_of, M, k, x, x); n += 1
+        if not s.n_shared and s.hidden <= 8192:
+            # the rows are final: the norm in front of the next layer (or the head) rides along
+            gain = w.f[f"blk.{il + 1}.attn_norm.weight" if il + 1 < s.n_layer else "output_norm.weight"]
+            G.moe_combine_norm(self.slot_out, self.pos_of, M, k, x, x, gain, s.rms_eps, xn); n += 1
+            self._normed = True
+        else:
+            G.moe_combine(self.slot_out, self.pos_of, M, k, x, x); n += 1
         if s.n_shared:
             n += self.shared_expert(il, M, xn, tiles, x, x)
             mark(il, "shared_expert")
@@ -347,11 +353,14 @@ class BatchDecode:
         x, xn = self.x[:M], self.xn[:M]
         n = 0
         self.embed(M, x); n += 1
+        self._normed = False                         # xn holds the normed rows already
         for il in range(s.n_layer):
             b = f"blk.{il}."
             mark = self.timing.mark
             mark(il, "ffn_tail")
-            G.rmsnorm_bf16(x, w.f[b + "attn_norm.weight"], s.rms_eps, xn); n += 1
+            if not self._normed:
+                G.rmsnorm_bf16(x, w.f[b + "attn_norm.weight"], s.rms_eps, xn); n += 1
+            self._normed = False
             mark(il, "norm")
             if s.mla:
                 n += self._attn_mla(il, M, xn, tiles)
@@ -362,10 +371,8 @@ class BatchDecode:
             mark(il, "o_proj")
             if s.layer_is_moe(il):
                 E, k = s.n_expert, s.n_used
-                K.router(x, w.f[b + "ffn_norm.weight"], s.rms_eps, w.q[b + "ffn_gate_inp.weight"], M, self.logits_r, None,
-                         None, None, e.fault, il); n += 1
-                K.route_rows(self.logits_r, e._rule(il), M, self.ids, self.wts, e.heat[il], e.fault, il); n += 1
-                G.rmsnorm_bf16(x, w.f[b + "ffn_norm.weight"], s.rms_eps, xn); n += 1
+                K.router_rows(x, w.f[b + "ffn_norm.weight"], s.rms_eps, w.q[b + "ffn_gate_inp.weight"], M, self.logits_r, xn); n += 1
+                K.route_rows(self.logits_r, e._rule(il), M, self.ids, self.wts, e.heat[il], e.fault, il, self.row_seq); n += 1
                 steps = self.experts(il, M, x, xn, self.ids[:M], self.wts[:M], tiles)
             else:
                 G.rmsnorm_bf16(x, w.f[b + "ffn_norm.weight"], s.rms_eps, xn); n += 1
@@ -375,7 +382,8 @@ class BatchDecode:
                     yield n                          # the ranks meet here
                 else:
                     n += got
-        G.rmsnorm_bf16(x, w.f["output_norm.weight"], s.rms_eps, xn); n += 1
+        if not self._normed:
+            G.rmsnorm_bf16(x, w.f["output_norm.weight"], s.rms_eps, xn); n += 1
         head_w = w.q.get("output.weight", w.q["token_embd.weight"])
         n += self._mm(xn, head_w, tiles, M, out_f32=self.logits[:M])
         K.argmax_rows(self.logits, s.vocab, M, self.am_blocks, self.am_v, self.am_i, self.counters[1:2], self.tokens_out,

@@ -469,7 +469,7 @@ class DecodeEngine:
         else:
             K.gate_up_sel(self.xq, self.xds, ids, None, gate, up, s.n_expert, s.n_used, M, self.actq, self.actds, None,
                           self.fault, il, route_logits=self.r_logits, rule=self._rule(il), wts=wts, heat=self.heat[il],
-                          down=down)
+                          down=down, row_seq=self.row_seq if M > 1 else None)
         extra, n = None, 3
         if s.n_shared:
             # the shared expert reads the router's q8 rows and lands as an extra addend of the combine

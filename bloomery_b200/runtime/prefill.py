@@ -203,6 +203,7 @@ class GemmPrefill:
             with torch.cuda.stream(side):
                 expand(0, "all")
                 ready[0].record(side)
+        normed = False                          # xn holds the layer's normed rows already
         for il in range(s.n_layer):
             b = f"blk.{il}."
             self.timing.mark(il, "ffn")
@@ -236,7 +237,9 @@ class GemmPrefill:
                         expand(il + 1, "all")
                         ready[il + 1].record(side)
                 main.wait_event(ready[il])
-            G.rmsnorm_bf16(x, w.f[b + "attn_norm.weight"], s.rms_eps, xn)
+            if not normed:
+                G.rmsnorm_bf16(x, w.f[b + "attn_norm.weight"], s.rms_eps, xn)
+            normed = False
             if direct:
                 lo = 0
                 for nm in ("attn_q", "attn_k", "attn_v"):
@@ -289,15 +292,16 @@ class GemmPrefill:
                         self._router_w[il] = wr
                     G.rmsnorm_hilo(x, w.f[b + "ffn_norm.weight"], s.rms_eps, xn3)
                     G.gemm_bf16(xn3, wr, dense_tiles, out_f32=logits, status=st)
+                    rows_in = xn3[:, :H]                # the high halves are the bf16 rows that the experts take
                 else:
-                    K.router(x, w.f[b + "ffn_norm.weight"], s.rms_eps, rw, T, logits, None, None, None, e.fault, il)
+                    K.router_rows(x, w.f[b + "ffn_norm.weight"], s.rms_eps, rw, T, logits, xn)
+                    rows_in = xn
                 self.timing.mark(il, "router_logits")
                 K.route_rows(logits, e._rule(il), T, ids, wts, e.heat[il], e.fault, il)
                 self.timing.mark(il, "route")
-                G.rmsnorm_bf16(x, w.f[b + "ffn_norm.weight"], s.rms_eps, xn)
                 G.moe_plan(ids, wts, E, moe_tiles, pos_of, dst_row, row_scale)
                 self.timing.mark(il, "count_scatter")
-                G.gather_rows_bf16(xn, dst_row, moe_tiles.offsets[E:E + 1], cap, k, Ap)
+                G.gather_rows_bf16(rows_in, dst_row, moe_tiles.offsets[E:E + 1], cap, k, Ap)
                 self.timing.mark(il, "dispatch")
                 if direct:
                     qg, qu, qd = (w.q[b + f"ffn_{n}_exps.weight"] for n in ("gate", "up", "down"))
@@ -315,7 +319,11 @@ class GemmPrefill:
                     self.timing.mark(il, "expand_down")
                     G.gemm_bf16(act, wd, moe_tiles, out_f32=slot_out, dst_row=dst_row, row_scale=row_scale, status=st)
                 self.timing.mark(il, "gemm_down")
-                G.moe_combine(slot_out, pos_of, T, k, x, x)
+                if il + 1 < s.n_layer and H <= 8192:
+                    G.moe_combine_norm(slot_out, pos_of, T, k, x, x, w.f[f"blk.{il + 1}.attn_norm.weight"], s.rms_eps, xn)
+                    normed = True
+                else:
+                    G.moe_combine(slot_out, pos_of, T, k, x, x)
                 self.timing.mark(il, "combine")
             else:
                 G.rmsnorm_bf16(x, w.f[b + "ffn_norm.weight"], s.rms_eps, xn)

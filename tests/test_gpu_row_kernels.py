@@ -1,0 +1,133 @@
+"""Kernels of decode rounds and short prompts at the sizes where their tiles and splits end: the tensor-core segment pass
+of decode attention, the expert plan shared by a cluster, the router of many rows, the combine with its norm."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _fault():
+    return torch.full((1,), -1, dtype=torch.int32, device=DEV)
+
+
+@pytest.mark.parametrize("head,n_q,n_kv", [(128, 32, 4), (128, 8, 8), (64, 14, 2), (64, 16, 2), (128, 24, 2)])
+@pytest.mark.parametrize("lengths,n_seg", [([1, 15, 16, 17, 31, 33], 3), ([64, 65, 500, 1021], 5), ([3000], 37), ([200, 7], 1)])
+def test_decode_attention_against_64_bits(head, n_q, n_kv, lengths, n_seg):
+    """Rows whose keys end inside a step, a tile and a page; queries of very different size per head."""
+    from bloomery_b200.ops import decode as K
+    g = torch.Generator().manual_seed(5)
+    M, mp = len(lengths), (max(lengths) + 63) // 64
+    k = torch.randn(M * mp, n_kv, 64, head, generator=g).half()
+    v = torch.randn(M * mp, n_kv, 64, head, generator=g).half()
+    table = torch.randperm(M * mp, generator=g).int().view(M, mp)
+    q = torch.randn(M, n_q, head, generator=g) * head ** -0.5 * torch.logspace(-3, 1, n_q).view(1, n_q, 1)
+    ref = torch.zeros(M, n_q * head, dtype=torch.float64)
+    for m, n in enumerate(lengths):
+        kk, vv = (c[table[m].long()].permute(1, 0, 2, 3).reshape(n_kv, -1, head)[:, :n].double() for c in (k, v))
+        s = q[m].double().view(n_kv, n_q // n_kv, head) @ kk.transpose(1, 2)
+        ref[m] = (torch.softmax(s, -1) @ vv).reshape(-1)
+        if n % 64 and n_q // n_kv <= 8:                  # what lies behind the last key is never part of a sum
+            k[table[m, n // 64], :, n % 64:] = float("nan")
+            v[table[m, n // 64], :, n % 64:] = float("nan")
+    k, v, table, q = k.to(DEV), v.to(DEV), table.contiguous().to(DEV), q.to(DEV)
+    pos = torch.tensor([n - 1 for n in lengths], dtype=torch.int32, device=DEV)
+    seq = torch.arange(M, dtype=torch.int32, device=DEV)
+    ml = torch.zeros(M * n_q * n_seg * 2, device=DEV)
+    acc = torch.zeros(M * n_q * n_seg * head, device=DEV)
+    out = torch.zeros(M, n_q * head, device=DEV)
+    oq = torch.zeros(M, n_q * head, dtype=torch.int8, device=DEV)
+    od = torch.zeros(M, n_q * head // 32, 2, device=DEV)
+    ob = torch.zeros(M, n_q * head, dtype=torch.bfloat16, device=DEV)
+    f = _fault()
+    K.flash_decode(q, k, v, pos, seq, table, M * mp, head, n_q, n_kv, M, n_seg, mp * 64, ml, acc, out, oq, od, f, 0)
+    K.flash_decode_bf16(q, k, v, pos, seq, table, M * mp, head, n_q, n_kv, M, n_seg, mp * 64, ml, acc, ob, f, 0)
+    torch.cuda.synchronize()
+    assert int(f) == -1
+    # scores of up to about 40 in fp32 steps of 2^-18 move a probability by as much; the exponential adds 2^-22
+    assert float((out.cpu().double() - ref).norm() / ref.norm()) < 1e-5
+    assert torch.equal(ob, out.bfloat16())
+
+
+@pytest.mark.parametrize("n,E,tile", [(1, 4, 32), (2048, 128, 32), (2049, 128, 128), (4100, 40, 128), (32768, 512, 128), (8192, 1, 64)])
+def test_expert_plan_of_one_block_and_of_a_cluster(n, E, tile):
+    from bloomery_b200.ops import gemm as G
+    g = torch.Generator().manual_seed(n)
+    ids = torch.randint(-1, E, (n,), generator=g, dtype=torch.int32)
+    wts = torch.rand(n, generator=g)
+    tiles = G.TileTable(n, E, DEV, tile)
+    cap = n + 128
+    pos = torch.full((n,), -7, dtype=torch.int32, device=DEV)
+    dst = torch.full((cap,), -7, dtype=torch.int32, device=DEV)
+    sc = torch.zeros(cap, device=DEV)
+    G.moe_plan(ids.to(DEV), wts.to(DEV), E, tiles, pos, dst, sc)
+    torch.cuda.synchronize()
+    counts = torch.bincount(ids[ids >= 0].long(), minlength=E)
+    off = torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)])
+    assert torch.equal(tiles.offsets.cpu().long(), off)
+    want = [(e, r, int(off[e + 1])) for e in range(E) for r in range(int(off[e]), int(off[e + 1]), tile)]
+    assert int(tiles.n_mtiles) == len(want) and [tuple(r[:3]) for r in tiles.mtiles[:len(want)].tolist()] == want
+    pos, dst, sc = pos.cpu().long(), dst.cpu().long(), sc.cpu()
+    assert bool((pos[ids < 0] == -1).all()) and bool((dst[int(off[E]):] == -1).all())
+    used = (ids >= 0).nonzero().flatten()
+    assert torch.equal(dst[pos[used]], used) and torch.equal(sc[pos[used]], wts[used])
+    assert bool((pos[used] >= off[ids[used].long()]).all()) and bool((pos[used] < off[ids[used].long() + 1]).all())
+
+
+@pytest.mark.parametrize("t", ["F32", "F16", "BF16"])
+@pytest.mark.parametrize("M,E,K", [(9, 128, 2048), (64, 128, 2048), (17, 6, 256), (127, 30, 4096)])
+def test_router_of_many_rows_agrees_with_the_router(t, M, E, K):
+    from bloomery_b200.ops import decode as D
+    torch.manual_seed(7)
+    dt = {"F32": torch.float32, "F16": torch.float16, "BF16": torch.bfloat16}[t]
+    w = D.QWeight((torch.randn(E, K, device=DEV) * 0.05).to(dt).view(torch.uint8), t, K)
+    x, gain = torch.randn(M, K, device=DEV) * 3, torch.rand(K, device=DEV) + 0.5
+    a, b = torch.zeros(M, E, device=DEV), torch.zeros(M, E, device=DEV)
+    xn = torch.zeros(M, K, dtype=torch.bfloat16, device=DEV)
+    D.router(x, gain, 1e-6, w, M, a, None, None, None, _fault(), 0)
+    D.router_rows(x, gain, 1e-6, w, M, b, xn)
+    torch.cuda.synchronize()
+    # the same sums in the same order; the compiler may contract the squares of the norm differently
+    assert torch.allclose(a, b, rtol=1e-6, atol=1e-6)
+    ref = x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + 1e-6) * gain
+    assert torch.allclose(xn.float(), ref, rtol=2 ** -8, atol=1e-6)      # one rounding to bf16 and a few fp32 ones
+
+
+@pytest.mark.parametrize("T,k,H", [(1, 8, 2048), (33, 2, 4), (5, 3, 8192), (7, 8, 1028)])
+def test_combine_with_the_next_norm(T, k, H):
+    from bloomery_b200.ops import gemm as G
+    torch.manual_seed(8)
+    slot, x, gain = torch.randn(T * k, H, device=DEV), torch.randn(T, H, device=DEV), torch.rand(H, device=DEV) + 0.5
+    pos = torch.arange(T * k, dtype=torch.int32, device=DEV)
+    pos[::5] = -1
+    slot[::5] = float("nan")                                             # dropped slots are not read
+    y, z = torch.zeros(T, H, device=DEV), x.clone()
+    xn = torch.zeros(T, H, dtype=torch.bfloat16, device=DEV)
+    G.moe_combine(slot, pos, T, k, x, y)
+    G.moe_combine_norm(slot, pos, T, k, z, z, gain, 1e-6, xn)            # in place, as the layers use it
+    torch.cuda.synchronize()
+    assert torch.equal(y, z)
+    ref = y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + 1e-6) * gain
+    assert torch.allclose(xn.float(), ref, rtol=2 ** -8, atol=1e-6)
+
+
+@pytest.mark.parametrize("n,start", [(12, 0), (33, 0), (64, 40), (100, 3), (128, 0), (129, 0)])
+def test_short_prompts_over_quantised_blocks_agree_with_the_bf16_copies(n, start):
+    from bloomery_b200.models.spec import tiny_qwen3moe
+    from bloomery_b200.models.weights import Weights, synth_tensors
+    from bloomery_b200.runtime.engine import DecodeEngine
+    spec = tiny_qwen3moe()
+    w = Weights.from_items(spec, synth_tensors(spec, "cpu", seed=0), "cpu").to(DEV)
+    g = torch.Generator().manual_seed(n)
+    ids = torch.randint(0, spec.vocab, (start + n,), generator=g).tolist()
+    out = []
+    for rows in (128, 0):
+        eng = DecodeEngine(w, n_slots=1, slot_ctx=512)
+        eng._gemm_prefill = eng._new_gemm_prefill()
+        eng._gemm_prefill.direct_rows = rows
+        if start:
+            eng.prefill(0, ids[:start], gemm=False)
+        eng.prefill(0, ids[start:], start, gemm=True)
+        out.append(eng.logits[0].double().cpu())
+    # the same bf16 operands, their fp32 sums in another order: a layer's roundings to bf16 differ in places, four layers deep
+    assert float((out[0] - out[1]).norm() / out[1].norm()) < 2e-2
