@@ -5,15 +5,15 @@
 // (16 .. 128 per tile), so a decode batch of a few rows per expert pays for the tokens it has instead of a 128-row
 // tile, and a prompt tile expands each weight once for 128 tokens.
 //
-//   * weights: eight producer warps decode 64-value units in registers and store bf16 into the 128-byte-swizzled A
-//     stage (generic-proxy stores, fence.proxy.async, mbarrier arrive) -- the bf16 form of a weight never exists in
-//     HBM.  The quantised super-blocks of the tile's 128 rows reach the producers through a ring of raw TMA boxes
-//     ([128 rows x one super-block] of bytes, several in flight per SM, which is what a pass bound by weight
-//     streaming needs), or, where the ring does not fit beside the operand stages (gate+up at 128 tokens, Q8_0),
-//     by register loads one stage ahead;
-//   * tokens: one TMA thread loads [tokens x 64] bf16 boxes into the B stage of the same ring;
-//   * one elected thread issues tcgen05.mma (M = 128, N = tokens, K = 16) into TMEM, two accumulator buffers, so four
-//     epilogue warps read tile i back with tcgen05.ld while tile i + 1 accumulates;
+//   * weights: sixteen producer warps decode 64-value units in registers and store bf16 into the MMA's A operand in
+//     tensor memory (tcgen05.st, lane = weight row) -- the bf16 form of a weight never exists in HBM or shared memory
+//     (in shared memory its writes and the MMA's reads bound the launch).  The quantised super-blocks of the tile's 128
+//     rows reach the producers through a ring of raw TMA boxes ([128 rows x one super-block] of bytes, several in
+//     flight per SM, which is what a pass bound by weight streaming needs), or, for types without super-blocks, by
+//     register loads one item ahead;
+//   * tokens: one TMA thread loads [tokens x 64] bf16 boxes into the B stage of the same index;
+//   * one elected thread issues tcgen05.mma (M = 128, N = tokens, K = 16) into TMEM, two accumulators (one for gate+up
+//     at 128 tokens), so four epilogue warps read tile i back with tcgen05.ld while tile i + 1 accumulates;
 //   * "dual" mode runs gate and up in one main loop and the epilogue writes silu(gate) * up;
 //   * the epilogue scatters and scales like the bf16 GEMM (dst_row / row_scale / resid): lane = weight row, so one
 //     token's 32 outputs of a warp are one contiguous 128-byte (fp32) or 64-byte (bf16) store.

@@ -632,8 +632,9 @@ class DecodeEngine:
 
     def prefill(self, slot: int, tokens: Sequence[int], start: int = 0, gemm: Optional[bool] = None) -> int:
         """Feed a prompt; returns the greedy token after it.  Prompts of at least
-        ``gemm_threshold`` rows go through the tcgen05 GEMM path in micro-batches, shorter
-        ones through passes of up to 8 rows of the decode chain."""
+        ``gemm_threshold`` rows (``direct_threshold`` where it multiplies the quantised blocks themselves) go
+        through the tcgen05 GEMM path in micro-batches, shorter ones through passes of up to 8 rows of the decode
+        chain."""
         n = len(tokens)
         use_gemm = gemm if gemm is not None else (self.gemm_threshold > 0 and (n >= self.gemm_threshold or self._direct_prompt(n)))
         use_gemm = use_gemm and not self.mtp_on        # the draft layer's prompt rows run on the pass path
