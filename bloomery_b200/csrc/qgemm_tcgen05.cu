@@ -179,15 +179,18 @@ __device__ __forceinline__ uint4 short8(uint32_t w0, uint32_t w1, uint32_t s2, u
 //   widens to f32, takes the block scale and is rounded to bf16 once.
 //   NVFP4 (E2M1 codes, E4M3 scale per 16 values, f32 tensor scale): a code's magnitude is one of eight values, so two
 //   byte permutes with the code nibbles as selectors look up the low and the high byte of bf16(2 * magnitude) for four
-//   codes at once; the sign bits are gathered with two more permutes, and a packed bf16 multiply applies the group
-//   scale (rounded to bf16: the code values have two significant bits, so the product is exact in bf16 but for that
-//   rounding of the scale).
-template <class T> struct ChunkUnit { static constexpr bool kHas = false; };
+//   codes at once; the sign bits are gathered with two more permutes.  Exact form: the pair widens to f32, takes the f32
+//   scale and is rounded to bf16 once, as the expander of the bf16 copies does.  Short form: one packed bf16 multiply by
+//   the scale rounded to bf16, so a weight is rounded twice (relative weight error over random codes and scales 2.1e-3
+//   against 1.5e-3 once).
+template <class T> struct ChunkUnit { static constexpr bool kHas = false, kOneForm = true; };
 
 template <> struct ChunkUnit<Fp8B128> {
   static constexpr bool kHas = true;
+  static constexpr bool kOneForm = true;
   struct Pre { float sc; };
   static __device__ __forceinline__ Pre pre(const Fp8B128::Regs& r) { return Pre{r.sc}; }
+  template <bool EXACT>
   static __device__ __forceinline__ uint4 chunk(const Fp8B128::Regs& r, const Pre& pr, int j) {
     const u32x4& q = r.q[j >> 1];
     const uint32_t w0 = (j & 1) ? q.z : q.x, w1 = (j & 1) ? q.w : q.y;
@@ -202,29 +205,39 @@ template <> struct ChunkUnit<Fp8B128> {
 
 template <> struct ChunkUnit<NvFp4> {
   static constexpr bool kHas = true;
-  struct Pre { uint32_t s2[4]; };
+  static constexpr bool kOneForm = false;
+  struct Pre { float sc[4]; };
   static __device__ __forceinline__ Pre pre(const NvFp4::Regs& r) {
-    float sc[4];
-    e4m3x4_to_float(r.sc, sc);
     Pre pr;
+    e4m3x4_to_float(r.sc, pr.sc);
 #pragma unroll
-    for (int g = 0; g < 4; ++g) pr.s2[g] = bf2_dup(sc[g] * r.g * 0.5f);   // the table below holds 2 * magnitude
+    for (int g = 0; g < 4; ++g) pr.sc[g] = pr.sc[g] * r.g * 0.5f;                  // the table below holds 2 * magnitude
     return pr;
   }
+  template <bool EXACT>
   static __device__ __forceinline__ uint4 chunk(const NvFp4::Regs& r, const Pre& pr, int j) {
     const uint32_t w = j == 0 ? r.q0.x : j == 1 ? r.q0.y : j == 2 ? r.q0.z : j == 3 ? r.q0.w
                      : j == 4 ? r.q1.x : j == 5 ? r.q1.y : j == 6 ? r.q1.z : r.q1.w;
     const uint32_t sel = w & 0x77777777u;
     const uint32_t sodd = w & 0x80808080u, seven = (w << 4) & 0x80808080u;   // signs of the odd / the even codes
-    const uint32_t s2 = pr.s2[j >> 1];
+    const float sc = pr.sc[j >> 1];
+    const uint32_t s2 = EXACT ? 0u : bf2_dup(sc);
     uint32_t o[4];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const uint32_t c = h ? sel >> 16 : sel;
       const uint32_t lo4 = __byte_perm(0x40008000u, 0x4000C080u, c);
       const uint32_t hi4 = __byte_perm(0x40403F00u, 0x41414040u, c) | __byte_perm(seven, sodd, h ? 0x7362 : 0x5140);
-      o[2 * h] = bf2_fma(__byte_perm(lo4, hi4, 0x5140), s2, 0u);
-      o[2 * h + 1] = bf2_fma(__byte_perm(lo4, hi4, 0x7362), s2, 0u);
+      const uint32_t m[2] = {__byte_perm(lo4, hi4, 0x5140), __byte_perm(lo4, hi4, 0x7362)};
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        if constexpr (EXACT) {
+          const __nv_bfloat162 p = __floats2bfloat162_rn(__uint_as_float(m[i] << 16) * sc, __uint_as_float(m[i] & 0xFFFF0000u) * sc);
+          o[2 * h + i] = *reinterpret_cast<const uint32_t*>(&p);
+        } else {
+          o[2 * h + i] = bf2_fma(m[i], s2, 0u);
+        }
+      }
     }
     return make_uint4(o[0], o[1], o[2], o[3]);
   }
@@ -255,7 +268,7 @@ __device__ __forceinline__ void expand_unit(const typename Unit<T>::Regs& regs, 
   } else if constexpr (ChunkUnit<T>::kHas) {
     const typename ChunkUnit<T>::Pre pr = ChunkUnit<T>::pre(regs);
 #pragma unroll
-    for (int g = 0; g < 4; ++g) put(g, ChunkUnit<T>::chunk(regs, pr, 2 * g), ChunkUnit<T>::chunk(regs, pr, 2 * g + 1));
+    for (int g = 0; g < 4; ++g) put(g, ChunkUnit<T>::template chunk<EXACT>(regs, pr, 2 * g), ChunkUnit<T>::template chunk<EXACT>(regs, pr, 2 * g + 1));
   } else {
     float v[64];
     Unit<T>::decodeu(regs, u, v);
@@ -600,7 +613,7 @@ static int qgemm_go(const CUtensorMap& mx, const QGemmArgs& a, int n_groups, int
 
 template <class T, bool DUAL>
 static int qgemm_pick(bool exact, int bn, const CUtensorMap& mx, const QGemmArgs& a, int n_groups, int grid, cudaStream_t st) {
-  constexpr bool kOne = !FastUnit<T>::kHas;                          // the other types have one form
+  constexpr bool kOne = !FastUnit<T>::kHas && ChunkUnit<T>::kOneForm;   // types with an exact form only
   if (bn == 128) return qgemm_go<T, DUAL, 128, true>(mx, a, n_groups, grid, st);
   if (bn == 64) return exact ? qgemm_go<T, DUAL, 64, true>(mx, a, n_groups, grid, st) : qgemm_go<T, DUAL, 64, kOne>(mx, a, n_groups, grid, st);
   if (bn == 32) return exact ? qgemm_go<T, DUAL, 32, true>(mx, a, n_groups, grid, st) : qgemm_go<T, DUAL, 32, kOne>(mx, a, n_groups, grid, st);

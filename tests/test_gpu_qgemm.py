@@ -40,12 +40,36 @@ def test_dense_qgemm(t, rows, tile):
     assert int(st) == 0
     ref = X.float() @ ref_w.bfloat16().float().T + R
     # tiles below 128 tokens use the short expander (scale and offset of a block rounded to bf16 before the FMA)
-    # (and NVFP4 rounds its group scale to bf16 at every tile size)
-    tol = dict(rtol=1e-3, atol=1e-2) if tile == 128 and t != "NVFP4" else dict(rtol=1e-2, atol=3e-2)
+    # (NVFP4 rounds its group scale to bf16 there)
+    tol = dict(rtol=1e-3, atol=1e-2) if tile == 128 else dict(rtol=1e-2, atol=3e-2)
     assert torch.allclose(C, ref, **tol), (C - ref).abs().max()
     C2 = torch.zeros_like(C)
     G.qgemm(X, qw, tiles, out_f32=C2, resid=R, status=st)
     assert torch.equal(C, C2)                                   # bit-identical rerun
+
+
+@pytest.mark.parametrize("t", ["Q8_0", "FP8_B128", "NVFP4", "IQ4_NL"])
+@pytest.mark.parametrize("tile", [32, 64, 128])
+def test_the_exact_form_multiplies_the_weights_of_the_bf16_copies(t, tile):
+    """Rows of the identity read every weight out of the product as it was multiplied: the fp32 value rounded to bf16
+    once, bit for bit what the bf16 copies hold; the SwiGLU pair too."""
+    from bloomery_b200.ops import gemm as G
+    N, K = 136, 512
+    (w, _), (w2, _) = _weight(t, (N,), K, 21), _weight(t, (N,), K, 22)
+    copies = [torch.zeros(N, K, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+    for q, c in zip((w, w2), copies):
+        G.dequant_bf16(q, c)
+    X = torch.eye(K, dtype=torch.bfloat16, device=DEV)
+    st, tiles = _status(), G.TileTable.dense(K, DEV, tile)
+    C, D = (torch.full((K, N), float("nan"), device=DEV) for _ in range(2))
+    G.qgemm(X, w, tiles, out_f32=C, status=st, exact=True)
+    G.qgemm(X, w, tiles, out_f32=D, W2=w2, status=st, exact=True)
+    torch.cuda.synchronize()
+    assert int(st) == 0
+    g, u = (c.float().T for c in copies)
+    assert torch.equal(C, g)
+    # fp32 exponential and division: a few 2^-22
+    assert torch.allclose(D, torch.nn.functional.silu(g) * u, rtol=4e-6, atol=1e-12)
 
 
 @pytest.mark.parametrize("gt,dt", [("Q4_K", "Q6_K"), ("FP8_B128", "FP8_B128"), ("NVFP4", "NVFP4")])
