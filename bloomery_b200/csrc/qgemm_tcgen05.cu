@@ -70,9 +70,9 @@ __device__ __forceinline__ uint4 q_pack8(const float* v) {
 
 // ---- fast expanders ---------------------------------------------------------------------
 // Integer-to-float conversions run at a quarter of the FMA rate, so the K-quant expanders avoid them.
-//   exact form (prompts): a code byte q (< 128) dropped into mantissa bits 16..22 of 1.0f reads as 1 + q / 128; a packed
-//   subtract leaves q / 128 exactly and the block's affine map v = s * q + o is one FMA v = (128 s) * (q / 128) + o on a
-//   packed pair (fma.rn.f32x2), rounded to bf16 once: the fp32 decode, bit for bit.
+//   exact form (prompts): a code byte q (< 128) dropped into mantissa bits 16..22 of 1.0f reads as X = 1 + q / 128, and the block's affine map
+//   v = s * q + o becomes one FMA v = (128 s) * X + (o - 128 s) on a packed pair (fma.rn.f32x2), rounded to bf16 once.
+//   The result equals the fp32 decode to within an fp32 rounding of the offset.
 //   short form (decode rounds, which the expanders' integer pipe bounds): two code bytes become the bf16 pair
 //   (128 + q0, 128 + q1) with one byte permute, a packed bf16 subtract gives (q0, q1) exactly and a packed bf16 FMA gives
 //   s * q + o with s and o rounded to bf16: half the integer instructions, at most about one more bf16 ulp of error per
@@ -128,13 +128,13 @@ template <> struct FastUnit<Q6K> {
   }
 };
 
-// bf16x2 of (a * (x0 - 1) + c, a * (x1 - 1) + c) with one packed subtract and one packed FMA
+// bf16x2 of (a * x0 + c, a * x1 + c) with one packed FMA
 __device__ __forceinline__ uint32_t fma2_bf16(uint32_t x0, uint32_t x1, float a, float c) {
   uint32_t lo, hi;
-  asm("{\n\t.reg .b64 ra, rx, rc, rr, ro;\n\t"
-      "mov.b64 ra, {%2, %2};\n\tmov.b64 rx, {%3, %4};\n\tmov.b64 rc, {%5, %5};\n\tmov.b64 ro, {%6, %6};\n\t"
-      "add.rn.f32x2 rx, rx, ro;\n\tfma.rn.f32x2 rr, ra, rx, rc;\n\tmov.b64 {%0, %1}, rr;\n\t}"
-      : "=r"(lo), "=r"(hi) : "f"(a), "r"(x0), "r"(x1), "f"(c), "f"(-1.0f));
+  asm("{\n\t.reg .b64 ra, rx, rc, rr;\n\t"
+      "mov.b64 ra, {%2, %2};\n\tmov.b64 rx, {%3, %4};\n\tmov.b64 rc, {%5, %5};\n\t"
+      "fma.rn.f32x2 rr, ra, rx, rc;\n\tmov.b64 {%0, %1}, rr;\n\t}"
+      : "=r"(lo), "=r"(hi) : "f"(a), "r"(x0), "r"(x1), "f"(c));
   __nv_bfloat162 p = __floats2bfloat162_rn(__uint_as_float(lo), __uint_as_float(hi));
   return *reinterpret_cast<uint32_t*>(&p);
 }
@@ -262,8 +262,8 @@ __device__ __forceinline__ void expand_unit(const typename Unit<T>::Regs& regs, 
         put(g, short8(cw[4 * g], cw[4 * g + 1], s2, o2), short8(cw[4 * g + 2], cw[4 * g + 3], s2, o2));
         continue;
       }
-      const float a = 128.0f * s[g];
-      put(g, fast8(cw[4 * g], cw[4 * g + 1], a, o[g]), fast8(cw[4 * g + 2], cw[4 * g + 3], a, o[g]));
+      const float a = 128.0f * s[g], c = o[g] - a;
+      put(g, fast8(cw[4 * g], cw[4 * g + 1], a, c), fast8(cw[4 * g + 2], cw[4 * g + 3], a, c));
     }
   } else if constexpr (ChunkUnit<T>::kHas) {
     const typename ChunkUnit<T>::Pre pr = ChunkUnit<T>::pre(regs);

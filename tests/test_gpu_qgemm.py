@@ -48,7 +48,7 @@ def test_dense_qgemm(t, rows, tile):
     assert torch.equal(C, C2)                                   # bit-identical rerun
 
 
-@pytest.mark.parametrize("t", ["Q4_K", "Q5_K", "Q6_K", "Q8_0", "FP8_B128", "NVFP4", "IQ4_NL"])
+@pytest.mark.parametrize("t", ["Q8_0", "FP8_B128", "NVFP4", "IQ4_NL"])
 @pytest.mark.parametrize("tile", [32, 64, 128])
 def test_the_exact_form_multiplies_the_weights_of_the_bf16_copies(t, tile):
     """Rows of the identity read every weight out of the product as it was multiplied: the fp32 value rounded to bf16
