@@ -68,11 +68,31 @@ __device__ __forceinline__ uint4 q_pack8(const float* v) {
   return o;
 }
 
+// eight values as bf16 and as bf16 of what that leaves (exact in fp32)
+__device__ __forceinline__ void q_split8(const float* v, uint4& hi, uint4& lo) {
+  hi = q_pack8(v);
+  const uint32_t h[4] = {hi.x, hi.y, hi.z, hi.w};
+  float r[8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    r[2 * i] = v[2 * i] - __uint_as_float(h[i] << 16);
+    r[2 * i + 1] = v[2 * i + 1] - __uint_as_float(h[i] & 0xFFFF0000u);
+  }
+  lo = q_pack8(r);
+}
+
+// How a weight reaches the tensor cores; see the expanders below.
+enum QForm { Q_SHORT = 0, Q_EXACT = 1, Q_SPLIT = 2 };
+
 // ---- fast expanders ---------------------------------------------------------------------
 // Integer-to-float conversions run at a quarter of the FMA rate, so the K-quant expanders avoid them.
-//   exact form (prompts): a code byte q (< 128) dropped into mantissa bits 16..22 of 1.0f reads as X = 1 + q / 128, and the block's affine map
-//   v = s * q + o becomes one FMA v = (128 s) * X + (o - 128 s) on a packed pair (fma.rn.f32x2), rounded to bf16 once.
-//   The result equals the fp32 decode to within an fp32 rounding of the offset.
+//   exact form (prompts): a code byte q (< 128) dropped into mantissa bits 16..22 of 1.0f reads as X = 1 + q / 128, and the
+//   block's affine map v = s * q + o becomes one FMA v = (128 s) * X + (o - 128 s) on a packed pair (fma.rn.f32x2), rounded
+//   to bf16 once.  The result equals the fp32 decode to within an fp32 rounding of the offset (a scale is an f16 times a
+//   small integer, so the offset is exact unless s and o are far apart).
+//   split form (prompts that would otherwise run on the chain, whose integer dots round no weight): the same fp32 value as a
+//   bf16 and a bf16 remainder, 16 bits together.  The halves fill two consecutive stages over the same tokens, so the tensor
+//   cores do twice the products, of which there is room, and the expanders write twice.
 //   short form (decode rounds, which the expanders' integer pipe bounds): two code bytes become the bf16 pair
 //   (128 + q0, 128 + q1) with one byte permute, a packed bf16 subtract gives (q0, q1) exactly and a packed bf16 FMA gives
 //   s * q + o with s and o rounded to bf16: half the integer instructions, at most about one more bf16 ulp of error per
@@ -128,24 +148,19 @@ template <> struct FastUnit<Q6K> {
   }
 };
 
-// bf16x2 of (a * x0 + c, a * x1 + c) with one packed FMA
-__device__ __forceinline__ uint32_t fma2_bf16(uint32_t x0, uint32_t x1, float a, float c) {
-  uint32_t lo, hi;
+// (a * x0 + c, a * x1 + c) with one packed FMA
+__device__ __forceinline__ void fma2_f32(uint32_t x0, uint32_t x1, float a, float c, float* v) {
   asm("{\n\t.reg .b64 ra, rx, rc, rr;\n\t"
       "mov.b64 ra, {%2, %2};\n\tmov.b64 rx, {%3, %4};\n\tmov.b64 rc, {%5, %5};\n\t"
       "fma.rn.f32x2 rr, ra, rx, rc;\n\tmov.b64 {%0, %1}, rr;\n\t}"
-      : "=r"(lo), "=r"(hi) : "f"(a), "r"(x0), "r"(x1), "f"(c));
-  __nv_bfloat162 p = __floats2bfloat162_rn(__uint_as_float(lo), __uint_as_float(hi));
-  return *reinterpret_cast<uint32_t*>(&p);
+      : "=f"(v[0]), "=f"(v[1]) : "f"(a), "r"(x0), "r"(x1), "f"(c));
 }
-__device__ __forceinline__ uint4 fast8(uint32_t w0, uint32_t w1, float a, float c) {
+__device__ __forceinline__ void fast8(uint32_t w0, uint32_t w1, float a, float c, float* v) {
   w0 |= 0x80808080u; w1 |= 0x80808080u;
-  uint4 out;
-  out.x = fma2_bf16(__byte_perm(w0, 0x3F000000u, 0x7044), __byte_perm(w0, 0x3F000000u, 0x7144), a, c);
-  out.y = fma2_bf16(__byte_perm(w0, 0x3F000000u, 0x7244), __byte_perm(w0, 0x3F000000u, 0x7344), a, c);
-  out.z = fma2_bf16(__byte_perm(w1, 0x3F000000u, 0x7044), __byte_perm(w1, 0x3F000000u, 0x7144), a, c);
-  out.w = fma2_bf16(__byte_perm(w1, 0x3F000000u, 0x7244), __byte_perm(w1, 0x3F000000u, 0x7344), a, c);
-  return out;
+  fma2_f32(__byte_perm(w0, 0x3F000000u, 0x7044), __byte_perm(w0, 0x3F000000u, 0x7144), a, c, v);
+  fma2_f32(__byte_perm(w0, 0x3F000000u, 0x7244), __byte_perm(w0, 0x3F000000u, 0x7344), a, c, v + 2);
+  fma2_f32(__byte_perm(w1, 0x3F000000u, 0x7044), __byte_perm(w1, 0x3F000000u, 0x7144), a, c, v + 4);
+  fma2_f32(__byte_perm(w1, 0x3F000000u, 0x7244), __byte_perm(w1, 0x3F000000u, 0x7344), a, c, v + 6);
 }
 
 // bf16x2 FMA on raw register pairs
@@ -174,7 +189,7 @@ __device__ __forceinline__ uint4 short8(uint32_t w0, uint32_t w1, uint32_t s2, u
 }
 
 // ---- float-coded types ---------------------------------------------------------------------
-// ChunkUnit<T>::chunk(regs, j) yields values 8j .. 8j+7 of the unit as eight bf16, never holding the unit's 64 floats.
+// ChunkUnit<T>::values(regs, pre, j) yields values 8j .. 8j+7 of the unit, never holding the unit's 64 floats.
 //   FP8 (E4M3 codes, one f32 scale per 128 values): the hardware converter takes two codes to an f16 pair; the pair
 //   widens to f32, takes the block scale and is rounded to bf16 once.
 //   NVFP4 (E2M1 codes, E4M3 scale per 16 values, f32 tensor scale): a code's magnitude is one of eight values, so two
@@ -190,16 +205,13 @@ template <> struct ChunkUnit<Fp8B128> {
   static constexpr bool kOneForm = true;
   struct Pre { float sc; };
   static __device__ __forceinline__ Pre pre(const Fp8B128::Regs& r) { return Pre{r.sc}; }
-  template <bool EXACT>
-  static __device__ __forceinline__ uint4 chunk(const Fp8B128::Regs& r, const Pre& pr, int j) {
+  static __device__ __forceinline__ void values(const Fp8B128::Regs& r, const Pre& pr, int j, float* f) {
     const u32x4& q = r.q[j >> 1];
     const uint32_t w0 = (j & 1) ? q.z : q.x, w1 = (j & 1) ? q.w : q.y;
-    float f[8];
     e4m3x4_to_float(w0, f);
     e4m3x4_to_float(w1, f + 4);
 #pragma unroll
     for (int i = 0; i < 8; ++i) f[i] *= pr.sc;
-    return q_pack8(f);
   }
 };
 
@@ -214,42 +226,54 @@ template <> struct ChunkUnit<NvFp4> {
     for (int g = 0; g < 4; ++g) pr.sc[g] = pr.sc[g] * r.g * 0.5f;                  // the table below holds 2 * magnitude
     return pr;
   }
-  template <bool EXACT>
-  static __device__ __forceinline__ uint4 chunk(const NvFp4::Regs& r, const Pre& pr, int j) {
+  // bf16 pairs of 2 * magnitude with their signs
+  static __device__ __forceinline__ void codes(const NvFp4::Regs& r, int j, uint32_t* m) {
     const uint32_t w = j == 0 ? r.q0.x : j == 1 ? r.q0.y : j == 2 ? r.q0.z : j == 3 ? r.q0.w
                      : j == 4 ? r.q1.x : j == 5 ? r.q1.y : j == 6 ? r.q1.z : r.q1.w;
     const uint32_t sel = w & 0x77777777u;
     const uint32_t sodd = w & 0x80808080u, seven = (w << 4) & 0x80808080u;   // signs of the odd / the even codes
-    const float sc = pr.sc[j >> 1];
-    const uint32_t s2 = EXACT ? 0u : bf2_dup(sc);
-    uint32_t o[4];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const uint32_t c = h ? sel >> 16 : sel;
       const uint32_t lo4 = __byte_perm(0x40008000u, 0x4000C080u, c);
       const uint32_t hi4 = __byte_perm(0x40403F00u, 0x41414040u, c) | __byte_perm(seven, sodd, h ? 0x7362 : 0x5140);
-      const uint32_t m[2] = {__byte_perm(lo4, hi4, 0x5140), __byte_perm(lo4, hi4, 0x7362)};
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        if constexpr (EXACT) {
-          const __nv_bfloat162 p = __floats2bfloat162_rn(__uint_as_float(m[i] << 16) * sc, __uint_as_float(m[i] & 0xFFFF0000u) * sc);
-          o[2 * h + i] = *reinterpret_cast<const uint32_t*>(&p);
-        } else {
-          o[2 * h + i] = bf2_fma(m[i], s2, 0u);
-        }
-      }
+      m[2 * h] = __byte_perm(lo4, hi4, 0x5140);
+      m[2 * h + 1] = __byte_perm(lo4, hi4, 0x7362);
     }
-    return make_uint4(o[0], o[1], o[2], o[3]);
+  }
+  static __device__ __forceinline__ void values(const NvFp4::Regs& r, const Pre& pr, int j, float* f) {
+    uint32_t m[4];
+    codes(r, j, m);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      f[2 * i] = __uint_as_float(m[i] << 16) * pr.sc[j >> 1];
+      f[2 * i + 1] = __uint_as_float(m[i] & 0xFFFF0000u) * pr.sc[j >> 1];
+    }
+  }
+  static __device__ __forceinline__ uint4 short8(const NvFp4::Regs& r, const Pre& pr, int j) {
+    uint32_t m[4];
+    codes(r, j, m);
+    const uint32_t s2 = bf2_dup(pr.sc[j >> 1]);
+    return make_uint4(bf2_fma(m[0], s2, 0u), bf2_fma(m[1], s2, 0u), bf2_fma(m[2], s2, 0u), bf2_fma(m[3], s2, 0u));
   }
 };
 
 // Unit u (64 values of this thread's weight row) of stage kb into the A operand in tensor memory: lane = weight row,
 // 32-bit column c of the stage holds values 2c and 2c + 1.  A unit's groups of 16 values are contiguous in the row, so
-// each is one 8-column store.  Warp-collective.
-template <class T, bool EXACT>
-__device__ __forceinline__ void expand_unit(const typename Unit<T>::Regs& regs, int u, int kb, uint32_t ta) {
-  auto put = [&](int g, const uint4& x, const uint4& y) {
-    tmem_st8(ta + (uint32_t)((Unit<T>::pos(u, 16 * g) - QBK * kb) >> 1), x, y);
+// each is one 8-column store (split form: a second one at the next stage, `ta_lo`).  Warp-collective.
+template <class T, int FORM>
+__device__ __forceinline__ void expand_unit(const typename Unit<T>::Regs& regs, int u, int kb, uint32_t ta, uint32_t ta_lo) {
+  auto col = [&](int g) { return (uint32_t)((Unit<T>::pos(u, 16 * g) - QBK * kb) >> 1); };
+  auto put = [&](int g, const float* v) {
+    if constexpr (FORM == Q_SPLIT) {
+      uint4 h0, h1, l0, l1;
+      q_split8(v, h0, l0);
+      q_split8(v + 8, h1, l1);
+      tmem_st8(ta + col(g), h0, h1);
+      tmem_st8(ta_lo + col(g), l0, l1);
+    } else {
+      tmem_st8(ta + col(g), q_pack8(v), q_pack8(v + 8));
+    }
   };
   if constexpr (FastUnit<T>::kHas) {
     uint32_t cw[16];
@@ -257,23 +281,36 @@ __device__ __forceinline__ void expand_unit(const typename Unit<T>::Regs& regs, 
     FastUnit<T>::codes(regs, u, cw, s, o);
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
-      if constexpr (!EXACT) {
+      if constexpr (FORM == Q_SHORT) {
         const uint32_t s2 = bf2_dup(s[g]), o2 = bf2_dup(o[g]);
-        put(g, short8(cw[4 * g], cw[4 * g + 1], s2, o2), short8(cw[4 * g + 2], cw[4 * g + 3], s2, o2));
-        continue;
+        tmem_st8(ta + col(g), short8(cw[4 * g], cw[4 * g + 1], s2, o2), short8(cw[4 * g + 2], cw[4 * g + 3], s2, o2));
+      } else {
+        const float a = 128.0f * s[g], c = o[g] - a;
+        float v[16];
+        fast8(cw[4 * g], cw[4 * g + 1], a, c, v);
+        fast8(cw[4 * g + 2], cw[4 * g + 3], a, c, v + 8);
+        put(g, v);
       }
-      const float a = 128.0f * s[g], c = o[g] - a;
-      put(g, fast8(cw[4 * g], cw[4 * g + 1], a, c), fast8(cw[4 * g + 2], cw[4 * g + 3], a, c));
     }
   } else if constexpr (ChunkUnit<T>::kHas) {
-    const typename ChunkUnit<T>::Pre pr = ChunkUnit<T>::pre(regs);
+    using C = ChunkUnit<T>;
+    const typename C::Pre pr = C::pre(regs);
 #pragma unroll
-    for (int g = 0; g < 4; ++g) put(g, ChunkUnit<T>::template chunk<EXACT>(regs, pr, 2 * g), ChunkUnit<T>::template chunk<EXACT>(regs, pr, 2 * g + 1));
+    for (int g = 0; g < 4; ++g) {
+      if constexpr (FORM == Q_SHORT && !C::kOneForm) {
+        tmem_st8(ta + col(g), C::short8(regs, pr, 2 * g), C::short8(regs, pr, 2 * g + 1));
+      } else {
+        float v[16];
+        C::values(regs, pr, 2 * g, v);
+        C::values(regs, pr, 2 * g + 1, v + 8);
+        put(g, v);
+      }
+    }
   } else {
     float v[64];
     Unit<T>::decodeu(regs, u, v);
 #pragma unroll
-    for (int g = 0; g < 4; ++g) put(g, q_pack8(v + 16 * g), q_pack8(v + 16 * g + 8));
+    for (int g = 0; g < 4; ++g) put(g, v + 16 * g);
   }
 }
 
@@ -297,7 +334,7 @@ __host__ __device__ constexpr int q_raw_slots(int sb_bytes, bool dual, int bn) {
 
 // 768 threads: warp 0 = TMA of the token tiles, warp 1 = MMA issuer and TMEM owner, warps 2..5 = epilogue, warp 6 = TMA
 // of the raw weight super-blocks, warp 7 idle, warps 8..23 = weight expanders (warp id modulo 4 = TMEM lane quarter).
-template <class T, bool DUAL, int BN, bool EXACT>
+template <class T, bool DUAL, int BN, int FORM>
 __global__ void __launch_bounds__(QTHREADS, 1)
 qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUtensorMap tma_w,
              const __grid_constant__ CUtensorMap tma_w2, const QGemmArgs a) {
@@ -313,6 +350,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
   constexpr int ACC_COLS = (DUAL ? 2 : 1) * BN;
   constexpr int A_MAT = QBK / 2;                                     // columns of one matrix's stage
   constexpr int A_COLS = (DUAL ? 2 : 1) * A_MAT;
+  constexpr int HALVES = FORM == Q_SPLIT ? 2 : 1;                    // stages that hold one 128-deep block of weights
   constexpr int FILLERS = DUAL ? QPRODUCERS / 32 : QPRODUCERS / 64;  // warps that write one stage
   __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
   __shared__ __align__(8) uint64_t raw_full[RS > 0 ? RS : 1], raw_empty[RS > 0 ? RS : 1];
@@ -357,7 +395,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
       for (int t = blockIdx.x; t < total_tiles && !*abort_flag; t += gridDim.x) {
         const QTile mt = a.tiles[t / a.splits / a.tiles_w];
         const int kb0 = (t % a.splits) * kblocks;
-        for (int kb = kb0; kb < kb0 + kblocks; ++kb) {
+        for (int s = kb0 * HALVES; s < (kb0 + kblocks) * HALVES; ++s) {
+          const int kb = s / HALVES;
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) break;
           uint8_t* sb = smem + (size_t)stage * B_STAGE;
           mbar_expect_tx(&full_bar[stage], B_STAGE);
@@ -386,7 +425,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
         tc_fence_after();
         const uint32_t d0 = tmem_base + ab * ACC_COLS;
         bool ok = true;
-        for (int kb = 0; kb < kblocks; ++kb) {
+        for (int s = 0; s < kblocks * HALVES; ++s) {
           if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sb = smem_u32(smem + (size_t)stage * B_STAGE);
@@ -394,7 +433,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
 #pragma unroll
           for (int k = 0; k < QBK / UMMA_K; ++k) {
             const uint64_t db = umma_desc(sb + (k >> 2) * B_ATOM) + (uint64_t)((k & 3) * UMMA_K * 2 / 16);
-            const uint32_t acc = (kb > 0 || k > 0) ? 1u : 0u;
+            const uint32_t acc = (s > 0 || k > 0) ? 1u : 0u;
             umma_bf16_ta(d0, ta + k * (UMMA_K / 2), db, idesc, acc);
             if (DUAL) umma_bf16_ta(d0 + BN, ta + A_MAT + k * (UMMA_K / 2), db, idesc, acc);
           }
@@ -522,19 +561,24 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
     const int row = q * 32 + lane, mat = DUAL ? grp >> 1 : 0, half = grp & 1;
     const int kb_first = DUAL ? 0 : grp >> 1;
     const uint32_t ta0 = tmem_a + ((uint32_t)(q * 32) << 16) + mat * A_MAT;
-    unsigned lin = (unsigned)kb_first;                               // stages of this CTA so far, over all its tiles
+    unsigned lin = (unsigned)kb_first * HALVES;                      // stages of this CTA so far, over all its tiles
     bool ok = true;
     auto emit = [&](int kb, const typename U::Regs& r) {
       const unsigned stage = lin % STAGES, phase = (lin / STAGES) & 1;
-      lin += STEP;
+      const unsigned next = (lin + 1) % STAGES, next_phase = ((lin + 1) / STAGES) & 1;    // split form: the remainders' stage
+      lin += STEP * HALVES;
       ok = __all_sync(0xFFFFFFFFu, mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag));
+      if (ok && HALVES == 2) ok = __all_sync(0xFFFFFFFFu, mbar_wait(&empty_bar[next], next_phase ^ 1, abort_flag));
       if (!ok) return;
       tc_fence_after();
-      expand_unit<T, EXACT>(r, 2 * kb + half, kb, ta0 + stage * A_COLS);
+      expand_unit<T, FORM>(r, 2 * kb + half, kb, ta0 + stage * A_COLS, ta0 + next * A_COLS);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&full_bar[stage]);
+      if (lane == 0) {
+        mbar_arrive(&full_bar[stage]);
+        if (HALVES == 2) mbar_arrive(&full_bar[next]);
+      }
     };
     if constexpr (RS > 0) {
       // raw ring: the tile's super-blocks arrive by TMA; a thread reads its row's units out of shared memory
@@ -588,7 +632,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
   if (threadIdx.x == 0 && s_abort && a.status) atomicMax(a.status, 1u);
 }
 
-template <class T, bool DUAL, int BN, bool EXACT>
+template <class T, bool DUAL, int BN, int FORM>
 static int qgemm_go(const CUtensorMap& mx, const QGemmArgs& a, int n_groups, int grid, cudaStream_t st) {
   constexpr int SB = SbBytes<T>::v;
   constexpr int RS = q_raw_slots(SB, DUAL, BN);
@@ -605,23 +649,29 @@ static int qgemm_go(const CUtensorMap& mx, const QGemmArgs& a, int n_groups, int
   }
   static bool set = false;
   if (!set) {
-    cudaFuncSetAttribute(qgemm_kernel<T, DUAL, BN, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(qgemm_kernel<T, DUAL, BN, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     set = true;
   }
-  return (int)launch(qgemm_kernel<T, DUAL, BN, EXACT>, dim3(grid), dim3(QTHREADS), smem, st, mx, mw, mw2, a);
+  return (int)launch(qgemm_kernel<T, DUAL, BN, FORM>, dim3(grid), dim3(QTHREADS), smem, st, mx, mw, mw2, a);
 }
 
 template <class T, bool DUAL>
-static int qgemm_pick(bool exact, int bn, const CUtensorMap& mx, const QGemmArgs& a, int n_groups, int grid, cudaStream_t st) {
-  constexpr bool kOne = !FastUnit<T>::kHas && ChunkUnit<T>::kOneForm;   // types with an exact form only
-  if (bn == 128) return qgemm_go<T, DUAL, 128, true>(mx, a, n_groups, grid, st);
-  if (bn == 64) return exact ? qgemm_go<T, DUAL, 64, true>(mx, a, n_groups, grid, st) : qgemm_go<T, DUAL, 64, kOne>(mx, a, n_groups, grid, st);
-  if (bn == 32) return exact ? qgemm_go<T, DUAL, 32, true>(mx, a, n_groups, grid, st) : qgemm_go<T, DUAL, 32, kOne>(mx, a, n_groups, grid, st);
+static int qgemm_pick(int form, int bn, const CUtensorMap& mx, const QGemmArgs& a, int n_groups, int grid, cudaStream_t st) {
+  constexpr int kShort = !FastUnit<T>::kHas && ChunkUnit<T>::kOneForm ? Q_EXACT : Q_SHORT;   // types without a short form
+  if (form == Q_SPLIT) {
+    if (bn == 32) return qgemm_go<T, DUAL, 32, Q_SPLIT>(mx, a, n_groups, grid, st);
+    if constexpr (!DUAL) { if (bn == 64) return qgemm_go<T, false, 64, Q_SPLIT>(mx, a, n_groups, grid, st); }
+    return BL_ERR_SHAPE;
+  }
+  const bool exact = form == Q_EXACT;
+  if (bn == 128) return qgemm_go<T, DUAL, 128, Q_EXACT>(mx, a, n_groups, grid, st);
+  if (bn == 64) return exact ? qgemm_go<T, DUAL, 64, Q_EXACT>(mx, a, n_groups, grid, st) : qgemm_go<T, DUAL, 64, kShort>(mx, a, n_groups, grid, st);
+  if (bn == 32) return exact ? qgemm_go<T, DUAL, 32, Q_EXACT>(mx, a, n_groups, grid, st) : qgemm_go<T, DUAL, 32, kShort>(mx, a, n_groups, grid, st);
   return BL_ERR_SHAPE;
 }
 template <class T>
-static int qgemm_pick(bool dual, bool exact, int bn, const CUtensorMap& mx, const QGemmArgs& a, int n_groups, int grid, cudaStream_t st) {
-  return dual ? qgemm_pick<T, true>(exact, bn, mx, a, n_groups, grid, st) : qgemm_pick<T, false>(exact, bn, mx, a, n_groups, grid, st);
+static int qgemm_pick(bool dual, int form, int bn, const CUtensorMap& mx, const QGemmArgs& a, int n_groups, int grid, cudaStream_t st) {
+  return dual ? qgemm_pick<T, true>(form, bn, mx, a, n_groups, grid, st) : qgemm_pick<T, false>(form, bn, mx, a, n_groups, grid, st);
 }
 
 }  // namespace bl
@@ -640,18 +690,20 @@ int bl_qgemm_supports(int wtype) {
 //   X [rows_x, K] bf16 (ldx elements); W, W2 [n_groups, N, row_bytes] resident blocks of type wtype;
 //   tiles: {group, row0, row_end, -} token tiles of at most tile_rows (32, 64 or 128) rows; exactly one of c_f32 / c_bf16;
 //   W2 != null: output = silu(X W^T) * (X W2^T).  status: device word, set to 1 when a wait ran out.
-//   exact: the weights' fp32 values rounded to bf16 once, at every tile size (see the expanders above).
+//   form: 0 short (exact at 128-row tiles), 1 exact, 2 split (tiles of 32 rows, and of 64 with one matrix); see the
+//   expanders above.
 //   fixed_tiles: the table has exactly max_tiles tiles and no launch in flight writes it.  splits > 1 (fixed tiles, one
 //   matrix, K / 256 divisible): that many CTAs share a tile's depth; partial: max_tiles * ceil(N / 128) * splits *
 //   tile_rows * 128 floats, tickets: max_tiles * ceil(N / 128) * 4 zeroed words, both of one stream at a time.
 int bl_qgemm_split(const void* X, long ldx, long rows_x, const void* W, const void* W2, int wtype, int n_groups, int N, int K,
              const void* tiles, const int* n_tiles, int max_tiles, int tile_rows, float* c_f32, void* c_bf16, long ldc,
              const int* dst_row, const float* row_scale, const float* resid, long ldr, unsigned* status, int sm_count,
-             int fixed_tiles, int exact, int splits, float* partial, int* tickets, cudaStream_t st) {
+             int fixed_tiles, int form, int splits, float* partial, int* tickets, cudaStream_t st) {
   BL_REQUIRE(K >= 256 && K % 256 == 0 && N >= 1 && rows_x >= 1 && n_groups >= 1 && max_tiles >= 1, BL_ERR_SHAPE);
   BL_REQUIRE(tile_rows == 32 || tile_rows == 64 || tile_rows == 128, BL_ERR_SHAPE);
   BL_REQUIRE(ldx % 8 == 0 && ((uintptr_t)X & 15) == 0 && ((uintptr_t)W & 15) == 0 && ((uintptr_t)W2 & 15) == 0, BL_ERR_ALIGN);
   BL_REQUIRE((c_f32 != nullptr) != (c_bf16 != nullptr), BL_ERR_SHAPE);
+  BL_REQUIRE(form >= Q_SHORT && form <= Q_SPLIT && (form != Q_SPLIT || tile_rows <= (W2 ? 32 : 64)), BL_ERR_SHAPE);
   BL_REQUIRE(splits == 1 || (splits > 1 && fixed_tiles && !W2 && partial && tickets && (K / 256) % splits == 0), BL_ERR_SHAPE);
   const long rb = resident_row_bytes(wtype, K);
   BL_REQUIRE(rb > 0 && bl_qgemm_supports(wtype), BL_ERR_TYPE);
@@ -675,13 +727,13 @@ int bl_qgemm_split(const void* X, long ldx, long rows_x, const void* W, const vo
   const int grid = (int)(tiles_total < sm_count ? tiles_total : sm_count);
   const bool dual = W2 != nullptr;
   switch (wtype) {
-    case WT_Q4_K: return qgemm_pick<Q4K>(dual, exact != 0, tile_rows, mx, a, n_groups, grid, st);
-    case WT_Q5_K: return qgemm_pick<Q5K>(dual, exact != 0, tile_rows, mx, a, n_groups, grid, st);
-    case WT_Q6_K: return qgemm_pick<Q6K>(dual, exact != 0, tile_rows, mx, a, n_groups, grid, st);
-    case WT_Q8_0: return qgemm_pick<Q80>(dual, exact != 0, tile_rows, mx, a, n_groups, grid, st);
-    case WT_FP8_B128: return qgemm_pick<Fp8B128>(dual, exact != 0, tile_rows, mx, a, n_groups, grid, st);
-    case WT_NVFP4: return qgemm_pick<NvFp4>(dual, exact != 0, tile_rows, mx, a, n_groups, grid, st);
-    case WT_Q8_F32: return qgemm_pick<Q8F>(dual, exact != 0, tile_rows, mx, a, n_groups, grid, st);
+    case WT_Q4_K: return qgemm_pick<Q4K>(dual, form, tile_rows, mx, a, n_groups, grid, st);
+    case WT_Q5_K: return qgemm_pick<Q5K>(dual, form, tile_rows, mx, a, n_groups, grid, st);
+    case WT_Q6_K: return qgemm_pick<Q6K>(dual, form, tile_rows, mx, a, n_groups, grid, st);
+    case WT_Q8_0: return qgemm_pick<Q80>(dual, form, tile_rows, mx, a, n_groups, grid, st);
+    case WT_FP8_B128: return qgemm_pick<Fp8B128>(dual, form, tile_rows, mx, a, n_groups, grid, st);
+    case WT_NVFP4: return qgemm_pick<NvFp4>(dual, form, tile_rows, mx, a, n_groups, grid, st);
+    case WT_Q8_F32: return qgemm_pick<Q8F>(dual, form, tile_rows, mx, a, n_groups, grid, st);
   }
   return BL_ERR_TYPE;
 }

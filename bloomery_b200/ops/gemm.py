@@ -253,12 +253,13 @@ def qgemm_splits(n_tiles: int, depth_blocks: int, sm: int) -> int:
 def qgemm(X: torch.Tensor, W: QWeight, tiles: TileTable, *, out_f32: Optional[torch.Tensor] = None,
           out_bf16: Optional[torch.Tensor] = None, W2: Optional[QWeight] = None, dst_row=None, row_scale=None,
           resid=None, status: Optional[torch.Tensor] = None, work: Optional[QgemmWork] = None,
-          exact: bool = False) -> None:
+          exact: bool = False, fine: bool = False) -> None:
     """C = X @ W[g].T per token tile with W left block-quantised (``csrc/qgemm_tcgen05.cu``): X [rows, K] bf16, W (and
     W2) resident Q4_K / Q5_K / Q6_K / Q8_0 / FP8_B128 / NVFP4 / Q8_F32 matrices [N, bytes] or stacks [G, N, bytes]; tiles of
     32, 64 or 128 token rows.
     With W2 the output is silu(X W^T) * (X W2^T).  With ``work`` a product of few tiles splits its depth over CTAs.
-    ``exact``: K-quant weights are rounded to bf16 once from their fp32 values in tiles of 32 and 64 rows too."""
+    ``exact``: weights are rounded to bf16 once from their fp32 values in tiles of 32 and 64 rows too.  ``fine``: they enter as
+    a bf16 value and a bf16 remainder, 16 bits together (tiles of 32 rows, with one matrix of 64 too)."""
     assert X.dtype == torch.bfloat16 and X.stride(-1) == 1 and W.data.is_contiguous() and tiles.tile_rows in (32, 64, 128)
     assert W2 is None or (W2.wt == W.wt and W2.data.shape == W.data.shape and W2.data.is_contiguous())
     G = W.data.shape[0] if W.data.dim() == 3 else 1
@@ -272,8 +273,8 @@ def qgemm(X: torch.Tensor, W: QWeight, tiles: TileTable, *, out_f32: Optional[to
                                I(G), I(N), I(W.k), p(tiles.mtiles), p(tiles.n_mtiles), I(tiles.fixed or tiles.max_mtiles),
                                I(tiles.tile_rows), p(out_f32), p(out_bf16), L(out.stride(0)), p(dst_row), p(row_scale),
                                p(resid), L(resid.stride(0) if resid is not None else 0), p(status), I(sm),
-                               I(1 if tiles.fixed else 0), I(1 if exact else 0), I(splits), p(work.partial if splits > 1 else None),
-                               p(work.tickets if splits > 1 else None), stream())
+                               I(1 if tiles.fixed else 0), I(2 if fine else 1 if exact else 0), I(splits),
+                               p(work.partial if splits > 1 else None), p(work.tickets if splits > 1 else None), stream())
     check(rc, "bl_qgemm_split")
 
 

@@ -26,6 +26,7 @@ from ..ops import decode as K
 from .kv import PAGE, KvPool
 
 MAX_ROWS = 8
+GEMM_THRESHOLD = 64         # prompts of at least this many ids take the GEMM path unless the caller moves the line
 FAULT_CLEAN = 0xFFFFFFFF
 
 FAULT_SITES = {1: "token id out of range", 2: "non-finite activation", 3: "non-finite router logit",
@@ -184,7 +185,7 @@ class DecodeEngine:
         self.launches_per_step = 0
         self.steps = 0
         # prompts at least this long use the GEMM path (0 = never; the GEMM path serves the GQA + routed-expert plan)
-        self.gemm_threshold = 0 if (s.mla or s.n_shared or layers is not None or self.kv_q8) else 64
+        self.gemm_threshold = 0 if (s.mla or s.n_shared or layers is not None or self.kv_q8) else GEMM_THRESHOLD
         # shorter ones too where that path multiplies the quantised blocks themselves: a pass of the chain over eight rows took
         # 7.3 ms on the 30 B shape, that path 13 ms for 36 rows; from 32 ids on it has won by a factor of two
         self.direct_threshold = 32

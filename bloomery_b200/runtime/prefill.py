@@ -28,6 +28,7 @@ import torch
 
 from ..ops import decode as K
 from ..ops import gemm as G
+from .engine import GEMM_THRESHOLD
 from .kv import PAGE
 
 
@@ -95,14 +96,17 @@ class GemmPrefill:
         for p in range(start, start + n, PAGE):
             e.kv.own(slot, p)
         e.kv.sync_table()
+        # A prompt that would run on the 8-row chain if it were not here keeps what the chain gives it: weights that are not
+        # rounded to bf16 (value and remainder) and queries, probabilities, keys and values as decode attention has them.
+        fine = n < GEMM_THRESHOLD and self._direct(n)
         i = 0
         while i < n:
             chunk = tokens[i:i + self.ubatch]
-            self._ubatch(slot, chunk, start + i)
+            self._ubatch(slot, chunk, start + i, fine)
             i += len(chunk)
         e.slot_len[slot] = max(e.slot_len[slot], start + n)
 
-    def _ubatch(self, slot: int, tokens: Sequence[int], p0: int) -> None:
+    def _ubatch(self, slot: int, tokens: Sequence[int], p0: int, fine: bool = False) -> None:
         e = self.e
         s, w, dev = e.spec, e.w, e.device
         T = len(tokens)
@@ -124,7 +128,15 @@ class GemmPrefill:
         nset = 2 if ahead else 1
         wqkv_s = [None if direct else self._get(f"wqkv{i}", (qkv_w, H), bf) for i in range(nset)]
         wo_s = [None if direct else self._get(f"wo{i}", (H, s.q_rows), bf) for i in range(nset)]
-        q_bf = self._get("q_bf", (s.n_q, T, s.head_dim), bf)
+        form = dict(fine=True) if fine else dict(exact=True)
+        if fine:
+            # key segments as in a decode round: about eight blocks a processor
+            n_seg = max(1, min(e.n_seg, 8 * K.sm_count(dev) // (s.n_kv * T)))
+            q_rows = self._get("q_rows", (T, s.n_q, s.head_dim), f32)
+            part_ml = self._get("part_ml", (T * s.n_q * n_seg * 2,), f32)
+            part_acc = self._get("part_acc", (T * s.n_q * n_seg * s.head_dim,), f32)
+        else:
+            q_bf = self._get("q_bf", (s.n_q, T, s.head_dim), bf)
         attn = self._get("attn", (T, s.q_rows), bf)
         if direct:
             dense_tiles = G.TileTable.dense(T, dev, 32 if T <= 32 else 64 if T <= 64 else 128, host=True)
@@ -134,8 +146,9 @@ class GemmPrefill:
             dense_tiles = G.TileTable.dense(T, dev)
         n_keys = p0 + T
         T_pad = (n_keys + 127) // 128 * 128
-        Kb = self._get("Kb", (s.n_kv, T_pad, s.head_dim), bf)
-        Vt = self._get("Vt", (s.n_kv, s.head_dim, T_pad), bf)
+        if not fine:
+            Kb = self._get("Kb", (s.n_kv, T_pad, s.head_dim), bf)
+            Vt = self._get("Vt", (s.n_kv, s.head_dim, T_pad), bf)
         Tq_max = max(128, min(T, self.score_bytes // (s.n_q * T_pad * 4) // 128 * 128))
         Gq = s.n_q // s.n_kv
         if s.is_moe:
@@ -244,41 +257,50 @@ class GemmPrefill:
                 lo = 0
                 for nm in ("attn_q", "attn_k", "attn_v"):
                     wq = w.q[b + nm + ".weight"]
-                    G.qgemm(xn, wq, dense_tiles, out_f32=qkv[:, lo:lo + wq.rows], status=st, work=self._work, exact=True)
+                    G.qgemm(xn, wq, dense_tiles, out_f32=qkv[:, lo:lo + wq.rows], status=st, work=self._work, **form)
                     lo += wq.rows
             else:
                 if not ahead and not resident:
                     expand(il, "attn")
                 G.gemm_bf16(xn, wqkv, dense_tiles, out_f32=qkv, status=st)
             self.timing.mark(il, "qkv_gemm")
-            G.qk_norm_rope_append_prefill(qkv, w.f.get(b + "attn_q_norm.weight"), w.f.get(b + "attn_k_norm.weight"),
-                                          e.inv_freq, s.rms_eps, 1.0 / math.sqrt(s.head_dim), s.head_dim, s.n_q, s.n_kv,
-                                          T, row_pos, row_seq, e.kv.table, e.kv.n_pages, e.kv.k[il], e.kv.v[il], q_bf,
-                                          e.fault, il)
-            self.timing.mark(il, "rope_append")
-            G.kv_gather_bf16(e.kv.k[il], e.kv.v[il], e.kv.table[slot], e.kv.n_pages, s.n_kv, s.head_dim, n_keys, T_pad,
-                             Kb, Vt)
-            self.timing.mark(il, "qkv")
-            if s.head_dim == 128 and self.flash:
-                # scores, softmax and values in one tcgen05 launch: the score matrix stays in tensor memory
-                G.flash_prefill(q_bf, Kb, Vt, attn, p0, st)
+            if fine:
+                K.qk_norm_rope_append(qkv, w.f.get(b + "attn_q_norm.weight"), w.f.get(b + "attn_k_norm.weight"), e.inv_freq,
+                                      s.rms_eps, e.attn_scale, s.head_dim, s.n_q, s.n_kv, T, row_pos, row_seq, e.kv.table,
+                                      e.kv.n_pages, e.kv.k[il], e.kv.v[il], q_rows, e.fault, il)
+                self.timing.mark(il, "rope_append")
+                K.flash_decode_bf16(q_rows, e.kv.k[il], e.kv.v[il], row_pos, row_seq, e.kv.table, e.kv.n_pages, s.head_dim,
+                                    s.n_q, s.n_kv, T, n_seg, e.slot_ctx, part_ml, part_acc, attn, e.fault, il)
                 self.timing.mark(il, "flash")
-            for c0 in range(0, T if not (s.head_dim == 128 and self.flash) else 0, Tq_max):
-                Tq = min(Tq_max, T - c0)
-                rows = s.n_q * Tq
-                S = self._get("S", (rows, T_pad), f32)
-                P = self._get("P", (rows, T_pad), bf)
-                qk_tiles, pv_tiles, map_s, map_o = self._attn_tables(T, Tq, c0, s.n_q, Gq, p0)
-                G.gemm_bf16(q_bf.view(s.n_q * T, s.head_dim), Kb, qk_tiles, out_f32=S, dst_row=map_s, status=st)
-                self.timing.mark(il, "scores")
-                G.softmax_causal(S, rows, Tq, p0 + c0, T_pad, P)
-                self.timing.mark(il, "softmax")
-                G.gemm_bf16(P, Vt, pv_tiles, out_bf16=attn.view(T * s.n_q, s.head_dim), dst_row=map_o, status=st)
-                self.timing.mark(il, "values")
+            else:
+                G.qk_norm_rope_append_prefill(qkv, w.f.get(b + "attn_q_norm.weight"), w.f.get(b + "attn_k_norm.weight"),
+                                              e.inv_freq, s.rms_eps, 1.0 / math.sqrt(s.head_dim), s.head_dim, s.n_q, s.n_kv,
+                                              T, row_pos, row_seq, e.kv.table, e.kv.n_pages, e.kv.k[il], e.kv.v[il], q_bf,
+                                              e.fault, il)
+                self.timing.mark(il, "rope_append")
+                G.kv_gather_bf16(e.kv.k[il], e.kv.v[il], e.kv.table[slot], e.kv.n_pages, s.n_kv, s.head_dim, n_keys, T_pad,
+                                 Kb, Vt)
+                self.timing.mark(il, "qkv")
+                if s.head_dim == 128 and self.flash:
+                    # scores, softmax and values in one tcgen05 launch: the score matrix stays in tensor memory
+                    G.flash_prefill(q_bf, Kb, Vt, attn, p0, st)
+                    self.timing.mark(il, "flash")
+                for c0 in range(0, T if not (s.head_dim == 128 and self.flash) else 0, Tq_max):
+                    Tq = min(Tq_max, T - c0)
+                    rows = s.n_q * Tq
+                    S = self._get("S", (rows, T_pad), f32)
+                    P = self._get("P", (rows, T_pad), bf)
+                    qk_tiles, pv_tiles, map_s, map_o = self._attn_tables(T, Tq, c0, s.n_q, Gq, p0)
+                    G.gemm_bf16(q_bf.view(s.n_q * T, s.head_dim), Kb, qk_tiles, out_f32=S, dst_row=map_s, status=st)
+                    self.timing.mark(il, "scores")
+                    G.softmax_causal(S, rows, Tq, p0 + c0, T_pad, P)
+                    self.timing.mark(il, "softmax")
+                    G.gemm_bf16(P, Vt, pv_tiles, out_bf16=attn.view(T * s.n_q, s.head_dim), dst_row=map_o, status=st)
+                    self.timing.mark(il, "values")
             self.timing.mark(il, "attention")
             if direct:
                 G.qgemm(attn, w.q[b + "attn_output.weight"], dense_tiles, out_f32=x, resid=x, status=st, work=self._work,
-                        exact=True)
+                        **form)
             else:
                 G.gemm_bf16(attn, wo, dense_tiles, out_f32=x, resid=x, status=st)
             self.timing.mark(il, "o_proj")
@@ -305,9 +327,9 @@ class GemmPrefill:
                 self.timing.mark(il, "dispatch")
                 if direct:
                     qg, qu, qd = (w.q[b + f"ffn_{n}_exps.weight"] for n in ("gate", "up", "down"))
-                    G.qgemm(Ap, qg, moe_tiles, out_bf16=act, W2=qu, status=st, exact=True)
+                    G.qgemm(Ap, qg, moe_tiles, out_bf16=act, W2=qu, status=st, **form)
                     self.timing.mark(il, "gemm_gate_up")
-                    G.qgemm(act, qd, moe_tiles, out_f32=slot_out, dst_row=dst_row, row_scale=row_scale, status=st, exact=True)
+                    G.qgemm(act, qd, moe_tiles, out_f32=slot_out, dst_row=dst_row, row_scale=row_scale, status=st, **form)
                 else:
                     if not ahead and not resident:
                         expand(il, "gate_up")

@@ -72,6 +72,36 @@ def test_the_exact_form_multiplies_the_weights_of_the_bf16_copies(t, tile):
     assert torch.allclose(D, torch.nn.functional.silu(g) * u, rtol=4e-6, atol=1e-12)
 
 
+@pytest.mark.parametrize("t", ["Q4_K", "Q5_K", "Q6_K", "Q8_0", "FP8_B128", "NVFP4", "IQ4_NL"])
+@pytest.mark.parametrize("tile,K", [(32, 256), (32, 2304), (64, 256), (64, 2304)])
+def test_the_split_form_keeps_sixteen_bits_of_every_weight(t, tile, K):
+    """Identity rows again: value and remainder add up to the fp32 weight to 2^-17 of it; depths of one super-block and of
+    several turns of the operand ring, the SwiGLU pair and a depth shared by several CTAs too."""
+    from bloomery_b200.ops import gemm as G
+    N = 136
+    (w, v), (w2, v2) = _weight(t, (N,), K, 23), _weight(t, (N,), K, 24)
+    X = torch.eye(K, dtype=torch.bfloat16, device=DEV)[:97 if K > 256 else K].contiguous()
+    X[5, K - 1] = 1                                              # a row that reaches both ends of the depth
+    st, tiles = _status(), G.TileTable.dense(X.shape[0], DEV, tile)
+    C, S, D = (torch.full((X.shape[0], N), float("nan"), device=DEV) for _ in range(3))
+    G.qgemm(X, w, tiles, out_f32=C, status=st, fine=True)
+    G.qgemm(X, w, tiles, out_f32=S, status=st, fine=True, work=G.QgemmWork(DEV))
+    if tile == 32:
+        G.qgemm(X, w, tiles, out_f32=D, W2=w2, status=st, fine=True)
+    torch.cuda.synchronize()
+    assert int(st) == 0
+    g, u = (X.float() @ m.T for m in (v, v2))
+    # what the remainder's own rounding leaves is 2^-18 of a weight; row 5 adds two weights
+    bound = 2 ** -17 * (X.float() @ v.abs().T)
+    assert bool(((C - g).abs() <= bound).all()), (C - g).abs().max()
+    assert bool(((S - g).abs() <= bound).all())
+    if tile == 32:
+        # the slope of silu is below 1.1; its fp32 exponential and division add a few 2^-22
+        silu = torch.nn.functional.silu(g)
+        bound2 = 1.1 * u.abs() * bound + silu.abs() * 2 ** -17 * (X.float() @ v2.abs().T) + 4e-6 * (silu * u).abs()
+        assert bool(((D - silu * u).abs() <= bound2).all()), (D - silu * u).abs().max()
+
+
 @pytest.mark.parametrize("gt,dt", [("Q4_K", "Q6_K"), ("FP8_B128", "FP8_B128"), ("NVFP4", "NVFP4")])
 @pytest.mark.parametrize("tile,T", [(128, 700), (32, 24)])
 def test_grouped_dual_swiglu_and_scatter_quantised(tile, T, gt, dt):

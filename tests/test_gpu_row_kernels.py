@@ -131,3 +131,37 @@ def test_short_prompts_over_quantised_blocks_agree_with_the_bf16_copies(n, start
         out.append(eng.logits[0].double().cpu())
     # the same bf16 operands, their fp32 sums in another order: a layer's roundings to bf16 differ in places, four layers deep
     assert float((out[0] - out[1]).norm() / out[1].norm()) < 2e-2
+
+
+@pytest.mark.parametrize("n", [32, 33, 63])
+@pytest.mark.parametrize("mix", ["Q4_K_M", "NVFP4"])
+def test_prompts_below_the_gemm_threshold_round_activations_and_nothing_else(n, mix):
+    """Keys and values behind the first layer against the fp32 oracle.  The bf16 copies round weights, queries,
+    probabilities, keys and values as well, the chain rounds activations to eight bits."""
+    from bloomery_b200.models.cpu_ref import CpuModel
+    from bloomery_b200.models.spec import tiny_qwen3moe
+    from bloomery_b200.models.weights import Weights, synth_tensors
+    from bloomery_b200.runtime.engine import DecodeEngine
+    spec = tiny_qwen3moe()
+    w = Weights.from_items(spec, synth_tensors(spec, "cpu", seed=0, mix=mix), "cpu")
+    g = torch.Generator().manual_seed(n)
+    ids = torch.randint(0, spec.vocab, (n,), generator=g)
+    oracle = CpuModel(w, quantize_acts=False)
+    oracle.forward(ids)
+    w = w.to(DEV)
+    err = {}
+    for route in ("chain", "blocks", "copies"):
+        eng = DecodeEngine(w, n_slots=1, slot_ctx=512)
+        eng._gemm_prefill = eng._new_gemm_prefill()
+        eng._gemm_prefill.direct_rows = 128 if route == "blocks" else 0
+        assert eng._gemm_prefill._direct(n) == (route == "blocks")
+        eng.prefill(0, ids.tolist(), gemm=route != "chain")
+        pages = torch.tensor(eng.kv.pages[0], device=DEV)
+        new = [c[1, pages].permute(0, 2, 1, 3).reshape(-1, spec.n_kv, spec.head_dim)[:n].float().cpu()
+               for c in (eng.kv.k, eng.kv.v)]
+        want = [oracle.k[1], oracle.v[1]]
+        # a median over the rows: where two experts are all but equal, one rounding chooses another
+        err[route] = float(torch.stack([((a - b).flatten(1).norm(dim=1) / b.flatten(1).norm(dim=1)).median()
+                                        for a, b in zip(new, want)]).mean())
+    # rounding weights and activations alike adds 1.41 times what activations alone add
+    assert err["blocks"] < 0.85 * err["copies"] and err["blocks"] < 0.5 * err["chain"], err

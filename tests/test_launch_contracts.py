@@ -33,6 +33,15 @@ def test_quantised_gemm_refuses_before_it_launches():
     assert cuda().bl_qgemm_supports(I(WT_F32)) == 0
 
 
+def test_forms_of_a_weight_that_the_quantised_gemm_has_no_kernel_for_are_refused():
+    def call(form, tile_rows, pair):
+        return cuda().bl_qgemm_split(P(A), L(1024), L(64), P(A), P(A if pair else 0), I(WT_Q4_K), I(1), I(256), I(1024), P(A), P(A), I(4),
+                                     I(tile_rows), P(A), P(0), L(256), P(0), P(0), P(0), L(0), P(0), I(148), I(0), I(form), I(1),
+                                     P(0), P(0), P(0))
+    assert call(3, 32, False) == SHAPE and call(-1, 32, False) == SHAPE
+    assert call(2, 128, False) == SHAPE and call(2, 64, True) == SHAPE and call(2, 128, True) == SHAPE
+
+
 def _fp8_gemm(K=1024, tile_rows=32, x=A, ldx=None, c_f32=A, c_bf16=0):
     return cuda().bl_fp8_gemm(P(x), L(K if ldx is None else ldx), L(64), P(A), P(A), P(0), I(1), I(256), I(K), P(A), P(A), I(4),
                               I(tile_rows), P(c_f32), P(c_bf16), L(256), P(0), P(0), P(0), L(0), P(0), I(148), P(0))
