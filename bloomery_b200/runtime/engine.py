@@ -186,8 +186,9 @@ class DecodeEngine:
         self.steps = 0
         # prompts at least this long use the GEMM path (0 = never; the GEMM path serves the GQA + routed-expert plan)
         self.gemm_threshold = 0 if (s.mla or s.n_shared or layers is not None or self.kv_q8) else GEMM_THRESHOLD
-        # shorter ones too where that path multiplies the quantised blocks themselves: a pass of the chain over eight rows took
-        # 7.3 ms on the 30 B shape, that path 13 ms for 36 rows; from 32 ids on it has won by a factor of two
+        # Shorter ones, from this many ids on, where a caller asks for them (short_prompt_on_blocks).  Eight layers of the 30 B
+        # shape, milliseconds on the chain and over the blocks: Q4_K_M 16 ids 2.8 / 2.9, 24 ids 4.0 / 3.4, 32 ids 5.3 / 3.5,
+        # 63 ids 10.2 / 4.2; FP8 32 ids 9.0 / 3.6; NVFP4 32 ids 10.4 / 3.9.  The chain is left where it loses by a half.
         self.direct_threshold = 32
         self.ubatch = 4096
         self._gemm_prefill = None
@@ -624,8 +625,11 @@ class DecodeEngine:
         from .prefill import GemmPrefill
         return GemmPrefill(self, ubatch=self.ubatch)
 
-    def _direct_prompt(self, n: int) -> bool:
-        if n < self.direct_threshold or type(self) is not DecodeEngine or not self.spec.is_moe:
+    def short_prompt_on_blocks(self, n: int) -> bool:
+        """Whether a prompt of ``n`` ids below ``gemm_threshold`` is fed faster, and with no bit less, by ``gemm=True``: the
+        GEMM path over the quantised blocks.  Only for callers that read no logits of it: the chain leaves the rows of
+        its last pass in ``logits``, the GEMM path the last row alone."""
+        if not self.direct_threshold <= n < self.gemm_threshold or type(self) is not DecodeEngine or not self.spec.is_moe:
             return False
         if self._gemm_prefill is None:
             self._gemm_prefill = self._new_gemm_prefill()
@@ -633,11 +637,10 @@ class DecodeEngine:
 
     def prefill(self, slot: int, tokens: Sequence[int], start: int = 0, gemm: Optional[bool] = None) -> int:
         """Feed a prompt; returns the greedy token after it.  Prompts of at least
-        ``gemm_threshold`` rows (``direct_threshold`` where it multiplies the quantised blocks themselves) go
-        through the tcgen05 GEMM path in micro-batches, shorter ones through passes of up to 8 rows of the decode
-        chain."""
+        ``gemm_threshold`` rows go through the tcgen05 GEMM path in micro-batches, shorter
+        ones through passes of up to 8 rows of the decode chain."""
         n = len(tokens)
-        use_gemm = gemm if gemm is not None else (self.gemm_threshold > 0 and (n >= self.gemm_threshold or self._direct_prompt(n)))
+        use_gemm = gemm if gemm is not None else (self.gemm_threshold > 0 and n >= self.gemm_threshold)
         use_gemm = use_gemm and not self.mtp_on        # the draft layer's prompt rows run on the pass path
         if use_gemm and n > 1:
             if self._gemm_prefill is None:

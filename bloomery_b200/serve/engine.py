@@ -167,7 +167,12 @@ class GpuEngine(Engine):
         from ..runtime.engine import EngineFault, EngineStalled
         try:
             if len(ids):
-                self.dec.prefill(slot, list(ids), start)
+                # a prompt's logits are not read here (its last id opens the first round), so short ones may take the blocks
+                blocks = getattr(self.dec, "short_prompt_on_blocks", None)
+                if blocks is not None and blocks(len(ids)):
+                    self.dec.prefill(slot, list(ids), start, gemm=True)
+                else:
+                    self.dec.prefill(slot, list(ids), start)
         except (EngineFault, EngineStalled) as exc:
             raise EngineError(str(exc)) from exc
 

@@ -165,3 +165,23 @@ def test_prompts_below_the_gemm_threshold_round_activations_and_nothing_else(n, 
                                         for a, b in zip(new, want)]).mean())
     # rounding weights and activations alike adds 1.41 times what activations alone add
     assert err["blocks"] < 0.85 * err["copies"] and err["blocks"] < 0.5 * err["chain"], err
+
+
+def test_a_short_prompt_leaves_the_logits_of_its_last_rows_unless_the_server_feeds_it():
+    from bloomery_b200.models.spec import tiny_qwen3moe
+    from bloomery_b200.models.weights import Weights, synth_tensors
+    from bloomery_b200.runtime.engine import DecodeEngine
+    from bloomery_b200.serve.engine import GpuEngine
+    from bloomery_b200.serve.tokenizer import ByteTokenizer
+    spec = tiny_qwen3moe()
+    w = Weights.from_items(spec, synth_tensors(spec, "cpu", seed=0), "cpu").to(DEV)
+    g = torch.Generator().manual_seed(9)
+    ids = torch.randint(0, spec.vocab, (45,), generator=g).tolist()
+    eng = [DecodeEngine(w, n_slots=2, slot_ctx=256) for _ in range(2)]
+    first = eng[0].prefill(0, ids), eng[1].prefill(0, ids, gemm=False)
+    assert first[0] == first[1] and torch.equal(eng[0].logits[:5], eng[1].logits[:5])
+    GpuEngine(eng[0], ByteTokenizer(), "m").prefill(1, ids, 0)
+    eng[1].prefill(1, ids, gemm=True)
+    rows = [e.kv.k[:, e.kv.pages[1][0], :, :45] for e in eng]
+    assert torch.equal(*rows)
+    assert not torch.equal(rows[0], eng[0].kv.k[:, eng[0].kv.pages[0][0], :, :45])
