@@ -628,8 +628,11 @@ class DecodeEngine:
     def short_prompt_on_blocks(self, n: int) -> bool:
         """Whether a prompt of ``n`` ids below ``gemm_threshold`` is fed faster, and with no bit less, by ``gemm=True``: the
         GEMM path over the quantised blocks.  Only for callers that read no logits of it: the chain leaves the rows of
-        its last pass in ``logits``, the GEMM path the last row alone."""
-        if not self.direct_threshold <= n < self.gemm_threshold or type(self) is not DecodeEngine or not self.spec.is_moe:
+        its last pass in ``logits``, the GEMM path the last row alone.  A ``gemm_threshold`` that somebody moved is
+        taken at its word."""
+        if self.gemm_threshold != GEMM_THRESHOLD or not self.direct_threshold <= n < GEMM_THRESHOLD:
+            return False
+        if type(self) is not DecodeEngine or not self.spec.is_moe:
             return False
         if self._gemm_prefill is None:
             self._gemm_prefill = self._new_gemm_prefill()

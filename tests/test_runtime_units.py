@@ -636,3 +636,19 @@ def test_native_cpu_engine_slots_share_save_and_restore():
     assert v is not None and abs(float(np.linalg.norm(v)) - 1.0) < 1e-4
     assert eng.props()["engine"] == "cpu-native"
     eng.close()
+
+
+def _engine_with(**over):
+    """A decode engine's routing rule without a card."""
+    from types import SimpleNamespace
+    from bloomery_b200.runtime.engine import GEMM_THRESHOLD, DecodeEngine
+    eng = object.__new__(DecodeEngine)
+    vars(eng).update(dict(gemm_threshold=GEMM_THRESHOLD, direct_threshold=32, spec=SimpleNamespace(is_moe=True),
+                          _gemm_prefill=SimpleNamespace(_direct=lambda n: n <= 128), route_trace=None, check_finite=False), **over)
+    return eng
+
+
+def test_short_prompts_go_over_the_blocks_only_below_an_untouched_gemm_threshold():
+    assert [n for n in range(0, 200) if _engine_with().short_prompt_on_blocks(n)] == list(range(32, 64))
+    for moved in (0, 16, 48, 63, 65, 1000):
+        assert not any(_engine_with(gemm_threshold=moved).short_prompt_on_blocks(n) for n in range(0, 200))
