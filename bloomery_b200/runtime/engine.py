@@ -632,6 +632,8 @@ class DecodeEngine:
         taken at its word."""
         if self.gemm_threshold != GEMM_THRESHOLD or not self.direct_threshold <= n < GEMM_THRESHOLD:
             return False
+        if self.route_trace is not None or self.check_finite:      # both look at the rows of a pass of the chain
+            return False
         if type(self) is not DecodeEngine or not self.spec.is_moe:
             return False
         if self._gemm_prefill is None:

@@ -652,3 +652,8 @@ def test_short_prompts_go_over_the_blocks_only_below_an_untouched_gemm_threshold
     assert [n for n in range(0, 200) if _engine_with().short_prompt_on_blocks(n)] == list(range(32, 64))
     for moved in (0, 16, 48, 63, 65, 1000):
         assert not any(_engine_with(gemm_threshold=moved).short_prompt_on_blocks(n) for n in range(0, 200))
+
+
+def test_short_prompts_stay_on_the_chain_under_a_route_trace_or_the_finite_check():
+    assert not _engine_with(route_trace=object()).short_prompt_on_blocks(40)
+    assert not _engine_with(check_finite=True).short_prompt_on_blocks(40)
