@@ -638,7 +638,7 @@ class DecodeEngine:
             return False
         if self._gemm_prefill is None:
             self._gemm_prefill = self._new_gemm_prefill()
-        return self._gemm_prefill._direct(n)
+        return self._gemm_prefill._direct(n, short=True)
 
     def prefill(self, slot: int, tokens: Sequence[int], start: int = 0, gemm: Optional[bool] = None) -> int:
         """Feed a prompt; returns the greedy token after it.  Prompts of at least

@@ -68,9 +68,11 @@ class GemmPrefill:
         from .timing import PromptTiming
         self.timing = PromptTiming()            # arm() it to get per-unit milliseconds of the next micro-batch
         # Micro-batches of at most this many tokens multiply the block-quantised weights as they are (csrc/qgemm_tcgen05.cu)
-        # instead of their bf16 copies: a layer's copies are 1.2 GB on the 30 B shape, its blocks 0.35 GB, and with few rows
-        # an expert nothing but those bytes counts (64 rows: gate+up and down 182 us a layer, 185 us just to read the copies;
-        # 512 rows: 231 us, 200 us over the copies).
+        # where every prompt would have to expand them to bf16 first: a layer of the 30 B shape is 0.35 GB of blocks and 1.2 GB
+        # of copies that are written and read.  Eight layers, 64 / 128 tokens, milliseconds: Q4_K_M 3.1 / 4.1 over the blocks,
+        # 6.0 / 5.8 with the expansion; FP8 3.3 / 4.3 and 9.9 / 10.1; NVFP4 3.6 / 4.6 and 6.2 / 6.5.  Copies that are kept
+        # are the faster ones from about 64 tokens on (3.2 to 3.6 / 3.5 in all three), so there the blocks are left to the
+        # prompts below it, which need their bits (run).
         self.direct_rows = 128
         self._direct_ok = None
         self._work = None
@@ -98,7 +100,7 @@ class GemmPrefill:
         e.kv.sync_table()
         # A prompt that would run on the 8-row chain if it were not here keeps what the chain gives it: weights that are not
         # rounded to bf16 (value and remainder) and queries, probabilities, keys and values as decode attention has them.
-        fine = n < GEMM_THRESHOLD and self._direct(n)
+        fine = n < GEMM_THRESHOLD and self._direct(n, short=True)
         i = 0
         while i < n:
             chunk = tokens[i:i + self.ubatch]
@@ -122,7 +124,7 @@ class GemmPrefill:
         qkv = self._get("qkv", (T, qkv_w), f32)
         # Quantised weights are expanded to bf16 one layer AHEAD of their use, on a side stream: the expansion is bound
         # by HBM traffic, the products by the tensor cores, so the two overlap.  Two sets of bf16 buffers alternate.
-        direct = self._direct(T)
+        direct = fine or self._direct(T)
         resident = not direct and self._use_resident()
         ahead = self.expert_source is None and self.expand_ahead and not resident and not direct
         nset = 2 if ahead else 1
@@ -363,9 +365,10 @@ class GemmPrefill:
         if int(st.item()) != 0:
             raise RuntimeError("a bounded wait inside the GEMM kernel ran out (status word set)")
 
-    def _direct(self, T: int) -> bool:
-        """Whether a micro-batch of T tokens multiplies the quantised blocks themselves: short ones of a model whose layers
-        are all routed and whose matrices all have a kernel for that (and whose experts are on the card)."""
+    def _direct(self, T: int, short: bool = False) -> bool:
+        """Whether a micro-batch of T tokens multiplies the quantised blocks themselves: a small one of a model whose layers
+        are all routed and whose matrices all have a kernel for that (and whose experts are on the card), where no bf16
+        copies are kept; ``short``: a whole prompt below the GEMM threshold, whatever is kept."""
         if T > self.direct_rows or self.expert_source is not None:
             return False
         if self._direct_ok is None:
@@ -375,7 +378,7 @@ class GemmPrefill:
                 s.layer_is_moe(il) and all(G.qgemm_supports(w.q[f"blk.{il}.{n}.weight"]) for n in names)
                 and w.q[f"blk.{il}.ffn_gate_exps.weight"].qtype == w.q[f"blk.{il}.ffn_up_exps.weight"].qtype
                 for il in range(s.n_layer))
-        return self._direct_ok
+        return self._direct_ok and (short or not self._use_resident())
 
     def _use_resident(self) -> bool:
         """Whether the layers' bf16 copies stay in HBM between prompts (decided once, before the first copy exists)."""

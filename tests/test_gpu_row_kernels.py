@@ -125,6 +125,8 @@ def test_short_prompts_over_quantised_blocks_agree_with_the_bf16_copies(n, start
         eng = DecodeEngine(w, n_slots=1, slot_ctx=512)
         eng._gemm_prefill = eng._new_gemm_prefill()
         eng._gemm_prefill.direct_rows = rows
+        eng._gemm_prefill.resident_bf16 = rows == 0              # the blocks are for prompts without kept copies, or short ones
+        assert eng._gemm_prefill._direct(n, short=n < 64) == (n <= rows)
         if start:
             eng.prefill(0, ids[:start], gemm=False)
         eng.prefill(0, ids[start:], start, gemm=True)
@@ -154,7 +156,7 @@ def test_prompts_below_the_gemm_threshold_round_activations_and_nothing_else(n, 
         eng = DecodeEngine(w, n_slots=1, slot_ctx=512)
         eng._gemm_prefill = eng._new_gemm_prefill()
         eng._gemm_prefill.direct_rows = 128 if route == "blocks" else 0
-        assert eng._gemm_prefill._direct(n) == (route == "blocks")
+        assert eng._gemm_prefill._direct(n, short=True) == (route == "blocks")
         eng.prefill(0, ids.tolist(), gemm=route != "chain")
         pages = torch.tensor(eng.kv.pages[0], device=DEV)
         new = [c[1, pages].permute(0, 2, 1, 3).reshape(-1, spec.n_kv, spec.head_dim)[:n].float().cpu()

@@ -644,7 +644,7 @@ def _engine_with(**over):
     from bloomery_b200.runtime.engine import GEMM_THRESHOLD, DecodeEngine
     eng = object.__new__(DecodeEngine)
     vars(eng).update(dict(gemm_threshold=GEMM_THRESHOLD, direct_threshold=32, spec=SimpleNamespace(is_moe=True),
-                          _gemm_prefill=SimpleNamespace(_direct=lambda n: n <= 128), route_trace=None, check_finite=False), **over)
+                          _gemm_prefill=SimpleNamespace(_direct=lambda n, short: short and n <= 128), route_trace=None, check_finite=False), **over)
     return eng
 
 
@@ -657,3 +657,14 @@ def test_short_prompts_go_over_the_blocks_only_below_an_untouched_gemm_threshold
 def test_short_prompts_stay_on_the_chain_under_a_route_trace_or_the_finite_check():
     assert not _engine_with(route_trace=object()).short_prompt_on_blocks(40)
     assert not _engine_with(check_finite=True).short_prompt_on_blocks(40)
+
+
+def test_kept_bf16_copies_serve_all_but_the_prompts_below_the_gemm_threshold():
+    from bloomery_b200.runtime.prefill import GemmPrefill
+    for kept in (False, True):
+        pre = object.__new__(GemmPrefill)
+        vars(pre).update(direct_rows=128, expert_source=None, _direct_ok=True, _use_resident=lambda: kept)
+        assert [pre._direct(n) for n in (5, 64, 128, 129)] == [not kept] * 3 + [False]
+        assert [pre._direct(n, short=True) for n in (5, 63, 129)] == [True, True, False]
+    vars(pre).update(_use_resident=lambda: False, expert_source=object())
+    assert not pre._direct(40, short=True)                       # experts streamed from the host: no stack to multiply
