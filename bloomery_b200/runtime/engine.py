@@ -16,6 +16,7 @@ from __future__ import annotations
 import math
 import threading
 import time
+import weakref
 from typing import Dict, List, Optional, Sequence, Tuple
 
 import torch
@@ -622,8 +623,11 @@ class DecodeEngine:
             return out[:len(rows)]
 
     def _new_gemm_prefill(self):
+        # this engine owns the object and outlives it, so it is handed a weak reference: no cycle, and the engine goes with
+        # its last reference and not in some later garbage collection, which could release its CUDA graphs inside another
+        # engine's capture
         from .prefill import GemmPrefill
-        return GemmPrefill(self, ubatch=self.ubatch)
+        return GemmPrefill(weakref.proxy(self), ubatch=self.ubatch)
 
     def short_prompt_on_blocks(self, n: int) -> bool:
         """Whether a prompt of ``n`` ids below ``gemm_threshold`` is fed faster, and with no bit less, by ``gemm=True``: the

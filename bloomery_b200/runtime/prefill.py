@@ -19,7 +19,6 @@ band test covers it, as the reference does (``ubatch.rs:19-30``).
 from __future__ import annotations
 
 import math
-import weakref
 from typing import List, Optional, Sequence
 
 import os
@@ -44,9 +43,7 @@ def _poison() -> bool:
 
 class GemmPrefill:
     def __init__(self, engine, ubatch: int = 2048, score_bytes: int = 1 << 30):
-        # the engine owns this object: no cycle, so an engine goes with its last reference and not in some later garbage
-        # collection, which could release its CUDA graphs inside another engine's capture
-        self.e = weakref.proxy(engine)
+        self.e = engine
         self.ubatch = ubatch
         self.score_bytes = score_bytes
         self._buf = {}

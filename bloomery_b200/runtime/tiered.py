@@ -11,6 +11,7 @@ reference's ``router -> handoff -> go -> [card experts] -> wait -> add``,
 """
 from __future__ import annotations
 
+import weakref
 from typing import Optional
 
 import torch
@@ -67,7 +68,7 @@ class TieredEngine(DecodeEngine):
         stream: ``crates/gpu/src/host/xstream.rs``; there only the hottest host experts move, here the whole layer,
         which the GEMM then reads as one stack)."""
         from .prefill import GemmPrefill
-        pre = GemmPrefill(self, ubatch=self.ubatch)
+        pre = GemmPrefill(weakref.proxy(self), ubatch=self.ubatch)
         pre.expert_source = ExpertStreamer(self.tiered, self.device).get
         return pre
 

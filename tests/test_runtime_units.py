@@ -668,3 +668,25 @@ def test_kept_bf16_copies_serve_all_but_the_prompts_below_the_gemm_threshold():
         assert [pre._direct(n, short=True) for n in (5, 63, 129)] == [True, True, False]
     vars(pre).update(_use_resident=lambda: False, expert_source=object())
     assert not pre._direct(40, short=True)                       # experts streamed from the host: no stack to multiply
+
+
+def test_a_prompt_path_keeps_the_engine_it_was_given_and_an_engine_not_itself(monkeypatch):
+    import weakref
+    from bloomery_b200.runtime.engine import DecodeEngine
+    from bloomery_b200.runtime.prefill import GemmPrefill
+    from bloomery_b200.runtime.tiered import TieredEngine
+
+    class Stub:
+        device, slot_ctx = "cpu", 7
+
+    pre = GemmPrefill(Stub())
+    assert pre.e.slot_ctx == 7                                   # nobody else holds the engine
+    for cls in (DecodeEngine, TieredEngine):
+        eng = object.__new__(cls)
+        vars(eng).update(device="cpu", ubatch=64, tiered=None, slot_ctx=8)
+        monkeypatch.setattr("bloomery_b200.runtime.tiered.ExpertStreamer", lambda *a: type("S", (), {"get": None}))
+        eng._gemm_prefill = eng._new_gemm_prefill()
+        assert eng._gemm_prefill.e.slot_ctx == 8
+        gone = weakref.ref(eng)
+        del eng
+        assert gone() is None                                    # by reference count alone
