@@ -692,7 +692,8 @@ int bl_qgemm_supports(int wtype) {
 //   W2 != null: output = silu(X W^T) * (X W2^T).  status: device word, set to 1 when a wait ran out.
 //   form: 0 short (exact at 128-row tiles), 1 exact, 2 split (tiles of 32 rows, and of 64 with one matrix); see the
 //   expanders above.
-//   fixed_tiles: the table has exactly max_tiles tiles and no launch in flight writes it.  splits > 1 (fixed tiles, one
+//   fixed_tiles: the table has exactly max_tiles tiles, and no launch in flight writes the table, W or W2: the warps that
+//   stream and expand weights read all three without waiting for the launch in front of this one.  splits > 1 (fixed tiles, one
 //   matrix, K / 256 divisible): that many CTAs share a tile's depth; partial: max_tiles * ceil(N / 128) * splits *
 //   tile_rows * 128 floats, tickets: max_tiles * ceil(N / 128) * 4 zeroed words, both of one stream at a time.
 int bl_qgemm_split(const void* X, long ldx, long rows_x, const void* W, const void* W2, int wtype, int n_groups, int N, int K,

@@ -30,6 +30,7 @@ class TileTable:
         """group_rows int32 [n_groups] on the device.  Rows of group g follow group g-1 in A
         (or start at ``base + g * group_stride`` when ``group_stride`` > 0) and use B matrix
         ``g // group_div``."""
+        self.fixed = 0                          # a launch writes the table now, and its number of tiles is on the device
         if causal_kind:
             # causal_kind 1: the product's columns are keys (scores), 2: its depth is keys (values); row r of a group
             # is the query at position causal_pos0 + r: tiles beyond the diagonal are skipped / cut short
@@ -219,6 +220,7 @@ def softmax_causal(S, rows: int, Tq: int, pos0: int, T_pad: int, P) -> None:
 def moe_plan(ids, wts, E: int, tiles: "TileTable", pos_of, dst_row, row_scale) -> None:
     """Count, offsets, tile table and scatter of a micro-batch's routed slots in one launch (``ids`` / ``wts`` flat)."""
     n = ids.numel()
+    tiles.fixed = 0
     rc = cuda().bl_moe_plan(p(ids), p(wts), I(n), I(E), I(dst_row.numel()), p(tiles.offsets), p(pos_of), p(dst_row),
                             p(row_scale), p(tiles.mtiles), p(tiles.n_mtiles), I(tiles.max_mtiles), I(tiles.tile_rows),
                             stream())

@@ -79,3 +79,20 @@ def test_every_code_has_a_name_and_check_raises_it():
     with pytest.raises(KernelError, match=r"bl_qgemm: .* \(code -2\)"):
         check(_qgemm(K=1000), "bl_qgemm")
     check(0, "nothing")
+
+
+def test_a_tile_table_that_a_launch_writes_is_no_longer_fixed(monkeypatch):
+    """qgemm takes a fixed table's tile count from the host and reads the table before the launch in front of it ends."""
+    import torch
+    from types import SimpleNamespace
+    from bloomery_b200.ops import gemm as G
+    done = lambda *a: 0                                                                                  # noqa: E731
+    monkeypatch.setattr(G, "cuda", lambda: SimpleNamespace(bl_gemm_build_tiles=done, bl_gemm_build_tiles_causal=done, bl_moe_plan=done))
+    monkeypatch.setattr(G, "stream", lambda: P(0))
+    rows = torch.tensor([70], dtype=torch.int32)
+    for again in (lambda t: t.build(rows), lambda t: t.build(rows, causal_pos0=0, causal_kind=1),
+                  lambda t: G.moe_plan(rows, rows.float(), 1, t, rows, rows, rows.float())):
+        t = G.TileTable.dense(70, "cpu", 32)
+        assert t.fixed == 3
+        again(t)
+        assert t.fixed == 0
