@@ -36,6 +36,10 @@ __device__ __forceinline__ void wf_split(float x, float y, uint32_t& hi, uint32_
   lo = *reinterpret_cast<const uint32_t*>(&r);
 }
 
+// The two partial products of one element.  An infinite key or value makes the remainder's product 0 * inf; the high one
+// is then the answer, as in a plain fp32 sum (a key of score -inf weighs nothing, an infinite value stays infinite).
+__device__ __forceinline__ float wf_join(float hi, float lo) { return fabsf(hi) < INFINITY ? hi + lo : hi; }
+
 template <int HEAD>
 struct WarpFlash {
   static constexpr int kKeys = 16;                       // keys a step
@@ -109,7 +113,7 @@ struct WarpFlash {
     for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const float x = ((c[nt][0][i] + c[nt][1][i]) + (c[nt][0][2 + i] + c[nt][1][2 + i])) * q_inv;
+        const float x = wf_join(c[nt][0][i] + c[nt][1][i], c[nt][0][2 + i] + c[nt][1][2 + i]) * q_inv;
         s[nt][i] = nt * 8 + 2 * t + i < n_valid ? x : -INFINITY;
       }
     float nm = fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1]));
@@ -150,7 +154,7 @@ struct WarpFlash {
 #pragma unroll
     for (int j = 0; j < ND; ++j)
       *reinterpret_cast<float2*>(out + g * HEAD + 8 * j + 2 * t) =
-          make_float2((o[j][0] + o[j][2]) * (1.f / 1024.f), (o[j][1] + o[j][3]) * (1.f / 1024.f));
+          make_float2(wf_join(o[j][0], o[j][2]) * (1.f / 1024.f), wf_join(o[j][1], o[j][3]) * (1.f / 1024.f));
   }
 };
 

@@ -49,6 +49,34 @@ def test_decode_attention_against_64_bits(head, n_q, n_kv, lengths, n_seg):
     assert torch.equal(ob, out.bfloat16())
 
 
+@pytest.mark.parametrize("head,n_q,n_kv", [(128, 32, 4), (64, 8, 8)])
+def test_decode_attention_over_infinite_keys_and_values(head, n_q, n_kv):
+    """f16 caches hold an infinity where a key or value left the range: a score of -inf weighs nothing, an infinite value
+    stays one, and neither touches the other dimensions."""
+    from bloomery_b200.ops import decode as K
+    g = torch.Generator().manual_seed(6)
+    n, mp, n_seg = 150, 3, 2
+    k, v = (torch.randn(mp, n_kv, 64, head, generator=g).half() for _ in range(2))
+    q = torch.randn(1, n_q, head, generator=g) * head ** -0.5
+    q[:, :, 3] = q[:, :, 3].abs() + 0.01
+    k[0, :, 7, 3] = -float("inf")
+    v[1, :, 20, 5] = float("inf")
+    v[2, :, 1, 9] = -float("inf")
+    kk, vv = (c.permute(1, 0, 2, 3).reshape(n_kv, -1, head)[:, :n].double() for c in (k, v))
+    ref = (torch.softmax(q[0].double().view(n_kv, n_q // n_kv, head) @ kk.transpose(1, 2), -1) @ vv).reshape(-1)
+    table = torch.arange(mp, dtype=torch.int32, device=DEV).view(1, mp)
+    pos, seq = torch.tensor([n - 1], dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    ml, acc = torch.zeros(n_q * n_seg * 2, device=DEV), torch.zeros(n_q * n_seg * head, device=DEV)
+    out = torch.zeros(1, n_q * head, device=DEV)
+    oq, od = torch.zeros(1, n_q * head, dtype=torch.int8, device=DEV), torch.zeros(1, n_q * head // 32, 2, device=DEV)
+    K.flash_decode(q.to(DEV), k.to(DEV), v.to(DEV), pos, seq, table, mp, head, n_q, n_kv, 1, n_seg, mp * 64, ml, acc, out, oq,
+                   od, _fault(), 0)
+    torch.cuda.synchronize()
+    out, wild = out[0].cpu().double(), ref.isinf()
+    assert int(wild.sum()) == 2 * n_q and torch.equal(out[wild], ref[wild])
+    assert float((out[~wild] - ref[~wild]).norm() / ref[~wild].norm()) < 1e-5       # as in the test above
+
+
 @pytest.mark.parametrize("n,E,tile", [(1, 4, 32), (2048, 128, 32), (2049, 128, 128), (4100, 40, 128), (32768, 512, 128), (8192, 1, 64)])
 def test_expert_plan_of_one_block_and_of_a_cluster(n, E, tile):
     from bloomery_b200.ops import gemm as G
