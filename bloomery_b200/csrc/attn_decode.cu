@@ -669,6 +669,7 @@ static int flash_decode_go(const float* q, const void* k_cache, const void* v_ca
   dim3 grid(n_seg, n_kv, M);
   size_t smem = (size_t)G * head * 4 + 2 * kKeyTile * (head + 8) * 2 + 2 * kKeyTile * head * 2;
   cudaError_t e;
+  // a kernel's shared-memory limit belongs to a device, and stages of one process may sit on several: set on every call
   if (kv_q8) {
     // q8_0 caches: the fp32 segment kernel with tiles expanded to f16 as they are staged
     if (head == 128) {
@@ -683,24 +684,22 @@ static int flash_decode_go(const float* q, const void* k_cache, const void* v_ca
     }
   } else if (g_flash_mma) {
     const size_t sm2 = (size_t)(16 + 4 * kKeyTile) * (head + 8) * 2 + (16 * 33 + 512) * 4 + 16 * 40 * 2 + 64;
-    static bool set128 = false, set64 = false;
     if (head == 128) {
-      if (!set128) { cudaFuncSetAttribute(flash_decode_seg_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2); set128 = true; }
+      cudaFuncSetAttribute(flash_decode_seg_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2);
       e = launch(flash_decode_seg_mma_kernel<128>, grid, dim3(256), sm2, st, a);
     } else {
-      if (!set64) { cudaFuncSetAttribute(flash_decode_seg_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2); set64 = true; }
+      cudaFuncSetAttribute(flash_decode_seg_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2);
       e = launch(flash_decode_seg_mma_kernel<64>, grid, dim3(256), sm2, st, a);
     }
   } else if (G <= 8) {
     // up to eight heads a group: both halves of the split operands fit one tile
-    static bool wf128 = false, wf64 = false;
     if (head == 128) {
       constexpr int sm3 = 8 * 128 * 4 + kWfWarps * kWfStages * WarpFlash<128>::kStageBytes;
-      if (!wf128) { cudaFuncSetAttribute(flash_decode_seg_wf_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm3); wf128 = true; }
+      cudaFuncSetAttribute(flash_decode_seg_wf_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm3);
       e = launch(flash_decode_seg_wf_kernel<128>, grid, dim3(kWfWarps * 32), sm3, st, a);
     } else {
       constexpr int sm3 = 8 * 64 * 4 + kWfWarps * kWfStages * WarpFlash<64>::kStageBytes;
-      if (!wf64) { cudaFuncSetAttribute(flash_decode_seg_wf_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm3); wf64 = true; }
+      cudaFuncSetAttribute(flash_decode_seg_wf_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm3);
       e = launch(flash_decode_seg_wf_kernel<64>, grid, dim3(kWfWarps * 32), sm3, st, a);
     }
   } else if (head == 128) {

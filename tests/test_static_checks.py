@@ -114,3 +114,9 @@ def test_comments_stand_alone():
                 if w in ln:
                     bad.append(f"{name}:{i + 1}: names {w!r}")
     assert not bad, "\n".join(bad)
+
+
+def test_decode_attention_sets_its_shared_memory_limits_on_every_device():
+    """A flag that remembers one call leaves the second device of a process at 48 KB, where the launch is refused."""
+    text = open(os.path.join(ROOT, "bloomery_b200", "csrc", "attn_decode.cu")).read()
+    assert text.count("MaxDynamicSharedMemorySize") >= 4 and "static bool" not in text
