@@ -121,6 +121,51 @@ def test_router_of_many_rows_agrees_with_the_router(t, M, E, K):
     assert torch.allclose(xn.float(), ref, rtol=2 ** -8, atol=1e-6)      # one rounding to bf16 and a few fp32 ones
 
 
+@pytest.mark.parametrize("seqs", [[0, -1], [3, 1, 2, 0, 4, -1, -1, -1], [-1, 5, -1, 6], [0, 1, 2, 3]])
+def test_rows_that_fill_a_bucket_route_nowhere(seqs):
+    """Both calls that route: a dead row's ids are -1 and its weights 0 whatever its logits hold, it counts nowhere, the
+    launch behind leaves its residual as it is, and the rows beside it keep their bits."""
+    from bloomery_b200.formats.resident import quantize_resident
+    from bloomery_b200.ops import decode as D
+    torch.manual_seed(12)
+    M, E, n, H, I_ = len(seqs), 16, 4, 512, 256
+    q = [D.QWeight(quantize_resident(torch.randn(E * r, k) * 0.05, "Q4_K", values=False)[0].to(DEV).reshape(E, r, -1).contiguous(), "Q4_K", k)
+         for r, k in ((I_, H), (I_, H), (H, I_))]
+    wr = D.QWeight((torch.randn(E, H, device=DEV) * 0.05).view(torch.uint8), "F32", H)
+    x, gain = torch.randn(M, H, device=DEV), torch.ones(H, device=DEV)
+    xq, xds = torch.zeros(M, H, dtype=torch.int8, device=DEV), torch.zeros(M, H // 32, 2, device=DEV)
+    logits, rule = torch.zeros(M, E, device=DEV), D.RouteRule(n)
+    D.router(x, gain, 1e-6, wr, M, logits, xq, xds, None, _fault(), 0)
+    seq = torch.tensor(seqs, dtype=torch.int32, device=DEV)
+    dead, poison = seq < 0, logits.clone()
+    poison[dead] = float("nan")
+
+    def run(lg, row_seq, rows):
+        ids, wts = torch.full((M, n), 7, dtype=torch.int32, device=DEV), torch.full((M, n), float("nan"), device=DEV)
+        heat, f = torch.zeros(E, dtype=torch.int32, device=DEV), _fault()
+        actq = torch.full((M, n, I_), 99, dtype=torch.int8, device=DEV)
+        actds = torch.full((M, n, I_ // 32, 2), float("nan"), device=DEV)
+        y = torch.full((M, H), float("nan"), device=DEV)
+        if rows:
+            D.route_rows(lg, rule, M, ids, wts, heat, f, 0, row_seq)
+        else:
+            D.gate_up_sel(xq, xds, ids, None, q[0], q[1], E, n, M, actq, actds, None, f, 0, route_logits=lg, rule=rule, wts=wts,
+                          heat=heat, row_seq=row_seq)
+            D.down_combine(actq, actds, ids, wts, None, q[2], E, n, M, x, None, y, f, 0)
+        torch.cuda.synchronize()
+        assert int(f) == -1
+        return ids, wts, heat, y
+
+    for rows in (True, False):
+        ids, wts, heat, y = run(logits, None, rows)              # every row alive
+        got = run(poison, seq, rows)
+        assert bool((got[0][dead] == -1).all()) and bool((got[1][dead] == 0).all())
+        assert torch.equal(got[0][~dead], ids[~dead]) and torch.equal(got[1][~dead], wts[~dead])
+        assert torch.equal(got[2].long(), torch.bincount(ids[~dead].flatten().long(), minlength=E))
+        if not rows:
+            assert torch.equal(got[3][dead], x[dead]) and torch.equal(got[3][~dead], y[~dead])
+
+
 @pytest.mark.parametrize("T,k,H", [(1, 8, 2048), (33, 2, 4), (5, 3, 8192), (7, 8, 1028)])
 def test_combine_with_the_next_norm(T, k, H):
     from bloomery_b200.ops import gemm as G

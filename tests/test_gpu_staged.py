@@ -191,6 +191,15 @@ def test_attn_fused_without_qk_norm_and_with_one_segment():
     _attn_case(128, 8, 2, [(0, 200), (1, 17)], n_seg=1, ctx=256, qk_norm=False)
 
 
+@pytest.mark.parametrize("head,n_q,n_kv", [(128, 32, 4), (64, 8, 2)])
+def test_attn_fused_segments_that_turn_the_ring_over(head, n_q, n_kv):
+    # a warp holds two steps of 16 keys and eight warps share a segment: past 256 keys its ring comes round again
+    _attn_case(head, n_q, n_kv, [(0, 700), (1, 255), (-1, 0), (2, 256), (3, 271)], n_seg=1, ctx=704)
+    _attn_case(head, n_q, n_kv, [(0, 1500)], n_seg=3, ctx=1536, seed=9)
+    # rows of this pass in a stage that has come round, across a step's and a page's end
+    _attn_case(head, n_q, n_kv, [(0, 572 + i) for i in range(8)], n_seg=1, ctx=640, seed=10)
+
+
 def test_attn_fused_bad_key_count_is_a_fault_word_not_a_trap():
     from bloomery_b200.ops import decode as K
     head, n_q, n_kv, M, n_seg, ctx = 128, 8, 2, 2, 4, 128
