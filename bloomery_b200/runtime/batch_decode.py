@@ -77,10 +77,11 @@ class BatchDecode:
             self.part_ml = torch.zeros(cells * 2, **f32)
             self.part_acc = torch.zeros(cells * s.head_dim, **f32)
             aw = s.q_rows
-        self.attn = torch.zeros(R, aw, **f32)
         self.attn_bf = torch.zeros(R, aw, **bf)
-        self.attn_q = torch.zeros(R, aw, dtype=torch.int8, device=dev)
-        self.attn_ds = torch.zeros(R, aw // 32, 2, **f32)
+        if s.mla:                                    # its merge writes these forms; the grouped-query one writes bf16 rows alone
+            self.attn = torch.zeros(R, aw, **f32)
+            self.attn_q = torch.zeros(R, aw, dtype=torch.int8, device=dev)
+            self.attn_ds = torch.zeros(R, aw // 32, 2, **f32)
         if s.is_moe:
             E, k, I_ = s.n_expert, s.n_used, s.moe_inter
             n = R * k
@@ -151,8 +152,8 @@ class BatchDecode:
     def _mm(self, X, Wq, tiles, M, x8=None, W2=None, branch=0, **kw):
         """X [rows, K] bf16 times a resident matrix (or, with W2, the SwiGLU pair): FP8 weights against E4M3 rows on the
         tensor cores, other quantised types expanded in flight, the rest through a bf16 expansion launch.  ``x8``: the
-        rows' E4M3 form when the caller already made it (several products of one input).  ``branch``: 0 on the pass's own stream, 1 / 2 on its side streams.  Returns the
-        launch count."""
+        rows' E4M3 form when the caller already made it (several products of one input).  ``branch``: 0 on the pass's own
+        stream, 1 / 2 on its side streams.  Returns the launch count."""
         if self._native_fp8(Wq):
             n = 0
             if x8 is None:
