@@ -211,11 +211,29 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
       if (m != -INFINITY && (m_new - m) * kLog2e <= kLazy) m_new = m;     // both halves see the same numbers: same choice
       const float mb = (m_new == -INFINITY) ? 0.f : m_new * kLog2e;       // a row with no key yet keeps zeros
       const float corr = (m == -INFINITY) ? 0.f : ex2(m * kLog2e - mb);
-      // the previous value product has to be complete only when some row of this warp rescales its output
-      if (t > 0 && __any_sync(0xffffffffu, corr != 1.0f)) {
+      float rowsum = 0.f, rowsum1 = 0.f;
+      uint32_t pk[32];
+#pragma unroll
+      for (int i = 0; i < 64; i += 2) {
+        // (s0, s1) * log2(e) - mb as one packed FMA; masked scores are -inf and 2^-inf = 0 (a row without any key
+        // has mb = 0 and only -inf scores, so it needs no special case)
+        uint32_t e0, e1;
+        asm("{\n\t.reg .b64 rs, rk, rm, rr;\n\t"
+            "mov.b64 rs, {%2, %3};\n\tmov.b64 rk, {%4, %4};\n\tmov.b64 rm, {%5, %5};\n\t"
+            "fma.rn.f32x2 rr, rs, rk, rm;\n\tmov.b64 {%0, %1}, rr;\n\t}"
+            : "=r"(e0), "=r"(e1) : "r"(i < 32 ? v0[i & 31] : v1[i & 31]), "r"(i < 32 ? v0[(i & 31) + 1] : v1[(i & 31) + 1]),
+              "f"(kLog2e), "f"(-mb));
+        const float p0 = ex2(__uint_as_float(e0)), p1 = ex2(__uint_as_float(e1));
+        rowsum += p0; rowsum1 += p1;
+        pk[i >> 1] = pack_bf16(p0, p1);
+      }
+      // The value product of the last tile reads the probabilities' tile and adds into the output: it has to be complete
+      // before this tile's probabilities take their place, whether a row rescales its output or not.  (Waiting for it in
+      // every tile also keeps this barrier's parity: a wait two phases ahead of it would not wait at all.)
+      if (t > 0) {
         if (!mbar_wait(&o_done, (uint32_t)((t - 1) & 1), abort_flag)) { ok = false; break; }
         tc_fence_after();
-        {
+        if (__any_sync(0xffffffffu, corr != 1.0f)) {
 #pragma unroll 1
           for (int c = 0; c < 2; ++c) {
             uint32_t v[32];
@@ -228,30 +246,10 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
           tmem_st_wait();
         }
       }
-      float rowsum = 0.f, rowsum1 = 0.f;
       uint8_t* prow = sP + half * FHALF + (r >> 3) * 1024 + (r & 7) * 128;     // this half's swizzle atom
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t pk[16];
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          // (s0, s1) * log2(e) - mb as one packed FMA; masked scores are -inf and 2^-inf = 0 (a row without any key
-          // has mb = 0 and only -inf scores, so it needs no special case)
-          uint32_t e0, e1;
-          asm("{\n\t.reg .b64 rs, rk, rm, rr;\n\t"
-              "mov.b64 rs, {%2, %3};\n\tmov.b64 rk, {%4, %4};\n\tmov.b64 rm, {%5, %5};\n\t"
-              "fma.rn.f32x2 rr, rs, rk, rm;\n\tmov.b64 {%0, %1}, rr;\n\t}"
-              : "=r"(e0), "=r"(e1) : "r"(c ? v1[i] : v0[i]), "r"(c ? v1[i + 1] : v0[i + 1]), "f"(kLog2e), "f"(-mb));
-          const float p0 = ex2(__uint_as_float(e0)), p1 = ex2(__uint_as_float(e1));
-          rowsum += p0; rowsum1 += p1;
-          pk[i >> 1] = pack_bf16(p0, p1);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int chunk = (c * 4 + j) ^ (r & 7);
-          *reinterpret_cast<uint4*>(prow + chunk * 16) = make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
-        }
-      }
+      for (int j = 0; j < 8; ++j)
+        *reinterpret_cast<uint4*>(prow + (j ^ (r & 7)) * 16) = make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
       l = l * corr + (rowsum + rowsum1);
       m = m_new;
       tc_fence_before();

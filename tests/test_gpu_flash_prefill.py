@@ -50,6 +50,32 @@ def test_flash_prefill_matches_fp32_attention(n_q, n_kv, T, pos0):
     assert torch.equal(out, out2)                                   # bit-identical rerun
 
 
+@pytest.mark.parametrize("T", [200, 300, 511])
+def test_flash_prefill_repeats_itself_with_cold_caches(T):
+    """Values that arrive late hold a value product back; the next tile's probabilities must wait for it whether or not a
+    row rescales its output (scores this small never do), and so must the output.  Every launch reads from memory."""
+    from bloomery_b200.ops import gemm as G
+    g = torch.Generator(device=DEV).manual_seed(T)
+    n_q, n_kv, d = 32, 4, 128
+    t_pad = (T + 127) // 128 * 128
+    q = (torch.randn(n_q, T, d, device=DEV, generator=g) / d).bfloat16()
+    k, v = (torch.randn(n_kv, T, d, device=DEV, generator=g).bfloat16() for _ in range(2))
+    Kb, Vt = torch.zeros(n_kv, t_pad, d, device=DEV, dtype=torch.bfloat16), torch.zeros(n_kv, d, t_pad, device=DEV, dtype=torch.bfloat16)
+    Kb[:, :T], Vt[:, :, :T] = k, v.transpose(1, 2)
+    ref = _ref(q, k, v, 0).permute(1, 0, 2).reshape(T, n_q * d)
+    flush = torch.empty(256 << 20, dtype=torch.uint8, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    outs = torch.zeros(150, T, n_q * d, device=DEV, dtype=torch.bfloat16)
+    for out in outs:
+        flush.fill_(1)
+        G.flash_prefill(q, Kb, Vt, out, 0, status)
+    torch.cuda.synchronize()
+    assert int(status) == 0
+    # probabilities (near 1 before the division) and outputs in bf16: 2^-9 of a mean of unit values each, and fp32 below it
+    assert float((outs[0].float() - ref).norm() / ref.norm()) < 2 ** -7
+    assert [i for i, out in enumerate(outs) if not torch.equal(out, outs[0])] == []
+
+
 def test_engine_prompt_through_flash_matches_the_three_launch_path():
     """A prompt through the GEMM path with and without the fused attention: same greedy token, logits in band."""
     from bloomery_b200.models.spec import ModelSpec
