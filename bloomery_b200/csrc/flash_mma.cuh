@@ -39,6 +39,13 @@ __device__ __forceinline__ void wf_split(float x, float y, uint32_t& hi, uint32_
 // The two partial products of one element.  An infinite key or value makes the remainder's product 0 * inf; the high one
 // is then the answer, as in a plain fp32 sum (a key of score -inf weighs nothing, an infinite value stays infinite).
 __device__ __forceinline__ float wf_join(float hi, float lo) { return fabsf(hi) < INFINITY ? hi + lo : hi; }
+// The maximum that a NaN gets through: the vote on a new maximum then finds such a step, which costs the others nothing
+// (joining every score took 6 % of a row of 16,000 keys).
+__device__ __forceinline__ float wf_max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
 
 template <int HEAD>
 struct WarpFlash {
@@ -113,14 +120,27 @@ struct WarpFlash {
     for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const float x = wf_join(c[nt][0][i] + c[nt][1][i], c[nt][0][2 + i] + c[nt][1][2 + i]) * q_inv;
+        const float x = ((c[nt][0][i] + c[nt][1][i]) + (c[nt][0][2 + i] + c[nt][1][2 + i])) * q_inv;
         s[nt][i] = nt * 8 + 2 * t + i < n_valid ? x : -INFINITY;
       }
-    float nm = fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1]));
-    nm = fmaxf(nm, __shfl_xor_sync(0xffffffffu, nm, 1));
-    nm = fmaxf(nm, __shfl_xor_sync(0xffffffffu, nm, 2));
-    nm = fmaxf(m, nm);
+    float nm = wf_max_nan(wf_max_nan(s[0][0], s[0][1]), wf_max_nan(s[1][0], s[1][1]));
+    nm = wf_max_nan(nm, __shfl_xor_sync(0xffffffffu, nm, 1));
+    nm = wf_max_nan(nm, __shfl_xor_sync(0xffffffffu, nm, 2));
+    nm = wf_max_nan(m, nm);
     if (__any_sync(0xffffffffu, nm != m)) {
+      if (__any_sync(0xffffffffu, nm != nm)) {           // an infinite key (or a NaN, which stays one)
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const float x = wf_join(c[nt][0][i] + c[nt][1][i], c[nt][0][2 + i] + c[nt][1][2 + i]) * q_inv;
+            s[nt][i] = nt * 8 + 2 * t + i < n_valid ? x : -INFINITY;
+          }
+        nm = fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1]));
+        nm = fmaxf(nm, __shfl_xor_sync(0xffffffffu, nm, 1));
+        nm = fmaxf(nm, __shfl_xor_sync(0xffffffffu, nm, 2));
+        nm = fmaxf(m, nm);
+      }
       const float corr = (m == -INFINITY) ? 0.f : __expf(m - nm);
       l *= corr;
 #pragma unroll
