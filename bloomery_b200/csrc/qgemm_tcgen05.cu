@@ -2,7 +2,7 @@
 //   C[t, n] = sum_k X[t, k] * W[g][n, k]          W resident Q4_K / Q5_K / Q6_K / Q8_0, X bf16, fp32 accumulate
 //
 // The product is issued transposed: the 128 weight rows of a tile are the M side of the MMA and the tokens the N side
-// (16 .. 128 per tile), so a decode batch of a few rows per expert pays for the tokens it has instead of a 128-row
+// (32, 64 or 128 per tile), so a decode batch of a few rows per expert pays for the tokens it has instead of a 128-row
 // tile, and a prompt tile expands each weight once for 128 tokens.
 //
 //   * weights: sixteen producer warps decode 64-value units in registers and store bf16 into the MMA's A operand in
@@ -95,9 +95,9 @@ enum QForm { Q_SHORT = 0, Q_EXACT = 1, Q_SPLIT = 2 };
 //   cores do twice the products, of which there is room, and the expanders write twice.
 //   short form (decode rounds, which the expanders' integer pipe bounds): two code bytes become the bf16 pair
 //   (128 + q0, 128 + q1) with one byte permute, a packed bf16 subtract gives (q0, q1) exactly and a packed bf16 FMA gives
-//   s * q + o with s and o rounded to bf16: half the integer instructions, at most about one more bf16 ulp of error per
-//   weight than the exact form.  Gate+up of 24 rows, 100 of 128 experts (Q4_K, 768 x 2048): 97 us exact, 88 us short
-//   (35 us of blocks at the copy rate).
+//   s * q + o with s and o rounded to bf16: half the integer instructions.  Its error is at most 2^-9 (|s q| + |o|) and one bf16
+//   rounding of the sum, which is no bound in ulps of the weight: near zero s q and o nearly cancel (Q4_K, Q5_K).  Gate+up
+//   of 24 rows, 100 of 128 experts (Q4_K, 768 x 2048): 97 us exact, 88 us short (35 us of blocks at the copy rate).
 // FastUnit<T>::codes yields the unit's 64 code bytes in value order (16 words; word w belongs to group w / 4) and the
 // (scale, offset) pair of each of the four groups of 16 values.
 template <class T> struct FastUnit { static constexpr bool kHas = false; };

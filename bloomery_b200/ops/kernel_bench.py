@@ -6,7 +6,8 @@ CUDA events.
 
 NAME: chain (the six launches of a layer in order) | qkv | attn | o | router | gateup | down | rope | flash |
 flash_mma | gemm | gemmdist | pflash | prope | mplan | qgu | qdown | qo | qq | bgu | bdown | mla | sampler | sampler_split | gap.  ``--no-staged`` runs the register-streaming kernels
-instead of the shared-memory staged ones.  It is also the small workload the ncu summaries under ``profiles/``
+instead of the shared-memory staged ones; ``--form exact`` / ``--form fine`` picks how the weights of qgu / qdown are expanded.
+It is also the small workload the ncu summaries under ``profiles/``
 were captured on.
 """
 import math
@@ -38,6 +39,11 @@ def main(argv=None) -> int:
     if "--wtype" in argv:
         i = argv.index("--wtype")
         wtype = argv[i + 1]
+        del argv[i:i + 2]
+    form = {}                          # --form exact | fine: how qgu / qdown weights reach the tensor cores (default: short)
+    if "--form" in argv:
+        i = argv.index("--form")
+        form = {argv[i + 1]: True}
         del argv[i:i + 2]
     if "--dbg" in argv:
         i = argv.index("--dbg")
@@ -236,8 +242,8 @@ def main(argv=None) -> int:
             if which == "mplan": X["G"].moe_plan(X["mids"], X["mwts"], E, X["mtt"], X["mpos_of"], X["mdst"], X["mscale"])
             if which == "qo": X["G"].qgemm(X["xo"], l["o"], X["tt"], out_f32=X["oo"], status=X["gst"])
             if which == "qq": X["G"].qgemm(X["xh"], l["q"], X["tt"], out_f32=X["oq"], status=X["gst"])
-            if which == "qgu": X["G"].qgemm(X["xa"], l["g"], X["tt"], out_bf16=X["act"], W2=l["u"], status=X["gst"])
-            if which == "qdown": X["G"].qgemm(X["act"], l["d"], X["tt"], out_f32=X["so"], dst_row=X["dst"], row_scale=X["scale"], status=X["gst"])
+            if which == "qgu": X["G"].qgemm(X["xa"], l["g"], X["tt"], out_bf16=X["act"], W2=l["u"], status=X["gst"], **form)
+            if which == "qdown": X["G"].qgemm(X["act"], l["d"], X["tt"], out_f32=X["so"], dst_row=X["dst"], row_scale=X["scale"], status=X["gst"], **form)
             if which == "fgu": X["G"].fp8_gemm(X["xa8"], X["xas"], l["g"], X["tt"], out_bf16=X["act"], W2=l["u"], status=X["gst"])
             if which == "fdown": X["G"].fp8_gemm(X["act8"], X["acts"], l["d"], X["tt"], out_f32=X["so"], dst_row=X["dst"], row_scale=X["scale"], status=X["gst"])
             if which == "bgu":
