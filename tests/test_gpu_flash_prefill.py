@@ -96,3 +96,10 @@ def test_engine_prompt_through_flash_matches_the_three_launch_path():
     scale = outs[1][1].abs().max().item()
     assert (outs[0][1] - outs[1][1]).abs().max().item() < 3e-2 * scale
     assert outs[0][0] == outs[1][0]
+
+
+@pytest.mark.parametrize("n_q,n_kv,T,pos0", [(3, 1, 129, 0), (3, 1, 300, 65), (5, 1, 1, 0), (7, 7, 128, 1), (6, 2, 385, 1000), (1, 1, 640, 0)])
+def test_query_tiles_that_pair_across_positions(n_q, n_kv, T, pos0):
+    """An odd number of heads a KV head pairs the last tile of one position with the first of the one before it, whose keys end
+    earlier, and may leave a tile alone."""
+    test_flash_prefill_matches_fp32_attention(n_q, n_kv, T, pos0)
