@@ -70,6 +70,7 @@ struct GemmArgs {
   int n_owners;
   int dst_div;
   int src_rows;               // > 0: A is row-sharded; product row = tile's source rank * src_rows + row in the shard
+  int splits;                 // cluster form: CTAs of a cluster that share a tile's depth
   int wide_stores;            // fp32 output rows start on 32-byte boundaries: the epilogue may use 256-bit stores
 };
 
@@ -89,7 +90,22 @@ __device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, 
   asm volatile("red.relaxed.sys.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
-template <bool DUAL, bool DIST>
+// The cluster form (SPLIT): a product of fewer tiles than half the processors gives each tile to a cluster of 2, 4 or 8 CTAs,
+// which walk equal shares of its depth.  Every CTA parks its partial tile in its own (by then idle) operand ring, and
+// each adds up its share of the rows from all of them over distributed shared memory, in ascending order.  One CTA streams
+// its operands at about 0.47 us per 64-deep step, whatever the rest of the chip does: the output projection of a prompt of
+// 512 (32 tiles, 4,096 deep) took 36 us and the router (4 tiles, 6,144 deep) 40 us; as clusters of 4 and 8 the two take 34.
+constexpr int SPLIT_ROW = 256 + 4;             // floats of a parked row: 16-byte aligned, and rows start four banks apart
+
+__device__ __forceinline__ void cluster_arrive_release() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait_acquire() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ float4 ld_cluster_v4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
+template <bool DUAL, bool DIST, bool SPLIT = false>
 __global__ void __launch_bounds__(192, 1)
 gemm_bf16_kernel(const __grid_constant__ AMaps tma_a, const __grid_constant__ CUtensorMap tma_b,
                  const __grid_constant__ CUtensorMap tma_b2, const GemmArgs a) {
@@ -126,17 +142,21 @@ gemm_bf16_kernel(const __grid_constant__ AMaps tma_a, const __grid_constant__ CU
   const int n_mt = min(*a.n_mtiles, a.max_mtiles);
   const int total_tiles = n_mt * a.tiles_n;
   const int kblocks = a.K / BK;
+  // cluster form: this CTA's tile, and its share [kb_lo, kb_hi) of the depth; the cluster walks one tile
+  const int rank = SPLIT ? (int)(blockIdx.x % a.splits) : 0;
+  const int kb_lo = SPLIT ? kblocks * rank / a.splits : 0, kb_hi = SPLIT ? kblocks * (rank + 1) / a.splits : kblocks;
+  const int first = SPLIT ? (int)blockIdx.x / a.splits : (int)blockIdx.x, step = SPLIT ? total_tiles + (int)gridDim.x : (int)gridDim.x;
 
   if (warp == 0) {
     if (lane == 0) {
       int stage = 0; uint32_t phase = 0;
       int issued = 0;
-      for (int t = blockIdx.x; t < total_tiles && !*abort_flag; t += gridDim.x) {
+      for (int t = first; t < total_tiles && !*abort_flag; t += step) {
         const MTile mt = a.mtiles[t / a.tiles_n];
         const int n0 = (t % a.tiles_n) * BN;
         if (!DIST && tile_skipped(mt, n0)) continue;
-        const int kb_end = DIST ? kblocks : tile_kblocks(mt, kblocks);
-        for (int kb = 0; kb < kb_end; ++kb) {
+        const int kb_end = SPLIT ? kb_hi : DIST ? kblocks : tile_kblocks(mt, kblocks);
+        for (int kb = kb_lo; kb < kb_end; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) break;
           uint8_t* sa = smem + (size_t)stage * STAGE_BYTES;
           mbar_expect_tx(&full_bar[stage], STAGE_BYTES);
@@ -165,10 +185,10 @@ gemm_bf16_kernel(const __grid_constant__ AMaps tma_a, const __grid_constant__ CU
       constexpr uint32_t idesc = umma_idesc(BM, BN);
       int stage = 0; uint32_t phase = 0;
       int it = 0;
-      for (int t = blockIdx.x; t < total_tiles && !*abort_flag; t += gridDim.x) {
+      for (int t = first; t < total_tiles && !*abort_flag; t += step) {
         const MTile mt = a.mtiles[t / a.tiles_n];
         if (!DIST && tile_skipped(mt, (t % a.tiles_n) * BN)) continue;
-        const int kb_end = DIST ? kblocks : tile_kblocks(mt, kblocks);
+        const int kb_end = SPLIT ? kb_hi : DIST ? kblocks : tile_kblocks(mt, kblocks);
         const int ab = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
         ++it;
@@ -176,14 +196,14 @@ gemm_bf16_kernel(const __grid_constant__ AMaps tma_a, const __grid_constant__ CU
         tc_fence_after();
         const uint32_t d0 = tmem_base + ab * ACC_COLS;
         bool ok = true;
-        for (int kb = 0; kb < kb_end; ++kb) {
+        for (int kb = kb_lo; kb < kb_end; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + (size_t)stage * STAGE_BYTES);
           const uint64_t da = umma_desc(sa), db = umma_desc(sa + TILE_A_BYTES);
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint32_t acc = (kb > 0 || k > 0) ? 1u : 0u;
+            const uint32_t acc = (kb > kb_lo || k > 0) ? 1u : 0u;
             umma_bf16(d0, da + (uint64_t)(k * UMMA_K * 2 / 16), db + (uint64_t)(k * UMMA_K * 2 / 16), idesc, acc);
             if (DUAL) {
               const uint64_t db2 = umma_desc(sa + TILE_A_BYTES + TILE_B_BYTES);
@@ -197,10 +217,27 @@ gemm_bf16_kernel(const __grid_constant__ AMaps tma_a, const __grid_constant__ CU
         umma_commit(&acc_full[ab]);            // accumulator complete
       }
     }
+  } else if constexpr (SPLIT) {
+    // Park the partial tile: every operand of this CTA has been read by now (its accumulator is complete), so the ring is free.
+    const int q = warp & 3;
+    if (first < total_tiles && __all_sync(0xFFFFFFFFu, mbar_wait(&acc_full[0], 0, abort_flag))) {
+      tc_fence_after();
+      float* park = reinterpret_cast<float*>(smem) + (q * 32 + lane) * SPLIT_ROW;
+#pragma unroll 1
+      for (int c = 0; c < BN / 32; ++c) {
+        uint32_t v[32];
+        tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + c * 32, v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; i += 4)
+          *reinterpret_cast<uint4*>(park + c * 32 + i) = make_uint4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+      }
+      tc_fence_before();
+    }
   } else {
     const int q = warp & 3;                    // TMEM lane quarter of this warp
     int it = 0;
-    for (int t = blockIdx.x; t < total_tiles && !*abort_flag; t += gridDim.x) {
+    for (int t = first; t < total_tiles && !*abort_flag; t += step) {
       const MTile mt = a.mtiles[t / a.tiles_n];
       const int n0 = (t % a.tiles_n) * BN;
       if (!DIST && tile_skipped(mt, n0)) continue;
@@ -287,6 +324,54 @@ gemm_bf16_kernel(const __grid_constant__ AMaps tma_a, const __grid_constant__ CU
     }
   }
 
+  if constexpr (SPLIT) {
+    // Every CTA of the cluster comes here, whatever it waited for in vain: the barriers always complete.
+    __syncwarp();
+    cluster_arrive_release();
+    cluster_wait_acquire();
+    if (first < total_tiles) {
+      const MTile mt = a.mtiles[first / a.tiles_n];
+      const int n0 = (first % a.tiles_n) * BN, cols = min(BN, a.N - n0) / 4;
+      const int share = BM / a.splits, r_lo = rank * share;
+      const int rows = min(share, mt.row_end - mt.row0 - r_lo);
+      const uint32_t mine = smem_u32(smem);
+      uint32_t base[8];
+#pragma unroll
+      for (int sp = 0; sp < 8; ++sp)
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base[sp]) : "r"(mine), "r"(sp < a.splits ? sp : 0));
+      for (int i = threadIdx.x; i < rows * cols; i += 192) {
+        const int rr = r_lo + i / cols, c4 = (i % cols) * 4;
+        const uint32_t off = (uint32_t)(rr * SPLIT_ROW + c4) * 4;
+        float4 p[8];
+#pragma unroll
+        for (int sp = 0; sp < 8; ++sp)
+          if (sp < a.splits) p[sp] = ld_cluster_v4(base[sp] + off);
+        float4 f = p[0];
+#pragma unroll
+        for (int sp = 1; sp < 8; ++sp)
+          if (sp < a.splits) { f.x += p[sp].x; f.y += p[sp].y; f.z += p[sp].z; f.w += p[sp].w; }
+        const int r = mt.row0 + rr;
+        long orow = r;
+        if (a.dst_row) orow = a.dst_row[r];
+        if (orow < 0) continue;
+        if (a.row_scale) { const float sc = a.row_scale[r]; f.x *= sc; f.y *= sc; f.z *= sc; f.w *= sc; }
+        const int col = n0 + c4;
+        if (a.resid) {
+          const float4 x = *reinterpret_cast<const float4*>(a.resid + orow * a.ldr + col);
+          f.x += x.x; f.y += x.y; f.z += x.z; f.w += x.w;
+        }
+        if (a.c_f32) {
+          *reinterpret_cast<float4*>(a.c_f32 + orow * a.ldc + col) = f;
+        } else {
+          __nv_bfloat162 o[2] = {__floats2bfloat162_rn(f.x, f.y), __floats2bfloat162_rn(f.z, f.w)};
+          *reinterpret_cast<uint2*>(a.c_bf16 + orow * a.ldc + col) = *reinterpret_cast<const uint2*>(o);
+        }
+      }
+    }
+    __syncwarp();
+    cluster_arrive_release();                  // no CTA leaves while a peer still reads its ring
+    cluster_wait_acquire();
+  }
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -294,6 +379,15 @@ gemm_bf16_kernel(const __grid_constant__ AMaps tma_a, const __grid_constant__ CU
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
   }
   if (threadIdx.x == 0 && s_abort && a.status) atomicMax(a.status, 1u);
+}
+
+// CTAs that share the depth of each of `tiles` tiles: the most (up to 8) that leave every CTA a processor of its own and at
+// least eight 64-deep steps.  Eight steps are where a share still hides its start: prompts of 512 tokens, output projection
+// (32 tiles) and router (4 tiles).
+static int gemm_splits(long tiles, int K, int sm_count) {
+  int s = 1;
+  while (s < 8 && tiles * (2 * s) <= sm_count && K / BK >= 16 * s) s *= 2;
+  return s;
 }
 
 // ---- tile table ----------------------------------------------------------------------
@@ -379,7 +473,7 @@ static int gemm_launch(const void* const* A_of_rank, int n_src, long lda, long r
                        int n_groups, int N, int K, const void* mtiles, const int* n_mtiles, int max_mtiles, float* c_f32,
                        void* c_bf16, long ldc, const int* dst_row, const float* row_scale, const float* resid, long ldr,
                        float* const* own_base, int n_owners, int rows_per_owner, int dst_div, int src_rows,
-                       unsigned* status, int sm_count, cudaStream_t st) {
+                       unsigned* status, int sm_count, int fixed_tiles, cudaStream_t st) {
   BL_REQUIRE(K >= BK && K % BK == 0 && N >= 32 && N % 32 == 0, BL_ERR_SHAPE);
   BL_REQUIRE(lda % 8 == 0 && rows_a >= 1 && n_groups >= 1 && n_src >= 1 && n_src <= 8, BL_ERR_SHAPE);
   BL_REQUIRE(((uintptr_t)B & 15) == 0 && ((uintptr_t)B2 & 15) == 0, BL_ERR_ALIGN);
@@ -425,6 +519,17 @@ static int gemm_launch(const void* const* A_of_rank, int n_src, long lda, long r
   long tiles = (long)max_mtiles * a.tiles_n;
   int grid = (int)(tiles < sm_count ? tiles : sm_count);
   const size_t smem = (size_t)STAGES * (TILE_A_BYTES + 2 * TILE_B128_BYTES) + 1024;
+  static_assert(BM * SPLIT_ROW * 4 <= STAGES * (TILE_A_BYTES + 2 * TILE_B128_BYTES), "a parked tile fits the ring");
+  a.splits = fixed_tiles && !dist && !B2 ? gemm_splits(tiles, K, sm_count) : 1;
+  if (a.splits > 1) {
+    static bool set = false;
+    if (!set) {
+      cudaFuncSetAttribute(gemm_bf16_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      set = true;
+    }
+    return (int)launch_cluster(gemm_bf16_kernel<false, false, true>, dim3((unsigned)(tiles * a.splits)), dim3(192), smem, a.splits, st,
+                               ma, mb, mb2, a);
+  }
   auto go = [&](auto kernel, bool& set) {
     if (!set) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); set = true; }
     return (int)launch(kernel, dim3(grid), dim3(192), smem, st, ma, mb, mb2, a);
@@ -440,7 +545,17 @@ int bl_gemm_bf16(const void* A, long lda, long rows_a, const void* B, const void
                  int sm_count, cudaStream_t st) {
   const void* As[1] = {A};
   return gemm_launch(As, 1, lda, rows_a, B, B2, n_groups, N, K, mtiles, n_mtiles, max_mtiles, c_f32, c_bf16, ldc, dst_row,
-                     row_scale, resid, ldr, nullptr, 0, 0, 1, 0, status, sm_count, st);
+                     row_scale, resid, ldr, nullptr, 0, 0, 1, 0, status, sm_count, 0, st);
+}
+
+// The same over a table that holds exactly max_mtiles tiles: a product of few tiles shares their depth over clusters.
+int bl_gemm_bf16_fixed(const void* A, long lda, long rows_a, const void* B, const void* B2, int n_groups, int N, int K,
+                       const void* mtiles, const int* n_mtiles, int max_mtiles, float* c_f32, void* c_bf16, long ldc,
+                       const int* dst_row, const float* row_scale, const float* resid, long ldr, unsigned* status,
+                       int sm_count, cudaStream_t st) {
+  const void* As[1] = {A};
+  return gemm_launch(As, 1, lda, rows_a, B, B2, n_groups, N, K, mtiles, n_mtiles, max_mtiles, c_f32, c_bf16, ldc, dst_row,
+                     row_scale, resid, ldr, nullptr, 0, 0, 1, 0, status, sm_count, 1, st);
 }
 
 // The several-GPU form.  A_of_rank: one pointer per source rank (each [rows_a, K], the rank's shard; tiles pick
@@ -455,7 +570,7 @@ int bl_gemm_bf16_dist(const void* const* A_of_rank, int n_src, long lda, long ro
   BL_REQUIRE(n_src == 1 || (src_rows >= BM && src_rows % BM == 0 && rows_a >= src_rows), BL_ERR_SHAPE);
   return gemm_launch(A_of_rank, n_src, lda, rows_a, B, B2, n_groups, N, K, mtiles, n_mtiles, max_mtiles, c_f32, c_bf16, ldc,
                      dst_row, row_scale, nullptr, 0, own_base, n_owners, rows_per_owner, dst_div < 1 ? 1 : dst_div,
-                     n_src > 1 ? src_rows : 0, status, sm_count, st);
+                     n_src > 1 ? src_rows : 0, status, sm_count, 0, st);
 }
 
 }  // extern "C"

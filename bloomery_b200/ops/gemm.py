@@ -72,17 +72,19 @@ def gemm_bf16(A: torch.Tensor, B: torch.Tensor, tiles: TileTable, *, out_f32: Op
               out_bf16: Optional[torch.Tensor] = None, B2: Optional[torch.Tensor] = None, dst_row=None, row_scale=None,
               resid=None, status: Optional[torch.Tensor] = None) -> None:
     """C = A @ B[g].T per tile.  A [rows, K] bf16; B (and B2) [G, N, K] or [N, K] bf16.
-    With B2 the output is silu(A B^T) * (A B2^T)."""
+    With B2 the output is silu(A B^T) * (A B2^T).  A table that the host wrote (``TileTable.fixed``) tells the launch how
+    many tiles there are, and a product of few tiles shares their depth over clusters of CTAs."""
     assert A.dtype == torch.bfloat16 and B.dtype == torch.bfloat16 and A.stride(-1) == 1 and B.is_contiguous()
     if B.dim() == 2:
         B = B[None]
         B2 = B2[None] if B2 is not None else None
     G, N, Kd = B.shape
     out = out_f32 if out_f32 is not None else out_bf16
-    rc = cuda().bl_gemm_bf16(p(A), L(A.stride(0)), L(A.shape[0]), p(B), p(B2), I(G), I(N), I(Kd), p(tiles.mtiles),
-                             p(tiles.n_mtiles), I(tiles.max_mtiles), p(out_f32), p(out_bf16), L(out.stride(0)),
-                             p(dst_row), p(row_scale), p(resid), L(resid.stride(0) if resid is not None else 0),
-                             p(status), I(sm_count()), stream())
+    entry = cuda().bl_gemm_bf16_fixed if tiles.fixed else cuda().bl_gemm_bf16
+    rc = entry(p(A), L(A.stride(0)), L(A.shape[0]), p(B), p(B2), I(G), I(N), I(Kd), p(tiles.mtiles),
+               p(tiles.n_mtiles), I(tiles.fixed or tiles.max_mtiles), p(out_f32), p(out_bf16), L(out.stride(0)),
+               p(dst_row), p(row_scale), p(resid), L(resid.stride(0) if resid is not None else 0),
+               p(status), I(sm_count()), stream())
     check(rc, "bl_gemm_bf16")
 
 

@@ -142,7 +142,7 @@ class GemmPrefill:
             if self._work is None:
                 self._work = G.QgemmWork(dev, 128)
         else:
-            dense_tiles = G.TileTable.dense(T, dev)
+            dense_tiles = G.TileTable.dense(T, dev, host=True)
         n_keys = p0 + T
         T_pad = (n_keys + 127) // 128 * 128
         if not fine:

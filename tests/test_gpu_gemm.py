@@ -234,3 +234,38 @@ def test_kv_gather_rows_and_transposed_values(n_kv, head, n_keys, T_pad):
     v_ref[:, n_keys:] = 0
     assert torch.equal(Kb.float(), k_ref.bfloat16().float())
     assert torch.equal(Vt.float(), v_ref.bfloat16().float().transpose(1, 2))
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 6144), (127, 32, 1024), (129, 160, 1088), (511, 2048, 4096), (300, 5120, 2048),
+                                   (640, 288, 1024), (64, 256, 960), (700, 2048, 4096)])
+def test_product_of_few_tiles_over_a_cluster(M, N, K):
+    """Clusters of 8, 8, 8, 4, 2, 2, 1 (too shallow) and 2 CTAs: ragged last tiles on both sides and depths that the shares do
+    not divide, with residual, scatter and bf16 rows; the bits repeat."""
+    from bloomery_b200.ops import gemm as G
+    g = torch.Generator(device=DEV).manual_seed(M)
+    A = torch.randn(M, K, device=DEV, generator=g).bfloat16()
+    B = (torch.randn(N, K, device=DEV, generator=g) / K ** 0.5).bfloat16()
+    R = torch.randn(M, N, device=DEV, generator=g)
+    dst = torch.randperm(M, device=DEV, generator=g).int()
+    dst[M // 2] = -1 if M > 1 else 0                             # a dropped row
+    scale = torch.rand(M, device=DEV, generator=g)
+    st, tiles = _status(), G.TileTable.dense(M, DEV, host=True)
+    ref = A.double() @ B.double().T
+    C = torch.full((M, N), float("nan"), device=DEV)
+    G.gemm_bf16(A, B, tiles, out_f32=C, resid=R, status=st)
+    # products of bf16 are exact in fp32; sums of K terms of size about 1 / sqrt(K), in fp32
+    assert float((C.double() - ref - R.double()).abs().max()) < 2 ** -24 * K ** 0.5 * 16
+    again = torch.full((M, N), float("nan"), device=DEV)
+    for _ in range(20):
+        G.gemm_bf16(A, B, tiles, out_f32=again, resid=R, status=st)
+        assert torch.equal(C, again)
+    S = torch.full((M, N), 7.0, device=DEV)
+    G.gemm_bf16(A, B, tiles, out_f32=S, dst_row=dst, row_scale=scale, status=st)
+    keep = dst >= 0
+    want = torch.full((M, N), 7.0, device=DEV, dtype=torch.float64)
+    want[dst[keep].long()] = ref[keep] * scale[keep].double()[:, None]
+    assert float((S.double() - want).abs().max()) < 2 ** -23 * K ** 0.5 * 16
+    H = torch.full((M, N), float("nan"), device=DEV, dtype=torch.bfloat16)
+    G.gemm_bf16(A, B, tiles, out_bf16=H, status=st)
+    assert torch.equal(H, (again - R).bfloat16()) or torch.allclose(H.double(), ref, rtol=2 ** -7, atol=1e-4)
+    assert int(st) == 0
