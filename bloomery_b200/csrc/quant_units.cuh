@@ -670,18 +670,30 @@ struct NvFp4 {
     uint32_t gb = ld32(row + K / 2 + K / 16);
     __builtin_memcpy(&r.g, &gb, 4);
   }
-  // eight nibbles of one word -> two words of int8 (values x2)
+  // Eight nibbles of one word -> two words of int8 (values x2).  On the device four codes at a time: byte permutes whose
+  // selectors are the code nibbles look up the magnitude and its negative, a third one spreads the sign bits over their
+  // bytes, and a bitwise select takes one or the other: 11 instructions for eight codes against about 60 one by one (a token of
+  // the 30 B shape: 3.62 -> 2.34 ms).
   static BL_HD void expand(uint32_t w, uint32_t& lo4, uint32_t& hi4) {
+#if defined(__CUDA_ARCH__)
+    const uint32_t sel = w & 0x77777777u, seven = w << 4;          // sign bits of even codes: top bits of `seven`, of odd ones: of w
+    uint32_t s0, s1;
+    asm("prmt.b32 %0, %1, %2, 0xD9C8;" : "=r"(s0) : "r"(seven), "r"(w));   // selector bit 3: the byte's sign bit, eight times
+    asm("prmt.b32 %0, %1, %2, 0xFBEA;" : "=r"(s1) : "r"(seven), "r"(w));
+    lo4 = (__byte_perm(0x03020100u, 0x0C080604u, sel) & ~s0) | (__byte_perm(0xFDFEFF00u, 0xF4F8FAFCu, sel) & s0);
+    hi4 = (__byte_perm(0x03020100u, 0x0C080604u, sel >> 16) & ~s1) | (__byte_perm(0xFDFEFF00u, 0xF4F8FAFCu, sel >> 16) & s1);
+#else
     lo4 = 0; hi4 = 0;
-#pragma unroll
     for (int i = 0; i < 4; ++i) {
       lo4 |= (uint32_t)(uint8_t)e2m1_x2((w >> (4 * i)) & 0xF) << (8 * i);
       hi4 |= (uint32_t)(uint8_t)e2m1_x2((w >> (16 + 4 * i)) & 0xF) << (8 * i);
     }
+#endif
   }
   static BL_HD float dot(const Regs& r, const uint32_t* aq /*16 words*/, const float* ad /*d of the two 32-blocks*/) {
     const uint32_t w[8] = {r.q0.x, r.q0.y, r.q0.z, r.q0.w, r.q1.x, r.q1.y, r.q1.z, r.q1.w};
-    float acc = 0.f;
+    float acc = 0.f, sc[4];
+    e4m3x4_to_float(r.sc, sc);
 #pragma unroll
     for (int g = 0; g < 4; ++g) {                 // group g: values 16g..16g+15 = words 2g, 2g+1 of codes
       int s = 0;
@@ -692,7 +704,7 @@ struct NvFp4 {
         s = dot4(lo4, aq[4 * g + 2 * h], s);
         s = dot4(hi4, aq[4 * g + 2 * h + 1], s);
       }
-      acc += e4m3_to_float((uint8_t)(r.sc >> (8 * g))) * ad[g >> 1] * (float)s;
+      acc += sc[g] * ad[g >> 1] * (float)s;
     }
     return acc * r.g * 0.5f;
   }
