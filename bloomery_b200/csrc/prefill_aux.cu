@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(256) rope_append_prefill_kernel(const float* q
                                                                   const int* row_seq, const int* block_table, int max_pages,
                                                                   int n_pages, __half* k_cache, __half* v_cache,
                                                                   __nv_bfloat16* q_bf16, unsigned* fault, int layer) {
-  constexpr int DPL = HEAD / 32;
+  constexpr int DPL = HEAD / 32, kHeads = 5;
   pdl_wait();
   pdl_launch();
   const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -265,38 +265,56 @@ __global__ void __launch_bounds__(256) rope_append_prefill_kernel(const float* q
   const bool page_ok = page >= 0 && page < n_pages;
   if (!page_ok && threadIdx.x == 0) raise_fault(fault, layer, FS_PAGE);
   const float* row = qkv + (long)t * qkv_stride;
-  for (int head = warp; head < n_q + 2 * n_kv; head += 8) {
-    const bool is_q = head < n_q, is_k = !is_q && head < n_q + n_kv;
-    float x[DPL];
+  // kHeads heads of a warp at a time: their loads, and then their double-precision sums and roots, run side by side
+  for (int h0 = warp; h0 < n_q + 2 * n_kv; h0 += 8 * kHeads) {
+    float x[kHeads][DPL];
 #pragma unroll
-    for (int j = 0; j < DPL; ++j) x[j] = row[(long)head * HEAD + lane + 32 * j];
-    const float* gain = is_q ? q_gain : (is_k ? k_gain : nullptr);
-    if (gain) {
-      double ss = 0.0;
+    for (int b = 0; b < kHeads; ++b) {
+      const int head = h0 + 8 * b;
+      if (head < n_q + 2 * n_kv)
 #pragma unroll
-      for (int j = 0; j < DPL; ++j) ss += (double)(x[j] * x[j]);
-      ss = warp_sum_d(ss);
-      const float scale = (float)(1.0 / sqrt(ss / (double)HEAD + (double)eps));
-#pragma unroll
-      for (int j = 0; j < DPL; ++j) x[j] = (scale * gain[lane + 32 * j]) * x[j];
+        for (int j = 0; j < DPL; ++j) x[b][j] = row[(long)head * HEAD + lane + 32 * j];
     }
-    if (is_q || is_k) {
+    double ss[kHeads];
 #pragma unroll
-      for (int j = 0; j < DPL / 2; ++j) {
-        const float x0 = x[j], x1 = x[j + DPL / 2];
-        x[j] = fmaf(x0, cs[j], -(x1 * sn[j]));
-        x[j + DPL / 2] = fmaf(x0, sn[j], x1 * cs[j]);
+    for (int b = 0; b < kHeads; ++b) {
+      ss[b] = 0.0;
+#pragma unroll
+      for (int j = 0; j < DPL; ++j) ss[b] += (double)(x[b][j] * x[b][j]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int b = 0; b < kHeads; ++b) ss[b] += __shfl_xor_sync(0xffffffffu, ss[b], o);
+#pragma unroll
+    for (int b = 0; b < kHeads; ++b) {
+      const int head = h0 + 8 * b;
+      if (head >= n_q + 2 * n_kv) break;
+      const bool is_q = head < n_q, is_k = !is_q && head < n_q + n_kv;
+      const float* gain = is_q ? q_gain : (is_k ? k_gain : nullptr);
+      if (gain) {
+        const float scale = (float)(1.0 / sqrt(ss[b] / (double)HEAD + (double)eps));
+#pragma unroll
+        for (int j = 0; j < DPL; ++j) x[b][j] = (scale * gain[lane + 32 * j]) * x[b][j];
       }
-    }
-    if (is_q) {
-      __nv_bfloat16* q = q_bf16 + ((long)head * T + t) * HEAD;
+      if (is_q || is_k) {
 #pragma unroll
-      for (int j = 0; j < DPL; ++j) q[lane + 32 * j] = __float2bfloat16_rn(x[j] * q_scale);
-    } else if (page_ok) {
-      const int kvh = is_k ? head - n_q : head - n_q - n_kv;
-      __half* dst = (is_k ? k_cache : v_cache) + (((long)page * n_kv + kvh) * 64 + (pos % 64)) * HEAD;
+        for (int j = 0; j < DPL / 2; ++j) {
+          const float x0 = x[b][j], x1 = x[b][j + DPL / 2];
+          x[b][j] = fmaf(x0, cs[j], -(x1 * sn[j]));
+          x[b][j + DPL / 2] = fmaf(x0, sn[j], x1 * cs[j]);
+        }
+      }
+      if (is_q) {
+        __nv_bfloat16* q = q_bf16 + ((long)head * T + t) * HEAD;
 #pragma unroll
-      for (int j = 0; j < DPL; ++j) dst[lane + 32 * j] = __float2half_rn(x[j]);
+        for (int j = 0; j < DPL; ++j) q[lane + 32 * j] = __float2bfloat16_rn(x[b][j] * q_scale);
+      } else if (page_ok) {
+        const int kvh = is_k ? head - n_q : head - n_q - n_kv;
+        __half* dst = (is_k ? k_cache : v_cache) + (((long)page * n_kv + kvh) * 64 + (pos % 64)) * HEAD;
+#pragma unroll
+        for (int j = 0; j < DPL; ++j) dst[lane + 32 * j] = __float2half_rn(x[b][j]);
+      }
     }
   }
 }
@@ -386,30 +404,68 @@ __global__ void __launch_bounds__(256) moe_combine_norm_kernel(const float* slot
 //   Kb [n_kv][T_pad][HEAD], Vt [n_kv][HEAD][T_pad]; positions >= n_keys are zero.
 // One block per (cache page of 64 keys, KV head): rows are read and the key rows written whole; the values
 // pass through a shared tile so that the transposed rows are written 128 contiguous bytes at a time.
+// Rows of whole 16-byte pieces (VEC) move eight values at a time: 9,700 keys of four heads are 20 MB in and 20 MB out.
+__device__ __forceinline__ uint4 half8_to_bf16(const uint4& h) {
+  const uint32_t w[4] = {h.x, h.y, h.z, h.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+    const __nv_bfloat162 p = __floats2bfloat162_rn(f.x, f.y);
+    o[i] = *reinterpret_cast<const uint32_t*>(&p);
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+template <bool VEC>
 __global__ void __launch_bounds__(256) kv_gather_bf16_kernel(const __half* k_cache, const __half* v_cache, const int* block_table,
                                                             int n_pages, int n_kv, int head, int n_keys, int T_pad,
                                                             __nv_bfloat16* Kb, __nv_bfloat16* Vt) {
-  __shared__ __nv_bfloat16 sv[64][130];         // 65-word rows: the transposed read has no bank conflicts
+  __shared__ __align__(4) __nv_bfloat16 sv[64][130];   // 65-word rows: the transposed read has few bank conflicts
   pdl_wait();
   pdl_launch();
   const int t0 = blockIdx.x * 64, kvh = blockIdx.y, tid = threadIdx.x;
   int page = t0 < n_keys ? block_table[t0 / 64] : -1;
   if (page >= n_pages) page = -1;
   const long src0 = ((long)page * n_kv + kvh) * 64 * head;
-  for (int i = tid; i < 64 * head; i += 256) {
-    const int tt = i / head, d = i - tt * head;
-    float kv = 0.f, vv = 0.f;
-    if (page >= 0 && t0 + tt < n_keys) {
-      kv = __half2float(k_cache[src0 + i]);
-      vv = __half2float(v_cache[src0 + i]);
+  if constexpr (VEC) {
+    const int per = head / 8;
+    for (int i = tid; i < 64 * per; i += 256) {
+      const int tt = i / per, d = (i - tt * per) * 8;
+      uint4 kv = make_uint4(0u, 0u, 0u, 0u), vv = kv;
+      if (page >= 0 && t0 + tt < n_keys) {
+        kv = *reinterpret_cast<const uint4*>(k_cache + src0 + 8 * i);
+        vv = *reinterpret_cast<const uint4*>(v_cache + src0 + 8 * i);
+      }
+      *reinterpret_cast<uint4*>(Kb + ((long)kvh * T_pad + t0 + tt) * head + d) = half8_to_bf16(kv);
+      const uint4 vb = half8_to_bf16(vv);
+      uint32_t* s = reinterpret_cast<uint32_t*>(&sv[tt][d]);
+      s[0] = vb.x; s[1] = vb.y; s[2] = vb.z; s[3] = vb.w;
     }
-    Kb[((long)kvh * T_pad + t0 + tt) * head + d] = __float2bfloat16_rn(kv);
-    sv[tt][d] = __float2bfloat16_rn(vv);
-  }
-  __syncthreads();
-  for (int i = tid; i < 64 * head; i += 256) {
-    const int d = i >> 6, tt = i & 63;
-    Vt[((long)kvh * head + d) * T_pad + t0 + tt] = sv[tt][d];
+    __syncthreads();
+    for (int i = tid; i < 8 * head; i += 256) {
+      const int d = i >> 3, tt = (i & 7) * 8;
+      __nv_bfloat162 o[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) { o[j].x = sv[tt + 2 * j][d]; o[j].y = sv[tt + 2 * j + 1][d]; }
+      *reinterpret_cast<uint4*>(Vt + ((long)kvh * head + d) * T_pad + t0 + tt) = *reinterpret_cast<const uint4*>(o);
+    }
+  } else {
+    for (int i = tid; i < 64 * head; i += 256) {
+      const int tt = i / head, d = i - tt * head;
+      float kv = 0.f, vv = 0.f;
+      if (page >= 0 && t0 + tt < n_keys) {
+        kv = __half2float(k_cache[src0 + i]);
+        vv = __half2float(v_cache[src0 + i]);
+      }
+      Kb[((long)kvh * T_pad + t0 + tt) * head + d] = __float2bfloat16_rn(kv);
+      sv[tt][d] = __float2bfloat16_rn(vv);
+    }
+    __syncthreads();
+    for (int i = tid; i < 64 * head; i += 256) {
+      const int d = i >> 6, tt = i & 63;
+      Vt[((long)kvh * head + d) * T_pad + t0 + tt] = sv[tt][d];
+    }
   }
 }
 
@@ -522,8 +578,25 @@ __global__ void __launch_bounds__(256) rmsnorm_hilo_kernel(const float* x, long 
   pdl_launch();
   const int t = blockIdx.x, tid = threadIdx.x;
   const float* xr = x + (long)t * x_stride;
+  __nv_bfloat16* o = out + (long)t * 3 * K;
+  const bool vec = K % 4 == 0 && K <= 8192 && x_stride % 4 == 0 && ((((uintptr_t)x | (uintptr_t)gain) & 15) | ((uintptr_t)out & 7)) == 0;
+  float4 keep[8];                               // the row, read once (VEC: four values at a time)
   float ss = 0.f;
-  for (int i = tid; i < K; i += 256) { float v = xr[i]; ss += v * v; }
+  if (vec) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int i = (c * 256 + tid) * 4;
+      if (i >= K) break;
+      keep[c] = *reinterpret_cast<const float4*>(xr + i);
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      if ((c * 256 + tid) * 4 >= K) break;
+      ss += keep[c].x * keep[c].x + keep[c].y * keep[c].y + keep[c].z * keep[c].z + keep[c].w * keep[c].w;
+    }
+  } else {
+    for (int i = tid; i < K; i += 256) { float v = xr[i]; ss += v * v; }
+  }
   double tot = warp_sum_d((double)ss);
   if ((tid & 31) == 0) red[tid >> 5] = tot;
   __syncthreads();
@@ -531,12 +604,28 @@ __global__ void __launch_bounds__(256) rmsnorm_hilo_kernel(const float* x, long 
 #pragma unroll
   for (int w = 0; w < 8; ++w) all += red[w];
   const float scale = 1.0f / sqrtf((float)(all / (double)K) + eps);
-  __nv_bfloat16* o = out + (long)t * 3 * K;
-  for (int i = tid; i < K; i += 256) {
-    const float v = xr[i] * scale * gain[i];
-    const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-    o[i] = hi; o[K + i] = hi;
-    o[2 * K + i] = __float2bfloat16_rn(v - __bfloat162float(hi));
+  if (vec) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int i = (c * 256 + tid) * 4;
+      if (i >= K) break;
+      const float4 g = *reinterpret_cast<const float4*>(gain + i);
+      const float v[4] = {keep[c].x * scale * g.x, keep[c].y * scale * g.y, keep[c].z * scale * g.z, keep[c].w * scale * g.w};
+      __nv_bfloat162 hi[2] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3])};
+      __nv_bfloat162 lo[2] = {__floats2bfloat162_rn(v[0] - __low2float(hi[0]), v[1] - __high2float(hi[0])),
+                              __floats2bfloat162_rn(v[2] - __low2float(hi[1]), v[3] - __high2float(hi[1]))};
+      const uint2 h2 = *reinterpret_cast<const uint2*>(hi);
+      *reinterpret_cast<uint2*>(o + i) = h2;
+      *reinterpret_cast<uint2*>(o + K + i) = h2;
+      *reinterpret_cast<uint2*>(o + 2 * K + i) = *reinterpret_cast<const uint2*>(lo);
+    }
+  } else {
+    for (int i = tid; i < K; i += 256) {
+      const float v = xr[i] * scale * gain[i];
+      const __nv_bfloat16 hi = __float2bfloat16_rn(v);
+      o[i] = hi; o[K + i] = hi;
+      o[2 * K + i] = __float2bfloat16_rn(v - __bfloat162float(hi));
+    }
   }
 }
 
@@ -622,8 +711,10 @@ int bl_moe_combine(const float* slot_out, const int* pos_of, int T, int k, int H
 int bl_kv_gather_bf16(const void* k_cache, const void* v_cache, const int* block_table, int n_pages, int n_kv, int head,
                       int n_keys, int T_pad, void* Kb, void* Vt, cudaStream_t st) {
   BL_REQUIRE(head <= 128 && T_pad >= 64 && T_pad % 64 == 0 && n_keys <= T_pad, BL_ERR_SHAPE);
-  return (int)launch(kv_gather_bf16_kernel, dim3(T_pad / 64, n_kv), dim3(256), 0, st, (const __half*)k_cache, (const __half*)v_cache,
-                     block_table, n_pages, n_kv, head, n_keys, T_pad, (__nv_bfloat16*)Kb, (__nv_bfloat16*)Vt);
+  const bool vec = head % 8 == 0 && (((uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)Kb | (uintptr_t)Vt) & 15) == 0;
+  return (int)launch(vec ? kv_gather_bf16_kernel<true> : kv_gather_bf16_kernel<false>, dim3(T_pad / 64, n_kv), dim3(256), 0, st,
+                     (const __half*)k_cache, (const __half*)v_cache, block_table, n_pages, n_kv, head, n_keys, T_pad,
+                     (__nv_bfloat16*)Kb, (__nv_bfloat16*)Vt);
 }
 
 int bl_softmax_causal(const float* S, long ldS, long rows, int Tq, int pos0, int T_pad, void* P, long ldP, cudaStream_t st) {

@@ -141,6 +141,59 @@ __device__ __forceinline__ bool route_block(const RouteParams& p, int m, RouteSh
 }
 
 
+// The picks alone, by every warp for itself and without a block barrier, for the plain case: softmax over the chosen, one group,
+// 32, 64, 128 or 256 experts.  A lane holds the scores of E / 32 neighbouring experts as integers of the same order; a pick is
+// their maximum over the warp (redux) and the first lane that has it, so equal scores go to the smaller id as in rank
+// counting.  The first `n` picks come out in lanes 0 .. n - 1 (id and logit); false: some logit is not finite.
+__host__ __device__ __forceinline__ bool route_pick_ok(const RouteParams& p) {
+  return p.mode == 0 && p.renorm && p.n_group <= 1 && (p.E == 32 || p.E == 64 || p.E == 128 || p.E == 256);
+}
+
+__device__ __forceinline__ bool route_pick(const RouteParams& p, int m, int lane, int n, int& id, float& logit) {
+  const int per = p.E / 32;
+  const float* row = p.logits + (long)m * p.E + lane * per;
+  float l[8];
+  unsigned key[8];
+  bool nonfinite = false;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) l[i] = i < per ? __ldcg(row + i) : 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    nonfinite |= !isfinite(l[i]);
+    const unsigned b = __float_as_uint(l[i] + 0.0f);               // -0 and 0 are equal scores
+    key[i] = i < per ? ((b >> 31) ? ~b : b | 0x80000000u) : 0u;    // finite scores have keys above 0
+  }
+  id = 0; logit = 0.f;
+  if (__any_sync(0xffffffffu, nonfinite)) return false;
+  for (int r = 0; r < n; ++r) {
+    unsigned best = 0u;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) best = max(best, key[i]);
+    const unsigned top = __reduce_max_sync(0xffffffffu, best);
+    const int src = __ffs(__ballot_sync(0xffffffffu, best == top)) - 1;
+    int mine = 0;
+    float val = 0.f;
+#pragma unroll
+    for (int i = 7; i >= 0; --i)
+      if (key[i] == top) { mine = i; val = l[i]; }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (lane == src && i == mine) key[i] = 0u;
+    const int e = __shfl_sync(0xffffffffu, lane * per + mine, src);
+    const float v = __shfl_sync(0xffffffffu, val, src);
+    if (lane == r) { id = e; logit = v; }
+  }
+  return true;
+}
+
+// Weights of the picks in lanes 0 .. top_k - 1 (the arithmetic of route_block, softmax over the chosen).
+__device__ __forceinline__ float route_pick_weight(const RouteParams& p, int lane, float logit) {
+  const float ex = expf(logit - __shfl_sync(0xffffffffu, logit, 0));
+  double sum = 0.0;
+  for (int j = 0; j < p.top_k; ++j) sum += (double)__shfl_sync(0xffffffffu, ex, j);
+  return lane < p.top_k ? ex / (float)sum * p.scale : 0.f;
+}
+
 // The same routing by ONE warp, for the common shape (one expert group, at most 256 experts, a multiple of 32):
 // no block barriers, so a kernel can route in warp 0 while its other warps fetch activations.  Scores, ranks,
 // weights and tie rule are those of route_block (same sums in the same order: the results are bit-equal).

@@ -269,3 +269,36 @@ def test_product_of_few_tiles_over_a_cluster(M, N, K):
     G.gemm_bf16(A, B, tiles, out_bf16=H, status=st)
     assert torch.equal(H, (again - R).bfloat16()) or torch.allclose(H.double(), ref, rtol=2 ** -7, atol=1e-4)
     assert int(st) == 0
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("head", [64, 128, 40, 20])
+def test_kv_gather_of_whole_pieces_and_of_single_values(head, shift):
+    """Rows of whole 16-byte pieces, rows that have none (20 values) and buffers that do not start on one."""
+    from bloomery_b200.ops import gemm as G
+    g = torch.Generator(device=DEV).manual_seed(head)
+    n_kv, n_pages, n_keys, T_pad = 3, 7, 130, 256
+    kc, vc = (torch.randn(n_pages, n_kv, 64, head, device=DEV, generator=g).half() for _ in range(2))
+    table = torch.tensor([5, 0, 3, -1], dtype=torch.int32, device=DEV)
+    flat = [torch.full((n_kv * T_pad * head + shift,), float("nan"), device=DEV, dtype=torch.bfloat16) for _ in range(2)]
+    Kb, Vt = flat[0][shift:].view(n_kv, T_pad, head), flat[1][shift:].view(n_kv, head, T_pad)
+    G.kv_gather_bf16(kc, vc, table, n_pages, n_kv, head, n_keys, T_pad, Kb, Vt)
+    for got, cache in ((Kb, kc), (Vt.transpose(1, 2), vc)):
+        want = torch.zeros(n_kv, T_pad, head, device=DEV, dtype=torch.bfloat16)
+        want[:, :n_keys] = cache[table[:3].long()].transpose(0, 1).reshape(n_kv, 192, head)[:, :n_keys].bfloat16()
+        assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("K,shift", [(64, 0), (2048, 0), (8192, 0), (8196, 0), (1030, 0), (2048, 1)])
+def test_split_rows_of_the_router(K, shift):
+    """Rows that are read four values at a time (up to 8,192 of them) and rows that cannot be."""
+    from bloomery_b200.ops import gemm as G
+    g = torch.Generator(device=DEV).manual_seed(K)
+    x = torch.randn(5 * K + shift, device=DEV, generator=g)[shift:].view(5, K) * 3
+    gain = 1 + 0.1 * torch.randn(K, device=DEV, generator=g)
+    out = torch.full((5, 3 * K), float("nan"), device=DEV, dtype=torch.bfloat16)
+    G.rmsnorm_hilo(x, gain, 1e-6, out)
+    ref = x.double() / torch.sqrt((x.double() ** 2).mean(1, keepdim=True) + 1e-6) * gain.double()
+    assert torch.equal(out[:, :K], out[:, K:2 * K])
+    # value and remainder: 16 bits, and a few fp32 roundings of the scale
+    assert float(((out[:, :K].double() + out[:, 2 * K:].double() - ref) / ref.abs().clamp_min(1e-3)).abs().max()) < 2 ** -15

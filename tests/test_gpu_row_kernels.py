@@ -260,3 +260,61 @@ def test_a_short_prompt_leaves_the_logits_of_its_last_rows_unless_the_server_fee
     rows = [e.kv.k[:, e.kv.pages[1][0], :, :45] for e in eng]
     assert torch.equal(*rows)
     assert not torch.equal(rows[0], eng[0].kv.k[:, eng[0].kv.pages[0][0], :, :45])
+
+
+@pytest.mark.parametrize("E,k", [(32, 8), (64, 1), (128, 8), (256, 16), (96, 4)])
+def test_routing_by_a_warp_a_row(E, k):
+    """Rows of many ties, of zeros of both signs, of one finite huge value, and one row that is not finite, against a stable
+    sort of the same logits (96 experts take the block's counting)."""
+    from bloomery_b200.ops import decode as D
+    g = torch.Generator().manual_seed(E)
+    M = 19
+    lg = torch.randn(M, E, generator=g)
+    lg[1] = 0.0
+    lg[2] = torch.where(torch.rand(E, generator=g) < 0.5, 0.0, -0.0)
+    lg[3] = torch.randint(-2, 3, (E,), generator=g).float()
+    lg[4] = -torch.arange(E).float() - 1e30
+    lg[5, E - 1] = 3e38
+    lg[6] = -3.4028234663852886e38
+    lg[17, E // 2] = float("nan")
+    ids = torch.full((M, k), 7, dtype=torch.int32, device=DEV)
+    wts, heat, f = torch.full((M, k), 9.0, device=DEV), torch.zeros(E, dtype=torch.int32, device=DEV), _fault()
+    seq = torch.zeros(M, dtype=torch.int32, device=DEV)
+    seq[18] = -1
+    D.route_rows(lg.to(DEV), D.RouteRule(k), M, ids, wts, heat, f, 3, seq)
+    torch.cuda.synchronize()
+    assert int(f) != -1 and (int(f) >> 8) == 3                   # the row that is not finite
+    live = [m for m in range(M) if m not in (17, 18)]
+    order = torch.sort(lg[live], dim=1, descending=True, stable=True)
+    assert torch.equal(ids.cpu()[live].long(), order.indices[:, :k])
+    want = torch.softmax(order.values[:, :k].double(), 1)
+    assert torch.allclose(wts.cpu()[live].double(), want, rtol=1e-5, atol=1e-7)
+    assert bool(wts[17].isnan().all()) and bool((ids[17] == 0).all())
+    assert bool((ids[18] == -1).all()) and bool((wts[18] == 0).all())
+    assert torch.equal(heat.cpu().long(), torch.bincount(order.indices[:, :k].flatten(), minlength=E))
+
+
+@pytest.mark.parametrize("head,n_q,n_kv", [(128, 32, 4), (128, 1, 1), (64, 14, 2), (128, 40, 8), (64, 37, 1)])
+def test_prompt_rows_are_normed_and_rotated_as_decode_rows_are(head, n_q, n_kv):
+    """Cached keys and values bit for bit those of the decode launch, queries its fp32 rows rounded to bf16, for numbers of
+    heads that the warps' groups divide and do not."""
+    from bloomery_b200.ops import decode as D
+    from bloomery_b200.ops import gemm as G
+    g = torch.Generator(device=DEV).manual_seed(head + n_q)
+    T, n_pages = 9, 4
+    qkv = torch.randn(T, (n_q + 2 * n_kv) * head, device=DEV, generator=g)
+    qg, kg = (1 + 0.1 * torch.randn(head, device=DEV, generator=g) for _ in range(2))
+    inv = (1.0 / (1e6 ** (torch.arange(0, head, 2, dtype=torch.float64) / head))).float().to(DEV)
+    pos = torch.tensor([0, 1, 63, 64, 65, 127, 128, 190, 200], dtype=torch.int32, device=DEV)
+    seq = torch.zeros(T, dtype=torch.int32, device=DEV)
+    table = torch.tensor([[2, 0, 3, 1]], dtype=torch.int32, device=DEV)
+    caches = [[torch.zeros(n_pages, n_kv, 64, head, dtype=torch.float16, device=DEV) for _ in range(2)] for _ in range(2)]
+    q32 = torch.zeros(T, n_q, head, device=DEV)
+    qbf = torch.zeros(n_q, T, head, device=DEV, dtype=torch.bfloat16)
+    f = _fault()
+    D.qk_norm_rope_append(qkv, qg, kg, inv, 1e-6, 0.125, head, n_q, n_kv, T, pos, seq, table, n_pages, *caches[0], q32, f, 0)
+    G.qk_norm_rope_append_prefill(qkv, qg, kg, inv, 1e-6, 0.125, head, n_q, n_kv, T, pos, seq, table, n_pages, *caches[1], qbf, f, 0)
+    torch.cuda.synchronize()
+    assert int(f) == -1
+    assert torch.equal(caches[0][0], caches[1][0]) and torch.equal(caches[0][1], caches[1][1])
+    assert torch.equal(q32.bfloat16().transpose(0, 1), qbf)
