@@ -137,46 +137,44 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
       }
     }
   } else if (warp == 9) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc(FQ, FKEYS);
-      auto qk = [&](int x, int st) {
-        const uint64_t dQ0 = umma_desc(smem_u32(sQ + x * FTILE)), dQ1 = umma_desc(smem_u32(sQ + x * FTILE + FHALF));
-        const uint64_t dK0 = umma_desc(smem_u32(sK + st * FTILE)), dK1 = umma_desc(smem_u32(sK + st * FTILE + FHALF));
-        const uint32_t tS = tS0 + x * FKEYS;
+    constexpr uint32_t idesc = umma_idesc(FQ, FKEYS);
+    auto qk = [&](int x, int st) {
+      const uint64_t dQ0 = umma_desc(smem_u32(sQ + x * FTILE)), dQ1 = umma_desc(smem_u32(sQ + x * FTILE + FHALF));
+      const uint64_t dK0 = umma_desc(smem_u32(sK + st * FTILE)), dK1 = umma_desc(smem_u32(sK + st * FTILE + FHALF));
+      const uint32_t tS = tS0 + x * FKEYS;
 #pragma unroll
-        for (int k = 0; k < FATOM / UMMA_K; ++k) umma_bf16(tS, dQ0 + (uint64_t)(k * 2), dK0 + (uint64_t)(k * 2), idesc, k > 0 ? 1u : 0u);
+      for (int k = 0; k < FATOM / UMMA_K; ++k) umma_bf16(tS, dQ0 + (uint64_t)(k * 2), dK0 + (uint64_t)(k * 2), idesc, k > 0 ? 1u : 0u);
 #pragma unroll
-        for (int k = 0; k < FATOM / UMMA_K; ++k) umma_bf16(tS, dQ1 + (uint64_t)(k * 2), dK1 + (uint64_t)(k * 2), idesc, 1u);
-        umma_commit(&s_full[x]);
-      };
-      bool ok = mbar_wait(&q_full, 0, abort_flag) && mbar_wait(&k_full[0], 0, abort_flag);
-      if (ok) {
+      for (int k = 0; k < FATOM / UMMA_K; ++k) umma_bf16(tS, dQ1 + (uint64_t)(k * 2), dK1 + (uint64_t)(k * 2), idesc, 1u);
+      umma_commit(&s_full[x]);
+    };
+    bool ok = mbar_wait_warp(&q_full, 0, abort_flag) && mbar_wait_warp(&k_full[0], 0, abort_flag);
+    if (ok) {
+      tc_fence_after();
+      for (int x = 0; x < n_x; ++x) qk(x, 0);
+      umma_commit(&k_empty[0]);
+    }
+    for (int t = 0; ok && t < n_t; ++t) {
+      const int st = t & 1, nx = (t + 1) & 1;
+      const uint32_t par = (uint32_t)((t >> 1) & 1), nx_par = (uint32_t)(((t + 1) >> 1) & 1);
+      const uint64_t dV0 = umma_desc(smem_u32(sV + st * FTILE)), dV1 = umma_desc(smem_u32(sV + st * FTILE + FHALF));
+      for (int x = 0; x < n_x; ++x) {
+        if (x == 0 && !mbar_wait_warp(&v_full[st], par, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(&p_full[x], (uint32_t)(t & 1), abort_flag)) { ok = false; break; }
         tc_fence_after();
-        for (int x = 0; x < n_x; ++x) qk(x, 0);
-        umma_commit(&k_empty[0]);
-      }
-      for (int t = 0; ok && t < n_t; ++t) {
-        const int st = t & 1, nx = (t + 1) & 1;
-        const uint32_t par = (uint32_t)((t >> 1) & 1), nx_par = (uint32_t)(((t + 1) >> 1) & 1);
-        const uint64_t dV0 = umma_desc(smem_u32(sV + st * FTILE)), dV1 = umma_desc(smem_u32(sV + st * FTILE + FHALF));
-        for (int x = 0; x < n_x; ++x) {
-          if (x == 0 && !mbar_wait(&v_full[st], par, abort_flag)) { ok = false; break; }
-          if (!mbar_wait(&p_full[x], (uint32_t)(t & 1), abort_flag)) { ok = false; break; }
+        const uint32_t tP = tS0 + x * FKEYS, tO = tO0 + x * FD;
+#pragma unroll
+        for (int k = 0; k < FATOM / UMMA_K; ++k) umma_bf16_ta(tO, tP + k * 8, dV0 + (uint64_t)(k * 2), idesc, (t > 0 || k > 0) ? 1u : 0u);
+#pragma unroll
+        for (int k = 0; k < FATOM / UMMA_K; ++k) umma_bf16_ta(tO, tP + 32 + k * 8, dV1 + (uint64_t)(k * 2), idesc, 1u);
+        if (x == n_x - 1) umma_commit(&v_empty[st]);
+        if (t + 1 < n_t) {
+          if (x == 0 && !mbar_wait_warp(&k_full[nx], nx_par, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t tP = tS0 + x * FKEYS, tO = tO0 + x * FD;
-#pragma unroll
-          for (int k = 0; k < FATOM / UMMA_K; ++k) umma_bf16_ta(tO, tP + k * 8, dV0 + (uint64_t)(k * 2), idesc, (t > 0 || k > 0) ? 1u : 0u);
-#pragma unroll
-          for (int k = 0; k < FATOM / UMMA_K; ++k) umma_bf16_ta(tO, tP + 32 + k * 8, dV1 + (uint64_t)(k * 2), idesc, 1u);
-          if (x == n_x - 1) umma_commit(&v_empty[st]);
-          if (t + 1 < n_t) {
-            if (x == 0 && !mbar_wait(&k_full[nx], nx_par, abort_flag)) { ok = false; break; }
-            tc_fence_after();
-            qk(x, nx);
-            if (x == n_x - 1) umma_commit(&k_empty[nx]);
-          } else {
-            umma_commit(&o_done[x]);
-          }
+          qk(x, nx);
+          if (x == n_x - 1) umma_commit(&k_empty[nx]);
+        } else {
+          umma_commit(&o_done[x]);
         }
       }
     }

@@ -58,9 +58,10 @@ __host__ __device__ constexpr uint32_t f8_idesc(int m, int n) {
 }
 __device__ __forceinline__ void umma_f8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, e;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
+      "elect.sync _|e, 0xFFFFFFFF;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
@@ -131,30 +132,28 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = f8_idesc(F8_BM, F8_BN);
-      int stage = 0; uint32_t phase = 0;
-      uint32_t part = 0, pphase = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < total_tiles && ok && !*abort_flag; t += gridDim.x) {
-        for (int kb = 0; kb < kblocks; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
-          if (!mbar_wait(&part_empty[part], pphase ^ 1, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sa = smem_u32(smem + (size_t)stage * STAGE_BYTES);
-          const uint32_t d0 = tmem_base + part * ACC_COLS;
-          const uint64_t da = umma_desc(sa), db = umma_desc(sa + B_OFF);
+    constexpr uint32_t idesc = f8_idesc(F8_BM, F8_BN);
+    int stage = 0; uint32_t phase = 0;
+    uint32_t part = 0, pphase = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+      for (int kb = 0; kb < kblocks; ++kb) {
+        if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(&part_empty[part], pphase ^ 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t sa = smem_u32(smem + (size_t)stage * STAGE_BYTES);
+        const uint32_t d0 = tmem_base + part * ACC_COLS;
+        const uint64_t da = umma_desc(sa), db = umma_desc(sa + B_OFF);
 #pragma unroll
-          for (int k = 0; k < F8_BK / 32; ++k) {                     // K = 32 codes = 32 bytes per instruction
-            const uint64_t step = (uint64_t)(k * 32 / 16);
-            umma_f8(d0, da + step, db + step, idesc, k > 0 ? 1u : 0u);
-            if (DUAL) umma_f8(d0 + F8_BN, umma_desc(sa + F8_A_BYTES) + step, db + step, idesc, k > 0 ? 1u : 0u);
-          }
-          umma_commit(&empty_bar[stage]);
-          umma_commit(&part_full[part]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
-          if (++part == F8_PARTS) { part = 0; pphase ^= 1; }
+        for (int k = 0; k < F8_BK / 32; ++k) {                     // K = 32 codes = 32 bytes per instruction
+          const uint64_t step = (uint64_t)(k * 32 / 16);
+          umma_f8(d0, da + step, db + step, idesc, k > 0 ? 1u : 0u);
+          if (DUAL) umma_f8(d0 + F8_BN, umma_desc(sa + F8_A_BYTES) + step, db + step, idesc, k > 0 ? 1u : 0u);
         }
+        umma_commit(&empty_bar[stage]);
+        umma_commit(&part_full[part]);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        if (++part == F8_PARTS) { part = 0; pphase ^= 1; }
       }
     }
   } else {

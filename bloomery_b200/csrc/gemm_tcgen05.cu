@@ -181,41 +181,39 @@ gemm_bf16_kernel(const __grid_constant__ AMaps tma_a, const __grid_constant__ CU
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc(BM, BN);
-      int stage = 0; uint32_t phase = 0;
-      int it = 0;
-      for (int t = first; t < total_tiles && !*abort_flag; t += step) {
-        const MTile mt = a.mtiles[t / a.tiles_n];
-        if (!DIST && tile_skipped(mt, (t % a.tiles_n) * BN)) continue;
-        const int kb_end = SPLIT ? kb_hi : DIST ? kblocks : tile_kblocks(mt, kblocks);
-        const int ab = it & 1;
-        const uint32_t acc_phase = (it >> 1) & 1;
-        ++it;
-        if (!mbar_wait(&acc_empty[ab], acc_phase ^ 1, abort_flag)) break;
+    constexpr uint32_t idesc = umma_idesc(BM, BN);
+    int stage = 0; uint32_t phase = 0;
+    int it = 0;
+    for (int t = first; t < total_tiles; t += step) {
+      const MTile mt = a.mtiles[t / a.tiles_n];
+      if (!DIST && tile_skipped(mt, (t % a.tiles_n) * BN)) continue;
+      const int kb_end = SPLIT ? kb_hi : DIST ? kblocks : tile_kblocks(mt, kblocks);
+      const int ab = it & 1;
+      const uint32_t acc_phase = (it >> 1) & 1;
+      ++it;
+      if (!mbar_wait_warp(&acc_empty[ab], acc_phase ^ 1, abort_flag)) break;
+      tc_fence_after();
+      const uint32_t d0 = tmem_base + ab * ACC_COLS;
+      bool ok = true;
+      for (int kb = kb_lo; kb < kb_end; ++kb) {
+        if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d0 = tmem_base + ab * ACC_COLS;
-        bool ok = true;
-        for (int kb = kb_lo; kb < kb_end; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sa = smem_u32(smem + (size_t)stage * STAGE_BYTES);
-          const uint64_t da = umma_desc(sa), db = umma_desc(sa + TILE_A_BYTES);
+        const uint32_t sa = smem_u32(smem + (size_t)stage * STAGE_BYTES);
+        const uint64_t da = umma_desc(sa), db = umma_desc(sa + TILE_A_BYTES);
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint32_t acc = (kb > kb_lo || k > 0) ? 1u : 0u;
-            umma_bf16(d0, da + (uint64_t)(k * UMMA_K * 2 / 16), db + (uint64_t)(k * UMMA_K * 2 / 16), idesc, acc);
-            if (DUAL) {
-              const uint64_t db2 = umma_desc(sa + TILE_A_BYTES + TILE_B_BYTES);
-              umma_bf16(d0 + BN, da + (uint64_t)(k * UMMA_K * 2 / 16), db2 + (uint64_t)(k * UMMA_K * 2 / 16), idesc, acc);
-            }
+        for (int k = 0; k < BK / UMMA_K; ++k) {
+          const uint32_t acc = (kb > kb_lo || k > 0) ? 1u : 0u;
+          umma_bf16(d0, da + (uint64_t)(k * UMMA_K * 2 / 16), db + (uint64_t)(k * UMMA_K * 2 / 16), idesc, acc);
+          if (DUAL) {
+            const uint64_t db2 = umma_desc(sa + TILE_A_BYTES + TILE_B_BYTES);
+            umma_bf16(d0 + BN, da + (uint64_t)(k * UMMA_K * 2 / 16), db2 + (uint64_t)(k * UMMA_K * 2 / 16), idesc, acc);
           }
-          umma_commit(&empty_bar[stage]);      // the stage is free once these MMAs have read it
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-        if (!ok) break;
-        umma_commit(&acc_full[ab]);            // accumulator complete
+        umma_commit(&empty_bar[stage]);      // the stage is free once these MMAs have read it
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
+      if (!ok) break;
+      umma_commit(&acc_full[ab]);            // accumulator complete
     }
   } else if constexpr (SPLIT) {
     // Park the partial tile: every operand of this CTA has been read by now (its accumulator is complete), so the ring is free.

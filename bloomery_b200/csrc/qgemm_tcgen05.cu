@@ -413,36 +413,34 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc(QBM, BN);
-      int stage = 0; uint32_t phase = 0;
-      int it = 0;
-      for (int t = blockIdx.x; t < total_tiles && !*abort_flag; t += gridDim.x) {
-        const int ab = it % NACC;
-        const uint32_t acc_phase = (it / NACC) & 1;
-        ++it;
-        if (!mbar_wait(&acc_empty[ab], acc_phase ^ 1, abort_flag)) break;
+    constexpr uint32_t idesc = umma_idesc(QBM, BN);
+    int stage = 0; uint32_t phase = 0;
+    int it = 0;
+    for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
+      const int ab = it % NACC;
+      const uint32_t acc_phase = (it / NACC) & 1;
+      ++it;
+      if (!mbar_wait_warp(&acc_empty[ab], acc_phase ^ 1, abort_flag)) break;
+      tc_fence_after();
+      const uint32_t d0 = tmem_base + ab * ACC_COLS;
+      bool ok = true;
+      for (int s = 0; s < kblocks * HALVES; ++s) {
+        if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d0 = tmem_base + ab * ACC_COLS;
-        bool ok = true;
-        for (int s = 0; s < kblocks * HALVES; ++s) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sb = smem_u32(smem + (size_t)stage * B_STAGE);
-          const uint32_t ta = tmem_a + stage * A_COLS;
+        const uint32_t sb = smem_u32(smem + (size_t)stage * B_STAGE);
+        const uint32_t ta = tmem_a + stage * A_COLS;
 #pragma unroll
-          for (int k = 0; k < QBK / UMMA_K; ++k) {
-            const uint64_t db = umma_desc(sb + (k >> 2) * B_ATOM) + (uint64_t)((k & 3) * UMMA_K * 2 / 16);
-            const uint32_t acc = (s > 0 || k > 0) ? 1u : 0u;
-            umma_bf16_ta(d0, ta + k * (UMMA_K / 2), db, idesc, acc);
-            if (DUAL) umma_bf16_ta(d0 + BN, ta + A_MAT + k * (UMMA_K / 2), db, idesc, acc);
-          }
-          umma_commit(&empty_bar[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        for (int k = 0; k < QBK / UMMA_K; ++k) {
+          const uint64_t db = umma_desc(sb + (k >> 2) * B_ATOM) + (uint64_t)((k & 3) * UMMA_K * 2 / 16);
+          const uint32_t acc = (s > 0 || k > 0) ? 1u : 0u;
+          umma_bf16_ta(d0, ta + k * (UMMA_K / 2), db, idesc, acc);
+          if (DUAL) umma_bf16_ta(d0 + BN, ta + A_MAT + k * (UMMA_K / 2), db, idesc, acc);
         }
-        if (!ok) break;
-        umma_commit(&acc_full[ab]);
+        umma_commit(&empty_bar[stage]);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
+      if (!ok) break;
+      umma_commit(&acc_full[ab]);
     }
   } else if (warp < 6) {
     const int q = warp & 3;
