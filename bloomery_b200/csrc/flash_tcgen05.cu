@@ -19,6 +19,10 @@
 // behind the product that reads them, and a commit behind Q K^T says that the P V in front of it is complete too.
 // One tile a CTA with two threads a row took 234 us a layer for 4,096 tokens of the 30 B shape (32 heads over 4) and 258 us for 700
 // behind 9,000; this takes 154 and 174.
+// A few hundred queries behind a long prefix are fewer CTAs than processors, each with a long walk over the keys: there
+// `splits` CTAs share the key tiles of a pair.  Each leaves its unnormalised output, maximum and sum of every row in a buffer,
+// and the warp that arrives last at its 32 rows (a ticket) adds the parts up in ascending order, its own out of tensor memory.
+// 700 queries behind 9,000 keys: 96 CTAs of 76 key tiles, 174 us; 288 of 25, 130 us.
 // Roles: warps 0..3 softmax of the first tile, 4..7 of the second (warp id modulo 4 = TMEM lane quarter), warp 8 the TMA
 // producer (two-stage rings for keys and values), warp 9 the MMA issuer and TMEM owner.  Every TMA load is a plain tile load
 // of this GPU's own memory.
@@ -45,6 +49,10 @@ struct FlashPrefillArgs {
   int t_pad;                  // key rows per KV head in K = key columns per row in Vt
   __nv_bfloat16* out; long ldo;
   unsigned* status;
+  int splits;                 // CTAs that share a pair's keys
+  float4* part;               // splits > 1: [pair][split][tile][column / 4][row] unnormalised outputs
+  float2* part_ml;            // [pair][split][tile][row]: maximum, sum
+  int* tickets;               // [pair][tile][4 warps], zero between launches
 };
 
 __device__ __forceinline__ float ex2(float x) {
@@ -59,6 +67,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 }
 
 constexpr int FTHREADS = 320;
+constexpr int kMaxSplits = 4;
 constexpr float kLazy = 8.0f;                           // the maximum may lag by 2^8 before the output is rescaled
 
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
@@ -82,12 +91,14 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
   // Query tiles of a KV head in descending order of position, its heads side by side: tile i = heads i % group at
   // position tile n_qt - 1 - i / group.  A CTA takes two that follow each other; the ones with the most keys start first.
   const int n_qt = (a.T + FQ - 1) / FQ;
-  const int kvh = (int)blockIdx.x % a.n_kv, item0 = 2 * ((int)blockIdx.x / a.n_kv);
+  const int pair = (int)blockIdx.x / a.splits, split = (int)blockIdx.x % a.splits;
+  const int kvh = pair % a.n_kv, item0 = 2 * (pair / a.n_kv);
   const int n_x = item0 + 1 < n_qt * a.group ? 2 : 1;           // tiles of this CTA
   auto tile_q0 = [&](int x) { return (n_qt - 1 - (item0 + x) / a.group) * FQ; };
   auto tile_head = [&](int x) { return kvh * a.group + (item0 + x) % a.group; };
   const int last_q = a.pos0 + min(tile_q0(0) + FQ, a.T) - 1;    // position of the first tile's last query: no other is later
-  const int n_t = last_q / FKEYS + 1;                           // key tiles 0 .. n_t - 1
+  const int all_t = last_q / FKEYS + 1;                         // key tiles of the pair
+  const int t_lo = all_t * split / a.splits, n_t = all_t * (split + 1) / a.splits - t_lo;   // this CTA's: t_lo .. t_lo + n_t - 1
 
   if (threadIdx.x == 0) {
     mbar_init(&q_full, 1);
@@ -123,12 +134,12 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
         const uint32_t par = (uint32_t)((t >> 1) & 1);
         if (!mbar_wait(&k_empty[st], par ^ 1, abort_flag)) break;
         mbar_expect_tx(&k_full[st], FTILE);
-        tma_load_2d(sK + st * FTILE, &tma_k, 0, kvh * a.t_pad + t * FKEYS, &k_full[st]);
-        tma_load_2d(sK + st * FTILE + FHALF, &tma_k, FATOM, kvh * a.t_pad + t * FKEYS, &k_full[st]);
+        tma_load_2d(sK + st * FTILE, &tma_k, 0, kvh * a.t_pad + (t_lo + t) * FKEYS, &k_full[st]);
+        tma_load_2d(sK + st * FTILE + FHALF, &tma_k, FATOM, kvh * a.t_pad + (t_lo + t) * FKEYS, &k_full[st]);
         if (!mbar_wait(&v_empty[st], par ^ 1, abort_flag)) break;
         mbar_expect_tx(&v_full[st], FTILE);
-        tma_load_2d(sV + st * FTILE, &tma_v, t * FKEYS, kvh * FD, &v_full[st]);
-        tma_load_2d(sV + st * FTILE + FHALF, &tma_v, t * FKEYS + FATOM, kvh * FD, &v_full[st]);
+        tma_load_2d(sV + st * FTILE, &tma_v, (t_lo + t) * FKEYS, kvh * FD, &v_full[st]);
+        tma_load_2d(sV + st * FTILE + FHALF, &tma_v, (t_lo + t) * FKEYS + FATOM, kvh * FD, &v_full[st]);
       }
       if (*abort_flag) {
         // copies of ours may still be landing: give them a bounded moment before the block's memory goes away
@@ -197,12 +208,13 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
 #pragma unroll
       for (int c = 0; c < 4; ++c) tmem_ld32(tS + 32 * c, v[c]);
       tmem_ld_wait();
-      if (t * FKEYS + FKEYS - 1 > a.pos0 + q0) {                // some key of this tile lies past some query of it
+      const int key0 = (t_lo + t) * FKEYS;
+      if (key0 + FKEYS - 1 > a.pos0 + q0) {                     // some key of this tile lies past some query of it
 #pragma unroll
         for (int c = 0; c < 4; ++c)
 #pragma unroll
           for (int i = 0; i < 32; ++i)
-            if (t * FKEYS + 32 * c + i > qpos) v[c][i] = 0xff800000u;     // -inf
+            if (key0 + 32 * c + i > qpos) v[c][i] = 0xff800000u;          // -inf
       }
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};        // four chains instead of one
 #pragma unroll
@@ -252,22 +264,94 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
     }
     if (ok && __all_sync(0xffffffffu, mbar_wait(&o_done[x], 0, abort_flag))) {
       tc_fence_after();
-      const float inv = l > 0.f ? 1.0f / l : 0.f;
-      __nv_bfloat16* orow = a.out + (long)qrow * a.ldo + (long)h * FD;
+      constexpr int PART = FD / 4 * FQ;                         // float4 of a tile's output
+      const long base = ((long)pair * a.splits * 2 + x) * FQ;   // + 2 FQ a split
+      bool mine = true;
+      if (a.splits > 1) {
+        float4* own = a.part + (((long)pair * a.splits + split) * 2 + x) * PART + r;
 #pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t o[32];
-        tmem_ld32(tO + c * 32, o);
-        tmem_ld_wait();
-        if (qrow < a.T) {
+        for (int c = 0; c < 4; ++c) {
+          uint32_t o[32];
+          tmem_ld32(tO + c * 32, o);
+          tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            uint4 pk;
-            pk.x = pack_bf16(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
-            pk.y = pack_bf16(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
-            pk.z = pack_bf16(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
-            pk.w = pack_bf16(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
-            *reinterpret_cast<uint4*>(orow + c * 32 + i) = pk;
+          for (int i = 0; i < 32; i += 4)
+            __stcg(own + (c * 8 + i / 4) * FQ, make_float4(__uint_as_float(o[i]), __uint_as_float(o[i + 1]), __uint_as_float(o[i + 2]),
+                                                           __uint_as_float(o[i + 3])));
+        }
+        __stcg(a.part_ml + base + (long)split * 2 * FQ + r, make_float2(m, l));
+        __threadfence();
+        __syncwarp();
+        int last = 0;
+        if (lane == 0) {
+          int* ticket = a.tickets + ((long)pair * 2 + x) * 4 + (warp & 3);
+          last = atomicAdd(ticket, 1) == a.splits - 1;
+          if (last) *ticket = 0;                                // ready for the next launch
+        }
+        mine = __shfl_sync(0xffffffffu, last, 0) != 0;
+        if (mine) __threadfence();
+      }
+      if (mine) {
+        float w[kMaxSplits];                                    // what each part counts, the normalisation included
+        if (a.splits > 1) {
+          float top = -INFINITY, all = 0.f;
+#pragma unroll
+          for (int sp = 0; sp < kMaxSplits; ++sp) {
+            w[sp] = 0.f;
+            if (sp < a.splits) {
+              w[sp] = __ldcg(a.part_ml + base + (long)sp * 2 * FQ + r).x;
+              top = fmaxf(top, w[sp]);
+            }
+          }
+#pragma unroll
+          for (int sp = 0; sp < kMaxSplits; ++sp)
+            if (sp < a.splits) {
+              w[sp] = w[sp] == -INFINITY ? 0.f : ex2((w[sp] - top) * kLog2e);
+              all += w[sp] * __ldcg(a.part_ml + base + (long)sp * 2 * FQ + r).y;
+            }
+          const float inv = all > 0.f ? 1.0f / all : 0.f;
+#pragma unroll
+          for (int sp = 0; sp < kMaxSplits; ++sp) w[sp] *= inv;
+        } else {
+          w[0] = l > 0.f ? 1.0f / l : 0.f;
+        }
+        __nv_bfloat16* orow = a.out + (long)qrow * a.ldo + (long)h * FD;
+        const float4* parts = a.part + ((long)pair * a.splits * 2 + x) * PART + r;
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          uint32_t v[32];
+          tmem_ld32(tO + c * 32, v);
+          tmem_ld_wait();
+          float o[32];
+          if (a.splits > 1) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) o[i] = 0.f;
+#pragma unroll 1
+            for (int sp = 0; sp < a.splits; ++sp) {
+              float ws = w[0];
+#pragma unroll
+              for (int k = 1; k < kMaxSplits; ++k) ws = sp == k ? w[k] : ws;
+              if (sp == split) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) o[i] = fmaf(__uint_as_float(v[i]), ws, o[i]);
+              } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                  const float4 q = __ldcg(parts + (long)sp * 2 * PART + (c * 8 + i) * FQ);
+                  o[4 * i] = fmaf(q.x, ws, o[4 * i]); o[4 * i + 1] = fmaf(q.y, ws, o[4 * i + 1]);
+                  o[4 * i + 2] = fmaf(q.z, ws, o[4 * i + 2]); o[4 * i + 3] = fmaf(q.w, ws, o[4 * i + 3]);
+                }
+              }
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) o[i] = __uint_as_float(v[i]) * w[0];
+          }
+          if (qrow < a.T) {
+#pragma unroll
+            for (int i = 0; i < 32; i += 8)
+              *reinterpret_cast<uint4*>(orow + c * 32 + i) = make_uint4(pack_bf16(o[i], o[i + 1]), pack_bf16(o[i + 2], o[i + 3]),
+                                                                        pack_bf16(o[i + 4], o[i + 5]), pack_bf16(o[i + 6], o[i + 7]));
           }
         }
       }
@@ -292,8 +376,13 @@ extern "C" {
 // Causal attention of T query rows per head (positions pos0 .. pos0 + T - 1) over keys 0 .. pos0 + T - 1.
 //   q  bf16 [n_q][T][128]   k  bf16 [n_kv][t_pad][128]   vt  bf16 [n_kv][128][t_pad]   out  bf16 [T][ldo >= n_q * 128]
 // t_pad is a multiple of 128 that covers the keys; value columns past the last key must be finite (zero).
-int bl_flash_prefill(const void* q, const void* k, const void* vt, void* out, long ldo, int T, int n_q, int n_kv, int pos0,
-                     int t_pad, unsigned* status, cudaStream_t st) {
+// splits > 1 (up to 4; pos0 + 1 > 128 * splits, so that no share is empty): part holds 2 * pairs * splits * 16,384 floats,
+// part_ml 2 * pairs * splits * 256, tickets 8 * pairs zeroed words, with pairs = n_kv * ceil(ceil(T / 128) * (n_q / n_kv) / 2); all
+// of one stream at a time.
+int bl_flash_prefill_split(const void* q, const void* k, const void* vt, void* out, long ldo, int T, int n_q, int n_kv, int pos0,
+                           int t_pad, unsigned* status, int splits, float* part, float* part_ml, int* tickets, cudaStream_t st) {
+  BL_REQUIRE(splits >= 1 && splits <= kMaxSplits && (splits == 1 || (pos0 >= 128 * splits && part && part_ml && tickets)), BL_ERR_SHAPE);
+  BL_REQUIRE(((uintptr_t)part & 15) == 0 && ((uintptr_t)part_ml & 7) == 0, BL_ERR_ALIGN);
   BL_REQUIRE(T >= 1 && n_q >= 1 && n_kv >= 1 && n_q % n_kv == 0 && pos0 >= 0, BL_ERR_SHAPE);
   BL_REQUIRE(t_pad % 128 == 0 && t_pad >= pos0 + T && ldo >= (long)n_q * FD && ldo % 8 == 0, BL_ERR_SHAPE);
   BL_REQUIRE((((uintptr_t)q | (uintptr_t)k | (uintptr_t)vt | (uintptr_t)out) & 15) == 0, BL_ERR_ALIGN);
@@ -319,15 +408,21 @@ int bl_flash_prefill(const void* q, const void* k, const void* vt, void* out, lo
     int rc = make_map(&mv, vt, 2, dims, strides, box);
     if (rc) return rc;
   }
-  FlashPrefillArgs a{T, n_q, n_kv, n_q / n_kv, pos0, t_pad, (__nv_bfloat16*)out, ldo, status};
+  FlashPrefillArgs a{T, n_q, n_kv, n_q / n_kv, pos0, t_pad, (__nv_bfloat16*)out, ldo, status,
+                     splits, (float4*)part, (float2*)part_ml, tickets};
   static bool attr_set = false;
   if (!attr_set) {
     cudaFuncSetAttribute(flash_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FSMEM);
     attr_set = true;
   }
   const int items = (T + FQ - 1) / FQ * (n_q / n_kv);           // query tiles of a KV head
-  dim3 grid((unsigned)((items + 1) / 2 * n_kv));
+  dim3 grid((unsigned)((items + 1) / 2 * n_kv * splits));
   return (int)launch(flash_prefill_kernel, grid, dim3(FTHREADS), (size_t)FSMEM, st, mq, mk, mv, a);
+}
+
+int bl_flash_prefill(const void* q, const void* k, const void* vt, void* out, long ldo, int T, int n_q, int n_kv, int pos0,
+                     int t_pad, unsigned* status, cudaStream_t st) {
+  return bl_flash_prefill_split(q, k, vt, out, ldo, T, n_q, n_kv, pos0, t_pad, status, 1, nullptr, nullptr, nullptr, st);
 }
 
 }  // extern "C"

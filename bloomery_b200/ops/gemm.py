@@ -201,16 +201,48 @@ def kv_gather_bf16(k_cache, v_cache, block_table_row, n_pages: int, n_kv: int, h
                                    I(T_pad), p(Kb), p(Vt), stream()), "bl_kv_gather_bf16")
 
 
+class FlashWork:
+    """Partial outputs and tickets of prompt attention whose CTAs share their keys: one per stream that runs it."""
+
+    def __init__(self, device):
+        self.device = device
+        self.part = self.part_ml = self.tickets = None
+
+    def buffers(self, pairs: int, splits: int):
+        n = 2 * pairs * splits
+        if self.part is None or self.part.numel() < n * 16384:
+            self.part = torch.empty(n * 16384, dtype=torch.float32, device=self.device)
+            self.part_ml = torch.empty(n * 256, dtype=torch.float32, device=self.device)
+        if self.tickets is None or self.tickets.numel() < 8 * pairs:
+            self.tickets = torch.zeros(8 * pairs, dtype=torch.int32, device=self.device)
+        return self.part, self.part_ml, self.tickets
+
+
+def flash_splits(pairs: int, key_tiles: int, sm: int) -> int:
+    """CTAs that share the key tiles of a pair of query tiles: the number that ends first, counted in key tiles of a CTA times
+    waves of CTAs.  A share costs about four key tiles on top (its start, its partial output and the merge), so it has to
+    hold sixteen."""
+    cost = lambda s: -(-pairs * s // sm) * (-(-key_tiles // s) + (4 if s > 1 else 0))      # noqa: E731
+    return min((s for s in range(1, 5) if s == 1 or key_tiles >= 16 * s), key=cost)
+
+
 def flash_prefill(q_bf: torch.Tensor, Kb: torch.Tensor, Vt: torch.Tensor, out: torch.Tensor, pos0: int,
-                  status: Optional[torch.Tensor] = None) -> None:
+                  status: Optional[torch.Tensor] = None, work: Optional[FlashWork] = None) -> None:
     """Causal attention of a prompt chunk on tcgen05 tiles (``csrc/flash_tcgen05.cu``): queries bf16 [n_q, T, 128]
     (normalised, rotated, pre-scaled) at positions pos0.., keys bf16 [n_kv, T_pad, 128], values transposed bf16
-    [n_kv, 128, T_pad] (columns past the last key zero), output bf16 [T, n_q * 128]."""
+    [n_kv, 128, T_pad] (columns past the last key zero), output bf16 [T, n_q * 128].  With ``work`` the key tiles of few query
+    tiles behind a long prefix are shared by several CTAs."""
     n_q, T, hd = q_bf.shape
     n_kv, T_pad, _ = Kb.shape
     assert hd == 128 and Vt.shape == (n_kv, 128, T_pad) and q_bf.is_contiguous() and Kb.is_contiguous() and Vt.is_contiguous()
-    rc = cuda().bl_flash_prefill(p(q_bf), p(Kb), p(Vt), p(out), L(out.stride(0)), I(T), I(n_q), I(n_kv), I(pos0), I(T_pad),
-                                 p(status), stream())
+    splits, bufs = 1, (None, None, None)
+    if work is not None:
+        pairs = n_kv * (((T + 127) // 128 * (n_q // n_kv) + 1) // 2)
+        splits = flash_splits(pairs, (pos0 + 127) // 128, sm_count())
+        if splits > 1:
+            bufs = work.buffers(pairs, splits)
+    rc = cuda().bl_flash_prefill_split(p(q_bf), p(Kb), p(Vt), p(out), L(out.stride(0)), I(T), I(n_q), I(n_kv), I(pos0), I(T_pad),
+                                       p(status), I(splits), p(bufs[0]), p(bufs[1]), p(bufs[2]), stream())
     check(rc, "bl_flash_prefill")
 
 

@@ -73,6 +73,7 @@ class GemmPrefill:
         self.direct_rows = 128
         self._direct_ok = None
         self._work = None
+        self._flash_work = G.FlashWork(engine.device)
 
     def _get(self, name: str, shape, dtype) -> torch.Tensor:
         n = 1
@@ -282,7 +283,7 @@ class GemmPrefill:
                 self.timing.mark(il, "qkv")
                 if s.head_dim == 128 and self.flash:
                     # scores, softmax and values in one tcgen05 launch: the score matrix stays in tensor memory
-                    G.flash_prefill(q_bf, Kb, Vt, attn, p0, st)
+                    G.flash_prefill(q_bf, Kb, Vt, attn, p0, st, self._flash_work)
                     self.timing.mark(il, "flash")
                 for c0 in range(0, T if not (s.head_dim == 128 and self.flash) else 0, Tq_max):
                     Tq = min(Tq_max, T - c0)
@@ -360,6 +361,7 @@ class GemmPrefill:
             main.wait_stream(side)
         e.x[0].copy_(x[T - 1])
         if int(st.item()) != 0:
+            self._flash_work = G.FlashWork(dev)             # its tickets may not be back at zero
             raise RuntimeError("a bounded wait inside the GEMM kernel ran out (status word set)")
 
     def _direct(self, T: int, short: bool = False) -> bool:

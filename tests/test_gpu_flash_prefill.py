@@ -103,3 +103,30 @@ def test_query_tiles_that_pair_across_positions(n_q, n_kv, T, pos0):
     """An odd number of heads a KV head pairs the last tile of one position with the first of the one before it, whose keys end
     earlier, and may leave a tile alone."""
     test_flash_prefill_matches_fp32_attention(n_q, n_kv, T, pos0)
+
+
+@pytest.mark.parametrize("splits", [2, 3, 4])
+@pytest.mark.parametrize("n_q,n_kv,T,pos0", [(8, 2, 130, 512), (3, 1, 129, 1000), (5, 1, 1, 2048), (32, 4, 300, 3001)])
+def test_query_tiles_whose_keys_are_shared(n_q, n_kv, T, pos0, splits, monkeypatch):
+    """Shares of unequal length, a last share that some rows only see masked keys of, an odd tile that stays alone: the same
+    rows as without shares to the rounding of one bf16 output, and the same bits on every run whoever arrives last."""
+    from bloomery_b200.ops import gemm as G
+    g = torch.Generator(device=DEV).manual_seed(T + splits)
+    n_keys = pos0 + T
+    t_pad = (n_keys + 127) // 128 * 128
+    q = (torch.randn(n_q, T, 128, device=DEV, generator=g) / 128 ** 0.5).bfloat16()
+    k, v = (torch.randn(n_kv, n_keys, 128, device=DEV, generator=g).bfloat16() for _ in range(2))
+    k[:, n_keys // 3] *= 8                                        # a maximum that only one share holds
+    Kb, Vt = torch.zeros(n_kv, t_pad, 128, device=DEV, dtype=torch.bfloat16), torch.zeros(n_kv, 128, t_pad, device=DEV, dtype=torch.bfloat16)
+    Kb[:, :n_keys], Vt[:, :, :n_keys] = k, v.transpose(1, 2)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    work = G.FlashWork(DEV)
+    monkeypatch.setattr(G, "flash_splits", lambda *a: splits)
+    outs = torch.full((30, T, n_q * 128), float("nan"), device=DEV, dtype=torch.bfloat16)
+    for out in outs:
+        G.flash_prefill(q, Kb, Vt, out, pos0, status, work)
+    torch.cuda.synchronize()
+    assert int(status) == 0 and int(work.tickets.abs().sum()) == 0
+    assert [i for i, out in enumerate(outs) if not torch.equal(out, outs[0])] == []
+    ref = _ref(q, k, v, pos0).permute(1, 0, 2).reshape(T, n_q * 128)
+    assert float((outs[0].float() - ref).norm() / ref.norm()) < 2 ** -7          # as without shares
