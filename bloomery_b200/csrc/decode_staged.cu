@@ -170,6 +170,7 @@ struct AttnArgs {
   unsigned* fault; int layer;
   long long* probe;
   int recv_off;                            // cluster form: float offset of the merge buffer in dynamic shared memory
+  int seg_budget;                          // attn_fused: (row, segment) pairs of a KV head that fill the processors once
 };
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
@@ -237,7 +238,12 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
   const bool pad = seq < 0;
   const bool bad = !pad && (n_keys <= 0 || n_keys > a.ctx_limit);
   const int n_tiles = (pad || bad) ? 0 : (n_keys + kKeyTile - 1) / kKeyTile;
-  const int tps = max(1, (n_tiles + a.n_seg - 1) / a.n_seg);
+  // One block fits a processor, so the rows that live share the processors: segments of several rows beyond that would only
+  // queue, each with its own start (five rows of 1,500 keys in the bucket of eight: 480 blocks in 36 us a layer, 140 in 12).
+  int live = 0;
+  for (int mm = 0; mm < a.M; ++mm) live += a.row_seq[mm] >= 0 ? 1 : 0;
+  const int segs = min((int)gridDim.x, max(1, a.seg_budget / max(1, live)));
+  const int tps = max(1, (n_tiles + segs - 1) / segs);
   const int used = (n_tiles + tps - 1) / tps;
   const int t0 = seg * tps, t1 = min(n_tiles, t0 + tps);
   if (pad || bad) {
@@ -1306,12 +1312,19 @@ int bl_attn_fused(const float* qkv, long qkv_stride, const float* q_gain, const 
   const int G = n_q / n_kv;
   AttnArgs a{qkv, qkv_stride, q_gain, k_gain, inv_freq, eps, q_scale, n_q, n_kv, M, n_seg, ctx_limit, row_pos, row_seq,
              block_table, max_pages, n_pages, (__half*)k_cache, (__half*)v_cache, part_ml, part_acc, tickets, out, outq,
-             (float2*)outds, fault, layer, g_stage_probe, 0};
-  dim3 grid(n_seg, n_kv, M);
+             (float2*)outds, fault, layer, g_stage_probe, 0, 0};
   const int n_patch = M < kMaxPatch ? M : kMaxPatch;
   const size_t rings = G <= 8 ? (size_t)8 * kWfStages * (head == 128 ? WarpFlash<128>::kStageBytes : WarpFlash<64>::kStageBytes)
                               : (size_t)kStages * kKeyTile * (head + 8) * 2 + kStages * kKeyTile * head * 2;
   const size_t smem = (size_t)G * head * 4 + rings + (size_t)n_patch * 2 * head * 2;
+  // segments of the rows that live: as many blocks as the processors hold at once.  A bucket of M rows holds more than M / 2.
+  int dev = 0, sm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return BL_ERR_LIMIT;
+  const int resident = (int)(227 * 1024 / (smem + 2048));
+  a.seg_budget = M == 1 ? n_seg : sm * (resident < 1 ? 1 : resident > 2 ? 2 : resident) / n_kv;
+  const int most = a.seg_budget / (M / 2 + 1);
+  dim3 grid(M == 1 || most >= n_seg ? n_seg : most < 1 ? 1 : most, n_kv, M);
   static bool attr_set = false;
   if (!attr_set) {
     cudaFuncSetAttribute(attn_fused_kernel<128, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 180 * 1024);

@@ -361,3 +361,41 @@ def test_engine_tokens_do_not_depend_on_the_kernel_form():
         first = eng.prefill(0, prompt, gemm=False)
         toks.append([first] + eng.decode_chain(0, first, len(prompt), 24))
     assert toks[0] == toks[1]
+
+
+@pytest.mark.parametrize("head,n_q,n_kv", [(128, 32, 4), (64, 14, 2), (128, 48, 4)])
+@pytest.mark.parametrize("pos,dead", [([0, 700], []), ([1023, 5, 64], [1]), ([31, 32, 500, 900, 63, 0, 0, 0], [5, 6, 7]),
+                                      ([10, 900, 450, 33, 1, 31, 64, 800], [])])
+def test_attn_fused_rows_share_the_processors(head, n_q, n_kv, pos, dead):
+    """Fewer segments a row the more rows live: rows of one key up to a thousand, dead rows that count for nothing, against
+    softmax attention in 64 bits over the cache as the launch leaves it."""
+    from bloomery_b200.ops import decode as K
+    g = torch.Generator(device=DEV).manual_seed(head + len(pos))
+    M, ctx, n_seg = len(pos), 1024, 37
+    pages, n_pages = ctx // 64, M * (ctx // 64)
+    qkv = torch.randn(M, (n_q + 2 * n_kv) * head, device=DEV, generator=g)
+    inv = torch.zeros(head // 2, device=DEV)                       # angle 0: rows enter as they are
+    kc, vc = (torch.randn(n_pages, n_kv, 64, head, device=DEV, generator=g).half() for _ in range(2))
+    table = torch.arange(n_pages, dtype=torch.int32, device=DEV).view(M, pages)
+    rp = torch.tensor(pos, dtype=torch.int32, device=DEV)
+    rs = torch.tensor([-1 if m in dead else m for m in range(M)], dtype=torch.int32, device=DEV)
+    ml, acc = torch.zeros(M * n_q * n_seg * 2, device=DEV), torch.zeros(M * n_q * n_seg * head, device=DEV)
+    tickets, fault = torch.zeros(M * n_kv, dtype=torch.int32, device=DEV), torch.full((1,), -1, dtype=torch.int32, device=DEV)
+    out = torch.full((M, n_q * head), float("nan"), device=DEV)
+    outq, outds = torch.zeros(M, n_q * head, dtype=torch.int8, device=DEV), torch.zeros(M, n_q * head // 32, 2, device=DEV)
+    K.attn_fused(qkv, None, None, inv, 1e-6, head ** -0.5, head, n_q, n_kv, M, rp, rs, table, n_pages, kc, vc, n_seg, ctx, ml, acc,
+                 tickets, out, outq, outds, fault, 0)
+    torch.cuda.synchronize()
+    assert int(fault) == -1 and int(tickets.abs().sum()) == 0
+    for m in range(M):
+        if m in dead:
+            assert bool((out[m] == 0).all())
+            continue
+        L = pos[m] + 1
+        q = qkv[m, :n_q * head].view(n_q, head).double() * head ** -0.5
+        k, v = (c[table[m].long()].transpose(0, 1).reshape(n_kv, ctx, head)[:, :L].double() for c in (kc, vc))
+        assert torch.equal(k[:, -1].float(), qkv[m, n_q * head:(n_q + n_kv) * head].view(n_kv, head).half().float())
+        k, v = (t.repeat_interleave(n_q // n_kv, 0) for t in (k, v))
+        ref = torch.einsum("hk,hkd->hd", torch.softmax(torch.einsum("hd,hkd->hk", q, k), -1), v).reshape(-1)
+        # operands split into 22 bits, exponentials and sums in fp32
+        assert float((out[m].double() - ref).abs().max()) < 2e-4
