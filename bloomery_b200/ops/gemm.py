@@ -289,11 +289,12 @@ def qgemm_splits(n_tiles: int, depth_blocks: int, sm: int) -> int:
 def qgemm(X: torch.Tensor, W: QWeight, tiles: TileTable, *, out_f32: Optional[torch.Tensor] = None,
           out_bf16: Optional[torch.Tensor] = None, W2: Optional[QWeight] = None, dst_row=None, row_scale=None,
           resid=None, status: Optional[torch.Tensor] = None, work: Optional[QgemmWork] = None,
-          exact: bool = False, fine: bool = False) -> None:
+          exact: bool = False, fine: bool = False, room: int = 0) -> None:
     """C = X @ W[g].T per token tile with W left block-quantised (``csrc/qgemm_tcgen05.cu``): X [rows, K] bf16, W (and
     W2) resident Q4_K / Q5_K / Q6_K / Q8_0 / FP8_B128 / NVFP4 / Q8_F32 matrices [N, bytes] or stacks [G, N, bytes]; tiles of
     32, 64 or 128 token rows.
-    With W2 the output is silu(X W^T) * (X W2^T).  With ``work`` a product of few tiles splits its depth over CTAs.
+    With W2 the output is silu(X W^T) * (X W2^T).  With ``work`` a product of few tiles splits its depth over CTAs, as many as
+    ``room`` processors hold (0: all of them).
     ``exact``: weights are rounded to bf16 once from their fp32 values in tiles of 32 and 64 rows too.  ``fine``: they enter as
     a bf16 value and a bf16 remainder, 16 bits together (tiles of 32 rows, with one matrix of 64 too)."""
     assert X.dtype == torch.bfloat16 and X.stride(-1) == 1 and W.data.is_contiguous() and tiles.tile_rows in (32, 64, 128)
@@ -304,7 +305,7 @@ def qgemm(X: torch.Tensor, W: QWeight, tiles: TileTable, *, out_f32: Optional[to
     sm = sm_count()
     splits = 1
     if work is not None and tiles.fixed and W2 is None and tiles.tile_rows <= work.tile_rows:
-        splits = qgemm_splits(tiles.fixed * ((N + 127) // 128), W.k // 256, sm)
+        splits = qgemm_splits(tiles.fixed * ((N + 127) // 128), W.k // 256, min(room, sm) if room else sm)
     rc = cuda().bl_qgemm_split(p(X), L(X.stride(0)), L(X.shape[0]), p(W.data), p(W2.data if W2 is not None else None), I(W.wt),
                                I(G), I(N), I(W.k), p(tiles.mtiles), p(tiles.n_mtiles), I(tiles.fixed or tiles.max_mtiles),
                                I(tiles.tile_rows), p(out_f32), p(out_bf16), L(out.stride(0)), p(dst_row), p(row_scale),

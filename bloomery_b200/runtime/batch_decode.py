@@ -149,11 +149,12 @@ class BatchDecode:
     def _native_fp8(self, Wq) -> bool:
         return self.fp8_native and Wq.qtype == "FP8_B128" and Wq.k % 128 == 0
 
-    def _mm(self, X, Wq, tiles, M, x8=None, W2=None, branch=0, **kw):
+    def _mm(self, X, Wq, tiles, M, x8=None, W2=None, branch=0, room=0, **kw):
         """X [rows, K] bf16 times a resident matrix (or, with W2, the SwiGLU pair): FP8 weights against E4M3 rows on the
         tensor cores, other quantised types expanded in flight, the rest through a bf16 expansion launch.  ``x8``: the
         rows' E4M3 form when the caller already made it (several products of one input).  ``branch``: 0 on the pass's own
-        stream, 1 / 2 on its side streams.  Returns the launch count."""
+        stream, 1 / 2 on its side streams; ``room``: processors that a split product may take (0: all).  Returns the launch
+        count."""
         if self._native_fp8(Wq):
             n = 0
             if x8 is None:
@@ -163,7 +164,7 @@ class BatchDecode:
             G.fp8_gemm(x8[0], x8[1], Wq, tiles, W2=W2, status=self.status, **kw)
             return n + 1
         if G.qgemm_supports(Wq):
-            G.qgemm(X, Wq, tiles, W2=W2, status=self.status, work=self._work[branch], **kw)
+            G.qgemm(X, Wq, tiles, W2=W2, status=self.status, work=self._work[branch], room=room, **kw)
             return 1
         if Wq.qtype == "BF16":
             # bf16 rows need no expansion: the bf16 GEMM reads them in place (token tiles of 128 rows)
@@ -275,8 +276,11 @@ class BatchDecode:
         q_scale = 1.0 / math.sqrt(s.head_dim)
         n = 0
         # the three projections are small grids (32 + 4 + 4 weight tiles on the 30 B shape): K and V run on side
-        # streams beside Q (parallel branches of the captured graph)
+        # streams beside Q (parallel branches of the captured graph).  One CTA fits a processor: Q splits its depth over
+        # half of them and K and V over a quarter each, so that none of the three waits for another to end (Q over all of
+        # them, K and V behind it: 36 us a layer of a round of 24)
         main = torch.cuda.current_stream(e.device)
+        sm = K.sm_count(e.device)
         x8 = None
         if any(self._native_fp8(w.q[b + nm]) for nm in ("attn_q.weight", "attn_k.weight", "attn_v.weight")):
             x8 = self._q8(xn); n += 1                            # one E4M3 form of the rows for the three products
@@ -288,11 +292,11 @@ class BatchDecode:
             side = self._side[branch - 1]
             side.wait_event(fork)
             with torch.cuda.stream(side):
-                n += self._mm(xn, w.q[b + name], tiles, M, x8=x8, branch=branch, out_f32=self.qkv[:M, lo:hi])
+                n += self._mm(xn, w.q[b + name], tiles, M, x8=x8, branch=branch, room=sm // 4, out_f32=self.qkv[:M, lo:hi])
                 ev = torch.cuda.Event()
                 ev.record(side)
                 joins.append(ev)
-        n += self._mm(xn, w.q[b + "attn_q.weight"], tiles, M, x8=x8, out_f32=self.qkv[:M, :s.q_rows])
+        n += self._mm(xn, w.q[b + "attn_q.weight"], tiles, M, x8=x8, room=sm // 2, out_f32=self.qkv[:M, :s.q_rows])
         for ev in joins:
             main.wait_event(ev)
         kvp = e.kv
