@@ -188,6 +188,128 @@ __device__ __forceinline__ uint4 short8(uint32_t w0, uint32_t w1, uint32_t s2, u
   return out;
 }
 
+// ---- slabs: the short form of the super-block types ------------------------------------------
+// A slab is 64 consecutive values.  Slab<T>::Regs holds a row's 128 values of a stage (slabs i and i + 1 of its super-block
+// `sb`, i even) with their scales; codes() yields the x-th one's 64 code bytes in value order (16 words) and the (scale,
+// offset) pair of each of its four groups of 16.  The packed scales are taken apart four at a time, and a byte becomes a float
+// as the low mantissa byte of 2^23: half of an expander's integer instructions were those of its scales.
+template <class T> struct Slab;
+
+// byte `SEL` of w as a float, less `bias`
+template <int SEL>
+__device__ __forceinline__ float byte_float(uint32_t w, float bias = 8388608.0f) {
+  return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 + SEL)) - bias;
+}
+// scales and offsets of slab i: sub-blocks 2i and 2i + 1 of the eight 6-bit (scale, min) pairs of Q4_K and Q5_K
+__device__ __forceinline__ void k_scales(const u32x4& hdr, int i, float* s, float* o) {
+  uint32_t sw, mw;
+  if (i < 2) {
+    sw = hdr.y & 0x3F3F3F3Fu;
+    mw = hdr.z & 0x3F3F3F3Fu;
+  } else {
+    sw = (hdr.w & 0x0F0F0F0Fu) | ((hdr.y >> 2) & 0x30303030u);
+    mw = ((hdr.w >> 4) & 0x0F0F0F0Fu) | ((hdr.z >> 2) & 0x30303030u);
+  }
+  sw >>= 16 * (i & 1);
+  mw >>= 16 * (i & 1);
+  const float d = half_bits_to_float((uint16_t)(hdr.x & 0xFFFF)), dmin = half_bits_to_float((uint16_t)(hdr.x >> 16));
+  s[0] = s[1] = d * byte_float<0>(sw); o[0] = o[1] = -(dmin * byte_float<0>(mw));
+  s[2] = s[3] = d * byte_float<1>(sw); o[2] = o[3] = -(dmin * byte_float<1>(mw));
+}
+
+template <> struct Slab<Q4K> {
+  static constexpr bool kHas = true;
+  struct Regs { u32x4 hdr, q[4]; };
+  static __device__ __forceinline__ void load(const uint8_t* sb, int i, Regs& r) {
+    r.hdr = ld128(sb);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) r.q[x] = ld128(sb + 16 + 32 * i + 16 * x);
+  }
+  static __device__ __forceinline__ void codes(const Regs& r, int x, int i, uint32_t* cw, float* s, float* o) {
+    const u32x4 &a = r.q[2 * x], &b = r.q[2 * x + 1];
+    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int k = 0; k < 8; ++k) { cw[k] = w[k] & 0x0F0F0F0Fu; cw[8 + k] = (w[k] >> 4) & 0x0F0F0F0Fu; }
+    k_scales(r.hdr, i, s, o);
+  }
+};
+template <> struct Slab<Q5K> {
+  static constexpr bool kHas = true;
+  struct Regs { u32x4 hdr, h[2], q[4]; };
+  static __device__ __forceinline__ void load(const uint8_t* sb, int i, Regs& r) {
+    r.hdr = ld128(sb);
+    r.h[0] = ld128(sb + 16);
+    r.h[1] = ld128(sb + 32);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) r.q[x] = ld128(sb + 48 + 32 * i + 16 * x);
+  }
+  static __device__ __forceinline__ void codes(const Regs& r, int x, int i, uint32_t* cw, float* s, float* o) {
+    const u32x4 &a = r.q[2 * x], &b = r.q[2 * x + 1];
+    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    const uint32_t h[8] = {r.h[0].x, r.h[0].y, r.h[0].z, r.h[0].w, r.h[1].x, r.h[1].y, r.h[1].z, r.h[1].w};
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t hb = h[k] >> (2 * i);
+      cw[k] = (w[k] & 0x0F0F0F0Fu) | ((hb & 0x01010101u) << 4);
+      cw[8 + k] = ((w[k] >> 4) & 0x0F0F0F0Fu) | ((hb & 0x02020202u) << 3);
+    }
+    k_scales(r.hdr, i, s, o);
+  }
+};
+// Both slabs of a half super-block read the same bytes: the even one their low nibbles, the odd one the high ones.
+template <> struct Slab<Q6K> {
+  static constexpr bool kHas = true;
+  struct Regs { u32x4 l[4], h[2]; uint32_t sc[2], d; };
+  static __device__ __forceinline__ void load(const uint8_t* sb, int i, Regs& r) {
+    const uint8_t* p = sb + 64 * (i >> 1);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) r.l[x] = ld128(p + 16 * x);
+#pragma unroll
+    for (int x = 0; x < 2; ++x) r.h[x] = ld128(sb + 128 + 32 * (i >> 1) + 16 * x);
+#pragma unroll
+    for (int x = 0; x < 2; ++x) r.sc[x] = ld32(sb + 192 + 4 * (i + x));
+    r.d = ld32(sb + 208);
+  }
+  static __device__ __forceinline__ void codes(const Regs& r, int x, int i, uint32_t* cw, float* s, float* o) {
+    const int sh = 4 * x;
+    const uint32_t h[8] = {r.h[0].x, r.h[0].y, r.h[0].z, r.h[0].w, r.h[1].x, r.h[1].y, r.h[1].z, r.h[1].w};
+    const uint32_t w[16] = {r.l[0].x, r.l[0].y, r.l[0].z, r.l[0].w, r.l[1].x, r.l[1].y, r.l[1].z, r.l[1].w,
+                            r.l[2].x, r.l[2].y, r.l[2].z, r.l[2].w, r.l[3].x, r.l[3].y, r.l[3].z, r.l[3].w};
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t hb = h[k] >> sh;
+      cw[k] = ((w[k] >> sh) & 0x0F0F0F0Fu) | ((hb & 0x03030303u) << 4);
+      cw[8 + k] = ((w[8 + k] >> sh) & 0x0F0F0F0Fu) | ((hb & 0x0C0C0C0Cu) << 2);
+    }
+    const float d = half_bits_to_float((uint16_t)(r.d & 0xFFFF));
+    const uint32_t sc = r.sc[x] ^ 0x80808080u;                      // signed bytes, 128 up
+    s[0] = d * byte_float<0>(sc, 8388736.0f); s[1] = d * byte_float<1>(sc, 8388736.0f);
+    s[2] = d * byte_float<2>(sc, 8388736.0f); s[3] = d * byte_float<3>(sc, 8388736.0f);
+#pragma unroll
+    for (int g = 0; g < 4; ++g) o[g] = -32.0f * s[g];
+  }
+};
+
+// Slab x of `regs` into columns ta .. ta + 31.  `ready` waits for the stage behind the arithmetic, in front of the store.
+template <class T, class Ready>
+__device__ __forceinline__ bool expand_slab(const typename Slab<T>::Regs& regs, int x, int i, uint32_t ta, Ready ready) {
+  uint32_t cw[16], v[32];
+  float s[4], o[4];
+  Slab<T>::codes(regs, x, i + x, cw, s, o);
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    const uint32_t s2 = bf2_dup(s[g]), o2 = bf2_dup(o[g]);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint4 q = short8(cw[4 * g + 2 * h], cw[4 * g + 2 * h + 1], s2, o2);
+      v[8 * g + 4 * h] = q.x; v[8 * g + 4 * h + 1] = q.y; v[8 * g + 4 * h + 2] = q.z; v[8 * g + 4 * h + 3] = q.w;
+    }
+  }
+  if (!ready()) return false;
+  tmem_st32(ta, v);
+  return true;
+}
+
 // ---- float-coded types ---------------------------------------------------------------------
 // ChunkUnit<T>::values(regs, pre, j) yields values 8j .. 8j+7 of the unit, never holding the unit's 64 floats.
 //   FP8 (E4M3 codes, one f32 scale per 128 values): the hardware converter takes two codes to an f16 pair; the pair
@@ -281,16 +403,11 @@ __device__ __forceinline__ void expand_unit(const typename Unit<T>::Regs& regs, 
     FastUnit<T>::codes(regs, u, cw, s, o);
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
-      if constexpr (FORM == Q_SHORT) {
-        const uint32_t s2 = bf2_dup(s[g]), o2 = bf2_dup(o[g]);
-        tmem_st8(ta + col(g), short8(cw[4 * g], cw[4 * g + 1], s2, o2), short8(cw[4 * g + 2], cw[4 * g + 3], s2, o2));
-      } else {
-        const float a = 128.0f * s[g], c = o[g] - a;
-        float v[16];
-        fast8(cw[4 * g], cw[4 * g + 1], a, c, v);
-        fast8(cw[4 * g + 2], cw[4 * g + 3], a, c, v + 8);
-        put(g, v);
-      }
+      const float a = 128.0f * s[g], c = o[g] - a;
+      float v[16];
+      fast8(cw[4 * g], cw[4 * g + 1], a, c, v);
+      fast8(cw[4 * g + 2], cw[4 * g + 3], a, c, v + 8);
+      put(g, v);
     }
   } else if constexpr (ChunkUnit<T>::kHas) {
     using C = ChunkUnit<T>;
@@ -351,7 +468,9 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
   constexpr int A_MAT = QBK / 2;                                     // columns of one matrix's stage
   constexpr int A_COLS = (DUAL ? 2 : 1) * A_MAT;
   constexpr int HALVES = FORM == Q_SPLIT ? 2 : 1;                    // stages that hold one 128-deep block of weights
-  constexpr int FILLERS = DUAL ? QPRODUCERS / 32 : QPRODUCERS / 64;  // warps that write one stage
+  constexpr bool SLABS = RS > 0 && FORM == Q_SHORT;                  // a group of four warps fills a matrix's stage alone
+  constexpr int FILLERS = (DUAL ? 2 : 1) * (SLABS ? 4 : 8);          // warps that write one stage
+  constexpr int READERS = SLABS && !DUAL ? 8 : 16;                   // warps that read a raw slot
   __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
   __shared__ __align__(8) uint64_t raw_full[RS > 0 ? RS : 1], raw_empty[RS > 0 ? RS : 1];
   __shared__ uint32_t s_tmem_base;
@@ -363,7 +482,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1 + FILLERS); mbar_init(&empty_bar[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4); }
-    for (int r = 0; r < RS; ++r) { mbar_init(&raw_full[r], 1); mbar_init(&raw_empty[r], QPRODUCERS / 32); }
+    for (int r = 0; r < RS; ++r) { mbar_init(&raw_full[r], 1); mbar_init(&raw_empty[r], READERS); }
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -553,6 +672,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
   } else if (warp >= 8) {
     // Four groups of four warps, one per TMEM lane quarter: thread = weight row.  Gate+up: every group expands one unit
     // (matrix grp / 2, unit grp % 2) of every stage; one matrix: groups 0 and 1 the even stages, 2 and 3 the odd ones.
+    // Slabs: a group fills whole stages, gate+up: groups 2m and 2m + 1 the even and odd stages of matrix m; one matrix: stage n by
+    // group n % 4.
     using U = Unit<T>;
     constexpr int STEP = DUAL ? 1 : 2;                               // stages from one item of a group to its next
     const int grp = (warp - 8) >> 2, q = warp & 3;
@@ -578,7 +699,52 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
         if (HALVES == 2) mbar_arrive(&full_bar[next]);
       }
     };
-    if constexpr (RS > 0) {
+    if constexpr (SLABS) {
+      // The hand-over of a stage (its stores must have landed) waits until the next values are read, which covers the stores'
+      // latency.  It cannot lock the rings: a raw slot that this warp waits for is held up by a warp whose own stage is older
+      // than the one kept back here, and stages are used in order.
+      constexpr int NG = DUAL ? 2 : 4;                               // groups that share a matrix's stages, two a super-block
+      static_assert(NG <= STAGES, "a group's next stage lies at most one turn of the ring ahead");
+      const int mine = DUAL ? half : grp;
+      int rslot = 0, stage = mine, turn = 0, pending = -1;           // stage: this group's next one
+      uint32_t rphase = 0, phase = 0;
+      auto hand_over = [&]() {
+        if (pending < 0) return;
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full_bar[pending]);
+        pending = -1;
+      };
+      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+        for (int sbi = 0; sbi < kblocks / 2 && ok; ++sbi) {
+          const bool take = DUAL || turn == (mine >> 1);             // one matrix: the pairs of groups take super-blocks in turns
+          turn ^= 1;
+          if (take) {
+            ok = mbar_wait_warp(&raw_full[rslot], rphase, abort_flag);
+            if (!ok) break;
+            typename Slab<T>::Regs r;
+            Slab<T>::load(raw_ring + (size_t)rslot * RAW_SLOT + mat * RAW_MAT + row * SB, 2 * (mine & 1), r);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&raw_empty[rslot]);
+            hand_over();
+            auto ready = [&]() {
+              ok = mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag);
+              if (ok) tc_fence_after();
+              return ok;
+            };
+            const uint32_t ta = ta0 + stage * A_COLS;
+            if (!expand_slab<T>(r, 0, 2 * (mine & 1), ta, ready)) break;
+            expand_slab<T>(r, 1, 2 * (mine & 1), ta + 32, [] { return true; });
+            pending = stage;
+            stage += NG;
+            if (stage >= STAGES) { stage -= STAGES; phase ^= 1; }
+          }
+          if (++rslot == RS) { rslot = 0; rphase ^= 1; }
+        }
+      }
+      if (ok) hand_over();
+    } else if constexpr (RS > 0) {
       // raw ring: the tile's super-blocks arrive by TMA; a thread reads its row's units out of shared memory
       int rslot = 0; uint32_t rphase = 0;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
