@@ -492,8 +492,10 @@ __device__ __forceinline__ float down_row(const DownArgs& a, int m, int d, int l
   return warp_sum(y);
 }
 
-template <int UPL, int FAM>
-__global__ void __launch_bounds__(256, UPL <= 3 ? 2 : 1) down_combine_kernel(const DownArgs a) {
+// OCC = blocks a processor.  One row has 256 blocks for 148 processors and wants its registers (9.0 us a layer of the 30 B shape
+// with two, 10.6 with three); several rows queue for the processors (five rows: 34 us with two, 29 with three).
+template <int UPL, int FAM, int OCC>
+__global__ void __launch_bounds__(256, OCC) down_combine_kernel(const DownArgs a) {
   __shared__ int s_slot[kMaxTopK];
   __shared__ float s_w[kMaxTopK];
   const int m = blockIdx.y;
@@ -732,13 +734,13 @@ int bl_down_combine(const int8_t* actq, const float* actds, const int* ids, cons
   BL_REQUIRE(total <= 512, BL_ERR_LIMIT);
   dim3 grid((H + 7) / 8, M);
   if (is_plane_family(dtype)) {
-    if (total <= 96) return (int)launch(down_combine_kernel<3, 2>, grid, dim3(256), 0, st, a);
-    if (total <= 192) return (int)launch(down_combine_kernel<6, 2>, grid, dim3(256), 0, st, a);
-    return (int)launch(down_combine_kernel<16, 2>, grid, dim3(256), 0, st, a);
+    if (total <= 96) return (int)launch(M == 1 ? down_combine_kernel<3, 2, 2> : down_combine_kernel<3, 2, 3>, grid, dim3(256), 0, st, a);
+    if (total <= 192) return (int)launch(down_combine_kernel<6, 2, 1>, grid, dim3(256), 0, st, a);
+    return (int)launch(down_combine_kernel<16, 2, 1>, grid, dim3(256), 0, st, a);
   }
-  if (total <= 96) return (int)launch(down_combine_kernel<3, 0>, grid, dim3(256), 0, st, a);
-  if (total <= 192) return (int)launch(down_combine_kernel<6, 0>, grid, dim3(256), 0, st, a);
-  return (int)launch(down_combine_kernel<16, 0>, grid, dim3(256), 0, st, a);
+  if (total <= 96) return (int)launch(M == 1 ? down_combine_kernel<3, 0, 2> : down_combine_kernel<3, 0, 3>, grid, dim3(256), 0, st, a);
+  if (total <= 192) return (int)launch(down_combine_kernel<6, 0, 1>, grid, dim3(256), 0, st, a);
+  return (int)launch(down_combine_kernel<16, 0, 1>, grid, dim3(256), 0, st, a);
 }
 
 }  // extern "C"
