@@ -474,7 +474,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
   __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
   __shared__ __align__(8) uint64_t raw_full[RS > 0 ? RS : 1], raw_empty[RS > 0 ? RS : 1];
   __shared__ uint32_t s_tmem_base;
-  __shared__ int s_abort;
+  __shared__ int s_abort, s_last;
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* const raw_ring = smem + (size_t)STAGES * B_STAGE;
 
@@ -576,11 +576,9 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
       tc_fence_after();
       const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + ab * ACC_COLS;
       const int n_rows = min(BN, mt.row_end - mt.row0);            // token rows of this tile
-      // partial sums of a split tile: [tile][split][token][128 weight rows]
-      float* const part = a.partial + (long)tile * a.splits * (BN * QBM) + q * 32 + lane;
-      bool mine = true;                                            // this warp finishes its quarter of the tile
       if (!DUAL && a.splits > 1) {
-        float* const own = part + (long)(t % a.splits) * (BN * QBM);
+        // a share's sums: [tile][split][token][128 weight rows]; the CTA that arrives last adds them up, see the end
+        float* const own = a.partial + (long)t * (BN * QBM) + q * 32 + lane;
 #pragma unroll 1
         for (int c = 0; c < n_rows; c += 16) {
           uint32_t v[16];
@@ -590,34 +588,13 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
           for (int i = 0; i < 16; ++i) __stcg(own + (c + i) * QBM, __uint_as_float(v[i]));
         }
         __threadfence();
-        __syncwarp();
-        int last = 0;
-        if (lane == 0) {
-          last = atomicAdd(&a.tickets[tile * 4 + q], 1) == a.splits - 1;
-          if (last) a.tickets[tile * 4 + q] = 0;                   // ready for the next launch
-        }
-        mine = __shfl_sync(0xFFFFFFFFu, last, 0) != 0;
-        if (mine) __threadfence();
-      }
-      if (mine) {
+      } else {
 #pragma unroll 1
         for (int c = 0; c < n_rows; c += 16) {
           uint32_t v[16], u[DUAL ? 16 : 1];
-          if (!DUAL && a.splits > 1) {
-            // the splits' sums are added in ascending order whichever warp arrived last: same bits on every run
-            float f[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) f[i] = 0.f;
-            for (int sp = 0; sp < a.splits; ++sp)
-#pragma unroll
-              for (int i = 0; i < 16; ++i) f[i] += __ldcg(part + (long)sp * (BN * QBM) + (c + i) * QBM);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(f[i]);
-          } else {
-            tmem_ld16(tbase + c, v);
-            if constexpr (DUAL) tmem_ld16(tbase + BN + c, u);
-            tmem_ld_wait();
-          }
+          tmem_ld16(tbase + c, v);
+          if constexpr (DUAL) tmem_ld16(tbase + BN + c, u);
+          tmem_ld_wait();
           // lane i fetches the routing of token row i of this chunk; the store loop broadcasts it
           const int r_l = mt.row0 + c + (lane & 15);
           int orow_l = -1;
@@ -789,6 +766,47 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
 
   tc_fence_before();
   __syncthreads();
+  if constexpr (!DUAL) {
+    if (a.splits > 1) {
+      // One share a CTA.  The CTA that finishes a tile's last share adds all of them up with all of its threads, eight in flight
+      // each, in ascending order: same bits on every run.  (Four epilogue warps, one share after the other, took about 6 us of
+      // the 21 of an output projection of 24 rows.)
+      const int tile = (int)blockIdx.x / a.splits;
+      if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = tile < n_tt * a.tiles_w && atomicAdd(&a.tickets[tile * 4], 1) == a.splits - 1;
+        if (s_last) a.tickets[tile * 4] = 0;                           // ready for the next launch
+        __threadfence();
+      }
+      __syncthreads();
+      if (s_last) {
+        const QTile mt = a.tiles[tile / a.tiles_w];
+        const int n = (tile % a.tiles_w) * QBM + (threadIdx.x & (QBM - 1)), n_rows = min(BN, mt.row_end - mt.row0);
+        const float* part = a.partial + (long)tile * a.splits * (BN * QBM) + (threadIdx.x & (QBM - 1));
+        if (n < a.N) {
+#pragma unroll 2
+          for (int i = threadIdx.x / QBM; i < n_rows; i += QTHREADS / QBM) {
+            const int r = mt.row0 + i, orow = a.dst_row ? a.dst_row[r] : r;
+            float f = 0.f;
+            for (int sp0 = 0; sp0 < a.splits; sp0 += 8) {
+              float v[8];
+#pragma unroll
+              for (int k = 0; k < 8; ++k)
+                if (sp0 + k < a.splits) v[k] = __ldcg(part + ((long)(sp0 + k) * BN + i) * QBM);
+#pragma unroll
+              for (int k = 0; k < 8; ++k)
+                if (sp0 + k < a.splits) f += v[k];
+            }
+            if (orow < 0) continue;
+            if (a.row_scale) f *= a.row_scale[r];
+            if (a.resid) f += a.resid[(long)orow * a.ldr + n];
+            if (a.c_f32) a.c_f32[(long)orow * a.ldc + n] = f;
+            else a.c_bf16[(long)orow * a.ldc + n] = __float2bfloat16_rn(f);
+          }
+        }
+      }
+    }
+  }
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
@@ -889,7 +907,7 @@ int bl_qgemm_split(const void* X, long ldx, long rows_x, const void* W, const vo
   a.dst_row = dst_row; a.row_scale = row_scale; a.resid = resid; a.ldr = ldr; a.status = status;
   a.fixed_tiles = fixed_tiles; a.splits = splits; a.partial = partial; a.tickets = tickets;
   const long tiles_total = (long)max_tiles * a.tiles_w * splits;
-  const int grid = (int)(tiles_total < sm_count ? tiles_total : sm_count);
+  const int grid = (int)(splits > 1 || tiles_total < sm_count ? tiles_total : sm_count);   // a share has a CTA of its own
   const bool dual = W2 != nullptr;
   switch (wtype) {
     case WT_Q4_K: return qgemm_pick<Q4K>(dual, form, tile_rows, mx, a, n_groups, grid, st);
