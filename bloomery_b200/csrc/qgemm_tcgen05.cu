@@ -97,7 +97,7 @@ enum QForm { Q_SHORT = 0, Q_EXACT = 1, Q_SPLIT = 2 };
 //   (128 + q0, 128 + q1) with one byte permute, a packed bf16 subtract gives (q0, q1) exactly and a packed bf16 FMA gives
 //   s * q + o with s and o rounded to bf16: half the integer instructions.  Its error is at most 2^-9 (|s q| + |o|) and one bf16
 //   rounding of the sum, which is no bound in ulps of the weight: near zero s q and o nearly cancel (Q4_K, Q5_K).  Gate+up
-//   of 24 rows, 100 of 128 experts (Q4_K, 768 x 2048): 97 us exact, 88 us short (35 us of blocks at the copy rate).
+//   of 24 rows, 95 of 128 experts (Q4_K, 768 x 2048): 56 us short (33 us of blocks at the copy rate).
 // FastUnit<T>::codes yields the unit's 64 code bytes in value order (16 words; word w belongs to group w / 4) and the
 // (scale, offset) pair of each of the four groups of 16 values.
 template <class T> struct FastUnit { static constexpr bool kHas = false; };

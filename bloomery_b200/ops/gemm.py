@@ -278,7 +278,7 @@ class QgemmWork:
 def qgemm_splits(n_tiles: int, depth_blocks: int, sm: int) -> int:
     """CTAs that share the depth (in 256-value blocks) of each of ``n_tiles`` output tiles: as many as leave one CTA a
     processor, in equal shares.  A projection of a decode round has 4 to 32 tiles on 148 processors, and each tile walks
-    its whole depth in one serial pipeline (2,048 deep: about 12 us; an eighth of 4,096: about 5)."""
+    its whole depth in one serial pipeline (2,048 deep: about 12 us; an eighth of 4,096 and the adding up: 11 with the launch)."""
     best = 1
     for s in range(2, min(16, depth_blocks) + 1):
         if depth_blocks % s == 0 and n_tiles * s <= sm:
