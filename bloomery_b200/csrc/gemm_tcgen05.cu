@@ -520,11 +520,9 @@ static int gemm_launch(const void* const* A_of_rank, int n_src, long lda, long r
   static_assert(BM * SPLIT_ROW * 4 <= STAGES * (TILE_A_BYTES + 2 * TILE_B128_BYTES), "a parked tile fits the ring");
   a.splits = fixed_tiles && !dist && !B2 ? gemm_splits(tiles, K, sm_count) : 1;
   if (a.splits > 1) {
-    static bool set = false;
-    if (!set) {
-      cudaFuncSetAttribute(gemm_bf16_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      set = true;
-    }
+    // an attribute of the device's context: a process may have several
+    if (cudaFuncSetAttribute(gemm_bf16_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+      return BL_ERR_LIMIT;
     return (int)launch_cluster(gemm_bf16_kernel<false, false, true>, dim3((unsigned)(tiles * a.splits)), dim3(192), smem, a.splits, st,
                                ma, mb, mb2, a);
   }
