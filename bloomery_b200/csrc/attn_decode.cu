@@ -485,12 +485,12 @@ template <int HEAD>
 __global__ void __launch_bounds__(kWfWarps * 32, 3) flash_decode_seg_wf_kernel(const FlashArgs a) {
   using W = WarpFlash<HEAD>;
   extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ float s_ml[kWfWarps][16];
-  float* sq = reinterpret_cast<float*>(smem);                              // [G][HEAD]
+  __shared__ __align__(8) float s_ml[kWfWarps][16];
+  float* sq = reinterpret_cast<float*>(smem);                              // [G][kQ]
   const int G = a.n_q / a.n_kv;
   const int seg = blockIdx.x, kvh = blockIdx.y, m = blockIdx.z;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  uint8_t* const rings = smem + 8 * HEAD * 4;
+  uint8_t* const rings = smem + 8 * W::kQ * 4;
   __half* const ring = reinterpret_cast<__half*>(rings + (size_t)warp * kWfStages * W::kStageBytes);
   pdl_wait();
   pdl_launch();
@@ -519,7 +519,7 @@ __global__ void __launch_bounds__(kWfWarps * 32, 3) flash_decode_seg_wf_kernel(c
   };
 #pragma unroll
   for (int st = 0; st < kWfStages; ++st) issue(warp + st * kWfWarps, page_of(warp + st * kWfWarps), st);
-  for (int i = tid; i < G * HEAD; i += kWfWarps * 32) sq[i] = a.q[((long)m * a.n_q + (long)kvh * G) * HEAD + i];
+  for (int i = tid; i < G * HEAD; i += kWfWarps * 32) sq[i / HEAD * W::kQ + i % HEAD] = a.q[((long)m * a.n_q + (long)kvh * G) * HEAD + i];
   __syncthreads();
   W w;
   w.init(sq, G, lane);
@@ -696,11 +696,11 @@ static int flash_decode_go(const float* q, const void* k_cache, const void* v_ca
   } else if (G <= 8) {
     // up to eight heads a group: both halves of the split operands fit one tile
     if (head == 128) {
-      constexpr int sm3 = 8 * 128 * 4 + kWfWarps * kWfStages * WarpFlash<128>::kStageBytes;
+      constexpr int sm3 = 8 * WarpFlash<128>::kQ * 4 + kWfWarps * kWfStages * WarpFlash<128>::kStageBytes;
       cudaFuncSetAttribute(flash_decode_seg_wf_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm3);
       e = launch(flash_decode_seg_wf_kernel<128>, grid, dim3(kWfWarps * 32), sm3, st, a);
     } else {
-      constexpr int sm3 = 8 * 64 * 4 + kWfWarps * kWfStages * WarpFlash<64>::kStageBytes;
+      constexpr int sm3 = 8 * WarpFlash<64>::kQ * 4 + kWfWarps * kWfStages * WarpFlash<64>::kStageBytes;
       cudaFuncSetAttribute(flash_decode_seg_wf_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm3);
       e = launch(flash_decode_seg_wf_kernel<64>, grid, dim3(kWfWarps * 32), sm3, st, a);
     }

@@ -170,7 +170,6 @@ struct AttnArgs {
   unsigned* fault; int layer;
   long long* probe;
   int recv_off;                            // cluster form: float offset of the merge buffer in dynamic shared memory
-  int seg_budget;                          // attn_fused: (row, segment) pairs of a KV head that fill the processors once
 };
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
@@ -211,57 +210,101 @@ __device__ __forceinline__ void head_out_q8(const float (&o)[HEAD / 32], int lan
   if ((lane % LPB) == 0) a.outds[((long)m * width + col) / 32] = make_float2(dd, dd * (float)sum);
 }
 
-// grid (n_seg, n_kv, M); 256 threads = 8 warps.  Groups of up to eight query heads (HPW 1): every warp takes 16 keys a step
-// for all heads on tensor-core tiles (flash_mma.cuh) and the warps meet at the segment's end; larger groups: warp w serves
-// heads w and w + 8 over tiles that the block stages together.
-template <int HEAD, int HPW>
+// Key tiles of a row (0: it fills a bucket, or its key count is not one), how many of them a segment takes, and its segments.
+// Segments depend on the row alone, so its bits do not change with the rows beside it: a drafted token's row, or one of a
+// round of several users, is the row of a pass of one.
+struct RowSegs { int tiles, tps, used; };
+__device__ __forceinline__ RowSegs row_segs(const AttnArgs& a, int mm) {
+  const int nk = a.row_pos[mm] + 1;
+  if (a.row_seq[mm] < 0 || nk <= 0 || nk > a.ctx_limit) return RowSegs{0, 1, 0};
+  const int tiles = (nk + kKeyTile - 1) / kKeyTile, tps = (tiles + a.n_seg - 1) / a.n_seg;
+  return RowSegs{tiles, tps, (tiles + tps - 1) / tps};
+}
+
+// 256 threads = 8 warps.  Groups of up to eight query heads (HPW 1): every warp takes 16 keys a step for all heads on
+// tensor-core tiles (flash_mma.cuh) and the warps meet at a segment's end; larger groups: warp w serves heads w and w + 8
+// over tiles that the block stages together.
+// One row: grid (n_seg, n_kv, 1), a block a segment.  Several rows (DEAL): grid (blocks, n_kv), as many blocks as the processors
+// hold at once, because one fits a processor and each has a start of its own; they are dealt to the rows by their key tiles,
+// and a block walks several segments of its row.  30 B shape, us a layer, a block a segment / dealt: five rows of 900 to 2,200
+// keys (480 blocks) 30.8 / 14.6, eight of 3,000 20.2 dealt, eight of 5,000 68 / 25.5, eight of 15,000 103 / 57, one of 12,000
+// beside seven of 100 23.9 / 18.3.  (Longer segments where several rows live would be a little faster still, 13.0, 17.6, 22.4
+// and 48.7 for the first four, and would make a row's bits depend on the rows beside it.)
+template <int HEAD, int HPW, bool DEAL>
 __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const AttnArgs a) {
   constexpr int KSTR = HEAD + 8, DPL = HEAD / 32;
   extern __shared__ __align__(128) uint8_t smem[];
   const int G = a.n_q / a.n_kv;
-  float* sq = reinterpret_cast<float*>(smem);                              // [G][HEAD]
+  constexpr int QSTR = HPW == 1 ? WarpFlash<HEAD>::kQ : HEAD;
+  float* sq = reinterpret_cast<float*>(smem);                              // [G][QSTR]
   __half* sk = reinterpret_cast<__half*>(smem + (size_t)G * HEAD * 4);     // [kStages][32][KSTR]
   __half* sv = sk + kStages * kKeyTile * KSTR;                             // [kStages][32][HEAD]
   using W = WarpFlash<HEAD>;
-  uint8_t* const rings = smem + (size_t)G * HEAD * 4;                      // HPW 1: [8 warps][kWfStages] in their place
-  __half* snew = HPW == 1 ? reinterpret_cast<__half*>(rings + (size_t)8 * kWfStages * W::kStageBytes) : sv + kStages * kKeyTile * HEAD;                           // [patch rows][2][HEAD]: keys and values of this pass
+  uint8_t* const rings = smem + (size_t)G * QSTR * 4;                      // HPW 1: [8 warps][kWfStages] in their place
+  // results of the warps, HPW 1: [16 slots][8][kOut] for two turns of the eight warps, or each at the start of its own ring
+  float* const s_res = reinterpret_cast<float*>(rings + (DEAL ? (size_t)8 * kWfStages * W::kStageBytes : 0));
+  constexpr size_t kResStride = DEAL ? 8 * W::kOut : kWfStages * W::kStageBytes / 4;
+  __half* snew = HPW == 1 ? reinterpret_cast<__half*>(rings + (size_t)8 * kWfStages * W::kStageBytes + (DEAL ? (size_t)16 * 8 * W::kOut * 4 : 0))
+                          : sv + kStages * kKeyTile * HEAD;        // [patch rows][2][HEAD]: keys and values of this pass
   __shared__ int s_last, s_np;
   __shared__ int s_pm[kMaxPatch], s_ppos[kMaxPatch];
-  __shared__ float s_ml[HPW == 1 ? 8 : 1][16];
-  const int seg = blockIdx.x, kvh = blockIdx.y, m = blockIdx.z;
+  __shared__ __align__(8) float s_ml[HPW == 1 ? 16 : 1][16];
+  __shared__ __align__(8) uint64_t s_turn;                  // DEAL: the warps' results of a turn are there
+  const int kvh = blockIdx.y;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
   // positions, sequence and block table are step parameters: they do not depend on the predecessor kernel
-  const int seq = a.row_seq[m];
-  const int pos = a.row_pos[m];
-  const int n_keys = pos + 1;
-  const bool pad = seq < 0;
-  const bool bad = !pad && (n_keys <= 0 || n_keys > a.ctx_limit);
-  const int n_tiles = (pad || bad) ? 0 : (n_keys + kKeyTile - 1) / kKeyTile;
-  // One block fits a processor, so the rows that live share the processors: segments of several rows beyond that would only
-  // queue, each with its own start (five rows of 1,500 keys in the bucket of eight: 480 blocks in 36 us a layer, 140 in 12).
-  int live = 0;
-  for (int mm = 0; mm < a.M; ++mm) live += a.row_seq[mm] >= 0 ? 1 : 0;
-  const int segs = min((int)gridDim.x, max(1, a.seg_budget / max(1, live)));
-  const int tps = max(1, (n_tiles + segs - 1) / segs);
-  const int used = (n_tiles + tps - 1) / tps;
-  const int t0 = seg * tps, t1 = min(n_tiles, t0 + tps);
-  if (pad || bad) {
-    // padding rows and rows with a bad key count still publish rows for o_proj: zeros, or a NaN scale
-    if (seg != 0) return;
-    pdl_wait();
-    pdl_launch();
+  // This block's row and segments g0 .. g1 - 1, and the blocks that share the row.
+  int m = blockIdx.z, g0 = blockIdx.x, g1 = g0 + 1, sharers;
+  RowSegs rs;
+  bool publish = !DEAL && blockIdx.x == 0;         // rows without keys (row blockIdx.z, or blockIdx.x) are this block's to publish
+  if constexpr (DEAL) {
+    // Lane mm looks at row mm: it gets a block, and of the others its share by key tiles.  Any number from 1 to `used` blocks deals the
+    // segments out, so the quotient need not be exact, only the same in every block and no larger.
+    const RowSegs mine = lane < a.M ? row_segs(a, lane) : RowSegs{0, 1, 0};
+    const int spare = (int)gridDim.x - __popc(__ballot_sync(0xffffffffu, mine.used > 0));
+    const float per_tile = (float)spare * 0.9999f * __frcp_rn((float)max(1u, __reduce_add_sync(0xffffffffu, (unsigned)mine.tiles)));
+    const int n = min(mine.used, 1 + (int)((float)mine.tiles * per_tile));
+    int end = n;                                   // blocks of the rows up to this lane's
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) { const int o = __shfl_up_sync(0xffffffffu, end, off); if (lane >= off) end += o; }
+    m = __ffs(__ballot_sync(0xffffffffu, end > (int)blockIdx.x)) - 1;
+    publish = blockIdx.x < (unsigned)a.M && __shfl_sync(0xffffffffu, mine.used, blockIdx.x & 31) == 0;
+    const int src = max(m, 0);
+    rs = RowSegs{__shfl_sync(0xffffffffu, mine.tiles, src), __shfl_sync(0xffffffffu, mine.tps, src), __shfl_sync(0xffffffffu, mine.used, src)};
+    sharers = __shfl_sync(0xffffffffu, n, src);
+    const int i = (int)blockIdx.x - (__shfl_sync(0xffffffffu, end, src) - sharers);
+    g0 = m < 0 ? 0 : i * rs.used / sharers;
+    g1 = m < 0 ? 0 : (i + 1) * rs.used / sharers;
+  } else {
+    rs = row_segs(a, m);
+    sharers = rs.used;
+    publish = publish && rs.used == 0;
+  }
+  const int used = rs.used, tps = rs.tps;
+  const int t0 = g0 * tps, t1 = min(rs.tiles, g1 * tps);
+  // padding rows and rows with a bad key count still publish rows for o_proj: zeros, or a NaN scale
+  auto publish_empty = [&]() {
+    const int r = DEAL ? blockIdx.x : blockIdx.z;
+    const bool bad = a.row_seq[r] >= 0;
     if (bad && tid == 0 && kvh == 0) raise_fault(a.fault, a.layer, FS_KEY_COUNT);
     const long width = (long)a.n_q * HEAD;
     for (int i = tid; i < G * HEAD; i += 256) {
       const long col = (long)kvh * G * HEAD + i;
-      a.outq[(long)m * width + col] = 0;
-      if (a.out) a.out[(long)m * width + col] = bad ? kNaN : 0.f;
-      if ((i & 31) == 0) a.outds[((long)m * width + col) / 32] = bad ? make_float2(kNaN, 0.f) : make_float2(0.f, 0.f);
+      a.outq[(long)r * width + col] = 0;
+      if (a.out) a.out[(long)r * width + col] = bad ? kNaN : 0.f;
+      if ((i & 31) == 0) a.outds[((long)r * width + col) / 32] = bad ? make_float2(kNaN, 0.f) : make_float2(0.f, 0.f);
+    }
+  };
+  if (t0 >= t1) {                                  // no segment for this block
+    if (publish) {
+      pdl_wait();
+      pdl_launch();
+      publish_empty();
     }
     return;
   }
-  if (t0 >= t1) return;                            // past the row's last key tile
+  const int seq = a.row_seq[m], pos = a.row_pos[m], n_keys = pos + 1;
 
   const int* bt = a.block_table + (long)seq * a.max_pages;
   auto issue_tile = [&](int t, int stage) {
@@ -280,20 +323,84 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
   // keys of earlier positions are already in the cache: the first kStages tiles stream in while the predecessor
   // still runs (one copy group per stage, empty past the last tile, so the group count stays uniform)
   probe_mark(a.probe, 0);
-  const int key_lo = t0 * kKeyTile, key_hi = min(n_keys, t1 * kKeyTile);
-  const int n_steps = (key_hi - key_lo + W::kKeys - 1) / W::kKeys;         // HPW 1: warp w takes steps w, w + 8, ...
+  // HPW 1: a segment's step j belongs to its warp j % 8, and the block's warps take (segment, warp) pairs in turns: two or four
+  // segments a turn where one has two or four steps, otherwise one, which starts a remainder of eight further on each time so
+  // that all warps get as many steps.
+  const int key_hi = min(n_keys, t1 * kKeyTile), n_g = g1 - g0, per = tps < 3 ? 2 * tps : 8;
+  struct At { int g, w, j; };                                              // segment of this block, warp of it, step of it
+  auto key_of = [&](int g) { return (g0 + g) * tps * kKeyTile; };
+  auto steps_of = [&](int g) { return min(2 * tps, (key_hi - key_of(g) + W::kKeys - 1) / W::kKeys); };
+  auto next_turn = [&](At& c) {
+    c.g += 8 / per;
+    if (per == 8) c.w = (c.w - 2 * tps) & 7;
+    c.j = c.w;
+  };
+  At cur{warp / per, warp % per, warp % per}, ahead = cur;
   __half* const ring = reinterpret_cast<__half*>(rings + (size_t)warp * kWfStages * W::kStageBytes);
-  auto page_of = [&](int j) { return j < n_steps ? bt[(key_lo + j * W::kKeys) / kPage] : 0; };
-  auto issue_step = [&](int j, int page, int st) {
-    if (j < n_steps) {
-      const int key0 = key_lo + j * W::kKeys;
-      page = (page < 0 || page >= a.n_pages) ? 0 : page;
-      const long base = (((long)page * a.n_kv + kvh) * kPage + (key0 % kPage)) * HEAD;
-      W::issue(ring + (size_t)st * (W::kStageBytes / 2), a.k_cache + base, a.v_cache + base, n_keys - key0, lane);
+  // the step at `ahead`, which moves on to this warp's next one; its page is looked up a step early
+  auto settle = [&]() { while (ahead.g < n_g && ahead.j >= steps_of(ahead.g)) next_turn(ahead); };
+  auto page_ahead = [&]() { return ahead.g < n_g ? bt[(key_of(ahead.g) + ahead.j * W::kKeys) / kPage] : 0; };
+  auto issue_keys = [&](int key0, int page, int st) {
+    page = (page < 0 || page >= a.n_pages) ? 0 : page;
+    const long base = (((long)page * a.n_kv + kvh) * kPage + (key0 % kPage)) * HEAD;
+    W::issue(ring + (size_t)st * (W::kStageBytes / 2), a.k_cache + base, a.v_cache + base, n_keys - key0, lane);
+  };
+  auto issue_ahead = [&](int page, int st) {
+    if (ahead.g < n_g) {
+      issue_keys(key_of(ahead.g) + ahead.j * W::kKeys, page, st);
+      ahead.j += 8;
+      settle();
     }
     cp_async_commit();
   };
-  if constexpr (HPW == 1) {
+  // one segment: warp w takes steps w, w + 8, ... of it
+  const int key_lo = t0 * kKeyTile, n_steps = (key_hi - key_lo + W::kKeys - 1) / W::kKeys;
+  auto page_of = [&](int j) { return j < n_steps ? bt[(key_lo + j * W::kKeys) / kPage] : 0; };
+  auto issue_step = [&](int j, int page, int st) {
+    if (j < n_steps) issue_keys(key_lo + j * W::kKeys, page, st);
+    cp_async_commit();
+  };
+  // DEAL: a block of many short segments gives each to one warp, tiles of keys and then of values through a ring of four (see
+  // below).  In steps one behind the other: 2 tps for up to eight segments, against about two and a half a turn.  Eight rows of
+  // 3,000 keys, eight segments a block: 20.7 us alone, 26.6 in turns; three of 9,000, three a block: 27.7 and 22.4.
+  const bool alone = DEAL && HPW == 1 && used > 1 && 2 * tps <= W::kOut / 8 && 4 * tps * ((n_g + 7) / 8) < 5 * ((n_g * per + 7) / 8);
+  int a_n = 0, a_i = 0, a_w = 0, a_j = 0, a_page = 0;      // steps of this warp's segment; next tile to fetch, and its step
+  auto issue_alone = [&](int key0) {
+    if (a_i < 2 * a_n) {
+      const int step = a_i < a_n ? a_i : a_j, key = key0 + step * W::kKeys;
+      int page = __shfl_sync(0xffffffffu, a_page, key / kPage - key0 / kPage);
+      page = (page < 0 || page >= a.n_pages) ? 0 : page;
+      const long base = (((long)page * a.n_kv + kvh) * kPage + (key % kPage)) * HEAD;
+      W::issue_tile(ring + (a_i & 3) * W::kTile, (a_i < a_n ? a.k_cache : a.v_cache) + base, n_keys - key, lane);
+      if (a_i >= a_n && (a_j += 8) >= a_n) a_j = ++a_w;
+      ++a_i;
+    }
+    cp_async_commit();
+  };
+  auto open_alone = [&](int g) {                           // the first four tiles of segment g
+    a_n = g < n_g ? steps_of(g) : 0;
+    a_i = a_w = a_j = 0;
+    if (lane < 8 && key_of(g) / kPage + lane <= (key_hi - 1) / kPage) a_page = bt[key_of(g) / kPage + lane];
+    for (int i = 0; i < 4; ++i) issue_alone(key_of(g));
+  };
+  if (alone) {
+    open_alone(warp);
+  } else if constexpr (HPW == 1 && DEAL) {
+    settle();
+    int key0[kWfStages], page[kWfStages];              // pages of all first steps before their keys: one round trip
+#pragma unroll
+    for (int st = 0; st < kWfStages; ++st) {
+      key0[st] = ahead.g < n_g ? key_of(ahead.g) + ahead.j * W::kKeys : -1;
+      page[st] = page_ahead();
+      ahead.j += 8;
+      settle();
+    }
+#pragma unroll
+    for (int st = 0; st < kWfStages; ++st) {
+      if (key0[st] >= 0) issue_keys(key0[st], page[st], st);
+      cp_async_commit();
+    }
+  } else if constexpr (HPW == 1) {
 #pragma unroll
     for (int st = 0; st < kWfStages; ++st) issue_step(warp + 8 * st, page_of(warp + 8 * st), st);
   } else {
@@ -305,6 +412,7 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
   }
   pdl_wait();
   pdl_launch();
+  if (DEAL && publish) publish_empty();
   probe_mark(a.probe, 1);
 
   // ---- queries of this KV head's group: RMSNorm + RoPE into shared memory ---------------------------
@@ -345,7 +453,7 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
       float y[DPL];
       norm_rope(row + ((long)kvh * G + hg) * HEAD, a.q_gain, true, pos, y);
 #pragma unroll
-      for (int j = 0; j < DPL; ++j) sq[hg * HEAD + lane + 32 * j] = y[j] * a.q_scale;
+      for (int j = 0; j < DPL; ++j) sq[hg * QSTR + lane + 32 * j] = y[j] * a.q_scale;
     }
   }
   probe_mark(a.probe, 2);
@@ -353,7 +461,10 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
   // Rows of the pass that belong to the same sequence at or before this row's position are not in the cache
   // yet (their owner blocks write them in this same launch), so a block computes the ones that fall inside its
   // key range itself and patches them into the tiles; only the row's own block stores its row to the cache.
-  if (tid == 0) s_np = 0;
+  if (tid == 0) {
+    s_np = 0;
+    if constexpr (DEAL && HPW == 1) mbar_init(&s_turn, 8);
+  }
   __syncthreads();
   for (int mm = tid; mm < a.M; mm += 256) {
     if (a.row_seq[mm] == seq) {
@@ -366,6 +477,8 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
   }
   __syncthreads();
   const int np = min(s_np, kMaxPatch);
+  int first_new = 0x7fffffff;                        // tiles that end in front of this position take nothing from the pass
+  for (int idx = 0; idx < np; ++idx) first_new = min(first_new, s_ppos[idx]);
   for (int it = warp; it < 2 * np; it += 8) {
     const int idx = it >> 1, mm = s_pm[idx], pp = s_ppos[idx];
     const bool is_k = (it & 1) == 0;
@@ -390,47 +503,176 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
 
   probe_mark(a.probe, 3);
   float mx[HPW], l[HPW], acc[HPW][DPL];
+  auto clear = [&]() {
 #pragma unroll
-  for (int h = 0; h < HPW; ++h) {
-    mx[h] = -INFINITY; l[h] = 0.f;
+    for (int h = 0; h < HPW; ++h) {
+      mx[h] = -INFINITY; l[h] = 0.f;
 #pragma unroll
-    for (int d = 0; d < DPL; ++d) acc[h][d] = 0.f;
-  }
+      for (int d = 0; d < DPL; ++d) acc[h][d] = 0.f;
+    }
+  };
+  // segment g of this block is complete: the row when it is the only one, otherwise a part of it
+  auto emit = [&](int g) {
+#pragma unroll
+    for (int h = 0; h < HPW; ++h) {
+      const int hg = warp + 8 * h;
+      if (hg < G) {
+        if (used == 1) {
+          float o[DPL];
+#pragma unroll
+          for (int d = 0; d < DPL; ++d) o[d] = acc[h][d] / l[h];
+          head_out_q8<HEAD>(o, lane, ((long)kvh * G + hg) * HEAD, a, m);
+        } else {
+          const long pidx = ((long)m * a.n_q + (long)kvh * G + hg) * a.n_seg + g0 + g;
+          if (lane == 0) { a.part_ml[pidx * 2] = mx[h]; a.part_ml[pidx * 2 + 1] = l[h]; }
+          float* part = a.part_acc + pidx * HEAD + lane * DPL;
+          if constexpr (DPL == 4) *reinterpret_cast<float4*>(part) = make_float4(acc[h][0], acc[h][1], acc[h][2], acc[h][3]);
+          else *reinterpret_cast<float2*>(part) = make_float2(acc[h][0], acc[h][1]);
+        }
+      }
+    }
+  };
   if constexpr (HPW == 1) {
     __syncthreads();                                 // queries and this pass's keys and values are in shared memory
-    if (warp < n_steps) {
-      W w;
-      w.init(sq, G, lane);
-      int st = 0;
-      for (int j = warp; j < n_steps; j += 8) {
-        const int page = page_of(j + 8 * kWfStages);
-        cp_async_wait<kWfStages - 1>();
-        __syncwarp();
-        __half* tile = ring + (size_t)st * (W::kStageBytes / 2);
-        const int key0 = key_lo + j * W::kKeys;
-        for (int idx = 0; idx < np; ++idx) {
-          const int r = s_ppos[idx] - key0;
-          if (r >= 0 && r < W::kKeys)                            // a row of this pass: the copy raced its store
-            for (int i = lane; i < HEAD; i += 32) {
-              tile[r * W::kStr + i] = snew[(size_t)idx * 2 * HEAD + i];
-              tile[W::kTile + r * W::kStr + i] = snew[((size_t)idx * 2 + 1) * HEAD + i];
-            }
-        }
-        __syncwarp();
-        w.step(tile, n_keys - key0, lane);
-        __syncwarp();
-        issue_step(j + 8 * kWfStages, page, st);
-        st = st + 1 == kWfStages ? 0 : st + 1;
-      }
-      cp_async_wait<0>();
+    W w;
+    // a step over stage `st` of this warp's ring, keys from key0 on
+    auto step = [&](int key0, int st) {
+      cp_async_wait<kWfStages - 1>();
       __syncwarp();
-      w.store(s_ml[warp], reinterpret_cast<float*>(ring), lane);
+      __half* tile = ring + (size_t)st * (W::kStageBytes / 2);
+      if (key0 + W::kKeys > first_new) for (int idx = 0; idx < np; ++idx) {
+        const int r = s_ppos[idx] - key0;
+        if (r >= 0 && r < W::kKeys)                            // a row of this pass: the copy raced its store
+          for (int i = lane; i < HEAD; i += 32) {
+            tile[r * W::kStr + i] = snew[(size_t)idx * 2 * HEAD + i];
+            tile[W::kTile + r * W::kStr + i] = snew[((size_t)idx * 2 + 1) * HEAD + i];
+          }
+      }
+      __syncwarp();
+      w.step(tile, n_keys - key0, lane);
+      __syncwarp();
+    };
+    if constexpr (!DEAL) {
+      if (warp < n_steps) {
+        w.init(sq, G, lane);
+        int st = 0;
+        for (int j = warp; j < n_steps; j += 8) {
+          const int page = page_of(j + 8 * kWfStages);
+          step(key_lo + j * W::kKeys, st);
+          issue_step(j + 8 * kWfStages, page, st);
+          st = st + 1 == kWfStages ? 0 : st + 1;
+        }
+        cp_async_wait<0>();
+        __syncwarp();
+        w.store(s_ml[warp], s_res + warp * kResStride, lane);
+      }
+      __syncthreads();
+      if (warp < G) {
+        wf_merge<HEAD>(&s_ml[0][0], s_res, kResStride, min(8, n_steps), warp, lane, acc[0], mx[0], l[0]);
+        emit(0);
+      }
+    } else if (alone) {
+      // All scores of the segment first (they wait in shared memory), so its maximum is known and the outputs of its eight
+      // warps, computed one after the other, are added up in registers: the sums of the form below, without its round
+      // trip of every output through shared memory.
+      float4* const s_sc = reinterpret_cast<float4*>(s_res + warp * 2 * 8 * W::kOut);     // [step][lane], kOut / 8 steps
+      float* const s_mx = reinterpret_cast<float*>(s_sc + W::kOut / 8 / 2 * 2 * 32);
+      w.init(sq, G, lane);
+      for (int g = warp; g < n_g; g += 8) {
+        if (g != warp) open_alone(g);
+        const int n = a_n, key_g = key_of(g);
+        // tile i of the segment, landed: a row of this pass raced its store
+        auto landed = [&](int i, int step, bool values) {
+          cp_async_wait<3>();
+          __syncwarp();
+          __half* tile = ring + (i & 3) * W::kTile;
+          if (key_g + (step + 1) * W::kKeys > first_new) for (int idx = 0; idx < np; ++idx) {
+            const int r = s_ppos[idx] - (key_g + step * W::kKeys);
+            if (r >= 0 && r < W::kKeys)
+              for (int e = lane; e < HEAD; e += 32) tile[r * W::kStr + e] = snew[((size_t)idx * 2 + (values ? 1 : 0)) * HEAD + e];
+          }
+          __syncwarp();
+          return tile;
+        };
+        float top = -INFINITY;
+        for (int j = 0; j < n; ++j) {
+          float c[2][2][4], s[2][2];
+          w.products(landed(j, j, false), lane, c);
+          float nm = w.scores(c, n_keys - (key_g + j * W::kKeys), lane, s);
+          if (__any_sync(0xffffffffu, nm != nm)) nm = w.scores_joined(c, n_keys - (key_g + j * W::kKeys), lane, s);
+          top = fmaxf(top, nm);
+          s_sc[j * 32 + lane] = make_float4(s[0][0], s[0][1], s[1][0], s[1][1]);
+          if ((lane & 3) == 0) s_mx[j * 8 + (lane >> 2)] = nm;
+          __syncwarp();
+          issue_alone(key_g);
+        }
+        float sum = 0.f, part[W::ND][2];
+#pragma unroll
+        for (int d = 0; d < W::ND; ++d) part[d][0] = part[d][1] = 0.f;
+        int i = n;
+        for (int v = 0; v < min(8, n); ++v) {
+          w.reset();
+          for (int j = v; j < n; j += 8, ++i) {
+            const float4 q = s_sc[j * 32 + lane];
+            const float s[2][2] = {{q.x, q.y}, {q.z, q.w}};
+            const float nm = fmaxf(w.m, s_mx[j * 8 + (lane >> 2)]);
+            const __half* tile = landed(i, j, true);
+            if (__any_sync(0xffffffffu, nm != w.m)) w.rescale(nm);
+            w.values(s, tile, lane);
+            __syncwarp();
+            issue_alone(key_g);
+          }
+          w.add_to(part, sum, top);
+        }
+        const int hg = lane >> 2;
+        if (hg < G) {
+          const long pidx = ((long)m * a.n_q + (long)kvh * G + hg) * a.n_seg + g0 + g;
+          if ((lane & 3) == 0) { a.part_ml[pidx * 2] = top; a.part_ml[pidx * 2 + 1] = sum; }
+#pragma unroll
+          for (int d = 0; d < W::ND; ++d)
+            *reinterpret_cast<float2*>(a.part_acc + pidx * HEAD + 8 * d + 2 * (lane & 3)) = make_float2(part[d][0], part[d][1]);
+        }
+      }
+    } else {
+      w.init(sq, G, lane);
+      int page = page_ahead(), st = 0;
+      // A turn's results lie in one half of the slots.  A warp may run a turn ahead of the others: it waits for all to have left
+      // their results of the turn before, behind which nobody reads the half that this turn overwrites.
+      int done = 0;
+      auto merge_turn = [&](int turn) {                  // warp w: head w of the segments that this turn ended
+        for (; done < n_g && (done + 1) * per <= 8 * (turn + 1); ++done)
+          if (warp < G) {
+            wf_merge<HEAD>(&s_ml[0][0], s_res, kResStride, min(8, steps_of(done)), warp, lane, acc[0], mx[0], l[0], done * per);
+            emit(done);
+          }
+      };
+      const int n_turns = (n_g * per + 7) / 8;
+      for (int turn = 0; turn < n_turns; ++turn) {
+        const bool mine = cur.g < n_g && cur.w < steps_of(cur.g);
+        if (mine) {
+          if (turn > 0) w.reset();
+          const int n = steps_of(cur.g), key_g = key_of(cur.g);
+          for (int j = cur.w; j < n; j += 8) {
+            step(key_g + j * W::kKeys, st);
+            issue_ahead(page, st);
+            page = page_ahead();
+            st = st + 1 == kWfStages ? 0 : st + 1;
+          }
+        }
+        if (turn > 0) mbar_wait(&s_turn, (turn - 1) & 1, a.fault, a.layer);
+        const int slot = (turn & 1) * 8 + (per == 8 ? cur.w : warp);
+        if (mine) w.store(s_ml[slot], s_res + slot * kResStride, lane);
+        if (turn > 0) merge_turn(turn - 1);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_turn);
+        next_turn(cur);
+      }
+      mbar_wait(&s_turn, (n_turns - 1) & 1, a.fault, a.layer);
+      merge_turn(n_turns - 1);
     }
-    __syncthreads();
-    if (warp < G)
-      wf_merge<HEAD>(&s_ml[0][0], reinterpret_cast<const float*>(rings), kWfStages * W::kStageBytes / 4, min(8, n_steps), warp,
-                     lane, acc[0], mx[0], l[0]);
-  } else
+  } else {
+  clear();
+  int in_seg = 0, done = 0;
   for (int t = t0; t < t1; ++t) {
     const int stage = (t - t0) % kStages;
     cp_async_wait<kStages - 1>();                    // the oldest group in flight (tile t) has landed
@@ -498,39 +740,18 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
     __syncthreads();
     if (t + kStages < t1) issue_tile(t + kStages, stage);     // refill the stage just read
     else cp_async_commit();
+    if (++in_seg == tps || t + 1 == t1) { emit(done++); clear(); in_seg = 0; }
+  }
   }
 
   probe_mark(a.probe, 4);
-  if (used == 1) {
-    // one segment covers the whole row: finish here, nothing to merge
-#pragma unroll
-    for (int h = 0; h < HPW; ++h) {
-      const int hg = warp + 8 * h;
-      if (hg < G) {
-        float o[DPL];
-#pragma unroll
-        for (int d = 0; d < DPL; ++d) o[d] = acc[h][d] / l[h];
-        head_out_q8<HEAD>(o, lane, ((long)kvh * G + hg) * HEAD, a, m);
-      }
-    }
-    return;
-  }
-#pragma unroll
-  for (int h = 0; h < HPW; ++h) {
-    const int hg = warp + 8 * h;
-    if (hg < G) {
-      const long pidx = ((long)m * a.n_q + (long)kvh * G + hg) * a.n_seg + seg;
-      if (lane == 0) { a.part_ml[pidx * 2] = mx[h]; a.part_ml[pidx * 2 + 1] = l[h]; }
-#pragma unroll
-      for (int d = 0; d < DPL; ++d) a.part_acc[pidx * HEAD + lane * DPL + d] = acc[h][d];
-    }
-  }
+  if (used == 1) return;                             // one segment covers the whole row: nothing to merge
   // completion ticket: the block that arrives last for this (row, KV head) merges the segments
   __threadfence();
   __syncthreads();
   if (tid == 0) {
     const unsigned t = atomicAdd(a.tickets + (long)m * a.n_kv + kvh, 1u);
-    s_last = (t == (unsigned)used - 1u) ? 1 : 0;
+    s_last = (t == (unsigned)sharers - 1u) ? 1 : 0;
     if (s_last) a.tickets[(long)m * a.n_kv + kvh] = 0u;       // ready for the next launch (graph replay)
   }
   __syncthreads();
@@ -542,46 +763,48 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
     const int hg = warp + 8 * h;
     if (hg < G) {
       const long p0 = ((long)m * a.n_q + (long)kvh * G + hg) * a.n_seg;
-      // lanes fetch the segments' (max, sum) pairs side by side; the accumulators follow eight segments per
-      // round trip; the sums themselves still run over the segments in ascending order
-      float gm = -INFINITY;
-      for (int s0 = 0; s0 < used; s0 += 32) {
-        const int sg = s0 + lane;
-        if (sg < used) gm = fmaxf(gm, __ldcg(a.part_ml + (p0 + sg) * 2));
-      }
-      gm = warp_max(gm);
-      float den = 0.f, num[DPL];
+      // lanes fetch the segments' (max, sum) pairs side by side and the accumulators sixteen segments per round trip; the
+      // sums themselves run over the segments in ascending order
+      float v[16][DPL];
+      auto fetch = [&](int s0) {
 #pragma unroll
-      for (int d = 0; d < DPL; ++d) num[d] = 0.f;
-      for (int s0 = 0; s0 < used; s0 += 32) {
-        const int sg = s0 + lane;
-        float ms = -INFINITY, ls = 0.f;
-        if (sg < used) { const float2 v = __ldcg(reinterpret_cast<const float2*>(a.part_ml + (p0 + sg) * 2)); ms = v.x; ls = v.y; }
-        const float wl = (ms == -INFINITY) ? 0.f : __expf(ms - gm);
-        const int cnt = min(32, used - s0);
-        for (int k0 = 0; k0 < cnt; k0 += 8) {
-          float v[8][DPL];
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            if (k0 + k < cnt) {
-              const float* src = a.part_acc + (p0 + s0 + k0 + k) * HEAD + lane * DPL;
-              if constexpr (DPL == 4) {
-                const float4 t = __ldcg(reinterpret_cast<const float4*>(src));
-                v[k][0] = t.x; v[k][1] = t.y; v[k][2] = t.z; v[k][3] = t.w;
-              } else {
-                const float2 t = __ldcg(reinterpret_cast<const float2*>(src));
-                v[k][0] = t.x; v[k][1] = t.y;
-              }
+        for (int k = 0; k < 16; ++k) {
+          if (s0 + k < used) {
+            const float* src = a.part_acc + (p0 + s0 + k) * HEAD + lane * DPL;
+            if constexpr (DPL == 4) {
+              const float4 t = __ldcg(reinterpret_cast<const float4*>(src));
+              v[k][0] = t.x; v[k][1] = t.y; v[k][2] = t.z; v[k][3] = t.w;
+            } else {
+              const float2 t = __ldcg(reinterpret_cast<const float2*>(src));
+              v[k][0] = t.x; v[k][1] = t.y;
             }
           }
+        }
+      };
+      auto pair_of = [&](int sg) { return sg < used ? __ldcg(reinterpret_cast<const float2*>(a.part_ml + (p0 + sg) * 2)) : make_float2(-INFINITY, 0.f); };
+      const float2 first = pair_of(lane), second = pair_of(32 + lane);
+      fetch(0);
+      float gm = fmaxf(first.x, second.x);
+      for (int s0 = 64; s0 < used; s0 += 32) gm = fmaxf(gm, pair_of(s0 + lane).x);
+      gm = warp_max(gm);
+      float den = 0.f, num[DPL], wl = 0.f, ls = 0.f;
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            if (k0 + k < cnt) {
-              const float wk = __shfl_sync(0xffffffffu, wl, k0 + k), lk = __shfl_sync(0xffffffffu, ls, k0 + k);
-              den = fmaf(lk, wk, den);
+      for (int d = 0; d < DPL; ++d) num[d] = 0.f;
+      for (int s0 = 0; s0 < used; s0 += 16) {
+        if (s0 > 0) fetch(s0);
+        if ((s0 & 31) == 0) {
+          const float2 ml = s0 == 0 ? first : s0 == 32 ? second : pair_of(s0 + lane);
+          wl = (ml.x == -INFINITY) ? 0.f : __expf(ml.x - gm);
+          ls = ml.y;
+        }
+        const int cnt = min(16, used - s0);
 #pragma unroll
-              for (int d = 0; d < DPL; ++d) num[d] = fmaf(v[k][d], wk, num[d]);
-            }
+        for (int k = 0; k < 16; ++k) {
+          if (k < cnt) {
+            const float wk = __shfl_sync(0xffffffffu, wl, (s0 & 31) + k), lk = __shfl_sync(0xffffffffu, ls, (s0 & 31) + k);
+            den = fmaf(lk, wk, den);
+#pragma unroll
+            for (int d = 0; d < DPL; ++d) num[d] = fmaf(v[k][d], wk, num[d]);
           }
         }
       }
@@ -1312,31 +1535,35 @@ int bl_attn_fused(const float* qkv, long qkv_stride, const float* q_gain, const 
   const int G = n_q / n_kv;
   AttnArgs a{qkv, qkv_stride, q_gain, k_gain, inv_freq, eps, q_scale, n_q, n_kv, M, n_seg, ctx_limit, row_pos, row_seq,
              block_table, max_pages, n_pages, (__half*)k_cache, (__half*)v_cache, part_ml, part_acc, tickets, out, outq,
-             (float2*)outds, fault, layer, g_stage_probe, 0, 0};
+             (float2*)outds, fault, layer, g_stage_probe, 0};
   const int n_patch = M < kMaxPatch ? M : kMaxPatch;
   const size_t rings = G <= 8 ? (size_t)8 * kWfStages * (head == 128 ? WarpFlash<128>::kStageBytes : WarpFlash<64>::kStageBytes)
                               : (size_t)kStages * kKeyTile * (head + 8) * 2 + kStages * kKeyTile * head * 2;
-  const size_t smem = (size_t)G * head * 4 + rings + (size_t)n_patch * 2 * head * 2;
-  // segments of the rows that live: as many blocks as the processors hold at once.  A bucket of M rows holds more than M / 2.
-  int dev = 0, sm = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    return BL_ERR_LIMIT;
-  const int resident = (int)(227 * 1024 / (smem + 2048));
-  a.seg_budget = M == 1 ? n_seg : sm * (resident < 1 ? 1 : resident > 2 ? 2 : resident) / n_kv;
-  const int most = a.seg_budget / (M / 2 + 1);
-  dim3 grid(M == 1 || most >= n_seg ? n_seg : most < 1 ? 1 : most, n_kv, M);
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(attn_fused_kernel<128, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 180 * 1024);
-    cudaFuncSetAttribute(attn_fused_kernel<128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
-    cudaFuncSetAttribute(attn_fused_kernel<64, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
-    cudaFuncSetAttribute(attn_fused_kernel<64, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
-    attr_set = true;
+  const size_t smem = (size_t)G * (G <= 8 ? head + 8 : head) * 4 + rings + (size_t)n_patch * 2 * head * 2;
+  // Several rows: blocks for the processors (a warp's lanes look at the rows, so 32 of them at most), every row at least one.
+  const size_t deal_smem = smem + (G <= 8 ? (size_t)16 * 8 * (head + 8) * 4 : 0);
+  const bool deal = M > 1 && M <= 32;
+  dim3 grid(n_seg, n_kv, M);
+  if (deal) {
+    int dev = 0, sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      return BL_ERR_LIMIT;
+    const int resident = G > 8 && 2 * (deal_smem + 2048) <= 227 * 1024 ? 2 : 1;      // G <= 8: by its registers one
+    const int blocks = sm * resident / n_kv;
+    const long most = (long)n_seg * M;
+    grid = dim3((unsigned)(blocks < M ? M : blocks > most ? most : blocks), n_kv, 1);
   }
-  cudaError_t e;
-  if (head == 128) e = G <= 8 ? launch(attn_fused_kernel<128, 1>, grid, dim3(256), smem, st, a) : launch(attn_fused_kernel<128, 2>, grid, dim3(256), smem, st, a);
-  else e = G <= 8 ? launch(attn_fused_kernel<64, 1>, grid, dim3(256), smem, st, a) : launch(attn_fused_kernel<64, 2>, grid, dim3(256), smem, st, a);
-  return (int)e;
+  auto go = [&](auto kernel, size_t bytes) {
+    // a kernel's shared-memory limit belongs to a device, and stages of one process may sit on several: set on every call
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (G <= 8 ? 225 : 110) * 1024) != cudaSuccess) return (int)BL_ERR_LIMIT;
+    return (int)launch(kernel, grid, dim3(256), bytes, st, a);
+  };
+  if (deal) {
+    if (head == 128) return G <= 8 ? go(attn_fused_kernel<128, 1, true>, deal_smem) : go(attn_fused_kernel<128, 2, true>, deal_smem);
+    return G <= 8 ? go(attn_fused_kernel<64, 1, true>, deal_smem) : go(attn_fused_kernel<64, 2, true>, deal_smem);
+  }
+  if (head == 128) return G <= 8 ? go(attn_fused_kernel<128, 1, false>, smem) : go(attn_fused_kernel<128, 2, false>, smem);
+  return G <= 8 ? go(attn_fused_kernel<64, 1, false>, smem) : go(attn_fused_kernel<64, 2, false>, smem);
 }
 
 // route_logits != null: every block routes its row from the logits (block (0, 0, m) writes ids / wts / heat);

@@ -30,6 +30,9 @@ __device__ __forceinline__ void bulk_load_chunks(uint8_t* dst, const uint8_t* sr
 __device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 // Bounded wait (1 s on the global timer) for phase `parity`.  On expiry: fault site "device wait ran out",
 // false is returned and the caller writes NaN; the kernel still returns.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned* fault, int layer) {

@@ -5,7 +5,8 @@ The contract is the reference's (``crates/runtime/src/lib.rs:13-17``, ``speculat
 a draft changes which passes run and never a token.  Verification feeds the last accepted
 token and the k drafted ids as k+1 rows of one pass; rows of a pass are bit-equal to their
 own 1-row steps, so the greedy picks are the ones plain decoding would have made; the
-longest agreeing prefix is kept and the KV rows of the rest are cut.
+longest agreeing prefix is kept and the KV rows of the rest are cut.  (The optional cluster launch
+of one row, off by default, adds the experts' rows up in another order than passes of several.)
 
 * :class:`NgramDraft` -- prompt-lookup draft: the longest recent n-gram that occurred before
   proposes what followed it (the reference's n-gram lookup draft).

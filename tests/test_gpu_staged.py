@@ -367,8 +367,8 @@ def test_engine_tokens_do_not_depend_on_the_kernel_form():
 @pytest.mark.parametrize("pos,dead", [([0, 700], []), ([1023, 5, 64], [1]), ([31, 32, 500, 900, 63, 0, 0, 0], [5, 6, 7]),
                                       ([10, 900, 450, 33, 1, 31, 64, 800], [])])
 def test_attn_fused_rows_share_the_processors(head, n_q, n_kv, pos, dead):
-    """Fewer segments a row the more rows live: rows of one key up to a thousand, dead rows that count for nothing, against
-    softmax attention in 64 bits over the cache as the launch leaves it."""
+    """Rows of one key up to a thousand, dead rows that count for nothing, against softmax attention in 64 bits over the cache
+    as the launch leaves it."""
     from bloomery_b200.ops import decode as K
     g = torch.Generator(device=DEV).manual_seed(head + len(pos))
     M, ctx, n_seg = len(pos), 1024, 37
@@ -399,3 +399,74 @@ def test_attn_fused_rows_share_the_processors(head, n_q, n_kv, pos, dead):
         ref = torch.einsum("hk,hkd->hd", torch.softmax(torch.einsum("hd,hkd->hk", q, k), -1), v).reshape(-1)
         # operands split into 22 bits, exponentials and sums in fp32
         assert float((out[m].double() - ref).abs().max()) < 2e-4
+
+
+def _attn_rows(head, n_q, n_kv, qkv, pos, seq, kc, vc, table, n_seg, ctx):
+    """One launch over the rows; caches are changed in place.  Returns the fp32 rows, the q8 codes and the scales."""
+    from bloomery_b200.ops import decode as K
+    M = len(pos)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    ml = torch.full((M * n_q * n_seg * 2,), float("nan"), device=DEV)
+    acc = torch.full((M * n_q * n_seg * head,), float("nan"), device=DEV)
+    tickets, fault = torch.zeros(M * n_kv, **i32), torch.full((1,), -1, **i32)
+    out = torch.full((M, n_q * head), float("nan"), device=DEV)
+    outq, outds = torch.zeros(M, n_q * head, dtype=torch.int8, device=DEV), torch.zeros(M, n_q * head // 32, 2, device=DEV)
+    inv = (1.0 / (1e6 ** (torch.arange(0, head, 2, dtype=torch.float64) / head))).float().to(DEV)
+    for _ in range(3):                              # tickets come back to zero by themselves
+        K.attn_fused(qkv, None, None, inv, 1e-6, head ** -0.5, head, n_q, n_kv, M, torch.tensor(pos, **i32), torch.tensor(seq, **i32),
+                     table, kc.shape[0], kc, vc, n_seg, ctx, ml, acc, tickets, out, outq, outds, fault, 0)
+    assert int(fault) == -1 and int(tickets.abs().sum()) == 0
+    return out, outq, outds
+
+
+@pytest.mark.parametrize("head,n_q,n_kv", [(128, 32, 4), (64, 14, 2), (128, 48, 4)])
+@pytest.mark.parametrize("rows", [
+    [(0, 1300), (1, 1299)],                                                  # two users
+    [(0, 1300), (0, 1301), (0, 1302), (0, 1303), (0, 1304)],                 # a token and four drafted ones behind it
+    [(0, 2000), (-1, 0), (1, 40), (2, 1333), (3, 0), (-1, 0), (4, 640)],     # ragged, with rows that fill a bucket
+    [(0, 4000)] + [(s, 90 + s) for s in range(1, 8)],                        # one long conversation beside short ones
+    [(s, 1200 + 31 * s) for s in range(8)],
+    [(s, 3 * s) for s in range(8)],
+])
+def test_attn_fused_row_is_the_row_of_a_pass_of_one(head, n_q, n_kv, rows):
+    """A draft, or another user, changes which pass a row runs in and never its bits: the key segments and the order in which
+    they are added up come from the row's own length."""
+    g = torch.Generator(device=DEV).manual_seed(len(rows) + head)
+    ctx, n_seg, n_seq = 4096, 37, 8
+    pages = ctx // 64
+    kc, vc = (torch.randn(n_seq * pages, n_kv, 64, head, device=DEV, generator=g).half() for _ in range(2))
+    table = torch.randperm(n_seq * pages, device=DEV, generator=g).to(torch.int32).view(n_seq, pages)
+    qkv = torch.randn(len(rows), (n_q + 2 * n_kv) * head, device=DEV, generator=g)
+    k1, v1 = kc.clone(), vc.clone()
+    got = _attn_rows(head, n_q, n_kv, qkv, [p for _, p in rows], [s for s, _ in rows], kc, vc, table, n_seg, ctx)
+    for m, (s, p) in enumerate(rows):                                       # in order: a row reads the keys of the rows before it
+        if s >= 0:
+            one = _attn_rows(head, n_q, n_kv, qkv[m:m + 1], [p], [s], k1, v1, table, n_seg, ctx)
+            for a, b in zip(got, one):
+                assert torch.equal(a[m], b[0]), (m, s, p)
+        else:
+            assert all(float(a[m].float().abs().max()) == 0.0 for a in got)
+    assert torch.equal(kc, k1) and torch.equal(vc, v1)
+
+
+def test_engine_row_is_the_row_of_a_pass_of_one():
+    """The contract of drafts over the whole engine: the logits of a row in a pass of five are those of its own pass."""
+    from bloomery_b200.models.spec import tiny_qwen3moe
+    from bloomery_b200.models.weights import Weights, synth_tensors
+    from bloomery_b200.ops import decode as K
+    from bloomery_b200.runtime.engine import DecodeEngine
+    K.set_staged_parts("attn,prefetch")                # the defaults: the cluster launch sums the down rows in another order
+    spec = tiny_qwen3moe()
+    w = Weights.from_items(spec, synth_tensors(spec, DEV, seed=0), DEV)
+    eng = DecodeEngine(w, n_slots=2, slot_ctx=2048)
+    prompt = [(7 * i + 3) % spec.vocab for i in range(1300)]
+    for slot in (0, 1):
+        eng.prefill(slot, prompt, gemm=False)
+    drafted = [11, 500, 3, 77, 901]
+    one = []
+    for j, t in enumerate(drafted):
+        eng.step([(0, t, len(prompt) + j)])
+        one.append(eng.logits[0].clone())
+    eng.step([(1, t, len(prompt) + j) for j, t in enumerate(drafted)])
+    for j in range(len(drafted)):
+        assert torch.equal(eng.logits[j], one[j]), j
