@@ -1,6 +1,6 @@
 // Prompt (prefill) flash attention on the 5th-generation tensor cores: scores and the output accumulator live in
-// tensor memory, the probabilities go from registers to shared memory and straight back into the second product,
-// and nothing of the score matrix ever reaches HBM.
+// tensor memory, the probabilities go from registers back into the columns of their scores and from there into the second
+// product, and nothing of the score matrix ever reaches HBM.
 //
 // One CTA = two tiles of 128 query positions (the 128 lanes of tensor memory) that read the same keys: two query heads of
 // one KV head, as a rule.  Their softmaxes and products take turns, so that one tile's exponentials (16,384 at 16 a clock a
@@ -99,6 +99,9 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
   const int last_q = a.pos0 + min(tile_q0(0) + FQ, a.T) - 1;    // position of the first tile's last query: no other is later
   const int all_t = last_q / FKEYS + 1;                         // key tiles of the pair
   const int t_lo = all_t * split / a.splits, n_t = all_t * (split + 1) / a.splits - t_lo;   // this CTA's: t_lo .. t_lo + n_t - 1
+  // A second tile one position earlier (an odd number of heads) ends a key tile earlier: it must not meet the values behind it,
+  // where a probability of zero times infinity is NaN.  A share holds two key tiles when it is the last, so never none of its.
+  auto tiles_of = [&](int x) { return min(n_t, (a.pos0 + min(tile_q0(x) + FQ, a.T) - 1) / FKEYS + 1 - t_lo); };
 
   if (threadIdx.x == 0) {
     mbar_init(&q_full, 1);
@@ -160,6 +163,7 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
       umma_commit(&s_full[x]);
     };
     bool ok = mbar_wait_warp(&q_full, 0, abort_flag) && mbar_wait_warp(&k_full[0], 0, abort_flag);
+    const int n_tx[2] = {n_t, n_x > 1 ? tiles_of(1) : 0};
     if (ok) {
       tc_fence_after();
       for (int x = 0; x < n_x; ++x) qk(x, 0);
@@ -171,28 +175,30 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
       const uint64_t dV0 = umma_desc(smem_u32(sV + st * FTILE)), dV1 = umma_desc(smem_u32(sV + st * FTILE + FHALF));
       for (int x = 0; x < n_x; ++x) {
         if (x == 0 && !mbar_wait_warp(&v_full[st], par, abort_flag)) { ok = false; break; }
-        if (!mbar_wait_warp(&p_full[x], (uint32_t)(t & 1), abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t tP = tS0 + x * FKEYS, tO = tO0 + x * FD;
+        if (t < n_tx[x]) {
+          if (!mbar_wait_warp(&p_full[x], (uint32_t)(t & 1), abort_flag)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t tP = tS0 + x * FKEYS, tO = tO0 + x * FD;
 #pragma unroll
-        for (int k = 0; k < FATOM / UMMA_K; ++k) umma_bf16_ta(tO, tP + k * 8, dV0 + (uint64_t)(k * 2), idesc, (t > 0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < FATOM / UMMA_K; ++k) umma_bf16_ta(tO, tP + k * 8, dV0 + (uint64_t)(k * 2), idesc, (t > 0 || k > 0) ? 1u : 0u);
 #pragma unroll
-        for (int k = 0; k < FATOM / UMMA_K; ++k) umma_bf16_ta(tO, tP + 32 + k * 8, dV1 + (uint64_t)(k * 2), idesc, 1u);
+          for (int k = 0; k < FATOM / UMMA_K; ++k) umma_bf16_ta(tO, tP + 32 + k * 8, dV1 + (uint64_t)(k * 2), idesc, 1u);
+        }
         if (x == n_x - 1) umma_commit(&v_empty[st]);
-        if (t + 1 < n_t) {
-          if (x == 0 && !mbar_wait_warp(&k_full[nx], nx_par, abort_flag)) { ok = false; break; }
+        if (t + 1 < n_t && x == 0 && !mbar_wait_warp(&k_full[nx], nx_par, abort_flag)) { ok = false; break; }
+        if (t + 1 < n_tx[x]) {
           tc_fence_after();
           qk(x, nx);
-          if (x == n_x - 1) umma_commit(&k_empty[nx]);
-        } else {
+        } else if (t + 1 == n_tx[x]) {
           umma_commit(&o_done[x]);
         }
+        if (t + 1 < n_t && x == n_x - 1) umma_commit(&k_empty[nx]);
       }
     }
   } else if ((warp >> 2) < n_x) {
     // ---- softmax: a thread per query row ------------------------------------------------------------------
     const int x = warp >> 2;
-    const int q0 = tile_q0(x), h = tile_head(x);
+    const int q0 = tile_q0(x), h = tile_head(x), n_tx = tiles_of(x);
     const int r = (warp & 3) * 32 + lane;
     const int qrow = q0 + r;
     const int qpos = a.pos0 + qrow;
@@ -200,7 +206,7 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
     const uint32_t tS = tS0 + x * FKEYS + lane_base, tO = tO0 + x * FD + lane_base;
     float m = -INFINITY, l = 0.f;
     bool ok = true;
-    for (int t = 0; t < n_t; ++t) {
+    for (int t = 0; t < n_tx; ++t) {
       ok = __all_sync(0xffffffffu, mbar_wait(&s_full[x], (uint32_t)(t & 1), abort_flag));
       if (!ok) break;
       tc_fence_after();

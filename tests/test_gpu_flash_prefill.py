@@ -130,3 +130,31 @@ def test_query_tiles_whose_keys_are_shared(n_q, n_kv, T, pos0, splits, monkeypat
     assert [i for i, out in enumerate(outs) if not torch.equal(out, outs[0])] == []
     ref = _ref(q, k, v, pos0).permute(1, 0, 2).reshape(T, n_q * 128)
     assert float((outs[0].float() - ref).norm() / ref.norm()) < 2 ** -7          # as without shares
+
+
+@pytest.mark.parametrize("n_q,n_kv,T,pos0,splits", [(1, 1, 300, 0, 1), (3, 1, 300, 0, 1), (10, 2, 513, 70, 1), (8, 2, 300, 0, 1), (3, 1, 300, 1000, 3),
+                                                    (1, 1, 129, 512, 4)])
+def test_values_behind_a_row_reach_no_tile_in_front_of_theirs(n_q, n_kv, T, pos0, splits, monkeypatch):
+    """An infinite value weighs zero for earlier queries, and zero times infinity is NaN: rows whose key tiles end in front of its
+    tile must not meet it, whichever tile shares their CTA."""
+    from bloomery_b200.ops import gemm as G
+    g = torch.Generator(device=DEV).manual_seed(T)
+    n_keys = pos0 + T
+    t_pad = (n_keys + 127) // 128 * 128
+    q = (torch.randn(n_q, T, 128, device=DEV, generator=g) / 128 ** 0.5).bfloat16()
+    Kb, Vt = torch.zeros(n_kv, t_pad, 128, device=DEV, dtype=torch.bfloat16), torch.zeros(n_kv, 128, t_pad, device=DEV, dtype=torch.bfloat16)
+    Kb[:, :n_keys] = torch.randn(n_kv, n_keys, 128, device=DEV, generator=g).bfloat16()
+    Vt[:, :, :n_keys] = torch.randn(n_kv, 128, n_keys, device=DEV, generator=g).bfloat16()
+    monkeypatch.setattr(G, "flash_splits", lambda *a: splits)
+    status, outs = torch.zeros(1, dtype=torch.int32, device=DEV), []
+    for bad in (False, True):
+        if bad:
+            Vt[:, 5, n_keys - 1] = float("inf")
+        out = torch.zeros(T, n_q * 128, device=DEV, dtype=torch.bfloat16)
+        G.flash_prefill(q, Kb, Vt, out, pos0, status, G.FlashWork(DEV))
+        outs.append(out)
+    assert int(status) == 0
+    # rows of query tiles whose last key tile lies in front of the one that holds the value
+    clear = [t for t in range(T) if (pos0 + min(t // 128 * 128 + 128, T) - 1) // 128 < (n_keys - 1) // 128]
+    assert clear and torch.equal(outs[0][clear], outs[1][clear])
+    assert bool(torch.isinf(outs[1][T - 1].view(n_q, 128)[:, 5]).all())
