@@ -154,6 +154,7 @@ constexpr int kPage = 64;
 constexpr int kKeyTile = 32;
 constexpr int kStages = 4;        // key / value tiles in flight per block
 constexpr int kWfStages = 2;      // the same for a warp that walks keys on its own
+constexpr int kWfTiles = 3;       // several rows: tiles of 16 keys or of 16 values in flight per warp (at least)
 constexpr int kMaxPatch = 64;     // rows of one pass whose keys a block may have to take from the pass itself
 
 struct AttnArgs {
@@ -227,9 +228,9 @@ __device__ __forceinline__ RowSegs row_segs(const AttnArgs& a, int mm) {
 // One row: grid (n_seg, n_kv, 1), a block a segment.  Several rows (DEAL): grid (blocks, n_kv), as many blocks as the processors
 // hold at once, because one fits a processor and each has a start of its own; they are dealt to the rows by their key tiles,
 // and a block walks several segments of its row.  30 B shape, us a layer, a block a segment / dealt: five rows of 900 to 2,200
-// keys (480 blocks) 30.8 / 14.6, eight of 3,000 20.2 dealt, eight of 5,000 68 / 25.5, eight of 15,000 103 / 57, one of 12,000
-// beside seven of 100 23.9 / 18.3.  (Longer segments where several rows live would be a little faster still, 13.0, 17.6, 22.4
-// and 48.7 for the first four, and would make a row's bits depend on the rows beside it.)
+// keys (480 blocks) 30.8 / 15.1, eight of 5,000 68 / 25.9, eight of 15,000 103 / 61, one of 12,000 beside seven of 100 23.9 /
+// 19.0.  (Segments cut by the number of rows instead took 13.0, 22.4, 48.7 and 34.4, and made a row's bits depend on the rows
+// beside it.)
 template <int HEAD, int HPW, bool DEAL>
 __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const AttnArgs a) {
   constexpr int KSTR = HEAD + 8, DPL = HEAD / 32;
@@ -240,11 +241,16 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
   __half* sk = reinterpret_cast<__half*>(smem + (size_t)G * HEAD * 4);     // [kStages][32][KSTR]
   __half* sv = sk + kStages * kKeyTile * KSTR;                             // [kStages][32][HEAD]
   using W = WarpFlash<HEAD>;
-  uint8_t* const rings = smem + (size_t)G * QSTR * 4;                      // HPW 1: [8 warps][kWfStages] in their place
+  uint8_t* const rings = smem + (size_t)G * QSTR * 4;                      // HPW 1: [8 warps][RING] in their place
+  constexpr int RING = DEAL ? kWfTiles * W::kTile : kWfStages * (W::kStageBytes / 2);   // f16 values of a warp's ring
   // results of the warps, HPW 1: [16 slots][8][kOut] for two turns of the eight warps, or each at the start of its own ring
-  float* const s_res = reinterpret_cast<float*>(rings + (DEAL ? (size_t)8 * kWfStages * W::kStageBytes : 0));
-  constexpr size_t kResStride = DEAL ? 8 * W::kOut : kWfStages * W::kStageBytes / 4;
-  __half* snew = HPW == 1 ? reinterpret_cast<__half*>(rings + (size_t)8 * kWfStages * W::kStageBytes + (DEAL ? (size_t)16 * 8 * W::kOut * 4 : 0))
+  float* const s_res = reinterpret_cast<float*>(rings + (DEAL ? (size_t)8 * RING * 2 : 0));
+  constexpr int kAllTiles = 40;                            // DEAL: rings and results together
+  static_assert(8 * (kWfTiles * W::kTile * 2 + 2 * 8 * W::kOut * 4) == kAllTiles * W::kTile * 2, "whole tiles");
+  constexpr int kAloneSteps = HEAD / 8;                    // steps whose scores and maxima (17 float4 a lane group) fit two tiles
+  static_assert(kAloneSteps / 2 * (32 * 16 + 8 * 4) <= W::kTile * 2, "half of them fit one");
+  constexpr size_t kResStride = DEAL ? 8 * W::kOut : RING / 2;
+  __half* snew = HPW == 1 ? reinterpret_cast<__half*>(rings + (size_t)8 * RING * 2 + (DEAL ? (size_t)16 * 8 * W::kOut * 4 : 0))
                           : sv + kStages * kKeyTile * HEAD;        // [patch rows][2][HEAD]: keys and values of this pass
   __shared__ int s_last, s_np;
   __shared__ int s_pm[kMaxPatch], s_ppos[kMaxPatch];
@@ -336,70 +342,74 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
     c.j = c.w;
   };
   At cur{warp / per, warp % per, warp % per}, ahead = cur;
-  __half* const ring = reinterpret_cast<__half*>(rings + (size_t)warp * kWfStages * W::kStageBytes);
-  // the step at `ahead`, which moves on to this warp's next one; its page is looked up a step early
+  // DEAL: a block of many short segments gives each to one warp, tiles of keys and then of values (see below).  In steps one behind the other: 2 tps for up to eight segments, against about two and a half a turn.  Eight rows of
+  // 3,000 keys, eight segments a block: 20.6 us alone, 26.6 in turns; three of 9,000, three a block: 27.7 and 22.1.
+  const bool alone = DEAL && HPW == 1 && used > 1 && 2 * tps <= kAloneSteps && 4 * tps * ((n_g + 7) / 8) < 5 * ((n_g * per + 7) / 8);
+  // All tiles of shared memory are then the active warps' own: scores, and a ring that holds the whole segment where it can, so
+  // that keys and values arrive while the launch in front still runs.
+  const int mine_t = alone ? kAllTiles / min(8, n_g) : 0, score_t = 2 * tps > kAloneSteps / 2 ? 2 : 1;
+  const int left = mine_t - score_t, ring_n = !alone ? kWfTiles : left >= 8 ? 8 : left >= 6 ? 6 : left >= 4 ? 4 : 3;
+  __half* const ring = reinterpret_cast<__half*>(rings) + (size_t)(alone ? min(warp, n_g - 1) * mine_t * W::kTile : warp * RING);
+  auto base_of = [&](int key, int page) {
+    page = (page < 0 || page >= a.n_pages) ? 0 : page;
+    return (((long)page * a.n_kv + kvh) * kPage + (key % kPage)) * HEAD;
+  };
+  // DEAL: every fetch is one tile and one copy group (empty past the last tile, so the count stays uniform)
+  int put = 0, get = 0;                                    // ring positions of the next tile to fetch and to take
+  auto fetch = [&](bool values, int key, int page) {
+    W::issue_tile(ring + put * W::kTile, (values ? a.v_cache : a.k_cache) + base_of(key, page), n_keys - key, lane);
+  };
+  auto fetched = [&]() { cp_async_commit(); put = put + 1 == ring_n ? 0 : put + 1; };
+  // the keys and then the values of the step at `ahead`, which moves on to this warp's next one; its page is looked up early
   auto settle = [&]() { while (ahead.g < n_g && ahead.j >= steps_of(ahead.g)) next_turn(ahead); };
   auto page_ahead = [&]() { return ahead.g < n_g ? bt[(key_of(ahead.g) + ahead.j * W::kKeys) / kPage] : 0; };
-  auto issue_keys = [&](int key0, int page, int st) {
-    page = (page < 0 || page >= a.n_pages) ? 0 : page;
-    const long base = (((long)page * a.n_kv + kvh) * kPage + (key0 % kPage)) * HEAD;
-    W::issue(ring + (size_t)st * (W::kStageBytes / 2), a.k_cache + base, a.v_cache + base, n_keys - key0, lane);
-  };
-  auto issue_ahead = [&](int page, int st) {
+  bool values_next = false;
+  int page_next = 0;
+  auto fetch_ahead = [&]() {
     if (ahead.g < n_g) {
-      issue_keys(key_of(ahead.g) + ahead.j * W::kKeys, page, st);
-      ahead.j += 8;
-      settle();
+      fetch(values_next, key_of(ahead.g) + ahead.j * W::kKeys, page_next);
+      if (values_next) {
+        ahead.j += 8;
+        settle();
+        page_next = page_ahead();
+      }
+      values_next = !values_next;
     }
-    cp_async_commit();
+    fetched();
   };
   // one segment: warp w takes steps w, w + 8, ... of it
   const int key_lo = t0 * kKeyTile, n_steps = (key_hi - key_lo + W::kKeys - 1) / W::kKeys;
   auto page_of = [&](int j) { return j < n_steps ? bt[(key_lo + j * W::kKeys) / kPage] : 0; };
   auto issue_step = [&](int j, int page, int st) {
-    if (j < n_steps) issue_keys(key_lo + j * W::kKeys, page, st);
-    cp_async_commit();
-  };
-  // DEAL: a block of many short segments gives each to one warp, tiles of keys and then of values through a ring of four (see
-  // below).  In steps one behind the other: 2 tps for up to eight segments, against about two and a half a turn.  Eight rows of
-  // 3,000 keys, eight segments a block: 20.7 us alone, 26.6 in turns; three of 9,000, three a block: 27.7 and 22.4.
-  const bool alone = DEAL && HPW == 1 && used > 1 && 2 * tps <= W::kOut / 8 && 4 * tps * ((n_g + 7) / 8) < 5 * ((n_g * per + 7) / 8);
-  int a_n = 0, a_i = 0, a_w = 0, a_j = 0, a_page = 0;      // steps of this warp's segment; next tile to fetch, and its step
-  auto issue_alone = [&](int key0) {
-    if (a_i < 2 * a_n) {
-      const int step = a_i < a_n ? a_i : a_j, key = key0 + step * W::kKeys;
-      int page = __shfl_sync(0xffffffffu, a_page, key / kPage - key0 / kPage);
-      page = (page < 0 || page >= a.n_pages) ? 0 : page;
-      const long base = (((long)page * a.n_kv + kvh) * kPage + (key % kPage)) * HEAD;
-      W::issue_tile(ring + (a_i & 3) * W::kTile, (a_i < a_n ? a.k_cache : a.v_cache) + base, n_keys - key, lane);
-      if (a_i >= a_n && (a_j += 8) >= a_n) a_j = ++a_w;
-      ++a_i;
+    if (j < n_steps) {
+      const int key0 = key_lo + j * W::kKeys;
+      const long base = base_of(key0, page);
+      W::issue(ring + (size_t)st * (W::kStageBytes / 2), a.k_cache + base, a.v_cache + base, n_keys - key0, lane);
     }
     cp_async_commit();
   };
-  auto open_alone = [&](int g) {                           // the first four tiles of segment g
+  int a_n = 0, a_i = 0, a_w = 0, a_j = 0, a_page = 0;      // steps of this warp's segment; next tile to fetch, and its step
+  auto fetch_alone = [&](int key0) {
+    if (a_i < 2 * a_n) {
+      const int key = key0 + (a_i < a_n ? a_i : a_j) * W::kKeys;
+      fetch(a_i >= a_n, key, __shfl_sync(0xffffffffu, a_page, key / kPage - key0 / kPage));
+      if (a_i >= a_n && (a_j += 8) >= a_n) a_j = ++a_w;
+      ++a_i;
+    }
+    fetched();
+  };
+  auto open_alone = [&](int g) {                           // the first tiles of segment g
     a_n = g < n_g ? steps_of(g) : 0;
     a_i = a_w = a_j = 0;
     if (lane < 8 && key_of(g) / kPage + lane <= (key_hi - 1) / kPage) a_page = bt[key_of(g) / kPage + lane];
-    for (int i = 0; i < 4; ++i) issue_alone(key_of(g));
+    for (int i = 0; i < ring_n; ++i) fetch_alone(key_of(g));
   };
   if (alone) {
     open_alone(warp);
   } else if constexpr (HPW == 1 && DEAL) {
     settle();
-    int key0[kWfStages], page[kWfStages];              // pages of all first steps before their keys: one round trip
-#pragma unroll
-    for (int st = 0; st < kWfStages; ++st) {
-      key0[st] = ahead.g < n_g ? key_of(ahead.g) + ahead.j * W::kKeys : -1;
-      page[st] = page_ahead();
-      ahead.j += 8;
-      settle();
-    }
-#pragma unroll
-    for (int st = 0; st < kWfStages; ++st) {
-      if (key0[st] >= 0) issue_keys(key0[st], page[st], st);
-      cp_async_commit();
-    }
+    page_next = page_ahead();
+    for (int i = 0; i < kWfTiles; ++i) fetch_ahead();
   } else if constexpr (HPW == 1) {
 #pragma unroll
     for (int st = 0; st < kWfStages; ++st) issue_step(warp + 8 * st, page_of(warp + 8 * st), st);
@@ -535,30 +545,42 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
   if constexpr (HPW == 1) {
     __syncthreads();                                 // queries and this pass's keys and values are in shared memory
     W w;
-    // a step over stage `st` of this warp's ring, keys from key0 on
-    auto step = [&](int key0, int st) {
-      cp_async_wait<kWfStages - 1>();
+    // a row of this pass among the 16 keys (or values) from key0 on: the copy raced its store
+    // (which: 0 keys, 1 values, 2 both, the values' tile behind the keys')
+    auto patch = [&](__half* tile, int key0, int which) {
+      if (key0 + W::kKeys > first_new)
+        for (int idx = 0; idx < np; ++idx) {
+          const int r = s_ppos[idx] - key0;
+          if (r >= 0 && r < W::kKeys)
+            for (int i = lane; i < HEAD; i += 32) {
+              tile[r * W::kStr + i] = snew[((size_t)idx * 2 + (which & 1)) * HEAD + i];
+              if (which == 2) tile[W::kTile + r * W::kStr + i] = snew[((size_t)idx * 2 + 1) * HEAD + i];
+            }
+        }
+    };
+    // DEAL: the next tile, landed
+    auto landed = [&](int key0, int which) {
+      if (ring_n == 3) cp_async_wait<2>(); else if (ring_n == 4) cp_async_wait<3>(); else if (ring_n == 6) cp_async_wait<5>(); else cp_async_wait<7>();
       __syncwarp();
-      __half* tile = ring + (size_t)st * (W::kStageBytes / 2);
-      if (key0 + W::kKeys > first_new) for (int idx = 0; idx < np; ++idx) {
-        const int r = s_ppos[idx] - key0;
-        if (r >= 0 && r < W::kKeys)                            // a row of this pass: the copy raced its store
-          for (int i = lane; i < HEAD; i += 32) {
-            tile[r * W::kStr + i] = snew[(size_t)idx * 2 * HEAD + i];
-            tile[W::kTile + r * W::kStr + i] = snew[((size_t)idx * 2 + 1) * HEAD + i];
-          }
-      }
+      __half* tile = ring + get * W::kTile;
+      get = get + 1 == ring_n ? 0 : get + 1;
+      patch(tile, key0, which);
       __syncwarp();
-      w.step(tile, n_keys - key0, lane);
-      __syncwarp();
+      return tile;
     };
     if constexpr (!DEAL) {
       if (warp < n_steps) {
         w.init(sq, G, lane);
         int st = 0;
         for (int j = warp; j < n_steps; j += 8) {
-          const int page = page_of(j + 8 * kWfStages);
-          step(key_lo + j * W::kKeys, st);
+          const int page = page_of(j + 8 * kWfStages), key0 = key_lo + j * W::kKeys;
+          cp_async_wait<kWfStages - 1>();
+          __syncwarp();
+          __half* stage = ring + (size_t)st * (W::kStageBytes / 2);
+          patch(stage, key0, 2);
+          __syncwarp();
+          w.step(stage, n_keys - key0, lane);
+          __syncwarp();
           issue_step(j + 8 * kWfStages, page, st);
           st = st + 1 == kWfStages ? 0 : st + 1;
         }
@@ -575,52 +597,40 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
       // All scores of the segment first (they wait in shared memory), so its maximum is known and the outputs of its eight
       // warps, computed one after the other, are added up in registers: the sums of the form below, without its round
       // trip of every output through shared memory.
-      float4* const s_sc = reinterpret_cast<float4*>(s_res + warp * 2 * 8 * W::kOut);     // [step][lane], kOut / 8 steps
-      float* const s_mx = reinterpret_cast<float*>(s_sc + W::kOut / 8 / 2 * 2 * 32);
+      float4* const s_sc = reinterpret_cast<float4*>(ring + ring_n * W::kTile);           // [step][lane]
+      float* const s_mx = reinterpret_cast<float*>(s_sc + score_t * (kAloneSteps / 2) * 32);
       w.init(sq, G, lane);
       for (int g = warp; g < n_g; g += 8) {
         if (g != warp) open_alone(g);
         const int n = a_n, key_g = key_of(g);
-        // tile i of the segment, landed: a row of this pass raced its store
-        auto landed = [&](int i, int step, bool values) {
-          cp_async_wait<3>();
-          __syncwarp();
-          __half* tile = ring + (i & 3) * W::kTile;
-          if (key_g + (step + 1) * W::kKeys > first_new) for (int idx = 0; idx < np; ++idx) {
-            const int r = s_ppos[idx] - (key_g + step * W::kKeys);
-            if (r >= 0 && r < W::kKeys)
-              for (int e = lane; e < HEAD; e += 32) tile[r * W::kStr + e] = snew[((size_t)idx * 2 + (values ? 1 : 0)) * HEAD + e];
-          }
-          __syncwarp();
-          return tile;
-        };
         float top = -INFINITY;
         for (int j = 0; j < n; ++j) {
           float c[2][2][4], s[2][2];
-          w.products(landed(j, j, false), lane, c);
-          float nm = w.scores(c, n_keys - (key_g + j * W::kKeys), lane, s);
-          if (__any_sync(0xffffffffu, nm != nm)) nm = w.scores_joined(c, n_keys - (key_g + j * W::kKeys), lane, s);
+          const int key0 = key_g + j * W::kKeys;
+          w.products(landed(key0, 0), lane, c);
+          __syncwarp();
+          fetch_alone(key_g);
+          float nm = w.scores(c, n_keys - key0, lane, s);
+          if (__any_sync(0xffffffffu, nm != nm)) nm = w.scores_joined(c, n_keys - key0, lane, s);
           top = fmaxf(top, nm);
           s_sc[j * 32 + lane] = make_float4(s[0][0], s[0][1], s[1][0], s[1][1]);
           if ((lane & 3) == 0) s_mx[j * 8 + (lane >> 2)] = nm;
-          __syncwarp();
-          issue_alone(key_g);
         }
+        __syncwarp();
         float sum = 0.f, part[W::ND][2];
 #pragma unroll
         for (int d = 0; d < W::ND; ++d) part[d][0] = part[d][1] = 0.f;
-        int i = n;
         for (int v = 0; v < min(8, n); ++v) {
           w.reset();
-          for (int j = v; j < n; j += 8, ++i) {
+          for (int j = v; j < n; j += 8) {
             const float4 q = s_sc[j * 32 + lane];
             const float s[2][2] = {{q.x, q.y}, {q.z, q.w}};
             const float nm = fmaxf(w.m, s_mx[j * 8 + (lane >> 2)]);
-            const __half* tile = landed(i, j, true);
+            const __half* tile = landed(key_g + j * W::kKeys, 1);
             if (__any_sync(0xffffffffu, nm != w.m)) w.rescale(nm);
             w.values(s, tile, lane);
             __syncwarp();
-            issue_alone(key_g);
+            fetch_alone(key_g);
           }
           w.add_to(part, sum, top);
         }
@@ -635,7 +645,6 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
       }
     } else {
       w.init(sq, G, lane);
-      int page = page_ahead(), st = 0;
       // A turn's results lie in one half of the slots.  A warp may run a turn ahead of the others: it waits for all to have left
       // their results of the turn before, behind which nobody reads the half that this turn overwrites.
       int done = 0;
@@ -653,10 +662,15 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
           if (turn > 0) w.reset();
           const int n = steps_of(cur.g), key_g = key_of(cur.g);
           for (int j = cur.w; j < n; j += 8) {
-            step(key_g + j * W::kKeys, st);
-            issue_ahead(page, st);
-            page = page_ahead();
-            st = st + 1 == kWfStages ? 0 : st + 1;
+            float c[2][2][4], s[2][2];
+            const int key0 = key_g + j * W::kKeys;
+            w.products(landed(key0, 0), lane, c);
+            __syncwarp();
+            fetch_ahead();
+            w.softmax(c, n_keys - key0, lane, s);
+            w.values(s, landed(key0, 1), lane);
+            __syncwarp();
+            fetch_ahead();
           }
         }
         if (turn > 0) mbar_wait(&s_turn, (turn - 1) & 1, a.fault, a.layer);
@@ -763,12 +777,14 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
     const int hg = warp + 8 * h;
     if (hg < G) {
       const long p0 = ((long)m * a.n_q + (long)kvh * G + hg) * a.n_seg;
-      // lanes fetch the segments' (max, sum) pairs side by side and the accumulators sixteen segments per round trip; the
+      // lanes fetch the segments' (max, sum) pairs side by side and the accumulators kTrip segments per round trip (16: one row
+      // of 12,000 keys 13.2 us, eight 15.9; several rows run behind longer code, and more of it costs what it saves); the
       // sums themselves run over the segments in ascending order
-      float v[16][DPL];
+      constexpr int kTrip = DEAL ? 8 : 16;
+      float v[kTrip][DPL];
       auto fetch = [&](int s0) {
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
+        for (int k = 0; k < kTrip; ++k) {
           if (s0 + k < used) {
             const float* src = a.part_acc + (p0 + s0 + k) * HEAD + lane * DPL;
             if constexpr (DPL == 4) {
@@ -790,16 +806,16 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
       float den = 0.f, num[DPL], wl = 0.f, ls = 0.f;
 #pragma unroll
       for (int d = 0; d < DPL; ++d) num[d] = 0.f;
-      for (int s0 = 0; s0 < used; s0 += 16) {
+      for (int s0 = 0; s0 < used; s0 += kTrip) {
         if (s0 > 0) fetch(s0);
         if ((s0 & 31) == 0) {
           const float2 ml = s0 == 0 ? first : s0 == 32 ? second : pair_of(s0 + lane);
           wl = (ml.x == -INFINITY) ? 0.f : __expf(ml.x - gm);
           ls = ml.y;
         }
-        const int cnt = min(16, used - s0);
+        const int cnt = min(kTrip, used - s0);
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
+        for (int k = 0; k < kTrip; ++k) {
           if (k < cnt) {
             const float wk = __shfl_sync(0xffffffffu, wl, (s0 & 31) + k), lk = __shfl_sync(0xffffffffu, ls, (s0 & 31) + k);
             den = fmaf(lk, wk, den);
@@ -1541,7 +1557,8 @@ int bl_attn_fused(const float* qkv, long qkv_stride, const float* q_gain, const 
                               : (size_t)kStages * kKeyTile * (head + 8) * 2 + kStages * kKeyTile * head * 2;
   const size_t smem = (size_t)G * (G <= 8 ? head + 8 : head) * 4 + rings + (size_t)n_patch * 2 * head * 2;
   // Several rows: blocks for the processors (a warp's lanes look at the rows, so 32 of them at most), every row at least one.
-  const size_t deal_smem = smem + (G <= 8 ? (size_t)16 * 8 * (head + 8) * 4 : 0);
+  // (results of two turns, and smaller rings: what is left lets the launches before and after overlap with this one)
+  const size_t deal_smem = G > 8 ? smem : (size_t)(G + 16 * 8) * (head + 8) * 4 + (size_t)8 * kWfTiles * 16 * (head + 8) * 2 + (size_t)n_patch * 2 * head * 2;
   const bool deal = M > 1 && M <= 32;
   dim3 grid(n_seg, n_kv, M);
   if (deal) {

@@ -163,6 +163,14 @@ struct WarpFlash {
     for (int j = 0; j < ND; ++j) { o[j][0] *= corr; o[j][1] *= corr; o[j][2] *= corr; o[j][3] *= corr; }
     m = nm;
   }
+  // scores, with the maximum they bring
+  __device__ __forceinline__ void softmax(const float (&c)[2][2][4], int n_valid, int lane, float (&s)[2][2]) {
+    float nm = wf_max_nan(m, scores(c, n_valid, lane, s));
+    if (__any_sync(0xffffffffu, nm != m)) {
+      if (__any_sync(0xffffffffu, nm != nm)) nm = fmaxf(m, scores_joined(c, n_valid, lane, s));
+      rescale(nm);
+    }
+  }
   // probabilities of a tile's scores under the maximum, times its values
   __device__ __forceinline__ void values(const float (&s)[2][2], const __half* v, int lane) {
     uint32_t a[4];
@@ -186,11 +194,7 @@ struct WarpFlash {
   __device__ __forceinline__ void step(const __half* stage, int n_valid, int lane) {
     float c[2][2][4], s[2][2];
     products(stage, lane, c);
-    float nm = wf_max_nan(m, scores(c, n_valid, lane, s));
-    if (__any_sync(0xffffffffu, nm != m)) {
-      if (__any_sync(0xffffffffu, nm != nm)) nm = fmaxf(m, scores_joined(c, n_valid, lane, s));
-      rescale(nm);
-    }
+    softmax(c, n_valid, lane, s);
     values(s, stage + kTile, lane);
   }
 
@@ -223,18 +227,18 @@ struct WarpFlash {
 
 // Head hg of the results that n_w (up to eight) warps left, the w-th at slot s = (first + w) & mask, ml + 16 s and
 // out + s * stride: lane's HEAD / 32 dims, the maximum and the sum, warps in ascending order.
-template <int HEAD, bool ALL>
-__device__ __forceinline__ void wf_merge_n(const float* ml, const float* out, size_t stride, int n_w, int hg, int lane,
-                                           float (&acc)[HEAD / 32], float& m, float& l, int first, int mask) {
+template <int HEAD>
+__device__ __forceinline__ void wf_merge(const float* ml, const float* out, size_t stride, int n_w, int hg, int lane,
+                                         float (&acc)[HEAD / 32], float& m, float& l, int first = 0, int mask = 15) {
   constexpr int DPL = HEAD / 32;
   float mw = -INFINITY, lw = 0.f, o[8][DPL];             // lane w: maximum and sum of warp w
-  if (ALL || (lane & 7) < n_w) {
+  if ((lane & 7) < n_w) {
     const float2 v = *reinterpret_cast<const float2*>(ml + 16 * ((first + (lane & 7)) & mask) + 2 * hg);
     mw = fmaxf(mw, v.x); lw = v.y;
   }
 #pragma unroll
   for (int w = 0; w < 8; ++w)
-    if (ALL || w < n_w) {
+    if (w < n_w) {
       const float* src = out + ((first + w) & mask) * stride + hg * WarpFlash<HEAD>::kOut + lane * DPL;
       if constexpr (DPL == 4) {
         const float4 v = *reinterpret_cast<const float4*>(src);
@@ -254,18 +258,12 @@ __device__ __forceinline__ void wf_merge_n(const float* ml, const float* out, si
 #pragma unroll
   for (int w = 0; w < 8; ++w) {
     const float kw = __shfl_sync(0xffffffffu, k, w), ls = __shfl_sync(0xffffffffu, lw, w);
-    if (ALL || w < n_w) {
+    if (w < n_w) {
       l = fmaf(ls, kw, l);
 #pragma unroll
       for (int d = 0; d < DPL; ++d) acc[d] = fmaf(o[w][d], kw, acc[d]);
     }
   }
-}
-template <int HEAD>
-__device__ __forceinline__ void wf_merge(const float* ml, const float* out, size_t stride, int n_w, int hg, int lane,
-                                         float (&acc)[HEAD / 32], float& m, float& l, int first = 0, int mask = 15) {
-  if (n_w == 8) wf_merge_n<HEAD, true>(ml, out, stride, n_w, hg, lane, acc, m, l, first, mask);
-  else wf_merge_n<HEAD, false>(ml, out, stride, n_w, hg, lane, acc, m, l, first, mask);
 }
 
 }  // namespace bl
