@@ -162,7 +162,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     uint32_t part = 0, pphase = 0;
     bool ok = true;
     int ti = 0;
-    for (int t = blockIdx.x; t < total_tiles && ok && !*abort_flag; t += gridDim.x, ++ti) {
+    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++ti) {
       const F8Tile mt = a.tiles[t / a.tiles_w];
       const int n = (t % a.tiles_w) * F8_BM + q * 32 + lane;         // weight row = output column of this thread
       const bool n_ok = n < a.N;
@@ -175,14 +175,14 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
       const float4* ws24 = reinterpret_cast<const float4*>(ws2);
       float4 w_cur = ws4[0], w_nxt = w_cur, w2_cur = DUAL ? ws24[0] : make_float4(0.f, 0.f, 0.f, 0.f), w2_nxt = w2_cur;
       // the activation scales of this tile's 32 tokens, [kb][token]; rows past the tile scale by zero
-      if (ti > 0 && !mbar_wait(&xs_done, (uint32_t)(ti - 1) & 1u, abort_flag)) break;   // the previous tile's readers are done
+      if (ti > 0 && !mbar_wait_warp(&xs_done, (uint32_t)(ti - 1) & 1u, abort_flag)) break;   // the previous tile's readers are done
       for (int i = et; i < kblocks * F8_BN; i += 128) {
         const int kb = i >> 5, tok = i & 31;
         const int r = mt.row0 + tok;
         s_xs[i] = r < mt.row_end ? a.xs[(long)r * kblocks + kb] : 0.0f;
       }
       mbar_arrive(&xs_ready);
-      if (!mbar_wait(&xs_ready, (uint32_t)ti & 1u, abort_flag)) break;
+      if (!mbar_wait_warp(&xs_ready, (uint32_t)ti & 1u, abort_flag)) break;
       float acc[F8_BN], acc2[DUAL ? F8_BN : 1];
 #pragma unroll
       for (int i = 0; i < F8_BN; ++i) { acc[i] = 0.0f; if (DUAL) acc2[i] = 0.0f; }
@@ -194,7 +194,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
         }
         const float wsc = j == 0 ? w_cur.x : j == 1 ? w_cur.y : j == 2 ? w_cur.z : w_cur.w;
         const float wsc2 = j == 0 ? w2_cur.x : j == 1 ? w2_cur.y : j == 2 ? w2_cur.z : w2_cur.w;
-        if (!mbar_wait(&part_full[part], pphase, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(&part_full[part], pphase, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + part * ACC_COLS;
         uint32_t v[32], u[32];

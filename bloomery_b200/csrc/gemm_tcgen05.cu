@@ -218,7 +218,7 @@ gemm_bf16_kernel(const __grid_constant__ AMaps tma_a, const __grid_constant__ CU
   } else if constexpr (SPLIT) {
     // Park the partial tile: every operand of this CTA has been read by now (its accumulator is complete), so the ring is free.
     const int q = warp & 3;
-    if (first < total_tiles && __all_sync(0xFFFFFFFFu, mbar_wait(&acc_full[0], 0, abort_flag))) {
+    if (first < total_tiles && mbar_wait_warp(&acc_full[0], 0, abort_flag)) {
       tc_fence_after();
       float* park = reinterpret_cast<float*>(smem) + (q * 32 + lane) * SPLIT_ROW;
 #pragma unroll 1
@@ -235,14 +235,14 @@ gemm_bf16_kernel(const __grid_constant__ AMaps tma_a, const __grid_constant__ CU
   } else {
     const int q = warp & 3;                    // TMEM lane quarter of this warp
     int it = 0;
-    for (int t = first; t < total_tiles && !*abort_flag; t += step) {
+    for (int t = first; t < total_tiles; t += step) {
       const MTile mt = a.mtiles[t / a.tiles_n];
       const int n0 = (t % a.tiles_n) * BN;
       if (!DIST && tile_skipped(mt, n0)) continue;
       const int ab = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
       ++it;
-      if (!mbar_wait(&acc_full[ab], acc_phase, abort_flag)) break;
+      if (!mbar_wait_warp(&acc_full[ab], acc_phase, abort_flag)) break;
       tc_fence_after();
       const int r = mt.row0 + q * 32 + lane;                 // product row of this thread
       const bool live = r < mt.row_end;

@@ -52,7 +52,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
-// The wait of a whole warp, which stays converged.
+// The wait of a whole warp, which stays converged: a limit that runs out for some lanes ends it for all, as the tensor-memory
+// loads and the elections behind it need.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_flag)) != 0;
 }

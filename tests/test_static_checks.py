@@ -120,3 +120,18 @@ def test_decode_attention_sets_its_shared_memory_limits_on_every_device():
     """A flag that remembers one call leaves the second device of a process at 48 KB, where the launch is refused."""
     text = open(os.path.join(ROOT, "bloomery_b200", "csrc", "attn_decode.cu")).read()
     assert text.count("MaxDynamicSharedMemorySize") >= 4 and "static bool" not in text
+
+
+def test_waits_in_front_of_warp_wide_instructions_are_warp_wide():
+    """A limit that runs out may do so for some lanes only; a tensor-memory load, an election or a barrier that the others then
+    reach without them has no defined outcome.  Only the single threads that issue copies wait for themselves (for a free slot)."""
+    bad = []
+    for path in _device_sources():
+        text = open(path, encoding="utf-8").read()
+        if "tmem_ld" not in text or path.endswith("tc_common.cuh"):
+            continue
+        for i, ln in enumerate(text.splitlines()):
+            for name in re.findall(r"(?<!__all_sync\(0xFFFFFFFFu, )(?<!__all_sync\(0xffffffffu, )mbar_wait\(&(\w+)", ln):
+                if name not in ("empty_bar", "raw_empty", "k_empty", "v_empty"):
+                    bad.append(f"{os.path.relpath(path, ROOT)}:{i + 1}: lanes wait for {name} one by one")
+    assert not bad, "\n".join(bad)
