@@ -22,6 +22,8 @@
 // and bf16_mma_gemm in crates/gpu/src/q8f32.rs; the reference has no sm_100 path at all.
 #include "tc_common.cuh"
 
+#include <atomic>
+
 namespace bl {
 
 constexpr int BM = 128, BK = 64;               // BK * 2 bytes = 128 = one swizzle atom row
@@ -93,8 +95,8 @@ __device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, 
 // The cluster form (SPLIT): a product of fewer tiles than half the processors gives each tile to a cluster of 2, 4 or 8 CTAs,
 // which walk equal shares of its depth.  Every CTA parks its partial tile in its own (by then idle) operand ring, and
 // each adds up its share of the rows from all of them over distributed shared memory, in ascending order.  One CTA streams
-// its operands at about 0.47 us per 64-deep step, whatever the rest of the chip does: the output projection of a prompt of
-// 512 (32 tiles, 4,096 deep) took 36 us and the router (4 tiles, 6,144 deep) 40 us; as clusters of 4 and 8 the two take 34.
+// its operands at about 0.4 to 0.5 us per 64-deep step, whatever the rest of the chip does: the output projection of a prompt
+// of 512 (32 tiles, 64 steps) took 36 us and the router (4 tiles, 96 steps) 40 us; as clusters of 4 and 8 the two take 34.
 constexpr int SPLIT_ROW = 256 + 4;             // floats of a parked row: 16-byte aligned, and rows start four banks apart
 
 __device__ __forceinline__ void cluster_arrive_release() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
@@ -379,13 +381,40 @@ gemm_bf16_kernel(const __grid_constant__ AMaps tma_a, const __grid_constant__ CU
   if (threadIdx.x == 0 && s_abort && a.status) atomicMax(a.status, 1u);
 }
 
-// CTAs that share the depth of each of `tiles` tiles: the most (up to 8) that leave every CTA a processor of its own and at
+constexpr size_t kGemmSmem = (size_t)STAGES * (TILE_A_BYTES + 2 * TILE_B128_BYTES) + 1024;
+
+// Clusters of 2 << i CTAs of the cluster form that this device holds at once.  A CTA takes a processor, and a cluster lies within
+// one GPC, whose processors are no multiple of it: 15 clusters of 8 run at once, not 18 (the router of 2,048 ids, 16 tiles: 24.0
+// us in two waves of clusters of 8, 16.8 in clusters of 4).
+static int gemm_clusters(int i) {
+  static std::atomic<int> known[64][3];                   // 0: not asked yet
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return 0;
+  if ((n = known[dev][i].load(std::memory_order_relaxed)) > 0) return n;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 2u << i;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.gridDim = dim3(2u << i);
+  cfg.blockDim = dim3(192);
+  cfg.dynamicSmemBytes = kGemmSmem;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  auto kernel = gemm_bf16_kernel<false, false, true>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) return 0;
+  known[dev][i].store(n, std::memory_order_relaxed);
+  return n;
+}
+
+// CTAs that share the depth of each of `tiles` tiles: the most (up to 8) for which all clusters run at once and every CTA has at
 // least eight 64-deep steps.  Eight steps are where a share still hides its start: prompts of 512 tokens, output projection
 // (32 tiles) and router (4 tiles).
 static int gemm_splits(long tiles, int K, int sm_count) {
-  int s = 1;
-  while (s < 8 && tiles * (2 * s) <= sm_count && K / BK >= 16 * s) s *= 2;
-  return s;
+  for (int i = 2; i >= 0; --i)
+    if (K / BK >= 8 * (2 << i) && tiles * (2 << i) <= sm_count && tiles <= gemm_clusters(i)) return 2 << i;
+  return 1;
 }
 
 // ---- tile table ----------------------------------------------------------------------
@@ -516,7 +545,7 @@ static int gemm_launch(const void* const* A_of_rank, int n_src, long lda, long r
   a.tiles_n = (N + (B2 ? BN_DUAL : BN_SINGLE) - 1) / (B2 ? BN_DUAL : BN_SINGLE);
   long tiles = (long)max_mtiles * a.tiles_n;
   int grid = (int)(tiles < sm_count ? tiles : sm_count);
-  const size_t smem = (size_t)STAGES * (TILE_A_BYTES + 2 * TILE_B128_BYTES) + 1024;
+  const size_t smem = kGemmSmem;
   static_assert(BM * SPLIT_ROW * 4 <= STAGES * (TILE_A_BYTES + 2 * TILE_B128_BYTES), "a parked tile fits the ring");
   a.splits = fixed_tiles && !dist && !B2 ? gemm_splits(tiles, K, sm_count) : 1;
   if (a.splits > 1) {
@@ -533,6 +562,11 @@ static int gemm_launch(const void* const* A_of_rank, int n_src, long lda, long r
   static bool s00 = false, s01 = false, s10 = false, s11 = false;
   if (B2) return dist ? go(gemm_bf16_kernel<true, true>, s11) : go(gemm_bf16_kernel<true, false>, s10);
   return dist ? go(gemm_bf16_kernel<false, true>, s01) : go(gemm_bf16_kernel<false, false>, s00);
+}
+
+// CTAs over which a product of rows x N, K deep, of a table that the host wrote (bl_gemm_bf16_fixed) shares each tile's depth.
+int bl_gemm_splits(long rows, int N, int K, int sm_count) {
+  return gemm_splits((rows + BM - 1) / BM * ((N + BN_SINGLE - 1) / BN_SINGLE), K, sm_count);
 }
 
 int bl_gemm_bf16(const void* A, long lda, long rows_a, const void* B, const void* B2, int n_groups, int N, int K,

@@ -68,6 +68,11 @@ class TileTable:
         return t
 
 
+def gemm_splits(rows: int, N: int, K: int) -> int:
+    """CTAs that share the depth of each tile of a [rows, K] x [N, K] product over a table that the host wrote."""
+    return cuda().bl_gemm_splits(L(rows), I(N), I(K), I(sm_count()))
+
+
 def gemm_bf16(A: torch.Tensor, B: torch.Tensor, tiles: TileTable, *, out_f32: Optional[torch.Tensor] = None,
               out_bf16: Optional[torch.Tensor] = None, B2: Optional[torch.Tensor] = None, dst_row=None, row_scale=None,
               resid=None, status: Optional[torch.Tensor] = None) -> None:

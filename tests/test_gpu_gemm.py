@@ -239,7 +239,7 @@ def test_kv_gather_rows_and_transposed_values(n_kv, head, n_keys, T_pad):
 @pytest.mark.parametrize("M,N,K", [(1, 128, 6144), (127, 32, 1024), (129, 160, 1088), (511, 2048, 4096), (300, 5120, 2048),
                                    (640, 288, 1024), (64, 256, 960), (700, 2048, 4096)])
 def test_product_of_few_tiles_over_a_cluster(M, N, K):
-    """Clusters of 8, 8, 8, 4, 2, 2, 1 (too shallow) and 2 CTAs: ragged last tiles on both sides and depths that the shares do
+    """Clusters of 8, 2, 2, 4, 2, 2, 1 (too shallow) and 2 CTAs: ragged last tiles on both sides and depths that the shares do
     not divide, with residual, scatter and bf16 rows; the bits repeat."""
     from bloomery_b200.ops import gemm as G
     g = torch.Generator(device=DEV).manual_seed(M)
@@ -302,3 +302,13 @@ def test_split_rows_of_the_router(K, shift):
     assert torch.equal(out[:, :K], out[:, K:2 * K])
     # value and remainder: 16 bits, and a few fp32 roundings of the scale
     assert float(((out[:, :K].double() + out[:, 2 * K:].double() - ref) / ref.abs().clamp_min(1e-3)).abs().max()) < 2 ** -15
+
+
+@pytest.mark.parametrize("M,N,K,splits", [(127, 32, 4160, 8), (129, 160, 4224, 8), (512, 128, 6144, 8), (511, 2048, 2112, 4), (1, 128, 6144, 8),
+                                          (129, 160, 1088, 2), (64, 256, 960, 1), (2304, 128, 6144, 4)])
+def test_clusters_of_every_size(M, N, K, splits):
+    """Clusters of 8 whose ranks all have rows, ragged rows and columns in them and depths that 8 or 4 do not divide; 18 tiles,
+    whose clusters of 8 would not all run at once."""
+    from bloomery_b200.ops import gemm as G
+    assert G.gemm_splits(M, N, K) == splits
+    test_product_of_few_tiles_over_a_cluster(M, N, K)
