@@ -682,6 +682,10 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
       // than the one kept back here, and stages are used in order.
       constexpr int NG = DUAL ? 2 : 4;                               // groups that share a matrix's stages, two a super-block
       static_assert(NG <= STAGES, "a group's next stage lies at most one turn of the ring ahead");
+      // One matrix: a warp waits for every second raw slot only.  With an odd ring it skips every other phase of a slot, and a wait
+      // by parity would pass two phases early.  It cannot: the warp's own stage of super-block s - 2 waited for the MMAs of stage
+      // 2 (s - 2) - STAGES, so all super-blocks up to s - 2 - STAGES / 2 have been read, and s - RS is one of them.
+      static_assert(DUAL || RS % 2 == 0 || RS <= 2 + STAGES / 2, "no raw slot is two phases behind");
       const int mine = DUAL ? half : grp;
       int rslot = 0, stage = mine, turn = 0, pending = -1;           // stage: this group's next one
       uint32_t rphase = 0, phase = 0;

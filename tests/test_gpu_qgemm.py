@@ -282,3 +282,23 @@ def test_the_split_takes_equal_shares_and_no_more_ctas_than_processors():
         for blocks in (1, 2, 3, 8, 16, 30):
             s = G.qgemm_splits(tiles, blocks, 148)
             assert blocks % s == 0 and (s == 1 or tiles * s <= 148)
+
+
+@pytest.mark.parametrize("t", ["Q4_K", "Q5_K", "Q6_K"])
+def test_deep_products_of_64_rows_turn_every_ring_over(t):
+    """Fourteen super-blocks through raw rings of four to six slots, an odd one with Q5_K, of which each group of expanders waits
+    for every second slot; a slot that was read a turn early would bring another super-block's weights."""
+    from bloomery_b200.ops import gemm as G
+    N, K, rows = 200, 14 * 256, 64
+    qw, ref_w = _weight(t, (N,), K, 5)
+    torch.manual_seed(6)
+    X = (torch.randn(rows, K, device=DEV) * 0.5).bfloat16()
+    st, tiles = _status(), G.TileTable.dense(rows, DEV, 64)
+    C = torch.full((40, rows, N), float("nan"), device=DEV)
+    for c in C:
+        G.qgemm(X, qw, tiles, out_f32=c, status=st)
+    torch.cuda.synchronize()
+    assert int(st) == 0
+    # scales and offsets rounded to bf16: 2^-9 of terms of about 0.1 on each of K weights, times 0.5, added up at random
+    assert torch.allclose(C[0], X.float() @ ref_w.bfloat16().float().T, rtol=1e-2, atol=6e-2)
+    assert [i for i, c in enumerate(C) if not torch.equal(c, C[0])] == []
