@@ -426,9 +426,4 @@ int bl_flash_prefill_split(const void* q, const void* k, const void* vt, void* o
   return (int)launch(flash_prefill_kernel, grid, dim3(FTHREADS), (size_t)FSMEM, st, mq, mk, mv, a);
 }
 
-int bl_flash_prefill(const void* q, const void* k, const void* vt, void* out, long ldo, int T, int n_q, int n_kv, int pos0,
-                     int t_pad, unsigned* status, cudaStream_t st) {
-  return bl_flash_prefill_split(q, k, vt, out, ldo, T, n_q, n_kv, pos0, t_pad, status, 1, nullptr, nullptr, nullptr, st);
-}
-
 }  // extern "C"

@@ -56,7 +56,7 @@ struct QGemmArgs {
   int fixed_tiles;            // the table holds max_tiles tiles and was written before the launches in flight
   int splits;                 // CTAs that share a tile's depth (1 with w2)
   float* partial;             // splits > 1: [tiles][splits][tile rows][128] sums
-  int* tickets;               // splits > 1: four per tile, zero between launches
+  int* tickets;               // splits > 1: one per tile, zero between launches
 };
 
 __device__ __forceinline__ uint4 q_pack8(const float* v) {
@@ -778,8 +778,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
       const int tile = (int)blockIdx.x / a.splits;
       if (threadIdx.x == 0) {
         __threadfence();
-        s_last = tile < n_tt * a.tiles_w && atomicAdd(&a.tickets[tile * 4], 1) == a.splits - 1;
-        if (s_last) a.tickets[tile * 4] = 0;                           // ready for the next launch
+        s_last = tile < n_tt * a.tiles_w && atomicAdd(&a.tickets[tile], 1) == a.splits - 1;
+        if (s_last) a.tickets[tile] = 0;                           // ready for the next launch
         __threadfence();
       }
       __syncthreads();
@@ -881,7 +881,7 @@ int bl_qgemm_supports(int wtype) {
 //   fixed_tiles: the table has exactly max_tiles tiles, and no launch in flight writes the table, W or W2: the warps that
 //   stream and expand weights read all three without waiting for the launch in front of this one.  splits > 1 (fixed tiles, one
 //   matrix, K / 256 divisible): that many CTAs share a tile's depth; partial: max_tiles * ceil(N / 128) * splits *
-//   tile_rows * 128 floats, tickets: max_tiles * ceil(N / 128) * 4 zeroed words, both of one stream at a time.
+//   tile_rows * 128 floats, tickets: max_tiles * ceil(N / 128) zeroed words, both of one stream at a time.
 int bl_qgemm_split(const void* X, long ldx, long rows_x, const void* W, const void* W2, int wtype, int n_groups, int N, int K,
              const void* tiles, const int* n_tiles, int max_tiles, int tile_rows, float* c_f32, void* c_bf16, long ldc,
              const int* dst_row, const float* row_scale, const float* resid, long ldr, unsigned* status, int sm_count,

@@ -248,7 +248,7 @@ def flash_prefill(q_bf: torch.Tensor, Kb: torch.Tensor, Vt: torch.Tensor, out: t
             bufs = work.buffers(pairs, splits)
     rc = cuda().bl_flash_prefill_split(p(q_bf), p(Kb), p(Vt), p(out), L(out.stride(0)), I(T), I(n_q), I(n_kv), I(pos0), I(T_pad),
                                        p(status), I(splits), p(bufs[0]), p(bufs[1]), p(bufs[2]), stream())
-    check(rc, "bl_flash_prefill")
+    check(rc, "bl_flash_prefill_split")
 
 
 def softmax_causal(S, rows: int, Tq: int, pos0: int, T_pad: int, P) -> None:
@@ -277,7 +277,7 @@ class QgemmWork:
         self.tile_rows = tile_rows
         sm = sm_count(device)
         self.partial = torch.empty(sm * tile_rows * 128, dtype=torch.float32, device=device)
-        self.tickets = torch.zeros(sm * 4, dtype=torch.int32, device=device)
+        self.tickets = torch.zeros(sm, dtype=torch.int32, device=device)
 
 
 def qgemm_splits(n_tiles: int, depth_blocks: int, sm: int) -> int:
