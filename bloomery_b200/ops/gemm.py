@@ -291,6 +291,20 @@ def qgemm_splits(n_tiles: int, depth_blocks: int, sm: int) -> int:
     return best
 
 
+def qkv_rooms(q_tiles: int, kv_tiles: int, depth_blocks: int, sm: int):
+    """Processors that Q, and K and V each, may take when the three products of a round run side by side (a CTA fits a
+    processor, so what does not fit waits for another product to end).  K and V take up to a quarter each and Q what they leave:
+    on the 30 B shape (32, 4 and 4 tiles, eight blocks deep) 64, 32 and 32 CTAs, 24 rows in 15 us where Q over all of them with K
+    and V behind it took 36.  Where Q would get fewer shares that way than all three at equal shares (64 Q tiles sixteen
+    blocks deep: one, and a walk of 16 blocks, against two), equal shares are the shorter walk."""
+    kv = qgemm_splits(kv_tiles, depth_blocks, sm // 4)
+    left = max(0, sm - 2 * kv_tiles * kv)
+    equal = qgemm_splits(q_tiles + 2 * kv_tiles, depth_blocks, sm)
+    if equal > qgemm_splits(q_tiles, depth_blocks, left):
+        return q_tiles * equal, kv_tiles * equal
+    return max(1, left), sm // 4
+
+
 def qgemm(X: torch.Tensor, W: QWeight, tiles: TileTable, *, out_f32: Optional[torch.Tensor] = None,
           out_bf16: Optional[torch.Tensor] = None, W2: Optional[QWeight] = None, dst_row=None, row_scale=None,
           resid=None, status: Optional[torch.Tensor] = None, work: Optional[QgemmWork] = None,

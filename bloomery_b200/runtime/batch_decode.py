@@ -276,11 +276,10 @@ class BatchDecode:
         q_scale = 1.0 / math.sqrt(s.head_dim)
         n = 0
         # the three projections are small grids (32 + 4 + 4 weight tiles on the 30 B shape): K and V run on side
-        # streams beside Q (parallel branches of the captured graph).  One CTA fits a processor: Q splits its depth over
-        # half of them and K and V over a quarter each, so that none of the three waits for another to end (Q over all of
-        # them, K and V behind it: 36 us a layer of a round of 24)
+        # streams beside Q (parallel branches of the captured graph), each split over processors of its own
         main = torch.cuda.current_stream(e.device)
-        sm = K.sm_count(e.device)
+        n_tiles = lambda rows: tiles.fixed * ((rows + 127) // 128)                                    # noqa: E731
+        q_room, kv_room = G.qkv_rooms(n_tiles(s.q_rows), n_tiles(s.kv_rows), s.hidden // 256, K.sm_count(e.device))
         x8 = None
         if any(self._native_fp8(w.q[b + nm]) for nm in ("attn_q.weight", "attn_k.weight", "attn_v.weight")):
             x8 = self._q8(xn); n += 1                            # one E4M3 form of the rows for the three products
@@ -292,11 +291,11 @@ class BatchDecode:
             side = self._side[branch - 1]
             side.wait_event(fork)
             with torch.cuda.stream(side):
-                n += self._mm(xn, w.q[b + name], tiles, M, x8=x8, branch=branch, room=sm // 4, out_f32=self.qkv[:M, lo:hi])
+                n += self._mm(xn, w.q[b + name], tiles, M, x8=x8, branch=branch, room=kv_room, out_f32=self.qkv[:M, lo:hi])
                 ev = torch.cuda.Event()
                 ev.record(side)
                 joins.append(ev)
-        n += self._mm(xn, w.q[b + "attn_q.weight"], tiles, M, x8=x8, room=sm // 2, out_f32=self.qkv[:M, :s.q_rows])
+        n += self._mm(xn, w.q[b + "attn_q.weight"], tiles, M, x8=x8, room=q_room, out_f32=self.qkv[:M, :s.q_rows])
         for ev in joins:
             main.wait_event(ev)
         kvp = e.kv

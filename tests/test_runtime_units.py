@@ -690,3 +690,21 @@ def test_a_prompt_path_keeps_the_engine_it_was_given_and_an_engine_not_itself(mo
         gone = weakref.ref(eng)
         del eng
         assert gone() is None                                    # by reference count alone
+
+
+def test_q_k_and_v_share_the_processors():
+    """The three products of a round fit side by side wherever one of them is split, and Q is split as often as K and V leave room
+    for or as equal shares allow, whichever is more."""
+    from bloomery_b200.ops.gemm import qgemm_splits, qkv_rooms
+    shares = lambda q, kv, d, sm: tuple(qgemm_splits(t, d, r) for t, r in zip((q, kv), qkv_rooms(q, kv, d, sm)))      # noqa: E731
+    assert shares(32, 4, 8, 148) == (2, 8)               # 4,096 query rows over 2,048 hidden values
+    assert shares(64, 4, 16, 148) == (2, 2)              # 8,192 over 4,096: half of the processors would leave Q unsplit
+    assert shares(40, 8, 20, 148) == (2, 4)
+    for sm in (1, 16, 132, 148):
+        for q in (1, 4, 32, 40, 64, 128, 300):
+            for kv in (1, 2, 4, 8, 32):
+                for d in (1, 2, 8, 10, 16, 30):
+                    a, b = shares(q, kv, d, sm)
+                    assert d % a == 0 and d % b == 0
+                    assert a == b == 1 or q * a + 2 * kv * b <= sm or (a == 1 and 2 * kv * b <= sm // 2)
+                    assert a >= qgemm_splits(q + 2 * kv, d, sm)
