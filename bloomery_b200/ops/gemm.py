@@ -206,8 +206,12 @@ def kv_gather_bf16(k_cache, v_cache, block_table_row, n_pages: int, n_kv: int, h
                                    I(T_pad), p(Kb), p(Vt), stream()), "bl_kv_gather_bf16")
 
 
+FLASH_WORK_BYTES = 128 << 20          # what shares of prompt attention may leave in memory: four of 2,048 ids of 32 heads over 4
+
+
 class FlashWork:
-    """Partial outputs and tickets of prompt attention whose CTAs share their keys: one per stream that runs it."""
+    """Partial outputs and tickets of prompt attention whose CTAs share their keys: one per stream that runs it.  It grows to
+    the largest prompt it has seen, ``FLASH_WORK_BYTES`` at most (see ``flash_splits``)."""
 
     def __init__(self, device):
         self.device = device
@@ -226,9 +230,9 @@ class FlashWork:
 def flash_splits(pairs: int, key_tiles: int, sm: int) -> int:
     """CTAs that share the key tiles of a pair of query tiles: the number that ends first, counted in key tiles of a CTA times
     waves of CTAs.  A share costs about four key tiles on top (its start, its partial output and the merge), so it has to
-    hold sixteen."""
+    hold sixteen, and its two tiles leave 128 KB each of the bounded workspace."""
     cost = lambda s: -(-pairs * s // sm) * (-(-key_tiles // s) + (4 if s > 1 else 0))      # noqa: E731
-    return min((s for s in range(1, 5) if s == 1 or key_tiles >= 16 * s), key=cost)
+    return min((s for s in range(1, 5) if s == 1 or (key_tiles >= 16 * s and pairs * s << 17 <= FLASH_WORK_BYTES)), key=cost)
 
 
 def flash_prefill(q_bf: torch.Tensor, Kb: torch.Tensor, Vt: torch.Tensor, out: torch.Tensor, pos0: int,

@@ -708,3 +708,16 @@ def test_q_k_and_v_share_the_processors():
                     assert d % a == 0 and d % b == 0
                     assert a == b == 1 or q * a + 2 * kv * b <= sm or (a == 1 and 2 * kv * b <= sm // 2)
                     assert a >= qgemm_splits(q + 2 * kv, d, sm)
+
+
+def test_shares_of_prompt_attention_fit_their_workspace():
+    """Whatever the prompt and the model, the partial outputs that the shares leave stay within the stated bytes; few query tiles
+    behind a long prefix are still shared."""
+    from bloomery_b200.ops.gemm import FLASH_WORK_BYTES, FlashWork, flash_splits
+    for pairs in list(range(1, 1500, 7)) + [256, 512, 1024, 4096]:
+        for keys in (1, 15, 33, 71, 128, 1000):
+            s = flash_splits(pairs, keys, 148)
+            assert s == 1 or (keys >= 16 * s and 2 * pairs * s * 16384 * 4 <= FLASH_WORK_BYTES)
+    assert flash_splits(96, 71, 148) == 3 and flash_splits(256, 128, 148) == 4 and flash_splits(512, 500, 148) == 2
+    part, ml, tickets = FlashWork("cpu").buffers(3, 4)
+    assert part.numel() == 2 * 3 * 4 * 16384 and ml.numel() == 2 * 3 * 4 * 256 and int(tickets.abs().sum()) == 0
