@@ -1,6 +1,7 @@
 // Shared device helpers: fault word, programmatic dependent launch, reductions,
 // the block-level q8 activation quantiser and the launch wrapper.
 #pragma once
+#include <atomic>
 #include <cuda_runtime.h>
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
@@ -302,6 +303,17 @@ inline cudaError_t launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
   cfg.numAttrs = g_use_pdl ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
+
+// What is to be done once on every device that a process uses (a kernel's shared-memory limit belongs to a device):
+//   static PerDevice limit; if (limit.due()) { ...; limit.mark(); }
+class PerDevice {
+ public:
+  bool due() const { const int d = device(); return d < 0 || !(done_.load(std::memory_order_acquire) >> d & 1); }
+  void mark() { const int d = device(); if (d >= 0) done_.fetch_or(1ull << d, std::memory_order_release); }
+ private:
+  static int device() { int d = 0; return cudaGetDevice(&d) == cudaSuccess && d < 64 ? d : -1; }
+  std::atomic<unsigned long long> done_{0};
+};
 
 // Host-side launch contract: a failed check returns a negative code and launches nothing.
 #define BL_REQUIRE(cond, code) \

@@ -233,10 +233,10 @@ static size_t gemv_smem(int MB, int K, bool floatw) {
 template <int MB, int R, int C, bool NORM, int FAM>
 static cudaError_t gemv_launch(const GemvArgs& a, int grid, cudaStream_t st) {
   size_t smem = gemv_smem(MB, a.K, FAM == 1);
-  static bool attr_set = false;
-  if (!attr_set) {
+  static PerDevice limit;
+  if (limit.due()) {
     cudaFuncSetAttribute(gemv_kernel<MB, R, C, NORM, FAM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    attr_set = true;
+    limit.mark();
   }
   return launch(gemv_kernel<MB, R, C, NORM, FAM>, dim3(grid), dim3(256), smem, st, a);
 }

@@ -1425,10 +1425,10 @@ constexpr size_t kStagedSliceMax = 100 * 1024;   // a block's weight rows (two s
 
 template <int MB, bool NORM, int FAM>
 static cudaError_t gemv_staged_launch(const GemvArgs& a, int grid, size_t smem, cudaStream_t st) {
-  static bool attr_set = false;
-  if (!attr_set) {
+  static PerDevice limit;
+  if (limit.due()) {
     cudaFuncSetAttribute(gemv_staged_kernel<MB, NORM, FAM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStagedSmemMax);
-    attr_set = true;
+    limit.mark();
   }
   return launch(gemv_staged_kernel<MB, NORM, FAM>, dim3(grid), dim3(256), smem, st, a);
 }
@@ -1445,11 +1445,11 @@ static cudaError_t gemv_staged_dispatch(const GemvArgs& a, int mb, int grid, siz
 
 template <int HEAD, int HPW>
 static int attn_cluster_launch(const AttnArgs& a, int CL, int n_kv, int M, size_t smem, cudaStream_t st) {
-  static bool attr_set = false;
-  if (!attr_set) {
+  static PerDevice limit;
+  if (limit.due()) {
     cudaFuncSetAttribute(attn_cluster_kernel<HEAD, HPW>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     cudaFuncSetAttribute(attn_cluster_kernel<HEAD, HPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
-    attr_set = true;
+    limit.mark();
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(CL, n_kv, M);
@@ -1570,9 +1570,13 @@ int bl_attn_fused(const float* qkv, long qkv_stride, const float* q_gain, const 
     const long most = (long)n_seg * M;
     grid = dim3((unsigned)(blocks < M ? M : blocks > most ? most : blocks), n_kv, 1);
   }
+  static PerDevice limit[8];
   auto go = [&](auto kernel, size_t bytes) {
-    // a kernel's shared-memory limit belongs to a device, and stages of one process may sit on several: set on every call
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (G <= 8 ? 225 : 110) * 1024) != cudaSuccess) return (int)BL_ERR_LIMIT;
+    PerDevice& one = limit[(deal ? 4 : 0) + (head == 128 ? 2 : 0) + (G <= 8 ? 1 : 0)];
+    if (one.due()) {
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (G <= 8 ? 225 : 110) * 1024) != cudaSuccess) return (int)BL_ERR_LIMIT;
+      one.mark();
+    }
     return (int)launch(kernel, grid, dim3(256), bytes, st, a);
   };
   if (deal) {
@@ -1626,10 +1630,10 @@ int bl_gate_up_staged(const int8_t* xq, const float* xds, const float* route_log
   GateUpStagedArgs a{xq, (const float2*)xds, RouteParams{route_logits, bias, E, n_used, mode, renorm, scale, n_group, topk_group},
                      ids, wts, heat, slot_map, (const uint8_t*)gate, (const uint8_t*)up, wtype,
                      (const uint8_t*)down, down_expert_bytes, K, I, E, n_used, M, actq, (float2*)actds, act_f32, fault, layer, g_stage_probe};
-  static bool attr_set = false;
-  if (!attr_set) {
+  static PerDevice limit;
+  if (limit.due()) {
     cudaFuncSetAttribute(gate_up_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStagedSmemMax);
-    attr_set = true;
+    limit.mark();
   }
   return (int)launch(gate_up_staged_kernel, dim3(I / 32, n_used, M), dim3(256), smem, st, a);
 }
@@ -1656,15 +1660,15 @@ int bl_down_staged(const int8_t* actq, const float* actds, const int* ids, const
                    resid, resid_stride, extra, extra_stride, out, out_stride, fault, layer, PushOut{}, g_stage_probe};
   if (push_desc) { a.push = *(const PushOut*)push_desc; BL_REQUIRE(a.push.n_ranks <= kMaxRanks && M <= kMaxRows, BL_ERR_SHAPE); }
   dim3 grid((H + rpb - 1) / rpb, M);
-  static bool attr_set = false;
-  if (!attr_set) {
+  static PerDevice limit;
+  if (limit.due()) {
     cudaFuncSetAttribute(down_staged_kernel<3, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStagedSmemMax);
     cudaFuncSetAttribute(down_staged_kernel<6, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStagedSmemMax);
     cudaFuncSetAttribute(down_staged_kernel<16, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStagedSmemMax);
     cudaFuncSetAttribute(down_staged_kernel<3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStagedSmemMax);
     cudaFuncSetAttribute(down_staged_kernel<6, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStagedSmemMax);
     cudaFuncSetAttribute(down_staged_kernel<16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStagedSmemMax);
-    attr_set = true;
+    limit.mark();
   }
   if (staged_fam(dtype) == 0) {
     if (total <= 96) return (int)launch(down_staged_kernel<3, 0>, grid, dim3(256), smem, st, a);

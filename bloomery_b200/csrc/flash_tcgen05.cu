@@ -416,10 +416,10 @@ int bl_flash_prefill_split(const void* q, const void* k, const void* vt, void* o
   }
   FlashPrefillArgs a{T, n_q, n_kv, n_q / n_kv, pos0, t_pad, (__nv_bfloat16*)out, ldo, status,
                      splits, (float4*)part, (float2*)part_ml, tickets};
-  static bool attr_set = false;
-  if (!attr_set) {
+  static PerDevice limit;
+  if (limit.due()) {
     cudaFuncSetAttribute(flash_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FSMEM);
-    attr_set = true;
+    limit.mark();
   }
   const int items = (T + FQ - 1) / FQ * (n_q / n_kv);           // query tiles of a KV head
   dim3 grid((unsigned)((items + 1) / 2 * n_kv * splits));

@@ -328,10 +328,10 @@ static int fp8_gemm_go(const CUtensorMap& mx, const F8Args& a0, int n_groups, in
   if (rc) return rc;
   mw2 = mw;
   if (DUAL) { rc = make_map_any(&mw2, a.w2, 3, dims, str, box, CU_TENSOR_MAP_DATA_TYPE_UINT8, CU_TENSOR_MAP_SWIZZLE_128B); if (rc) return rc; }
-  static bool set = false;
-  if (!set) {
+  static PerDevice limit;
+  if (limit.due()) {
     cudaFuncSetAttribute(fp8_gemm_kernel<DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
-    set = true;
+    limit.mark();
   }
   return (int)launch(fp8_gemm_kernel<DUAL>, dim3(grid), dim3(F8_THREADS), smem, st, mx, mw, mw2, a);
 }

@@ -548,18 +548,15 @@ static int gemm_launch(const void* const* A_of_rank, int n_src, long lda, long r
   const size_t smem = kGemmSmem;
   static_assert(BM * SPLIT_ROW * 4 <= STAGES * (TILE_A_BYTES + 2 * TILE_B128_BYTES), "a parked tile fits the ring");
   a.splits = fixed_tiles && !dist && !B2 ? gemm_splits(tiles, K, sm_count) : 1;
-  if (a.splits > 1) {
-    // an attribute of the device's context: a process may have several
-    if (cudaFuncSetAttribute(gemm_bf16_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      return BL_ERR_LIMIT;
+  if (a.splits > 1) {                          // (gemm_clusters has set this device's shared-memory limit)
     return (int)launch_cluster(gemm_bf16_kernel<false, false, true>, dim3((unsigned)(tiles * a.splits)), dim3(192), smem, a.splits, st,
                                ma, mb, mb2, a);
   }
-  auto go = [&](auto kernel, bool& set) {
-    if (!set) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); set = true; }
+  auto go = [&](auto kernel, PerDevice& limit) {
+    if (limit.due()) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); limit.mark(); }
     return (int)launch(kernel, dim3(grid), dim3(192), smem, st, ma, mb, mb2, a);
   };
-  static bool s00 = false, s01 = false, s10 = false, s11 = false;
+  static PerDevice s00, s01, s10, s11;
   if (B2) return dist ? go(gemm_bf16_kernel<true, true>, s11) : go(gemm_bf16_kernel<true, false>, s10);
   return dist ? go(gemm_bf16_kernel<false, true>, s01) : go(gemm_bf16_kernel<false, false>, s00);
 }

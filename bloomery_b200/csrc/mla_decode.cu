@@ -478,10 +478,10 @@ int bl_mla_flash_decode(const float* q_lat, const void* cache, const int* row_po
   BL_REQUIRE(wtype == 0 || wtype == 30, BL_ERR_TYPE);
   const size_t smem = (size_t)kHeadsPerBlock * kRowPad * 2 + (size_t)2 * kTile * kRowPad * 2 +
                       (size_t)(kHeadsPerBlock * kSStride + 4 * 16 * 8) * 4 + (size_t)kHeadsPerBlock * kPStride * 2 + 16 * 4;
-  static bool attr_set = false;
-  if (!attr_set) {
+  static PerDevice limit;
+  if (limit.due()) {
     cudaFuncSetAttribute(mla_flash_seg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attr_set = true;
+    limit.mark();
   }
   MlaFlashArgs f{q_lat, (const __half*)cache, row_pos, row_seq, block_table, max_pages, n_pages, n_q, M, n_seg, ctx_limit,
                  part_ml, part_acc, fault, layer};

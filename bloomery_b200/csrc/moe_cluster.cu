@@ -426,7 +426,8 @@ static int moe_cluster_check(int H, int I, int E, int n_used, int rtype, int gty
 
 template <int FAM>
 static int moe_cluster_launch(const MoeClusterArgs& a, int smem, int n_used, cudaStream_t st, bool query_only) {
-  static int max_clusters = -1;
+  static PerDevice limit;
+  static std::atomic<int> max_clusters{0};                 // of one device as of another of its kind
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(kCl, n_used, 1);
   cfg.blockDim = dim3(256);
@@ -438,7 +439,7 @@ static int moe_cluster_launch(const MoeClusterArgs& a, int smem, int n_used, cud
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  if (max_clusters < 0) {
+  if (limit.due()) {
     cudaError_t e = cudaFuncSetAttribute(moe_cluster_kernel<FAM>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(moe_cluster_kernel<FAM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 217 * 1024);
     if (e != cudaSuccess) { cudaGetLastError(); return BL_ERR_LIMIT; }
@@ -447,6 +448,7 @@ static int moe_cluster_launch(const MoeClusterArgs& a, int smem, int n_used, cud
     e = cudaOccupancyMaxActiveClusters(&n, moe_cluster_kernel<FAM>, &cfg);
     if (e != cudaSuccess) { cudaGetLastError(); n = 0; }
     max_clusters = n;
+    limit.mark();
   }
   // every chosen expert's cluster must be resident at once, or the launch would run in waves
   if (max_clusters < n_used) return BL_ERR_LIMIT;

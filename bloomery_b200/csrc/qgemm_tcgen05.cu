@@ -833,10 +833,10 @@ static int qgemm_go(const CUtensorMap& mx, const QGemmArgs& a, int n_groups, int
     if (rc) return rc;
     if (DUAL) { rc = make_map_u8(&mw2, a.w2, 3, dims, str, box); if (rc) return rc; }
   }
-  static bool set = false;
-  if (!set) {
+  static PerDevice limit;
+  if (limit.due()) {
     cudaFuncSetAttribute(qgemm_kernel<T, DUAL, BN, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    set = true;
+    limit.mark();
   }
   return (int)launch(qgemm_kernel<T, DUAL, BN, FORM>, dim3(grid), dim3(QTHREADS), smem, st, mx, mw, mw2, a);
 }

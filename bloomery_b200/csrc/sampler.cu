@@ -406,8 +406,8 @@ int bl_sample_rows_split(const float* logits, long stride, int V, int M, const i
   const int per_blk = (V + kSelBlocks - 1) / kSelBlocks;
   const size_t smem = (size_t)per_blk * 4;
   BL_REQUIRE(smem <= 200 * 1024, BL_ERR_LIMIT);
-  static bool set = false;
-  if (!set) { cudaFuncSetAttribute(sample_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); set = true; }
+  static PerDevice limit;
+  if (limit.due()) { cudaFuncSetAttribute(sample_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); limit.mark(); }
   SelectArgs sa{logits, stride, V, recent, recent_stride, n_recent, params, cand_val, cand_id, cap};
   cudaError_t e = launch(sample_select_kernel, dim3(kSelBlocks, M), dim3(1024), smem, st, sa);
   if (e != cudaSuccess) return (int)e;

@@ -135,3 +135,13 @@ def test_waits_in_front_of_warp_wide_instructions_are_warp_wide():
                 if name not in ("empty_bar", "raw_empty", "k_empty", "v_empty"):
                     bad.append(f"{os.path.relpath(path, ROOT)}:{i + 1}: lanes wait for {name} one by one")
     assert not bad, "\n".join(bad)
+
+
+def test_kernel_attributes_are_set_on_every_device():
+    """A kernel's limits belong to a device, and stages of one process may sit on several: no flag of the process remembers them."""
+    bad = []
+    for path in _device_sources():
+        text = open(path, encoding="utf-8").read()
+        if "cudaFuncSetAttribute" in text:
+            bad += [f"{os.path.relpath(path, ROOT)}: {m}" for m in re.findall(r"static (?:bool|int) \w+ = (?:false|-1)[^;]*;", text)]
+    assert not bad, "\n".join(bad)
