@@ -228,8 +228,8 @@ __device__ __forceinline__ RowSegs row_segs(const AttnArgs& a, int mm) {
 // One row: grid (n_seg, n_kv, 1), a block a segment.  Several rows (DEAL): grid (blocks, n_kv), as many blocks as the processors
 // hold at once, because one fits a processor and each has a start of its own; they are dealt to the rows by their key tiles,
 // and a block walks several segments of its row.  30 B shape, us a layer, a block a segment / dealt: five rows of 900 to 2,200
-// keys (480 blocks) 30.8 / 15.1, eight of 5,000 68 / 25.9, eight of 15,000 103 / 61, one of 12,000 beside seven of 100 23.9 /
-// 19.0.  (Segments cut by the number of rows instead took 13.0, 22.4, 48.7 and 34.4, and made a row's bits depend on the rows
+// keys (480 blocks) 30.8 / 13.9, eight of 5,000 68 / 25.1, eight of 15,000 103 / 59, one of 12,000 beside seven of 100 23.9 /
+// 17.8.  (Segments cut by the number of rows instead took 13.0, 22.4, 48.7 and 34.4, and made a row's bits depend on the rows
 // beside it.)
 template <int HEAD, int HPW, bool DEAL>
 __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const AttnArgs a) {
@@ -249,6 +249,8 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
   static_assert(8 * (kWfTiles * W::kTile * 2 + 2 * 8 * W::kOut * 4) == kAllTiles * W::kTile * 2, "whole tiles");
   constexpr int kAloneSteps = HEAD / 8;                    // steps whose scores and maxima (17 float4 a lane group) fit two tiles
   static_assert(kAloneSteps / 2 * (32 * 16 + 8 * 4) <= W::kTile * 2, "half of them fit one");
+  // what the merge at the end may use from `rings` on
+  constexpr int kMergeBytes = DEAL && HPW == 1 ? kAllTiles * W::kTile * 2 : HPW == 1 ? 8 * RING * 2 : kStages * kKeyTile * (KSTR + HEAD) * 2;
   constexpr size_t kResStride = DEAL ? 8 * W::kOut : RING / 2;
   __half* snew = HPW == 1 ? reinterpret_cast<__half*>(rings + (size_t)8 * RING * 2 + (DEAL ? (size_t)16 * 8 * W::kOut * 4 : 0))
                           : sv + kStages * kKeyTile * HEAD;        // [patch rows][2][HEAD]: keys and values of this pass
@@ -343,7 +345,8 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
   };
   At cur{warp / per, warp % per, warp % per}, ahead = cur;
   // DEAL: a block of many short segments gives each to one warp, tiles of keys and then of values (see below).  In steps one behind the other: 2 tps for up to eight segments, against about two and a half a turn.  Eight rows of
-  // 3,000 keys, eight segments a block: 20.6 us alone, 26.6 in turns; three of 9,000, three a block: 27.7 and 22.1.
+  // 3,000 keys, eight segments a block: 20.6 us alone, 26.6 in turns; three of 9,000, three a block: 27.7 and 22.1
+  // (before the merge at the end read all parts at once).
   const bool alone = DEAL && HPW == 1 && used > 1 && 2 * tps <= kAloneSteps && 4 * tps * ((n_g + 7) / 8) < 5 * ((n_g * per + 7) / 8);
   // All tiles of shared memory are then the active warps' own: scores, and a ring that holds the whole segment where it can, so
   // that keys and values arrive while the launch in front still runs.
@@ -777,52 +780,50 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
     const int hg = warp + 8 * h;
     if (hg < G) {
       const long p0 = ((long)m * a.n_q + (long)kvh * G + hg) * a.n_seg;
-      // lanes fetch the segments' (max, sum) pairs side by side and the accumulators kTrip segments per round trip (16: one row
-      // of 12,000 keys 13.2 us, eight 15.9; several rows run behind longer code, and more of it costs what it saves); the
-      // sums themselves run over the segments in ascending order
-      constexpr int kTrip = DEAL ? 8 : 16;
-      float v[kTrip][DPL];
-      auto fetch = [&](int s0) {
-#pragma unroll
-        for (int k = 0; k < kTrip; ++k) {
-          if (s0 + k < used) {
-            const float* src = a.part_acc + (p0 + s0 + k) * HEAD + lane * DPL;
-            if constexpr (DPL == 4) {
-              const float4 t = __ldcg(reinterpret_cast<const float4*>(src));
-              v[k][0] = t.x; v[k][1] = t.y; v[k][2] = t.z; v[k][3] = t.w;
-            } else {
-              const float2 t = __ldcg(reinterpret_cast<const float2*>(src));
-              v[k][0] = t.x; v[k][1] = t.y;
-            }
-          }
-        }
+      // The accumulators of a head lie one behind the other: all of them (`cap` at a time) come into the warp's share of the
+      // rings in one round trip, in a short loop, while its lanes fetch the (max, sum) pairs; the sums run over the segments
+      // in ascending order.  (Eight or sixteen a round trip through registers: one row of 12,000 keys 13.2 us, 12.7 now; five of
+      // 1,500 15.1, 13.9 now.  Thirty-two: longer code, and slower behind the other launches of a layer.)
+      constexpr int cap = kMergeBytes / 8 / (HEAD * 4);
+      float* const buf = reinterpret_cast<float*>(rings) + warp * cap * HEAD;
+      auto copy = [&](int s0) {
+        const float* src = a.part_acc + (p0 + s0) * HEAD;
+        for (int c = lane; c < min(cap, used - s0) * (HEAD / 4); c += 32) cp_async16(buf + 4 * c, src + 4 * c);
+        cp_async_commit();
       };
       auto pair_of = [&](int sg) { return sg < used ? __ldcg(reinterpret_cast<const float2*>(a.part_ml + (p0 + sg) * 2)) : make_float2(-INFINITY, 0.f); };
+      copy(0);
       const float2 first = pair_of(lane), second = pair_of(32 + lane);
-      fetch(0);
       float gm = fmaxf(first.x, second.x);
       for (int s0 = 64; s0 < used; s0 += 32) gm = fmaxf(gm, pair_of(s0 + lane).x);
       gm = warp_max(gm);
       float den = 0.f, num[DPL], wl = 0.f, ls = 0.f;
 #pragma unroll
       for (int d = 0; d < DPL; ++d) num[d] = 0.f;
-      for (int s0 = 0; s0 < used; s0 += kTrip) {
-        if (s0 > 0) fetch(s0);
-        if ((s0 & 31) == 0) {
-          const float2 ml = s0 == 0 ? first : s0 == 32 ? second : pair_of(s0 + lane);
-          wl = (ml.x == -INFINITY) ? 0.f : __expf(ml.x - gm);
-          ls = ml.y;
-        }
-        const int cnt = min(kTrip, used - s0);
-#pragma unroll
-        for (int k = 0; k < kTrip; ++k) {
-          if (k < cnt) {
-            const float wk = __shfl_sync(0xffffffffu, wl, (s0 & 31) + k), lk = __shfl_sync(0xffffffffu, ls, (s0 & 31) + k);
-            den = fmaf(lk, wk, den);
-#pragma unroll
-            for (int d = 0; d < DPL; ++d) num[d] = fmaf(v[k][d], wk, num[d]);
+      for (int s0 = 0; s0 < used; s0 += cap) {
+        if (s0 > 0) copy(s0);
+        cp_async_wait<0>();
+        __syncwarp();
+#pragma unroll 4
+        for (int k = 0; k < min(cap, used - s0); ++k) {
+          const int sg = s0 + k;
+          if ((sg & 31) == 0) {
+            const float2 ml = sg == 0 ? first : sg == 32 ? second : pair_of(sg + lane);
+            wl = (ml.x == -INFINITY) ? 0.f : __expf(ml.x - gm);
+            ls = ml.y;
+          }
+          const float wk = __shfl_sync(0xffffffffu, wl, sg & 31), lk = __shfl_sync(0xffffffffu, ls, sg & 31);
+          den = fmaf(lk, wk, den);
+          const float* v = buf + k * HEAD + lane * DPL;
+          if constexpr (DPL == 4) {
+            const float4 t = *reinterpret_cast<const float4*>(v);
+            num[0] = fmaf(t.x, wk, num[0]); num[1] = fmaf(t.y, wk, num[1]); num[2] = fmaf(t.z, wk, num[2]); num[3] = fmaf(t.w, wk, num[3]);
+          } else {
+            const float2 t = *reinterpret_cast<const float2*>(v);
+            num[0] = fmaf(t.x, wk, num[0]); num[1] = fmaf(t.y, wk, num[1]);
           }
         }
+        __syncwarp();
       }
       float o[DPL];
 #pragma unroll
