@@ -470,3 +470,10 @@ def test_engine_row_is_the_row_of_a_pass_of_one():
     eng.step([(1, t, len(prompt) + j) for j, t in enumerate(drafted)])
     for j in range(len(drafted)):
         assert torch.equal(eng.logits[j], one[j]), j
+
+
+@pytest.mark.parametrize("head,n_q,n_kv", [(128, 8, 2), (64, 14, 2), (128, 24, 2)])
+@pytest.mark.parametrize("rows,n_seg", [([(0, 2530)], 80), ([(0, 2530), (1, 1150), (2, 1999)], 80), ([(0, 1150)], 37), ([(0, 1183), (1, 1100)], 37)])
+def test_attn_fused_merges_more_segments_than_its_buffer_holds(head, n_q, n_kv, rows, n_seg):
+    """Up to 80 segments a row: more than the merge's share of the rings (16 to 45) and than two pairs a lane."""
+    _attn_case(head, n_q, n_kv, rows, n_seg=n_seg, ctx=2560, seed=11)
