@@ -18,7 +18,7 @@
 // of t + 1 for one tile, then for the other.  MMAs of one thread execute in order: the new scores replace the probabilities
 // behind the product that reads them, and a commit behind Q K^T says that the P V in front of it is complete too.
 // One tile a CTA with two threads a row took 234 us a layer for 4,096 tokens of the 30 B shape (32 heads over 4) and 258 us for 700
-// behind 9,000; this takes 154 and 174.
+// behind 9,000; this takes 140 and 174.
 // A few hundred queries behind a long prefix are fewer CTAs than processors, each with a long walk over the keys: there
 // `splits` CTAs share the key tiles of a pair.  Each leaves its unnormalised output, maximum and sum of every row in a buffer,
 // and the warp that arrives last at its 32 rows (a ticket) adds the parts up in ascending order, its own out of tensor memory.
