@@ -173,13 +173,6 @@ struct AttnArgs {
   int recv_off;                            // cluster form: float offset of the merge buffer in dynamic shared memory
 };
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
 // One head's HEAD values held as DPL = HEAD / 32 consecutive values per lane -> q8 codes + {d, s} per 32 values.
 template <int HEAD>
 __device__ __forceinline__ void head_out_q8(const float (&o)[HEAD / 32], int lane, long col0, const AttnArgs& a, int m) {

@@ -41,6 +41,7 @@ struct GemvArgs {
   const uint8_t* pf_ptr[6];
   long pf_bytes[6];
   int n_pf;
+  const int* row_seq;      // optional (M > 1): rows with a negative entry only fill the pass's bucket and are not computed
 };
 
 // One thread per block: ask L2 to prefetch this block's 1 / gridDim.x share of each span (16-byte granules).
@@ -58,6 +59,17 @@ __device__ __forceinline__ void prefetch_spans_l2(const uint8_t* const* ptr, con
   }
 }
 
+
+// ---- asynchronous copies into shared memory ----------------------------------------------
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // ---- shared-memory layout of a q8 activation row ----------------------------------------
 // The codes of a K-value row are kept in 16-byte chunks.  Layout 0 is linear.  The staged kernels read a
@@ -102,6 +114,21 @@ template <> struct StagedAct<Q6K> {
 };
 __host__ __device__ inline int staged_layout(int wtype) { return wtype == WT_Q6_K ? 2 : 1; }
 
+// Copies a q8 row of K values (codes and {d, s} pairs) into shared memory in `layout`; the caller waits and synchronises.
+__device__ __forceinline__ void copy_q8_row(const int8_t* xq, const float2* xds, int K, int layout, int8_t* sq, float2* sds) {
+  for (int c = threadIdx.x; c < K / 16; c += blockDim.x) cp_async16(sq + 16 * act_chunk_pos(c, K / 64, layout), xq + 16 * (long)c);
+  for (int c = threadIdx.x; c < K / 32; c += blockDim.x) cp_async8(sds + c, xds + c);
+  cp_async_commit();
+}
+
+// Sum of eight squares, rounded the same way in every kernel that takes a row's.
+__device__ __forceinline__ float sum_sq8(const float4& a, const float4& b) {
+  float s = fma_rn(a.x, a.x, mul_rn(a.y, a.y));
+  s = fma_rn(a.z, a.z, s); s = fma_rn(a.w, a.w, s);
+  s = fma_rn(b.x, b.x, s); s = fma_rn(b.y, b.y, s); s = fma_rn(b.z, b.z, s);
+  return fma_rn(b.w, b.w, s);
+}
+
 // ---- activation prologue ------------------------------------------------------------
 // sq/sds receive q8(x * gain) WITHOUT the RMS scale; s_scale[m] receives the scale.
 template <int MB, bool FLOATW>
@@ -137,7 +164,7 @@ __device__ __forceinline__ void prologue_norm(const GemvArgs& a, int8_t* sq, flo
       }
       float4 g0 = __ldg(reinterpret_cast<const float4*>(a.gain + i0)), g1 = __ldg(reinterpret_cast<const float4*>(a.gain + i0 + 4));
       float v[8] = {x0.x * g0.x, x0.y * g0.y, x0.z * g0.z, x0.w * g0.w, x1.x * g1.x, x1.y * g1.y, x1.z * g1.z, x1.w * g1.w};
-      ss += x0.x * x0.x + x0.y * x0.y + x0.z * x0.z + x0.w * x0.w + x1.x * x1.x + x1.y * x1.y + x1.z * x1.z + x1.w * x1.w;
+      ss += sum_sq8(x0, x1);
       float amax = 0.f;
 #pragma unroll
       for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
@@ -190,5 +217,75 @@ __device__ __forceinline__ void prologue_q8in(const GemvArgs& a, int8_t* sq, flo
   __syncthreads();
 }
 
+// prologue_norm for passes of several rows (live: bit m): all of them come into shared memory (sx) in one round trip.  One
+// after the other, each with its own trip to L2, five rows took 7 us of the 27 of their projections on the 30 B shape; held in
+// registers, they made the weight rows that wait there spill.  The sums are prologue_norm's, in its order.  FLOATW: sx keeps
+// x * gain.
+template <bool FLOATW>
+__device__ __forceinline__ void prologue_norm_rows(const GemvArgs& a, unsigned live, int8_t* sq, float2* sds, float* sx, float* s_scale,
+                                                   double* red, int layout) {
+  const int K = a.K, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (unsigned left = live; left; left &= left - 1) {
+    const int m = __ffs(left) - 1;
+    for (int c = tid; c < K / 4; c += 256) cp_async16(sx + (long)m * K + 4 * c, a.x + (long)m * a.x_stride + 4 * c);
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+#pragma unroll 2
+  for (unsigned left = live; left; left &= left - 1) {
+    const int m = __ffs(left) - 1;
+    float* x = sx + (long)m * K;
+    float ss = 0.f;
+    for (int i0 = tid * 8; i0 < K; i0 += 2048) {      // K is a multiple of 256: a warp is in or out as a whole
+      const float4 x0 = *reinterpret_cast<const float4*>(x + i0), x1 = *reinterpret_cast<const float4*>(x + i0 + 4);
+      const float4 g0 = __ldg(reinterpret_cast<const float4*>(a.gain + i0)), g1 = __ldg(reinterpret_cast<const float4*>(a.gain + i0 + 4));
+      const float v[8] = {x0.x * g0.x, x0.y * g0.y, x0.z * g0.z, x0.w * g0.w, x1.x * g1.x, x1.y * g1.y, x1.z * g1.z, x1.w * g1.w};
+      ss += sum_sq8(x0, x1);
+      float amax = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
+      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+      const float d = amax / 127.0f, inv = d > 0.f ? 1.0f / d : 0.f;
+      int q[8], sum = 0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) { q[j] = max(-127, min(127, __float2int_rn(v[j] * inv))); sum += q[j]; }
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      uint2 packed;
+      packed.x = (q[0] & 0xFF) | ((q[1] & 0xFF) << 8) | ((q[2] & 0xFF) << 16) | ((unsigned)(q[3] & 0xFF) << 24);
+      packed.y = (q[4] & 0xFF) | ((q[5] & 0xFF) << 8) | ((q[6] & 0xFF) << 16) | ((unsigned)(q[7] & 0xFF) << 24);
+      *reinterpret_cast<uint2*>(sq + (long)m * K + act_chunk_pos(i0 >> 4, K / 64, layout) * 16 + (i0 & 15)) = packed;
+      if ((tid & 3) == 0) sds[(long)m * (K / 32) + i0 / 32] = make_float2(d, d * (float)sum);
+      if (FLOATW) {
+        *reinterpret_cast<float4*>(x + i0) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4*>(x + i0 + 4) = make_float4(v[4], v[5], v[6], v[7]);
+      }
+    }
+    const double tot = warp_sum_d((double)ss);
+    if (lane == 0) red[m * 8 + warp] = tot;
+  }
+  __syncthreads();
+  if (tid < kMaxRows && (live >> tid & 1)) {
+    double all = 0.0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) all += red[tid * 8 + w];
+    s_scale[tid] = 1.0f / sqrtf((float)(all / (double)K) + a.eps);
+  }
+  __syncthreads();
+}
+
+// prologue_q8in for passes of several rows: the copies of all live rows are in flight at once.
+__device__ __forceinline__ void prologue_q8_rows(const GemvArgs& a, unsigned live, int8_t* sq, float2* sds, float* s_scale, int layout) {
+  const int K = a.K;
+  for (unsigned left = live; left; left &= left - 1) {
+    const int m = __ffs(left) - 1;
+    copy_q8_row(a.xq + (long)m * K, a.xds + (long)m * (K / 32), K, layout, sq + (long)m * K, sds + (long)m * (K / 32));
+  }
+  if (threadIdx.x < kMaxRows) s_scale[threadIdx.x] = 1.0f;
+  cp_async_wait<0>();
+  __syncthreads();
+}
 
 }  // namespace bl

@@ -13,6 +13,7 @@
 // experts.rs:36-45); the elsewhere-sentinel for slots another tier serves
 // (crates/gpu/src/kquant/sel.rs doc).  The completion counter instead of a grid barrier
 // is the reference's measured choice (docs/gpu-design.md:52-64).
+#include "gemv_common.cuh"
 #include "route.cuh"
 
 namespace bl {
@@ -280,6 +281,8 @@ __global__ void __launch_bounds__(256) router_rows_kernel(const float* x, long x
 // gate·up·SwiGLU over device-side expert ids
 // grid (I/32, n_used, M), 256 threads: warp w computes activation rows 4w..4w+3 of the chunk
 // ------------------------------------------------------------------------------------
+constexpr int kMaxInput = 200 * 1024;       // bytes of a staged activation row
+
 struct GateUpArgs {
   const int8_t* xq; const float2* xds;   // [M, K] q8
   RouteParams route;                     // route.logits == null: ids are given
@@ -298,10 +301,10 @@ struct GateUpArgs {
   const int* row_seq;
 };
 
-// two activation outputs (2 gate rows + 2 up rows) of one warp
+// two activation outputs (2 gate rows + 2 up rows) of one warp, the activations in shared memory (in the chunk layout of T)
 template <class T>
 __device__ __forceinline__ void gate_up_rows(const uint8_t* g0, const uint8_t* u0, long rb, int K, int lane,
-                                             const int8_t* xq, const float2* xds, float (&gacc)[2], float (&uacc)[2]) {
+                                             const int8_t* sq, const float2* sds, float (&gacc)[2], float (&uacc)[2]) {
   using U = Unit<T>;
   const int nunits = K / 64;
 #pragma unroll
@@ -310,8 +313,8 @@ __device__ __forceinline__ void gate_up_rows(const uint8_t* g0, const uint8_t* u
     typename U::Regs rg[2], ru[2];
 #pragma unroll
     for (int r = 0; r < 2; ++r) { U::loadu(g0 + r * rb, u, K, rg[r]); U::loadu(u0 + r * rb, u, K, ru[r]); }
-    ActRegs act;   // activations straight from L2, behind the weight loads already in flight
-    ActOf<T>::load(reinterpret_cast<const uint32_t*>(xq), reinterpret_cast<const F2*>(xds), u, act);
+    ActRegs act;
+    StagedAct<T>::load(sq, sds, u, nunits, act);
 #pragma unroll
     for (int r = 0; r < 2; ++r) { gacc[r] += ActOf<T>::dot(rg[r], u, act); uacc[r] += ActOf<T>::dot(ru[r], u, act); }
   }
@@ -319,47 +322,78 @@ __device__ __forceinline__ void gate_up_rows(const uint8_t* g0, const uint8_t* u
   for (int r = 0; r < 2; ++r) { gacc[r] = warp_sum(gacc[r]); uacc[r] = warp_sum(uacc[r]); }
 }
 
-// grid (I/32, n_used, M), 256 threads: warp w computes activation rows 4w..4w+3 of the chunk.
-// When route.logits is set, warp 0 of every block routes row m itself (redundantly, from
-// the router launch's logits) so no block waits on a completion counter; block (0, 0, m)
-// also publishes ids / weights / heat for the launches that follow.
+// grid (I/32, n_used, M), 256 threads: warp w computes activation rows 2w, 2w+1, 16+2w and 17+2w of the chunk.
+// When route.logits is set the grid is one wider in x: every block routes row m itself (redundantly, from the router
+// launch's logits) so no block waits on a completion counter, and the block behind the chunks publishes ids / weights /
+// heat for the launches that follow, which takes the weights' arithmetic off the path of those that multiply.
+// One row is a chain of latencies (logits, picks, weights, sums), so what can overlap does: the activations come in under the
+// picks, which one warp takes where route_pick serves, and the rows of the second half are asked into L2 while the first half
+// is in flight.  30 B shape, one row, us behind the launch in front: 10.2 before and 9.9 now alone in the layer, of which 2
+// go to the picks, 3 to 5 to the first half (1 of them to HBM), 1.8 to the second; what bounds the halves is the issue of
+// some 100 instructions a weight row and lane, two blocks on a third of the processors.  Five rows 36 -> 34.
 // FAM 0 = ggml integer-dot types, FAM 2 = block-scaled float planes (one kernel per family keeps
 // the plane decoders out of the K-quant bodies' register budget)
 template <int FAM>
 __global__ void __launch_bounds__(256, 2) gate_up_sel_kernel(const GateUpArgs a) {
+  extern __shared__ __align__(16) uint8_t s_in[];
   const int K = a.K;
+  int8_t* sq = reinterpret_cast<int8_t*>(s_in);
+  float2* sds = reinterpret_cast<float2*>(s_in + K);
   __shared__ float s_act[32];
-  __shared__ int s_e;
+  __shared__ RouteShared rs;
   const int chunk = blockIdx.x, j = blockIdx.y, m = blockIdx.z;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool publisher = chunk == a.I / 32;
+  if (publisher && j != 0) return;
   pdl_wait();
   pdl_launch();
   if (a.row_seq && a.row_seq[m] < 0) {
-    if (chunk == 0 && j == 0 && tid < a.n_used) {
+    if (publisher && tid < a.n_used) {
       a.ids[(long)m * a.n_used + tid] = kExpertElsewhere;
       a.wts[(long)m * a.n_used + tid] = 0.f;
     }
     return;
   }
-  if (a.route.logits) {
-    // block-wide rank counting: measured faster here than top_k rounds of a single warp's arg-max
-    __shared__ RouteShared rs;
+  const bool pick = a.route.logits && route_pick_ok(a.route);
+  if (publisher) {
+    if (pick && warp != 0) return;
     int id; float w;
-    const bool ok = route_block(a.route, m, rs, id, w);
-    if (tid == 0) s_e = ok ? rs.ids[j] : -3;
-    if (chunk == 0 && j == 0 && warp == 0) {
-      if (!ok && lane == 0) raise_fault(a.fault, a.layer, FS_ROUTER);
-      if (lane < a.n_used) {
-        a.ids[(long)m * a.n_used + lane] = ok ? id : 0;
-        a.wts[(long)m * a.n_used + lane] = w;
-        if (ok && a.heat) atomicAdd(a.heat + id, 1u);
-      }
+    bool ok;
+    if (pick) {
+      float l;
+      ok = route_pick(a.route, m, lane, a.n_used, id, l);
+      w = ok ? route_pick_weight(a.route, lane, l) : __int_as_float(0x7fc00000);
+    } else {
+      ok = route_block(a.route, m, rs, id, w);
     }
-  } else if (tid == 0) {
-    s_e = a.ids[(long)m * a.n_used + j];
+    if (warp != 0) return;
+    if (!ok && lane == 0) raise_fault(a.fault, a.layer, FS_ROUTER);
+    if (lane < a.n_used) {
+      a.ids[(long)m * a.n_used + lane] = ok ? id : 0;
+      a.wts[(long)m * a.n_used + lane] = w;
+      if (ok && a.heat) atomicAdd(a.heat + id, 1u);
+    }
+    return;
   }
-  __syncthreads();
-  int e = s_e;
+  copy_q8_row(a.xq + (long)m * K, a.xds + (long)m * (K / 32), K, staged_layout(a.gtype), sq, sds);
+  __shared__ int s_e;
+  int e;
+  if (pick) {
+    if (warp == 0) {
+      int id;
+      float l;
+      const bool ok = route_pick(a.route, m, lane, j + 1, id, l);
+      if (lane == j) s_e = ok ? id : -3;
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    e = s_e;
+  } else if (a.route.logits) {
+    float w;
+    e = route_block(a.route, m, rs, e, w) ? rs.ids[j] : -3;
+  } else {
+    e = a.ids[(long)m * a.n_used + j];
+  }
   const long ob = ((long)m * a.n_used + j) * a.I + chunk * 32;
   bool skip = false, bad = false;
   if (e == kExpertElsewhere) skip = true;
@@ -367,6 +401,7 @@ __global__ void __launch_bounds__(256, 2) gate_up_sel_kernel(const GateUpArgs a)
   else if (e < 0 || e >= a.E) { skip = true; bad = true; if (tid == 0 && chunk == 0) raise_fault(a.fault, a.layer, FS_EXPERT_ID); }
   else if (a.slot_map) { e = a.slot_map[e]; if (e < 0) skip = true; }
   if (skip) {
+    cp_async_wait<0>();
     if (tid < 32) {
       a.actq[ob + tid] = 0;
       if (a.act_f32) a.act_f32[ob + tid] = bad ? __int_as_float(0x7fc00000) : 0.f;
@@ -374,42 +409,53 @@ __global__ void __launch_bounds__(256, 2) gate_up_sel_kernel(const GateUpArgs a)
     if (tid == 0) a.actds[ob / 32] = bad ? make_float2(__int_as_float(0x7fc00000), 0.f) : make_float2(0.f, 0.f);
     return;
   }
-  const long rb = resident_row_bytes(a.gtype, K);
-  const int8_t* xq = a.xq + (long)m * K;
-  const float2* xds = a.xds + (long)m * (K / 32);
+  const long rb = resident_row_bytes(a.gtype, K), first = (long)e * a.I + chunk * 32;
+  if (tid == 0 || tid == 128) {
+    // rows 16 .. 31 of the chunk, which the second half reads
+    const uint8_t* p = (tid == 0 ? a.gate : a.up) + (first + 16) * rb;
+    for (long o = 0; o < 16 * rb; o += 32768) {
+      const unsigned nb = (unsigned)((16 * rb - o) < 32768 ? (16 * rb - o) : 32768);
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p + o), "r"(nb) : "memory");
+    }
+  }
   if (a.down && tid == 32) {
-    // the down launch that follows streams expert e's matrix: this block asks L2 for its 1 / gridDim.x share
-    const long share = (a.down_expert_bytes / gridDim.x) & ~15L;
+    // the down launch that follows streams expert e's matrix: this block asks L2 for its share of it
+    const long share = (a.down_expert_bytes / (a.I / 32)) & ~15L;
     for (long o = 0; o < share; o += 32768) {
       const unsigned nb = (unsigned)((share - o) < 32768 ? (share - o) : 32768);
       asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a.down + (long)e * a.down_expert_bytes + (long)chunk * share + o), "r"(nb) : "memory");
     }
   }
+  if (!pick) {
+    cp_async_wait<0>();
+    __syncthreads();
+  }
 #pragma unroll 1
   for (int half = 0; half < 2; ++half) {
-    const long row0 = (long)e * a.I + chunk * 32 + warp * 4 + half * 2;
+    const long row0 = first + half * 16 + warp * 2;
     const uint8_t* g0 = a.gate + row0 * rb;
     const uint8_t* u0 = a.up + row0 * rb;
     float gacc[2], uacc[2];
+    auto rows = [&](auto t) { gate_up_rows<decltype(t)>(g0, u0, rb, K, lane, sq, sds, gacc, uacc); };
     if constexpr (FAM == 2) {
       switch (a.gtype) {
-        case WT_NVFP4: gate_up_rows<NvFp4>(g0, u0, rb, K, lane, xq, xds, gacc, uacc); break;
-        case WT_FP8_B128: gate_up_rows<Fp8B128>(g0, u0, rb, K, lane, xq, xds, gacc, uacc); break;
-        case WT_Q2_K: gate_up_rows<Q2K>(g0, u0, rb, K, lane, xq, xds, gacc, uacc); break;
-        case WT_Q3_K: gate_up_rows<Q3K>(g0, u0, rb, K, lane, xq, xds, gacc, uacc); break;
-        case WT_Q4_0: gate_up_rows<Q40>(g0, u0, rb, K, lane, xq, xds, gacc, uacc); break;
-        case WT_Q4_1: gate_up_rows<Q41>(g0, u0, rb, K, lane, xq, xds, gacc, uacc); break;
-        case WT_Q5_0: gate_up_rows<Q50>(g0, u0, rb, K, lane, xq, xds, gacc, uacc); break;
-        case WT_Q5_1: gate_up_rows<Q51>(g0, u0, rb, K, lane, xq, xds, gacc, uacc); break;
+        case WT_NVFP4: rows(NvFp4{}); break;
+        case WT_FP8_B128: rows(Fp8B128{}); break;
+        case WT_Q2_K: rows(Q2K{}); break;
+        case WT_Q3_K: rows(Q3K{}); break;
+        case WT_Q4_0: rows(Q40{}); break;
+        case WT_Q4_1: rows(Q41{}); break;
+        case WT_Q5_0: rows(Q50{}); break;
+        case WT_Q5_1: rows(Q51{}); break;
         default: gacc[0] = gacc[1] = __int_as_float(0x7fc00000); uacc[0] = uacc[1] = 0.f;
       }
     } else {
       switch (a.gtype) {
-        case WT_Q4_K: gate_up_rows<Q4K>(g0, u0, rb, K, lane, xq, xds, gacc, uacc); break;
-        case WT_Q5_K: gate_up_rows<Q5K>(g0, u0, rb, K, lane, xq, xds, gacc, uacc); break;
-        case WT_Q6_K: gate_up_rows<Q6K>(g0, u0, rb, K, lane, xq, xds, gacc, uacc); break;
-        case WT_Q8_0: gate_up_rows<Q80>(g0, u0, rb, K, lane, xq, xds, gacc, uacc); break;
-        case WT_Q8_F32: gate_up_rows<Q8F>(g0, u0, rb, K, lane, xq, xds, gacc, uacc); break;
+        case WT_Q4_K: rows(Q4K{}); break;
+        case WT_Q5_K: rows(Q5K{}); break;
+        case WT_Q6_K: rows(Q6K{}); break;
+        case WT_Q8_0: rows(Q80{}); break;
+        case WT_Q8_F32: rows(Q8F{}); break;
         default: gacc[0] = gacc[1] = __int_as_float(0x7fc00000); uacc[0] = uacc[1] = 0.f;
       }
     }
@@ -417,7 +463,7 @@ __global__ void __launch_bounds__(256, 2) gate_up_sel_kernel(const GateUpArgs a)
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         float g = gacc[r];
-        s_act[warp * 4 + half * 2 + r] = (g / (1.0f + expf(-g))) * uacc[r];
+        s_act[half * 16 + warp * 2 + r] = (g / (1.0f + expf(-g))) * uacc[r];
       }
     }
   }
@@ -449,105 +495,114 @@ struct DownArgs {
   PushOut push;                             // n_ranks > 0: the result is this rank's partial update
 };
 
-// UPL = units per lane (all loaded before any is used: one DRAM round trip per row)
-template <class T, int UPL>
-__device__ __forceinline__ float down_row(const DownArgs& a, int m, int d, int lane, const int* s_slot, const float* s_w) {
+// One row d of the sum over the chosen experts.  The activations of a row of the pass, slot by slot, are one row of
+// n_used * I values, whose units go to the lanes in turn (t = lane + 32 c).  UPL = units per lane (all loaded before any is
+// used: one DRAM round trip per row); lane j < n_used holds the expert and the weight of slot j.
+template <class T, int UPL, class Landed>
+__device__ __forceinline__ float down_row(const DownArgs& a, int d, int lane, const int (&slot)[UPL], const int (&unit)[UPL], int my_e, float my_w,
+                                          const int8_t* sq, const float2* sds, Landed&& landed) {
   using U = Unit<T>;
-  const int upe = a.I / 64;              // units per expert row
-  const int total = a.n_used * upe;
+  const int total = a.n_used * (a.I / 64);
   const long rb = resident_row_bytes(T::kType, a.I);
   typename U::Regs regs[UPL];
-  int jj[UPL], uu[UPL];
+  bool use[UPL];
 #pragma unroll
   for (int c = 0; c < UPL; ++c) {
-    const int t = lane + 32 * c;
-    jj[c] = -1; uu[c] = 0;
-    if (t < total) {
-      const int j = t / upe;
-      const int e = s_slot[j];
-      if (e >= 0) { jj[c] = j; uu[c] = t - j * upe; U::loadu(a.down + ((long)e * a.H + d) * rb, uu[c], a.I, regs[c]); }
-    }
+    const int e = __shfl_sync(0xffffffffu, my_e, slot[c]);
+    use[c] = lane + 32 * c < total && e >= 0;
+    if (use[c]) U::loadu(a.down + ((long)e * a.H + d) * rb, unit[c], a.I, regs[c]);
   }
-  // per-slot partial sums kept separate, then added in ascending slot order
-  float part[kMaxTopK];
-#pragma unroll
-  for (int j = 0; j < kMaxTopK; ++j) part[j] = 0.f;
+  landed();
+  // the lane's units of a slot are added up, the router-weighted sum runs over its slots in ascending order, then one butterfly
+  float y = 0.f, part = 0.f;
 #pragma unroll
   for (int c = 0; c < UPL; ++c) {
-    if (jj[c] >= 0) {
+    const float w = __shfl_sync(0xffffffffu, my_w, slot[c]);
+    if (use[c]) {
       ActRegs act;
-      const long ab = ((long)m * a.n_used + jj[c]) * a.I;
-      ActOf<T>::load(reinterpret_cast<const uint32_t*>(a.actq + ab), reinterpret_cast<const F2*>(a.actds + ab / 32), uu[c], act);
-      float v = ActOf<T>::dot(regs[c], uu[c], act);
-#pragma unroll
-      for (int j = 0; j < kMaxTopK; ++j) if (j == jj[c]) part[j] += v;
+      StagedAct<T>::load(sq, sds, lane + 32 * c, total, act);
+      part += ActOf<T>::dot(regs[c], unit[c], act);
+      if (c + 1 == UPL || lane + 32 * (c + 1) >= total || slot[c + 1 < UPL ? c + 1 : c] != slot[c]) { y = fmaf(w, part, y); part = 0.f; }
     }
-  }
-  // router-weighted sum over slots in ascending order inside the lane, then one butterfly
-  float y = 0.f;
-#pragma unroll
-  for (int j = 0; j < kMaxTopK; ++j) {
-    if (j < a.n_used) y = fmaf(s_w[j], part[j], y);
   }
   return warp_sum(y);
 }
 
-// OCC = blocks a processor.  One row has 256 blocks for 148 processors and wants its registers (9.0 us a layer of the 30 B shape
-// with two, 10.6 with three); several rows queue for the processors (five rows: 34 us with
-// two, 29 with three; FP8 rows 36 us either way).
+// OCC = blocks a processor.  One row has 256 blocks for 148 processors and wants its registers; several rows queue for the
+// processors (five rows: 34 us with two, 29 with three, before the activations were staged; FP8 rows 36 us either way).
+// The launch in front asked L2 for the weights, so a row is bound by latencies and by the load unit: activations read from L2
+// sixteen bytes in every 64 took half of a warp's 380 wavefronts.  With them in shared memory, one request for a super-block's
+// head and the residual asked for in front, one row takes 6.5 us a layer of the 30 B shape (9.0 before), five 23 (28).
 template <int UPL, int FAM, int OCC>
 __global__ void __launch_bounds__(256, OCC) down_combine_kernel(const DownArgs a) {
-  __shared__ int s_slot[kMaxTopK];
-  __shared__ float s_w[kMaxTopK];
+  extern __shared__ __align__(16) uint8_t s_in[];
+  const int width = a.n_used * a.I;
+  int8_t* sq = reinterpret_cast<int8_t*>(s_in);
+  float2* sds = reinterpret_cast<float2*>(s_in + width);
   const int m = blockIdx.y;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int upe = a.I / 64;              // units per expert row
+  int slot[UPL], unit[UPL];
+#pragma unroll
+  for (int c = 0; c < UPL; ++c) {
+    slot[c] = min((lane + 32 * c) / upe, a.n_used - 1);
+    unit[c] = lane + 32 * c - slot[c] * upe;
+  }
+  const int d = blockIdx.x * 8 + warp, dr = min(d, a.H - 1);
   pdl_wait();
   pdl_launch();
-  if (tid < a.n_used) {
-    int e = a.ids[(long)m * a.n_used + tid];
-    float w = a.wts[(long)m * a.n_used + tid];
-    if (e == kExpertElsewhere) e = -1;
-    else if (e < 0 || e >= a.E) { e = -2; }
-    else if (a.slot_map) { e = a.slot_map[e]; if (e < 0) e = -1; }
-    s_slot[tid] = e; s_w[tid] = w;
+  int my_e = -1;
+  float my_w = 0.f;
+  if (lane < a.n_used) {
+    my_e = a.ids[(long)m * a.n_used + lane];
+    my_w = a.wts[(long)m * a.n_used + lane];
   }
-  __syncthreads();
-  bool bad = false;
-  for (int j = 0; j < a.n_used; ++j) bad |= (s_slot[j] == -2);
-  const int d = blockIdx.x * 8 + warp;
-  if (d < a.H) {
-    float y;
-    if constexpr (FAM == 2) {
-      switch (a.dtype) {
-        case WT_NVFP4: y = down_row<NvFp4, UPL>(a, m, d, lane, s_slot, s_w); break;
-        case WT_FP8_B128: y = down_row<Fp8B128, UPL>(a, m, d, lane, s_slot, s_w); break;
-        case WT_Q2_K: y = down_row<Q2K, UPL>(a, m, d, lane, s_slot, s_w); break;
-        case WT_Q3_K: y = down_row<Q3K, UPL>(a, m, d, lane, s_slot, s_w); break;
-        case WT_Q4_0: y = down_row<Q40, UPL>(a, m, d, lane, s_slot, s_w); break;
-        case WT_Q4_1: y = down_row<Q41, UPL>(a, m, d, lane, s_slot, s_w); break;
-        case WT_Q5_0: y = down_row<Q50, UPL>(a, m, d, lane, s_slot, s_w); break;
-        case WT_Q5_1: y = down_row<Q51, UPL>(a, m, d, lane, s_slot, s_w); break;
-        default: y = __int_as_float(0x7fc00000);
-      }
-    } else {
-      switch (a.dtype) {
-        case WT_Q4_K: y = down_row<Q4K, UPL>(a, m, d, lane, s_slot, s_w); break;
-        case WT_Q6_K: y = down_row<Q6K, UPL>(a, m, d, lane, s_slot, s_w); break;
-        case WT_Q5_K: y = down_row<Q5K, UPL>(a, m, d, lane, s_slot, s_w); break;
-        case WT_Q8_0: y = down_row<Q80, UPL>(a, m, d, lane, s_slot, s_w); break;
-        case WT_Q8_F32: y = down_row<Q8F, UPL>(a, m, d, lane, s_slot, s_w); break;
-        default: y = __int_as_float(0x7fc00000);
-      }
+  copy_q8_row(a.actq + (long)m * width, a.actds + (long)m * (width / 32), width, staged_layout(a.dtype), sq, sds);
+  float add = 0.f, old = 0.f;
+  if (lane == 0) {
+    if (a.extra) add = a.extra[(long)m * a.extra_stride + dr];
+    if (a.resid && a.push.n_ranks == 0) old = a.resid[(long)m * a.resid_stride + dr];
+  }
+  if (my_e == kExpertElsewhere) my_e = -1;
+  else if (my_e < 0 || my_e >= a.E) my_e = -2;
+  else if (a.slot_map) { my_e = a.slot_map[my_e]; if (my_e < 0) my_e = -1; }
+  const bool bad = __any_sync(0xffffffffu, my_e == -2);
+  auto landed = [&]() {
+    cp_async_wait<0>();
+    __syncthreads();
+  };
+  float y;
+  auto row = [&](auto t) { y = down_row<decltype(t), UPL>(a, dr, lane, slot, unit, my_e, my_w, sq, sds, landed); };
+  if constexpr (FAM == 2) {
+    switch (a.dtype) {
+      case WT_NVFP4: row(NvFp4{}); break;
+      case WT_FP8_B128: row(Fp8B128{}); break;
+      case WT_Q2_K: row(Q2K{}); break;
+      case WT_Q3_K: row(Q3K{}); break;
+      case WT_Q4_0: row(Q40{}); break;
+      case WT_Q4_1: row(Q41{}); break;
+      case WT_Q5_0: row(Q50{}); break;
+      case WT_Q5_1: row(Q51{}); break;
+      default: y = __int_as_float(0x7fc00000);
     }
-    if (lane == 0) {
-      if (bad) { y = __int_as_float(0x7fc00000); if (d == 0) raise_fault(a.fault, a.layer, FS_EXPERT_ID); }
-      if (a.extra) y += a.extra[(long)m * a.extra_stride + d];
-      if (a.push.n_ranks > 0) {
-        push_store(a.push, site_epoch(a.push.step, a.push.sites_per_step, a.push.site_index), (long)m * a.out_stride + d, y);
-      } else {
-        if (a.resid) y += a.resid[(long)m * a.resid_stride + d];
-        a.out[(long)m * a.out_stride + d] = y;
-      }
+  } else {
+    switch (a.dtype) {
+      case WT_Q4_K: row(Q4K{}); break;
+      case WT_Q6_K: row(Q6K{}); break;
+      case WT_Q5_K: row(Q5K{}); break;
+      case WT_Q8_0: row(Q80{}); break;
+      case WT_Q8_F32: row(Q8F{}); break;
+      default: y = __int_as_float(0x7fc00000);
+    }
+  }
+  if (lane == 0 && d < a.H) {
+    if (bad) { y = __int_as_float(0x7fc00000); if (d == 0) raise_fault(a.fault, a.layer, FS_EXPERT_ID); }
+    if (a.extra) y += add;
+    if (a.push.n_ranks > 0) {
+      push_store(a.push, site_epoch(a.push.step, a.push.sites_per_step, a.push.site_index), (long)m * a.out_stride + d, y);
+    } else {
+      if (a.resid) y += old;
+      a.out[(long)m * a.out_stride + d] = y;
     }
   }
 }
@@ -716,8 +771,16 @@ int bl_gate_up_sel(const int8_t* xq, const float* xds, const float* route_logits
   BL_REQUIRE(((uintptr_t)down & 15) == 0 && down_expert_bytes % 16 == 0, BL_ERR_ALIGN);
   a.down = (const uint8_t*)down; a.down_expert_bytes = down_expert_bytes;
   a.row_seq = row_seq;
-  if (is_plane_family(gtype)) return (int)launch(gate_up_sel_kernel<2>, dim3(I / 32, n_used, M), dim3(256), 0, st, a);
-  return (int)launch(gate_up_sel_kernel<0>, dim3(I / 32, n_used, M), dim3(256), 0, st, a);
+  const size_t smem = (size_t)K + K / 4;
+  BL_REQUIRE(smem <= kMaxInput, BL_ERR_LIMIT);
+  static PerDevice limit;
+  if (limit.due()) {
+    cudaFuncSetAttribute(gate_up_sel_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxInput);
+    cudaFuncSetAttribute(gate_up_sel_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxInput);
+    limit.mark();
+  }
+  const dim3 grid(I / 32 + (route_logits ? 1 : 0), n_used, M);
+  return (int)launch(is_plane_family(gtype) ? gate_up_sel_kernel<2> : gate_up_sel_kernel<0>, grid, dim3(256), smem, st, a);
 }
 
 int bl_down_combine(const int8_t* actq, const float* actds, const int* ids, const float* wts, const int* slot_map,
@@ -733,15 +796,15 @@ int bl_down_combine(const int8_t* actq, const float* actds, const int* ids, cons
   if (push_desc) { a.push = *(const PushOut*)push_desc; BL_REQUIRE(a.push.n_ranks <= kMaxRanks && M <= kMaxRows, BL_ERR_SHAPE); }
   const long total = (long)n_used * (I / 64);
   BL_REQUIRE(total <= 512, BL_ERR_LIMIT);
-  dim3 grid((H + 7) / 8, M);
-  if (is_plane_family(dtype)) {
-    if (total <= 96) return (int)launch(M == 1 ? down_combine_kernel<3, 2, 2> : down_combine_kernel<3, 2, 3>, grid, dim3(256), 0, st, a);
-    if (total <= 192) return (int)launch(down_combine_kernel<6, 2, 1>, grid, dim3(256), 0, st, a);
-    return (int)launch(down_combine_kernel<16, 2, 1>, grid, dim3(256), 0, st, a);
+  const dim3 grid((H + 7) / 8, M);
+  const size_t smem = (size_t)total * 80;          // at most 40 KB
+  const bool planes = is_plane_family(dtype);
+  if (total <= 96) {
+    if (M == 1) return (int)launch(planes ? down_combine_kernel<3, 2, 2> : down_combine_kernel<3, 0, 2>, grid, dim3(256), smem, st, a);
+    return (int)launch(planes ? down_combine_kernel<3, 2, 3> : down_combine_kernel<3, 0, 3>, grid, dim3(256), smem, st, a);
   }
-  if (total <= 96) return (int)launch(M == 1 ? down_combine_kernel<3, 0, 2> : down_combine_kernel<3, 0, 3>, grid, dim3(256), 0, st, a);
-  if (total <= 192) return (int)launch(down_combine_kernel<6, 0, 1>, grid, dim3(256), 0, st, a);
-  return (int)launch(down_combine_kernel<16, 0, 1>, grid, dim3(256), 0, st, a);
+  if (total <= 192) return (int)launch(planes ? down_combine_kernel<6, 2, 1> : down_combine_kernel<6, 0, 1>, grid, dim3(256), smem, st, a);
+  return (int)launch(planes ? down_combine_kernel<16, 2, 1> : down_combine_kernel<16, 0, 1>, grid, dim3(256), smem, st, a);
 }
 
 }  // extern "C"

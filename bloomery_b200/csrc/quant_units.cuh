@@ -68,6 +68,32 @@ BL_HD int dot4_us(uint32_t a, uint32_t b, int c) {
 #endif
 }
 
+// The dots round where they say: which products a compiler would join with an addition depends on the code around them, and a
+// row's bits must not depend on the kernel that takes it.
+BL_HD float fma_rn(float a, float b, float c) {
+#if defined(__CUDA_ARCH__)
+  return __fmaf_rn(a, b, c);
+#else
+  return __builtin_fmaf(a, b, c);
+#endif
+}
+BL_HD float mul_rn(float a, float b) {
+#if defined(__CUDA_ARCH__)
+  return __fmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
+
+// Sums of products as floats.  The conversion instruction runs at a quarter of the rate of the others; an accumulator that starts
+// at the bits of 1.5 * 2^23 reads as that number plus the sum (below 2^22 in magnitude: exact).
+constexpr int kSum0 = 0x4B400000;
+BL_HD float sum_float(int bits) {
+  float f;
+  __builtin_memcpy(&f, &bits, 4);
+  return f - 12582912.0f;
+}
+
 BL_HD float half_bits_to_float(uint16_t h) {
 #if defined(__CUDA_ARCH__)
   return __half2float(__ushort_as_half(h));
@@ -137,8 +163,8 @@ struct Q4K {
     int j = u & 3;
     r.q0 = ld128(p + 16 + 32 * j);
     r.q1 = ld128(p + 32 + 32 * j);
-    r.dm = ld32(p);
-    r.s0 = ld32(p + 4); r.s1 = ld32(p + 8); r.s2 = ld32(p + 12);
+    const u32x4 h = ld128(p);          // one request for d, dmin and the twelve scale bytes
+    r.dm = h.x; r.s0 = h.y; r.s1 = h.z; r.s2 = h.w;
   }
   static BL_HD void scale_min(const Regs& r, int i, int& sc, int& mn) {
     // 6-bit (scale, min) pair i of 8 from the 12 packed bytes
@@ -152,7 +178,7 @@ struct Q4K {
   static BL_HD float dot(const Regs& r, int u, const ActUnit& a) {
     int j = u & 3;
     const uint32_t w[8] = {r.q0.x, r.q0.y, r.q0.z, r.q0.w, r.q1.x, r.q1.y, r.q1.z, r.q1.w};
-    int lo = 0, hi = 0;
+    int lo = kSum0, hi = kSum0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       lo = dot4_us(w[i] & 0x0F0F0F0Fu, a.q[i], lo);
@@ -163,9 +189,10 @@ struct Q4K {
     scale_min(r, 2 * j + 1, sc1, mn1);
     float d = half_bits_to_float((uint16_t)(r.dm & 0xFFFF));
     float dmin = half_bits_to_float((uint16_t)(r.dm >> 16));
-    float pos = a.d0 * (float)(sc0 * lo) + a.d1 * (float)(sc1 * hi);
-    float neg = a.s0 * (float)mn0 + a.s1 * (float)mn1;
-    return d * pos - dmin * neg;
+    // 63 * 32 * 31 * 127 < 2^24: the products of scales and sums are exact
+    const float pos = fma_rn(a.d0, mul_rn(sum_float(kSum0 + sc0), sum_float(lo)), mul_rn(a.d1, mul_rn(sum_float(kSum0 + sc1), sum_float(hi))));
+    const float neg = fma_rn(a.s0, sum_float(kSum0 + mn0), mul_rn(a.s1, sum_float(kSum0 + mn1)));
+    return fma_rn(d, pos, -mul_rn(dmin, neg));
   }
   // decode the unit's 64 values (for the embedding gather and the bf16 expander)
   static BL_HD void decode(const Regs& r, int u, float* out) {
@@ -199,8 +226,8 @@ struct Q5K {
   static BL_HD void load(const uint8_t* row, int u, Regs& r) {
     const uint8_t* p = row + (long)(u >> 2) * kSbBytes;
     int j = u & 3;
-    r.dm = ld32(p);
-    r.s0 = ld32(p + 4); r.s1 = ld32(p + 8); r.s2 = ld32(p + 12);
+    const u32x4 h = ld128(p);
+    r.dm = h.x; r.s0 = h.y; r.s1 = h.z; r.s2 = h.w;
     r.h0 = ld128(p + 16); r.h1 = ld128(p + 32);
     r.q0 = ld128(p + 48 + 32 * j);
     r.q1 = ld128(p + 64 + 32 * j);
@@ -221,7 +248,7 @@ struct Q5K {
     int j = u & 3;
     uint32_t l5[8], h5[8];
     codes(r, u, l5, h5);
-    int lo = 0, hi = 0;
+    int lo = kSum0, hi = kSum0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       lo = dot4_us(l5[i], a.q[i], lo);
@@ -233,9 +260,10 @@ struct Q5K {
     Q4K::scale_min(t, 2 * j + 1, sc1, mn1);
     float d = half_bits_to_float((uint16_t)(r.dm & 0xFFFF));
     float dmin = half_bits_to_float((uint16_t)(r.dm >> 16));
-    float pos = a.d0 * (float)(sc0 * lo) + a.d1 * (float)(sc1 * hi);
-    float neg = a.s0 * (float)mn0 + a.s1 * (float)mn1;
-    return d * pos - dmin * neg;
+    // 63 * 32 * 31 * 127 < 2^24: the products of scales and sums are exact
+    const float pos = fma_rn(a.d0, mul_rn(sum_float(kSum0 + sc0), sum_float(lo)), mul_rn(a.d1, mul_rn(sum_float(kSum0 + sc1), sum_float(hi))));
+    const float neg = fma_rn(a.s0, sum_float(kSum0 + mn0), mul_rn(a.s1, sum_float(kSum0 + mn1)));
+    return fma_rn(d, pos, -mul_rn(dmin, neg));
   }
   static BL_HD void decode(const Regs& r, int u, float* out) {
     int j = u & 3;
@@ -317,9 +345,9 @@ struct Q6K {
         sx = dot4(0x01010101u, x[i], sx);
       }
       s -= 32 * sx;
-      acc += ads[2 * (4 * n + g)] * (float)(scale(r, 8 * n + 2 * g + h) * s);
+      acc = fma_rn(ads[2 * (4 * n + g)], (float)(scale(r, 8 * n + 2 * g + h) * s), acc);
     }
-    return half_bits_to_float((uint16_t)r.d) * acc;
+    return mul_rn(half_bits_to_float((uint16_t)r.d), acc);
   }
   static BL_HD void decode(const Regs& r, int u, float* out /*64: g*16 + i*/) {
     int n = (u >> 1) & 1, h = u & 1;
@@ -358,7 +386,7 @@ struct Q80 {
   static BL_HD float dot(const Regs& r, const ActUnit& a) {
     const uint32_t w[16] = {r.q[0].x, r.q[0].y, r.q[0].z, r.q[0].w, r.q[1].x, r.q[1].y, r.q[1].z, r.q[1].w,
                             r.q[2].x, r.q[2].y, r.q[2].z, r.q[2].w, r.q[3].x, r.q[3].y, r.q[3].z, r.q[3].w};
-    int lo = 0, hi = 0;
+    int lo = kSum0, hi = kSum0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       lo = dot4(w[i], a.q[i], lo);
@@ -366,7 +394,7 @@ struct Q80 {
     }
     float d0 = half_bits_to_float((uint16_t)(r.dd & 0xFFFF));
     float d1 = half_bits_to_float((uint16_t)(r.dd >> 16));
-    return d0 * a.d0 * (float)lo + d1 * a.d1 * (float)hi;
+    return fma_rn(mul_rn(d0, a.d0), sum_float(lo), mul_rn(mul_rn(d1, a.d1), sum_float(hi)));
   }
   static BL_HD void decode(const Regs& r, float* out) {
     float d0 = half_bits_to_float((uint16_t)(r.dd & 0xFFFF));
@@ -406,13 +434,13 @@ struct Q8F {
   static BL_HD float dot(const Regs& r, const ActUnit& a) {
     const uint32_t w[16] = {r.q[0].x, r.q[0].y, r.q[0].z, r.q[0].w, r.q[1].x, r.q[1].y, r.q[1].z, r.q[1].w,
                             r.q[2].x, r.q[2].y, r.q[2].z, r.q[2].w, r.q[3].x, r.q[3].y, r.q[3].z, r.q[3].w};
-    int lo = 0, hi = 0;
+    int lo = kSum0, hi = kSum0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       lo = dot4(w[i], a.q[i], lo);
       hi = dot4(w[8 + i], a.q[8 + i], hi);
     }
-    return scale(r.d0) * a.d0 * (float)lo + scale(r.d1) * a.d1 * (float)hi;
+    return fma_rn(mul_rn(scale(r.d0), a.d0), sum_float(lo), mul_rn(mul_rn(scale(r.d1), a.d1), sum_float(hi)));
   }
   static BL_HD void decode(const Regs& r, float* out) {
     const float d0 = scale(r.d0), d1 = scale(r.d1);
@@ -462,7 +490,7 @@ struct Q2K {
         sx = dot4(0x01010101u, a.q[4 * g + i], sx);
       }
       const uint32_t scb = (r.sc >> (8 * g)) & 0xFF;
-      acc += ((g >> 1) ? a.d1 : a.d0) * (d * (float)(scb & 0xF) * (float)s - dmin * (float)(scb >> 4) * (float)sx);
+      acc = fma_rn((g >> 1) ? a.d1 : a.d0, fma_rn(mul_rn(d, (float)(scb & 0xF)), (float)s, -mul_rn(mul_rn(dmin, (float)(scb >> 4)), (float)sx)), acc);
     }
     return acc;
   }
@@ -520,9 +548,9 @@ struct Q3K {
         sx = dot4(0x01010101u, a.q[4 * g + i], sx);
       }
       const int sc = (int)(int8_t)((r.sc >> (8 * g)) & 0xFF);
-      acc += ((g >> 1) ? a.d1 : a.d0) * (float)(sc * (s + 4 * sh - 4 * sx));
+      acc = fma_rn((g >> 1) ? a.d1 : a.d0, (float)(sc * (s + 4 * sh - 4 * sx)), acc);
     }
-    return half_bits_to_float((uint16_t)r.d) * acc;
+    return mul_rn(half_bits_to_float((uint16_t)r.d), acc);
   }
   static BL_HD void decode(const Regs& r, int u, float* out) {
     const int n = (u >> 1) & 1, jp = u & 1;
@@ -591,8 +619,8 @@ struct Q32 {
       for (int j = 0; j < 8; ++j) s = dot4_us(c[j], a.q[8 * b + j], s);
       const float d = half_bits_to_float((uint16_t)(r.dd >> (16 * b)));
       const float da = b ? a.d1 : a.d0, sa = b ? a.s1 : a.s0;
-      if (HAS_MIN) acc += d * da * (float)s + half_bits_to_float((uint16_t)(r.mm >> (16 * b))) * sa;
-      else acc += d * (da * (float)s - (float)(BITS == 5 ? 16 : 8) * sa);
+      if (HAS_MIN) acc += fma_rn(mul_rn(d, da), (float)s, mul_rn(half_bits_to_float((uint16_t)(r.mm >> (16 * b))), sa));
+      else acc = fma_rn(d, fma_rn(da, (float)s, -mul_rn((float)(BITS == 5 ? 16 : 8), sa)), acc);
     }
     return acc;
   }
@@ -704,9 +732,9 @@ struct NvFp4 {
         s = dot4(lo4, aq[4 * g + 2 * h], s);
         s = dot4(hi4, aq[4 * g + 2 * h + 1], s);
       }
-      acc += sc[g] * ad[g >> 1] * (float)s;
+      acc = fma_rn(mul_rn(sc[g], ad[g >> 1]), (float)s, acc);
     }
-    return acc * r.g * 0.5f;
+    return mul_rn(mul_rn(acc, r.g), 0.5f);
   }
   static BL_HD void decode(const Regs& r, float* out) {
     const uint32_t w[8] = {r.q0.x, r.q0.y, r.q0.z, r.q0.w, r.q1.x, r.q1.y, r.q1.z, r.q1.w};
@@ -732,6 +760,15 @@ struct Fp8B128 {
     uint32_t sb = ld32(row + K + 4 * (u >> 1));
     __builtin_memcpy(&r.sc, &sb, 4);
   }
+  // signed byte b of a word (on the device by a byte permute into the bits of 2^23 + 128 + value: the conversion
+  // instruction runs at a quarter of the rate, and a unit has 64 of them)
+  static BL_HD float byte_float(uint32_t w, int b) {
+#if defined(__CUDA_ARCH__)
+    return __uint_as_float(__byte_perm(w ^ 0x80808080u, 0x4B000000u, 0x7440u | b)) - 8388736.0f;
+#else
+    return (float)(int8_t)((w >> (8 * b)) & 0xFF);
+#endif
+  }
   static BL_HD float dot(const Regs& r, const uint32_t* aq, const float* ad) {
     float acc0 = 0.f, acc1 = 0.f;
 #pragma unroll
@@ -744,12 +781,12 @@ struct Fp8B128 {
         e4m3x4_to_float(w[k], wv);
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-          const float xv = (float)(int8_t)((aq[4 * i + k] >> (8 * b)) & 0xFF);
-          if (i < 2) acc0 = wv[b] * xv + acc0; else acc1 = wv[b] * xv + acc1;
+          const float xv = byte_float(aq[4 * i + k], b);
+          if (i < 2) acc0 = fma_rn(wv[b], xv, acc0); else acc1 = fma_rn(wv[b], xv, acc1);
         }
       }
     }
-    return r.sc * (ad[0] * acc0 + ad[1] * acc1);
+    return mul_rn(r.sc, fma_rn(ad[0], acc0, mul_rn(ad[1], acc1)));
   }
   static BL_HD void decode(const Regs& r, float* out) {
 #pragma unroll
@@ -926,16 +963,16 @@ template <> struct ActOf<Q6K> {
     float acc = 0.f;
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
-      int s = 0, sx = 0;
+      int s = kSum0, sx = 0;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         s = dot4_us(c[g][i], a.q[4 * g + i], s);
         sx = dot4(0x01010101u, a.q[4 * g + i], sx);
       }
-      s -= 32 * sx;
-      acc += a.d[g] * (float)(Q6K::scale(r, 8 * n + 2 * g + h) * s);
+      s -= 32 * sx;                       // 128 * 16 * 63 * 127 < 2^24: the product with the scale is exact
+      acc = fma_rn(a.d[g], mul_rn(sum_float(kSum0 + Q6K::scale(r, 8 * n + 2 * g + h)), sum_float(s)), acc);
     }
-    return half_bits_to_float((uint16_t)r.d) * acc;
+    return mul_rn(half_bits_to_float((uint16_t)r.d), acc);
   }
 };
 

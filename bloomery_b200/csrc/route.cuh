@@ -146,44 +146,63 @@ __device__ __forceinline__ bool route_block(const RouteParams& p, int m, RouteSh
 // their maximum over the warp (redux) and the first lane that has it, so equal scores go to the smaller id as in rank
 // counting.  The first `n` picks come out in lanes 0 .. n - 1 (id and logit); false: some logit is not finite.
 __host__ __device__ __forceinline__ bool route_pick_ok(const RouteParams& p) {
-  return p.mode == 0 && p.renorm && p.n_group <= 1 && (p.E == 32 || p.E == 64 || p.E == 128 || p.E == 256);
+  return p.mode == 0 && p.renorm && p.n_group <= 1 && (p.E == 32 || p.E == 64 || p.E == 128 || p.E == 256) &&
+         ((uintptr_t)p.logits & 15) == 0;
 }
 
-__device__ __forceinline__ bool route_pick(const RouteParams& p, int m, int lane, int n, int& id, float& logit) {
-  const int per = p.E / 32;
-  const float* row = p.logits + (long)m * p.E + lane * per;
-  float l[8];
-  unsigned key[8];
+template <int PER>
+__device__ __forceinline__ bool route_pick_per(const RouteParams& p, int m, int lane, int n, int& id, float& logit) {
+  const float* row = p.logits + (long)m * p.E + lane * PER;
+  float l[PER];
+  unsigned key[PER];
   bool nonfinite = false;
+  if constexpr (PER % 4 == 0) {
 #pragma unroll
-  for (int i = 0; i < 8; ++i) l[i] = i < per ? __ldcg(row + i) : 0.f;
+    for (int i = 0; i < PER; i += 4) {
+      const float4 v = __ldcg(reinterpret_cast<const float4*>(row + i));
+      l[i] = v.x; l[i + 1] = v.y; l[i + 2] = v.z; l[i + 3] = v.w;
+    }
+  } else {
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < PER; ++i) l[i] = __ldcg(row + i);
+  }
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
     nonfinite |= !isfinite(l[i]);
     const unsigned b = __float_as_uint(l[i] + 0.0f);               // -0 and 0 are equal scores
-    key[i] = i < per ? ((b >> 31) ? ~b : b | 0x80000000u) : 0u;    // finite scores have keys above 0
+    key[i] = (b >> 31) ? ~b : b | 0x80000000u;                     // finite scores have keys above 0
   }
   id = 0; logit = 0.f;
   if (__any_sync(0xffffffffu, nonfinite)) return false;
+#pragma unroll 1
   for (int r = 0; r < n; ++r) {
-    unsigned best = 0u;
+    unsigned best = key[0];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) best = max(best, key[i]);
+    for (int i = 1; i < PER; ++i) best = max(best, key[i]);
     const unsigned top = __reduce_max_sync(0xffffffffu, best);
     const int src = __ffs(__ballot_sync(0xffffffffu, best == top)) - 1;
     int mine = 0;
     float val = 0.f;
 #pragma unroll
-    for (int i = 7; i >= 0; --i)
+    for (int i = PER - 1; i >= 0; --i)
       if (key[i] == top) { mine = i; val = l[i]; }
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < PER; ++i)
       if (lane == src && i == mine) key[i] = 0u;
-    const int e = __shfl_sync(0xffffffffu, lane * per + mine, src);
+    const int e = __shfl_sync(0xffffffffu, lane * PER + mine, src);
     const float v = __shfl_sync(0xffffffffu, val, src);
     if (lane == r) { id = e; logit = v; }
   }
   return true;
+}
+
+__device__ __forceinline__ bool route_pick(const RouteParams& p, int m, int lane, int n, int& id, float& logit) {
+  switch (p.E) {
+    case 32: return route_pick_per<1>(p, m, lane, n, id, logit);
+    case 64: return route_pick_per<2>(p, m, lane, n, id, logit);
+    case 128: return route_pick_per<4>(p, m, lane, n, id, logit);
+    default: return route_pick_per<8>(p, m, lane, n, id, logit);
+  }
 }
 
 // Weights of the picks in lanes 0 .. top_k - 1 (the arithmetic of route_block, softmax over the chosen).
