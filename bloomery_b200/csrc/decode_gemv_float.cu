@@ -1,0 +1,6 @@
+// The decode GEMV (decode_gemv.cu) of calls with F32 / F16 / BF16 rows among their weights.
+#include "gemv_kernel.cuh"
+
+namespace bl {
+template cudaError_t gemv_family<true, 1>(const GemvArgs&, int, int, int, cudaStream_t);
+}  // namespace bl

@@ -1,0 +1,336 @@
+// The kernel of the quantised GEMV (decode_gemv.cu), one translation unit a family of weight types.
+#pragma once
+#include "gemv_common.cuh"
+
+namespace bl {
+
+// ---- the rows of one warp ---------------------------------------------------------------
+// A warp owns rows [r_lo, r_hi) of its segment and walks them R at a time; every load of a
+// chunk is issued before anything is computed.  C = units per lane per inner step.
+// `between` runs once per block, after the very first loads are in flight.
+template <class T, int MB, int R, int C, class Between>
+__device__ __forceinline__ void rows_q(const GemvArgs& a, const GemvSeg& s, int r_lo, int r_hi, int out_col0,
+                                       const int8_t* sq, const float2* sds, const float* s_scale, Between&& between) {
+  using U = Unit<T>;
+  const int K = a.K, lane = threadIdx.x & 31;
+  const int nunits = K / 64;
+  const unsigned push_epoch = a.push.n_ranks > 0 ? site_epoch(a.push.step, a.push.sites_per_step, a.push.site_index) : 0u;
+  for (int r0 = r_lo; r0 < r_hi || r0 == r_lo; r0 += R) {
+    float acc[R][MB];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int m = 0; m < MB; ++m) acc[r][m] = 0.f;
+    for (int base = 0; base < nunits; base += 32 * C) {
+      typename U::Regs regs[R][C];
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          const int u = base + c * 32 + lane;
+          if (u < nunits && r0 + r < r_hi) U::loadu(s.w + (long)(r0 + r) * s.row_bytes, u, K, regs[r][c]);
+        }
+      between();
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        const int u = base + c * 32 + lane;
+        if (u < nunits) {
+#pragma unroll
+          for (int m = 0; m < MB; ++m) {
+            // the block's activation rows sit in the conflict-free chunk layout of its weight type
+            ActRegs act;
+            StagedAct<T>::load(sq + (long)m * K, sds + (long)m * (K / 32), u, nunits, act);
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+              if (r0 + r < r_hi) acc[r][m] += ActOf<T>::dot(regs[r][c], u, act);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int m = 0; m < MB; ++m) acc[r][m] = warp_sum(acc[r][m]);
+    if (lane == 0) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        if (r0 + r < r_hi) {
+          const int col = out_col0 + r0 + r;
+#pragma unroll
+          for (int m = 0; m < MB; ++m)
+            if (m < a.M) {
+              float v = acc[r][m] * s_scale[m];
+              if (a.push.n_ranks > 0) { push_store(a.push, push_epoch, (long)m * a.out_stride + col, v); continue; }
+              if (a.resid) v += a.resid[(long)m * a.resid_stride + col];
+              a.out[(long)m * a.out_stride + col] = v;
+            }
+        }
+      }
+    }
+    if (r0 + R >= r_hi) break;
+  }
+}
+
+// The same for passes of several rows whose weight rows are at most 32 C units long: the weights of R rows stay in registers
+// and the pass's rows walk past them one by one, so nothing is kept per (weight row, row of the pass) and the loop runs
+// over live rows only.  Sums are those of rows_q.  Lane m keeps the results of row m and stores them at the end.
+// (Accumulators of 2 x 8 instead spilled 1 KB a thread; five rows in a bucket of eight computed eight.)
+template <class T, int R, int C, class Between>
+__device__ __forceinline__ void rows_multi(const GemvArgs& a, const GemvSeg& s, int r_lo, int r_hi, int out_col0, unsigned live,
+                                           const int8_t* sq, const float2* sds, const float* s_scale, Between&& between) {
+  using U = Unit<T>;
+  const int K = a.K, lane = threadIdx.x & 31;
+  const int nunits = K / 64;
+  const bool mine = lane < kMaxRows && (live >> lane & 1);
+  const unsigned push_epoch = a.push.n_ranks > 0 ? site_epoch(a.push.step, a.push.sites_per_step, a.push.site_index) : 0u;
+  for (int r0 = r_lo; r0 < r_hi || r0 == r_lo; r0 += R) {
+    typename U::Regs regs[R][C];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int c = 0; c < C; ++c)
+        if (c * 32 + lane < nunits && r0 + r < r_hi) U::loadu(s.w + (long)(r0 + r) * s.row_bytes, c * 32 + lane, K, regs[r][c]);
+    between();
+    float res[R], old[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      res[r] = old[r] = 0.f;
+      if (a.resid && a.push.n_ranks == 0 && mine && r0 + r < r_hi) old[r] = a.resid[(long)lane * a.resid_stride + out_col0 + r0 + r];
+    }
+#pragma unroll 1
+    for (unsigned left = live; left; left &= left - 1) {
+      const int m = __ffs(left) - 1;
+      float acc[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) acc[r] = 0.f;
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        const int u = c * 32 + lane;
+        if (u < nunits) {
+          ActRegs act;
+          StagedAct<T>::load(sq + (long)m * K, sds + (long)m * (K / 32), u, nunits, act);
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+            if (r0 + r < r_hi) acc[r] += ActOf<T>::dot(regs[r][c], u, act);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const float v = warp_sum(acc[r]);
+        if (lane == m) res[r] = v;
+      }
+    }
+    if (mine) {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (r0 + r < r_hi) {
+          const long at = (long)lane * a.out_stride + out_col0 + r0 + r;
+          float v = res[r] * s_scale[lane];
+          if (a.push.n_ranks > 0) { push_store(a.push, push_epoch, at, v); continue; }
+          if (a.resid) v += old[r];
+          a.out[at] = v;
+        }
+    }
+    if (r0 + R >= r_hi) break;
+  }
+}
+
+// float weights (F32 / F16 / BF16) against fp32 x*gain rows
+template <int MB, int R, class Between>
+__device__ __forceinline__ void rows_f(const GemvArgs& a, const GemvSeg& s, int r_lo, int r_hi, int out_col0, unsigned live,
+                                       const float* sx, const float* s_scale, Between&& between) {
+  const int K = a.K, lane = threadIdx.x & 31;
+  const unsigned push_epoch = a.push.n_ranks > 0 ? site_epoch(a.push.step, a.push.sites_per_step, a.push.site_index) : 0u;
+  for (int r0 = r_lo; r0 < r_hi || r0 == r_lo; r0 += R) {
+    float acc[R][MB];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int m = 0; m < MB; ++m) acc[r][m] = 0.f;
+    for (int i = lane * 8; i < K; i += 256) {
+      float wv[R][8];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const uint8_t* row = s.w + (long)min(r0 + r, s.rows - 1) * s.row_bytes;
+        if (s.wtype == WT_F32) {
+          float4 p = __ldg(reinterpret_cast<const float4*>(row) + i / 4), q = __ldg(reinterpret_cast<const float4*>(row) + i / 4 + 1);
+          wv[r][0] = p.x; wv[r][1] = p.y; wv[r][2] = p.z; wv[r][3] = p.w; wv[r][4] = q.x; wv[r][5] = q.y; wv[r][6] = q.z; wv[r][7] = q.w;
+        } else {
+          uint4 p = __ldg(reinterpret_cast<const uint4*>(row) + i / 8);
+          const uint32_t ws[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            float2 f = (s.wtype == WT_F16) ? __half22float2(*reinterpret_cast<const __half2*>(&ws[j]))
+                                           : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ws[j]));
+            wv[r][2 * j] = f.x; wv[r][2 * j + 1] = f.y;
+          }
+        }
+      }
+      between();
+#pragma unroll
+      for (int m = 0; m < MB; ++m) {
+        if (!(live >> m & 1)) continue;
+        const float4 x0 = *reinterpret_cast<const float4*>(sx + (long)m * K + i);
+        const float4 x1 = *reinterpret_cast<const float4*>(sx + (long)m * K + i + 4);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          float t = acc[r][m];
+          t = fmaf(wv[r][0], x0.x, t); t = fmaf(wv[r][1], x0.y, t); t = fmaf(wv[r][2], x0.z, t); t = fmaf(wv[r][3], x0.w, t);
+          t = fmaf(wv[r][4], x1.x, t); t = fmaf(wv[r][5], x1.y, t); t = fmaf(wv[r][6], x1.z, t); t = fmaf(wv[r][7], x1.w, t);
+          acc[r][m] = t;
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int m = 0; m < MB; ++m) acc[r][m] = warp_sum(acc[r][m]);
+    if (lane == 0) {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (r0 + r < r_hi) {
+          const int col = out_col0 + r0 + r;
+#pragma unroll
+          for (int m = 0; m < MB; ++m)
+            if (m < a.M && (live >> m & 1)) {
+              float v = acc[r][m] * s_scale[m];
+              if (a.push.n_ranks > 0) { push_store(a.push, push_epoch, (long)m * a.out_stride + col, v); continue; }
+              if (a.resid) v += a.resid[(long)m * a.resid_stride + col];
+              a.out[(long)m * a.out_stride + col] = v;
+            }
+        }
+    }
+    if (r0 + R >= r_hi) break;
+  }
+}
+
+// FAM: 0 = ggml integer-dot types, 1 = those plus float rows, 2 = block-scaled float planes (NVFP4, FP8).
+// One kernel per family keeps the register budget of the K-quant bodies free of the plane decoders.
+// MULTI: rows_multi and the prologues that fetch all rows at once (two rows and more, weight rows of at most 32 C units);
+// otherwise MB rows as a whole.
+template <int MB, int R, int C, bool NORM, int FAM, bool MULTI>
+__global__ void __launch_bounds__(256, 2) gemv_kernel(const GemvArgs a) {
+  static_assert(!MULTI || MB == kMaxRows, "any number of rows");
+  extern __shared__ __align__(16) uint8_t smem[];
+  const int K = a.K;
+  int8_t* sq = reinterpret_cast<int8_t*>(smem);
+  const int rows_in = MULTI ? a.M : MB;
+  float2* sds = reinterpret_cast<float2*>(smem + (size_t)rows_in * K);
+  double* red = reinterpret_cast<double*>(sds + (size_t)rows_in * (K / 32));
+  float* s_scale = reinterpret_cast<float*>(red + rows_in * 8);
+  float* sx = s_scale + 8;  // float weights, or several rows to normalise
+  unsigned live = (1u << MB) - 1;      // MULTI: the pass's rows that do not just fill its bucket
+  if constexpr (MULTI) {
+    live = 0;
+#pragma unroll
+    for (int m = 0; m < kMaxRows; ++m) live |= (m < a.M && (!a.row_seq || a.row_seq[m] >= 0) ? 1u : 0u) << m;
+  }
+
+  if (a.n_pf > 0 && threadIdx.x == 0) prefetch_spans_l2(a.pf_ptr, a.pf_bytes, a.n_pf);
+  int si = 0, col0 = 0;
+#pragma unroll
+  for (int q = 1; q < 4; ++q)
+    if (q < a.nseg && (int)blockIdx.x >= a.seg[q].blk0) { si = q; }
+  for (int q = 0; q < si; ++q) col0 += a.seg[q].rows;
+  // a block serves one weight type: its q8 activation rows take the chunk layout that type's units read without
+  // bank conflicts (act_chunk_pos); float rows read the fp32 copy instead
+  const int act_layout = staged_layout(a.seg[si].wtype);
+  bool ready = false;
+  auto between = [&]() {
+    if (!ready) {
+      pdl_wait();
+      if constexpr (MULTI && NORM) {
+        prologue_norm_rows<FAM == 1>(a, live, sq, sds, sx, s_scale, red, act_layout);
+      } else if constexpr (MULTI) {
+        prologue_q8_rows(a, live, sq, sds, s_scale, act_layout);
+      } else if constexpr (NORM) {
+        prologue_norm<MB, FAM == 1>(a, sq, sds, sx, s_scale, red, act_layout);
+      } else {
+        prologue_q8in<MB>(a, sq, sds, s_scale, act_layout);
+      }
+      pdl_launch();
+      ready = true;
+    }
+  };
+  {
+    const GemvSeg& s = a.seg[si];
+    // even split of the segment's rows over its warps
+    const int W = s.nblk * 8, wg = ((int)blockIdx.x - s.blk0) * 8 + (threadIdx.x >> 5);
+    const int rpw = (s.rows + W - 1) / W;
+    const int r_lo = min(s.rows, wg * rpw), r_hi = min(s.rows, r_lo + rpw);
+    auto rows = [&](auto t) {
+      if constexpr (MULTI) rows_multi<decltype(t), R, C>(a, s, r_lo, r_hi, col0, live, sq, sds, s_scale, between);
+      else rows_q<decltype(t), MB, R, C>(a, s, r_lo, r_hi, col0, sq, sds, s_scale, between);
+    };
+    if constexpr (FAM == 2) {
+      switch (s.wtype) {
+        case WT_NVFP4: rows(NvFp4{}); break;
+        case WT_FP8_B128: rows(Fp8B128{}); break;
+        case WT_Q2_K: rows(Q2K{}); break;
+        case WT_Q3_K: rows(Q3K{}); break;
+        case WT_Q4_0: rows(Q40{}); break;
+        case WT_Q4_1: rows(Q41{}); break;
+        case WT_Q5_0: rows(Q50{}); break;
+        case WT_Q5_1: rows(Q51{}); break;
+        default: break;
+      }
+    } else {
+      switch (s.wtype) {
+        case WT_Q4_K: rows(Q4K{}); break;
+        case WT_Q6_K: rows(Q6K{}); break;
+        case WT_Q5_K: rows(Q5K{}); break;
+        case WT_Q8_0: rows(Q80{}); break;
+        case WT_Q8_F32: rows(Q8F{}); break;
+        default:
+          if (FAM == 1) rows_f<MB, R>(a, s, r_lo, r_hi, col0, live, sx, s_scale, between);
+      }
+    }
+  }
+  between();
+}
+
+// M rows of activations, with their fp32 values or without
+static inline size_t gemv_smem(int M, int K, bool values) {
+  size_t b = (size_t)M * K + (size_t)M * (K / 32) * 8 + M * 8 * 8 + 8 * 4;
+  if (values) b += (size_t)M * K * 4;
+  return b;
+}
+
+template <int MB, int R, int C, bool NORM, int FAM, bool MULTI>
+static cudaError_t gemv_launch(const GemvArgs& a, int grid, cudaStream_t st) {
+  const size_t smem = gemv_smem(MULTI ? a.M : MB, a.K, FAM == 1 || (MULTI && NORM));
+  static PerDevice limit;
+  if (limit.due()) {
+    cudaFuncSetAttribute(gemv_kernel<MB, R, C, NORM, FAM, MULTI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    limit.mark();
+  }
+  return launch(gemv_kernel<MB, R, C, NORM, FAM, MULTI>, dim3(grid), dim3(256), smem, st, a);
+}
+
+template <bool NORM, int FAM, int MB, bool MULTI>
+static cudaError_t gemv_dispatch_shape(const GemvArgs& a, int R, int C, int grid, cudaStream_t st) {
+  if (C == 2) return gemv_launch<MB, 1, 2, NORM, FAM, MULTI>(a, grid, st);
+  // several rows keep the decoded weights of float planes in registers from one row to the next, which leaves room for one
+  if constexpr (!MULTI || FAM == 0) {
+    if (R >= 3) return gemv_launch<MB, 3, 1, NORM, FAM, MULTI>(a, grid, st);
+  }
+  if constexpr (!MULTI || FAM != 2) {
+    if (R >= 2) return gemv_launch<MB, 2, 1, NORM, FAM, MULTI>(a, grid, st);
+  }
+  return gemv_launch<MB, 1, 1, NORM, FAM, MULTI>(a, grid, st);
+}
+
+// One row; several rows; several rows whose weight rows do not fit the registers of a warp (two columns of units a lane), or that
+// are sums over ranks.
+template <bool NORM, int FAM>
+cudaError_t gemv_family(const GemvArgs& a, int R, int C, int grid, cudaStream_t st) {
+  if (a.M == 1) return gemv_dispatch_shape<NORM, FAM, 1, false>(a, R, C, grid, st);
+  if (a.K / 64 > 32 * C || a.red.n_ranks > 0) {
+    if (a.M <= 2) return gemv_launch<2, 1, 2, NORM, FAM, false>(a, grid, st);
+    if (a.M <= 4) return gemv_launch<4, 1, 2, NORM, FAM, false>(a, grid, st);
+    return gemv_launch<kMaxRows, 1, 2, NORM, FAM, false>(a, grid, st);
+  }
+  return gemv_dispatch_shape<NORM, FAM, kMaxRows, true>(a, R, C, grid, st);
+}
+
+}  // namespace bl

@@ -122,9 +122,11 @@ def gemv(segs: Sequence[QWeight], M: int, out: torch.Tensor, *, x: Optional[torc
          gain: Optional[torch.Tensor] = None, eps: float = 1e-6, xq: Optional[torch.Tensor] = None,
          xds: Optional[torch.Tensor] = None, resid: Optional[torch.Tensor] = None,
          red: Optional[ReduceIn] = None, push: Optional[PushOut] = None,
-         fault: Optional[torch.Tensor] = None, layer: int = 0, prefetch: Optional[Sequence[torch.Tensor]] = None) -> None:
+         fault: Optional[torch.Tensor] = None, layer: int = 0, prefetch: Optional[Sequence[torch.Tensor]] = None,
+         row_seq: Optional[torch.Tensor] = None) -> None:
     """``prefetch``: up to six tensors a later launch will stream (the next layer's projections); the launch asks L2
-    for them before it waits for its predecessor."""
+    for them before it waits for its predecessor.  ``row_seq``: rows with a negative entry only fill the pass's bucket;
+    their results may be left out."""
     fams = [_family(sg.qtype) for sg in segs]
     if len(set(fams) - {1}) > 1 or (2 in fams and 1 in fams):
         # segments of different kernel families (e.g. a Q5_0 fallback tensor beside K-quants): one call per run
@@ -136,7 +138,7 @@ def gemv(segs: Sequence[QWeight], M: int, out: torch.Tensor, *, x: Optional[torc
             width = sum(sg.rows for sg in segs[i:j])
             gemv(segs[i:j], M, out[:, col:col + width], x=x, gain=gain, eps=eps, xq=xq, xds=xds,
                  resid=resid[:, col:col + width] if resid is not None else None, red=red if i == 0 else None,
-                 push=push, fault=fault, layer=layer, prefetch=prefetch if i == 0 else None)
+                 push=push, fault=fault, layer=layer, prefetch=prefetch if i == 0 else None, row_seq=row_seq)
             col += width
             i = j
         return
@@ -162,7 +164,7 @@ def gemv(segs: Sequence[QWeight], M: int, out: torch.Tensor, *, x: Optional[torc
     rc = cuda().bl_gemv(I(n), wp, rows, wts, I(K), I(M), I(1 if norm else 0),
                         p(x), L(x.stride(0) if norm else 0), p(gain), F(eps), p(xq), p(xds),
                         p(out), L(out.stride(0)), p(resid), L(resid.stride(0) if resid is not None else 0),
-                        _ref(red), _ref(push), p(fault), I(layer), I(sm_count()), I(len(pf)), pfp, pfb, stream())
+                        _ref(red), _ref(push), p(fault), I(layer), I(sm_count()), I(len(pf)), pfp, pfb, p(row_seq), stream())
     check(rc, "bl_gemv")
 
 

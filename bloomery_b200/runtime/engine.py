@@ -240,7 +240,7 @@ class DecodeEngine:
         if head and self.stage_last:
             head_w = w.q.get("output.weight", w.q["token_embd.weight"])
             K.gemv([head_w], M, self.logits, x=x, gain=w.f["output_norm.weight"], eps=s.rms_eps,
-                   fault=self.fault, layer=s.n_layer); n += 1
+                   fault=self.fault, layer=s.n_layer, row_seq=self.row_seq); n += 1
             K.argmax_rows(self.logits, s.vocab, M, self.am_blocks, self.am_v, self.am_i, self.counters[1:2],
                           self.tokens_out, None, self.fault); n += 1
             if advance:
@@ -258,7 +258,7 @@ class DecodeEngine:
             n += self._predict(il, M, x)
         n += self._attn(il, M, x)
         K.gemv([w.q[b + "attn_output.weight"]], M, x, xq=self.attn_q, xds=self.attn_ds, resid=x,
-               fault=self.fault, layer=il); n += 1
+               fault=self.fault, layer=il, row_seq=self.row_seq); n += 1
         if s.layer_is_moe(il):
             if M == 1 and type(self)._moe is DecodeEngine._moe and not s.n_shared and self._cluster_ok(il):
                 # one row: router, routing, the chosen experts and the weighted sum as ONE cluster launch
@@ -401,7 +401,7 @@ class DecodeEngine:
             return self._attn_mla(il, M, x)
         K.gemv([w.q[b + "attn_q.weight"], w.q[b + "attn_k.weight"], w.q[b + "attn_v.weight"]], M, self.qkv,
                x=x, gain=w.f[b + "attn_norm.weight"], eps=s.rms_eps, fault=self.fault, layer=il,
-               prefetch=self._static_next(il))
+               prefetch=self._static_next(il), row_seq=self.row_seq)
         cl = K.attn_cluster_size(s.n_kv, M) if (self.attn_clusters and not self.kv_q8) else 0
         if cl:
             K.attn_cluster(self.qkv, w.f.get(b + "attn_q_norm.weight"), w.f.get(b + "attn_k_norm.weight"), self.inv_freq,

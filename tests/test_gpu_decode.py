@@ -52,6 +52,36 @@ def test_gemv_norm_matches_fp32(t, M):
     assert torch.equal(o1[0], out[M - 1])
 
 
+@pytest.mark.parametrize("t", ["Q4_K", "Q6_K", "NVFP4", "FP8_B128", "F32"])
+@pytest.mark.parametrize("Kd,rows", [(256, 40), (2048, 5123), (4096, 301), (4352, 77)])
+def test_gemv_rows_of_a_pass_equal_single_rows(t, Kd, rows):
+    """Rows of passes of 2 to 8, some of them only filling the bucket, have the bits of passes of one: one, two and more
+    units a lane, a last warp with fewer rows than it could take, projections and residual form."""
+    from bloomery_b200.ops import decode as K
+    torch.manual_seed(11)
+    if t == "F32":
+        from bloomery_b200.ops.decode import QWeight
+        qw = QWeight((torch.randn(rows, Kd, device=DEV) * 0.02).view(torch.uint8).reshape(rows, -1), t, Kd)
+    else:
+        qw, _ = _qw(torch.randn(rows, Kd) * 0.02, t)
+    x, gain, resid = torch.randn(8, Kd, device=DEV), 1 + 0.1 * torch.randn(Kd, device=DEV), torch.randn(8, rows, device=DEV)
+    c, ds = (v.to(DEV) for v in Q.quantize_act_q8(x.cpu()))
+    one, one_r = torch.zeros(8, rows, device=DEV), torch.zeros(8, rows, device=DEV)
+    for m in range(8):
+        K.gemv([qw], 1, one[m:m + 1], x=x[m:m + 1], gain=gain, eps=1e-6)
+        if t != "F32":
+            K.gemv([qw], 1, one_r[m:m + 1], xq=c[m:m + 1], xds=ds[m:m + 1], resid=resid[m:m + 1])
+    for M, dead in [(2, ()), (3, (1,)), (8, (5, 6, 7)), (8, ())]:
+        seq = torch.tensor([-1 if m in dead else m for m in range(M)], dtype=torch.int32, device=DEV)
+        live = [m for m in range(M) if m not in dead]
+        out = torch.zeros(M, rows, device=DEV)
+        K.gemv([qw], M, out, x=x, gain=gain, eps=1e-6, row_seq=seq)
+        assert torch.equal(out[live], one[live])
+        if t != "F32":
+            K.gemv([qw], M, out, xq=c, xds=ds, resid=resid, row_seq=seq)
+            assert torch.equal(out[live], one_r[live])
+
+
 def test_gemv_q8in_resid_multiseg():
     from bloomery_b200.ops import decode as K
     torch.manual_seed(1)
@@ -137,12 +167,14 @@ def test_router_sigmoid_groups_and_fault():
     assert torch.isnan(wts[1]).all() and not torch.isnan(wts[0]).any()
 
 
-def test_gate_up_routes_like_route_rows():
-    """The routing done inside gate_up (from logits) equals the standalone routing launch."""
+@pytest.mark.parametrize("E", [16, 32, 128, 256])
+def test_gate_up_routes_like_route_rows(E):
+    """The routing done inside gate_up (from logits) equals the standalone routing launch: by the block, and by one warp with
+    one, four and eight experts a lane."""
     from bloomery_b200.ops import decode as K
     from bloomery_b200.ops.decode import RouteRule
     torch.manual_seed(8)
-    H, I, E, k, M = 512, 256, 16, 4, 3
+    H, I, k, M = 512, 256, 4, 3
     gate, _ = _qw(torch.randn(E, I, H) * 0.03, "Q4_K")
     up, _ = _qw(torch.randn(E, I, H) * 0.03, "Q4_K")
     x = torch.randn(M, H)
