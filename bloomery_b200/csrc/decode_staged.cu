@@ -207,6 +207,8 @@ __device__ __forceinline__ void head_out_q8(const float (&o)[HEAD / 32], int lan
 // Key tiles of a row (0: it fills a bucket, or its key count is not one), how many of them a segment takes, and its segments.
 // Segments depend on the row alone, so its bits do not change with the rows beside it: a drafted token's row, or one of a
 // round of several users, is the row of a pass of one.
+// (Segments of at least two or four tiles leave fewer parts to merge: one row of 100 keys 1.84 -> 1.74 ms a pass, of 512 1.89 ->
+// 1.85; but several rows then share the processors worse, five of 400 5.03 -> 5.17, five of 1,500 5.35 -> 5.50.)
 struct RowSegs { int tiles, tps, used; };
 __device__ __forceinline__ RowSegs row_segs(const AttnArgs& a, int mm) {
   const int nk = a.row_pos[mm] + 1;
@@ -416,6 +418,18 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
       else cp_async_commit();
     }
   }
+  // Nor do the angles of the row and the gains: one row takes them ahead of the wait (several rows take them where they are
+  // used; kept in registers over the wait they cost five rows 3 us a layer).
+  float row_sn[DPL / 2], row_cs[DPL / 2], q_ahead[DPL], k_ahead[DPL];
+  if constexpr (!DEAL) {
+#pragma unroll
+    for (int j = 0; j < DPL / 2; ++j) sincosf((float)pos * a.inv_freq[lane + 32 * j], &row_sn[j], &row_cs[j]);
+#pragma unroll
+    for (int j = 0; j < DPL; ++j) {
+      if (a.q_gain) q_ahead[j] = a.q_gain[lane + 32 * j];
+      if (a.k_gain) k_ahead[j] = a.k_gain[lane + 32 * j];
+    }
+  }
   pdl_wait();
   pdl_launch();
   if (DEAL && publish) publish_empty();
@@ -423,11 +437,12 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
 
   // ---- queries of this KV head's group: RMSNorm + RoPE into shared memory ---------------------------
   const float* row = a.qkv + (long)m * a.qkv_stride;
-  auto norm_rope = [&](const float* src, const float* gain, bool rope, int at, float (&y)[DPL]) {
+  auto fetch_head = [&](const float* src, float (&x)[DPL]) {
     // lane owns elements lane + 32 j; NEOX pairs are (i, i + HALF)
-    float x[DPL];
 #pragma unroll
     for (int j = 0; j < DPL; ++j) x[j] = src[lane + 32 * j];
+  };
+  auto norm_rope = [&](float (&x)[DPL], const float* gain, const float (&ahead)[DPL], int at, float (&y)[DPL]) {
     if (gain) {
       double ss = 0.0;
 #pragma unroll
@@ -435,62 +450,28 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
       ss = warp_sum_d(ss);
       const float scale = (float)(1.0 / sqrt(ss / (double)HEAD + (double)a.eps));
 #pragma unroll
-      for (int j = 0; j < DPL; ++j) x[j] = (scale * gain[lane + 32 * j]) * x[j];
+      for (int j = 0; j < DPL; ++j) x[j] = (scale * (DEAL ? gain[lane + 32 * j] : ahead[j])) * x[j];
     }
-    if (rope) {
 #pragma unroll
-      for (int j = 0; j < DPL / 2; ++j) {
-        const int i = lane + 32 * j;
-        float sn, cs;
-        sincosf((float)at * a.inv_freq[i], &sn, &cs);
-        const float x0 = x[j], x1 = x[j + DPL / 2];
-        y[j] = fmaf(x0, cs, -(x1 * sn));
-        y[j + DPL / 2] = fmaf(x0, sn, x1 * cs);
-      }
+    for (int j = 0; j < DPL / 2; ++j) {
+      float sn, cs;
+      if constexpr (!DEAL) { sn = row_sn[j]; cs = row_cs[j]; }
+      if (DEAL || at != pos) sincosf((float)at * a.inv_freq[lane + 32 * j], &sn, &cs);
+      const float x0 = x[j], x1 = x[j + DPL / 2];
+      y[j] = fmaf(x0, cs, -(x1 * sn));
+      y[j + DPL / 2] = fmaf(x0, sn, x1 * cs);
+    }
+  };
+  // row mm of the pass: its key (or value) of this KV head, to where tiles are patched from and, the block's own row, to the cache
+  auto new_head = [&](int mm, bool is_k) { return a.qkv + (long)mm * a.qkv_stride + ((long)a.n_q + (is_k ? 0 : a.n_kv) + kvh) * HEAD; };
+  auto append = [&](int idx, int mm, int pp, bool is_k, float (&x)[DPL]) {
+    float y[DPL];
+    if (is_k) {
+      norm_rope(x, a.k_gain, k_ahead, pp, y);
     } else {
 #pragma unroll
       for (int j = 0; j < DPL; ++j) y[j] = x[j];
     }
-  };
-#pragma unroll
-  for (int h = 0; h < HPW; ++h) {
-    const int hg = warp + 8 * h;
-    if (hg < G) {
-      float y[DPL];
-      norm_rope(row + ((long)kvh * G + hg) * HEAD, a.q_gain, true, pos, y);
-#pragma unroll
-      for (int j = 0; j < DPL; ++j) sq[hg * QSTR + lane + 32 * j] = y[j] * a.q_scale;
-    }
-  }
-  probe_mark(a.probe, 2);
-  // ---- keys and values that this very pass appends --------------------------------------------------
-  // Rows of the pass that belong to the same sequence at or before this row's position are not in the cache
-  // yet (their owner blocks write them in this same launch), so a block computes the ones that fall inside its
-  // key range itself and patches them into the tiles; only the row's own block stores its row to the cache.
-  if (tid == 0) {
-    s_np = 0;
-    if constexpr (DEAL && HPW == 1) mbar_init(&s_turn, 8);
-  }
-  __syncthreads();
-  for (int mm = tid; mm < a.M; mm += 256) {
-    if (a.row_seq[mm] == seq) {
-      const int pp = a.row_pos[mm];
-      if (pp <= pos && pp >= t0 * kKeyTile && pp < t1 * kKeyTile) {
-        const int idx = atomicAdd(&s_np, 1);
-        if (idx < kMaxPatch) { s_pm[idx] = mm; s_ppos[idx] = pp; }
-      }
-    }
-  }
-  __syncthreads();
-  const int np = min(s_np, kMaxPatch);
-  int first_new = 0x7fffffff;                        // tiles that end in front of this position take nothing from the pass
-  for (int idx = 0; idx < np; ++idx) first_new = min(first_new, s_ppos[idx]);
-  for (int it = warp; it < 2 * np; it += 8) {
-    const int idx = it >> 1, mm = s_pm[idx], pp = s_ppos[idx];
-    const bool is_k = (it & 1) == 0;
-    float y[DPL];
-    const float* src = a.qkv + (long)mm * a.qkv_stride + ((long)a.n_q + (is_k ? 0 : a.n_kv) + kvh) * HEAD;
-    norm_rope(src, is_k ? a.k_gain : nullptr, is_k, pp, y);
     __half* sn = snew + ((size_t)idx * 2 + (is_k ? 0 : 1)) * HEAD;
     __half* dst = nullptr;
     if (mm == m) {
@@ -505,7 +486,59 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
       sn[lane + 32 * j] = hv;
       if (dst) dst[lane + 32 * j] = hv;
     }
+  };
+  // One row: its own key and value come in beside the queries, in the last segment's block, which was 1.2 us behind the others
+  // (with the angles and gains ahead of the wait, one row of 12,000 keys 2.15 -> 2.11 ms a pass, of 100 1.89 -> 1.86).
+  const bool single = !DEAL && a.M == 1, newest = single && pos < t1 * kKeyTile;
+  float x_new[DPL];
+  if (newest && warp < 2) fetch_head(new_head(0, warp == 0), x_new);
+#pragma unroll
+  for (int h = 0; h < HPW; ++h) {
+    const int hg = warp + 8 * h;
+    if (hg < G) {
+      float x[DPL], y[DPL];
+      fetch_head(row + ((long)kvh * G + hg) * HEAD, x);
+      norm_rope(x, a.q_gain, q_ahead, pos, y);
+#pragma unroll
+      for (int j = 0; j < DPL; ++j) sq[hg * QSTR + lane + 32 * j] = y[j] * a.q_scale;
+    }
   }
+  probe_mark(a.probe, 2);
+  // ---- keys and values that this very pass appends --------------------------------------------------
+  // Rows of the pass that belong to the same sequence at or before this row's position are not in the cache
+  // yet (their owner blocks write them in this same launch), so a block computes the ones that fall inside its
+  // key range itself and patches them into the tiles; only the row's own block stores its row to the cache.
+  int np = 0;
+  if (single) {
+    np = newest ? 1 : 0;
+    if (tid == 0) s_ppos[0] = pos;
+    if (newest && warp < 2) append(0, 0, pos, warp == 0, x_new);
+  } else {
+    if (tid == 0) {
+      s_np = 0;
+      if constexpr (DEAL && HPW == 1) mbar_init(&s_turn, 8);
+    }
+    __syncthreads();
+    for (int mm = tid; mm < a.M; mm += 256) {
+      if (a.row_seq[mm] == seq) {
+        const int pp = a.row_pos[mm];
+        if (pp <= pos && pp >= t0 * kKeyTile && pp < t1 * kKeyTile) {
+          const int idx = atomicAdd(&s_np, 1);
+          if (idx < kMaxPatch) { s_pm[idx] = mm; s_ppos[idx] = pp; }
+        }
+      }
+    }
+    __syncthreads();
+    np = min(s_np, kMaxPatch);
+    for (int it = warp; it < 2 * np; it += 8) {
+      float x[DPL];
+      fetch_head(new_head(s_pm[it >> 1], (it & 1) == 0), x);
+      append(it >> 1, s_pm[it >> 1], s_ppos[it >> 1], (it & 1) == 0, x);
+    }
+  }
+  int first_new = single ? pos : 0x7fffffff;         // tiles that end in front of this position take nothing from the pass
+  if (!single)
+    for (int idx = 0; idx < np; ++idx) first_new = min(first_new, s_ppos[idx]);
 
   probe_mark(a.probe, 3);
   float mx[HPW], l[HPW], acc[HPW][DPL];
