@@ -188,7 +188,7 @@ __device__ __forceinline__ uint4 short8(uint32_t w0, uint32_t w1, uint32_t s2, u
   return out;
 }
 
-// ---- slabs: the short form of the super-block types ------------------------------------------
+// ---- slabs: the super-block types, whole stages at a time ------------------------------------
 // A slab is 64 consecutive values.  Slab<T>::Regs holds a row's 128 values of a stage (slabs i and i + 1 of its super-block
 // `sb`, i even) with their scales; codes() yields the x-th one's 64 code bytes in value order (16 words) and the (scale,
 // offset) pair of each of its four groups of 16.  The packed scales are taken apart four at a time, and a byte becomes a float
@@ -290,18 +290,29 @@ template <> struct Slab<Q6K> {
   }
 };
 
-// Slab x of `regs` into columns ta .. ta + 31.  `ready` waits for the stage behind the arithmetic, in front of the store.
-template <class T, class Ready>
+// Slab x of `regs` into columns ta .. ta + 31.  `ready` waits for the stage behind the arithmetic, in front of the store.  (The split
+// form goes unit by unit: in slabs the down products of 36 rows took the same time, and gate+up, whose three stages hold a
+// block and a half, 168 us instead of 148.)
+template <class T, int FORM, class Ready>
 __device__ __forceinline__ bool expand_slab(const typename Slab<T>::Regs& regs, int x, int i, uint32_t ta, Ready ready) {
-  uint32_t cw[16], v[32];
+  uint32_t cw[16];
   float s[4], o[4];
   Slab<T>::codes(regs, x, i + x, cw, s, o);
+  uint32_t v[32];
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
     const uint32_t s2 = bf2_dup(s[g]), o2 = bf2_dup(o[g]);
+    const float a = 128.0f * s[g], c = o[g] - a;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const uint4 q = short8(cw[4 * g + 2 * h], cw[4 * g + 2 * h + 1], s2, o2);
+      uint4 q;
+      if constexpr (FORM == Q_SHORT) {
+        q = short8(cw[4 * g + 2 * h], cw[4 * g + 2 * h + 1], s2, o2);
+      } else {
+        float f[8];
+        fast8(cw[4 * g + 2 * h], cw[4 * g + 2 * h + 1], a, c, f);
+        q = q_pack8(f);
+      }
       v[8 * g + 4 * h] = q.x; v[8 * g + 4 * h + 1] = q.y; v[8 * g + 4 * h + 2] = q.z; v[8 * g + 4 * h + 3] = q.w;
     }
   }
@@ -443,10 +454,18 @@ __host__ __device__ constexpr int q_stages(bool dual, int bn) {
   const int n = (512 - q_accs(dual, bn) * (dual ? 2 : 1) * bn) / ((dual ? 2 : 1) * (QBK / 2));
   return n > 6 ? 6 : n;
 }
-__host__ __device__ constexpr int q_raw_slots(int sb_bytes, bool dual, int bn) {
+// Whole stages by groups of four warps
+__host__ __device__ constexpr bool q_slabs(int sb_bytes, int form) { return sb_bytes > 0 && form != Q_SPLIT; }
+// One matrix in slabs: a warp waits for every second raw slot only.  With an odd ring it skips every other phase of a slot, and a
+// wait by parity would pass where the copy of super-block s - slots has not landed yet.  It has where s - slots is among those
+// that are known to have been read: the warp's own stage of s - 2 waited for the MMAs of one turn of the ring before, so all
+// super-blocks up to s - 2 - ceil(stages / 2) have been.
+__host__ __device__ constexpr int q_raw_slots(int sb_bytes, bool dual, int bn, int form) {
   if (sb_bytes == 0) return 0;
-  const int n = (220 * 1024 - q_stages(dual, bn) * 2 * bn * 128) / ((dual ? 2 : 1) * QBM * sb_bytes);
-  return n > 6 ? 6 : n;
+  int n = (220 * 1024 - q_stages(dual, bn) * 2 * bn * 128) / ((dual ? 2 : 1) * QBM * sb_bytes);
+  if (n > 6) n = 6;
+  if (!dual && q_slabs(sb_bytes, form) && n % 2 == 1 && n < 2 + (q_stages(dual, bn) + 1) / 2) --n;
+  return n;
 }
 
 // 768 threads: warp 0 = TMA of the token tiles, warp 1 = MMA issuer and TMEM owner, warps 2..5 = epilogue, warp 6 = TMA
@@ -458,7 +477,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   constexpr int SB = SbBytes<T>::v;
   constexpr int STAGES = q_stages(DUAL, BN);
-  constexpr int RS = q_raw_slots(SB, DUAL, BN);                      // raw ring slots (0: register loads)
+  constexpr int RS = q_raw_slots(SB, DUAL, BN, FORM);                // raw ring slots (0: register loads)
   constexpr int RAW_MAT = QBM * SB;                                  // one matrix's 128 super-blocks
   constexpr int RAW_SLOT = (DUAL ? 2 : 1) * RAW_MAT;
   constexpr int B_ATOM = BN * 128;
@@ -468,7 +487,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
   constexpr int A_MAT = QBK / 2;                                     // columns of one matrix's stage
   constexpr int A_COLS = (DUAL ? 2 : 1) * A_MAT;
   constexpr int HALVES = FORM == Q_SPLIT ? 2 : 1;                    // stages that hold one 128-deep block of weights
-  constexpr bool SLABS = RS > 0 && FORM == Q_SHORT;                  // a group of four warps fills a matrix's stage alone
+  constexpr bool SLABS = q_slabs(SB, FORM);                          // a group of four warps fills a matrix's stage alone
   constexpr int FILLERS = (DUAL ? 2 : 1) * (SLABS ? 4 : 8);          // warps that write one stage
   constexpr int READERS = SLABS && !DUAL ? 8 : 16;                   // warps that read a raw slot
   __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
@@ -572,10 +591,25 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
       const int ab = it % NACC;
       const uint32_t acc_phase = (it / NACC) & 1;
       ++it;
+      const int n_rows = min(BN, mt.row_end - mt.row0);            // token rows of this tile
+      // lane l fetches the routing of token rows l, l + 32, ... while the products run; the store loop broadcasts it
+      int out_row[BN / 32];
+      float out_scale[BN / 32];
+      if (DUAL || a.splits == 1) {
+#pragma unroll
+        for (int b = 0; b < BN / 32; ++b) {
+          const int r_l = mt.row0 + 32 * b + lane;
+          out_row[b] = -1;
+          out_scale[b] = 1.0f;
+          if (32 * b + lane < n_rows) {
+            out_row[b] = a.dst_row ? a.dst_row[r_l] : r_l;
+            if (a.row_scale) out_scale[b] = a.row_scale[r_l];
+          }
+        }
+      }
       if (!__all_sync(0xFFFFFFFFu, mbar_wait(&acc_full[ab], acc_phase, abort_flag))) break;
       tc_fence_after();
       const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + ab * ACC_COLS;
-      const int n_rows = min(BN, mt.row_end - mt.row0);            // token rows of this tile
       if (!DUAL && a.splits > 1) {
         // a share's sums: [tile][split][token][128 weight rows]; the CTA that arrives last adds them up, see the end
         float* const own = a.partial + (long)t * (BN * QBM) + q * 32 + lane;
@@ -589,31 +623,29 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
         }
         __threadfence();
       } else {
-#pragma unroll 1
-        for (int c = 0; c < n_rows; c += 16) {
-          uint32_t v[16], u[DUAL ? 16 : 1];
-          tmem_ld16(tbase + c, v);
-          if constexpr (DUAL) tmem_ld16(tbase + BN + c, u);
-          tmem_ld_wait();
-          // lane i fetches the routing of token row i of this chunk; the store loop broadcasts it
-          const int r_l = mt.row0 + c + (lane & 15);
-          int orow_l = -1;
-          float sc_l = 1.0f;
-          if (r_l < mt.row_end) {
-            orow_l = a.dst_row ? a.dst_row[r_l] : r_l;
-            if (a.row_scale) sc_l = a.row_scale[r_l];
-          }
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const int orow = __shfl_sync(0xFFFFFFFFu, orow_l, i);
-            const float sc = __shfl_sync(0xFFFFFFFFu, sc_l, i);
-            if (orow < 0 || !n_ok) continue;
-            float f = __uint_as_float(v[i]);
-            if constexpr (DUAL) f = (f / (1.0f + __expf(-f))) * __uint_as_float(u[i]);
-            f *= sc;
-            if (a.resid) f += a.resid[(long)orow * a.ldr + n];
-            if (a.c_f32) a.c_f32[(long)orow * a.ldc + n] = f;
-            else a.c_bf16[(long)orow * a.ldc + n] = __float2bfloat16_rn(f);
+        for (int b = 0; b < BN / 32; ++b) {
+          if (32 * b >= n_rows) break;
+#pragma unroll 1
+          for (int h = 0; h < 32 && 32 * b + h < n_rows; h += 16) {
+            uint32_t v[16], u[DUAL ? 16 : 1];
+            tmem_ld16(tbase + 32 * b + h, v);
+            if constexpr (DUAL) tmem_ld16(tbase + BN + 32 * b + h, u);
+            tmem_ld_wait();
+            const int left = n_rows - 32 * b - h;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              if (!DUAL && i >= left) break;             // (gate+up of 24 rows 62 us without, 66 with)
+              const int orow = __shfl_sync(0xFFFFFFFFu, out_row[b], h + i);
+              const float sc = __shfl_sync(0xFFFFFFFFu, out_scale[b], h + i);
+              if (orow < 0 || !n_ok) continue;
+              float f = __uint_as_float(v[i]);
+              if constexpr (DUAL) f = (f / (1.0f + __expf(-f))) * __uint_as_float(u[i]);
+              f *= sc;
+              if (a.resid) f += a.resid[(long)orow * a.ldr + n];
+              if (a.c_f32) a.c_f32[(long)orow * a.ldc + n] = f;
+              else a.c_bf16[(long)orow * a.ldc + n] = __float2bfloat16_rn(f);
+            }
           }
         }
       }
@@ -682,10 +714,6 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
       // than the one kept back here, and stages are used in order.
       constexpr int NG = DUAL ? 2 : 4;                               // groups that share a matrix's stages, two a super-block
       static_assert(NG <= STAGES, "a group's next stage lies at most one turn of the ring ahead");
-      // One matrix: a warp waits for every second raw slot only.  With an odd ring it skips every other phase of a slot, and a wait
-      // by parity would pass two phases early.  It cannot: the warp's own stage of super-block s - 2 waited for the MMAs of stage
-      // 2 (s - 2) - STAGES, so all super-blocks up to s - 2 - STAGES / 2 have been read, and s - RS is one of them.
-      static_assert(DUAL || RS % 2 == 0 || RS <= 2 + STAGES / 2, "no raw slot is two phases behind");
       const int mine = DUAL ? half : grp;
       int rslot = 0, stage = mine, turn = 0, pending = -1;           // stage: this group's next one
       uint32_t rphase = 0, phase = 0;
@@ -715,8 +743,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
               return ok;
             };
             const uint32_t ta = ta0 + stage * A_COLS;
-            if (!expand_slab<T>(r, 0, 2 * (mine & 1), ta, ready)) break;
-            expand_slab<T>(r, 1, 2 * (mine & 1), ta + 32, [] { return true; });
+            if (!expand_slab<T, FORM>(r, 0, 2 * (mine & 1), ta, ready)) break;
+            expand_slab<T, FORM>(r, 1, 2 * (mine & 1), ta + 32, [] { return true; });
             pending = stage;
             stage += NG;
             if (stage >= STAGES) { stage -= STAGES; phase ^= 1; }
@@ -821,7 +849,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ 
 template <class T, bool DUAL, int BN, int FORM>
 static int qgemm_go(const CUtensorMap& mx, const QGemmArgs& a, int n_groups, int grid, cudaStream_t st) {
   constexpr int SB = SbBytes<T>::v;
-  constexpr int RS = q_raw_slots(SB, DUAL, BN);
+  constexpr int RS = q_raw_slots(SB, DUAL, BN, FORM);
   constexpr size_t smem = (size_t)q_stages(DUAL, BN) * 2 * BN * 128 + (size_t)RS * (DUAL ? 2 : 1) * QBM * SB + 1024;
   static_assert(q_stages(DUAL, BN) >= 2 && (SB == 0 || RS >= 2), "operand rings");
   CUtensorMap mw = mx, mw2 = mx;

@@ -70,8 +70,16 @@ class GemmPrefill:
         # 6.0 / 5.8 with the expansion; FP8 3.3 / 4.3 and 9.9 / 10.1; NVFP4 3.6 / 4.6 and 6.2 / 6.5.  Copies that are kept
         # are the faster ones from about 64 tokens on (3.2 to 3.6 / 3.5 in all three), so there the blocks are left to the
         # prompts below it, which need their bits (run).
+        # (0: no micro-batch multiplies blocks.)
         self.direct_rows = 128
+        # Experts alone take their blocks further, copies or not, up to this many rows an expert on average: the products are then
+        # bound by what they read, and the blocks are a quarter of the copies, or half.  Types whose expander keeps up with
+        # that; NVFP4 (231 against 221 at 256 ids) and Q8_0 (242) do not.  Gate+up and down of the 30 B shape, us a layer, copies
+        # / Q4_K / Q6_K / FP8: 160 ids 219 / 163 / 182 / 181, 384 ids 224 / 180 / 204 / 209, 512 ids 227 / 192 / 216 / 220, 700
+        # ids 231 / 203 / 230 / 233, 1,000 ids 238 / 262 / 294 / 299.
+        self.block_rows = {"Q4_K": 44, "Q5_K": 32, "Q6_K": 32, "FP8_B128": 32}
         self._direct_ok = None
+        self._block_limit = None
         self._work = None
         self._flash_work = G.FlashWork(engine.device)
 
@@ -123,6 +131,7 @@ class GemmPrefill:
         # Quantised weights are expanded to bf16 one layer AHEAD of their use, on a side stream: the expansion is bound
         # by HBM traffic, the products by the tensor cores, so the two overlap.  Two sets of bf16 buffers alternate.
         direct = fine or self._direct(T)
+        blocks = direct or self._expert_blocks(T)           # the routed experts' weights are multiplied as they are
         resident = not direct and self._use_resident()
         ahead = self.expert_source is None and self.expand_ahead and not resident and not direct
         nset = 2 if ahead else 1
@@ -155,9 +164,9 @@ class GemmPrefill:
             E, I_, k = s.n_expert, s.moe_inter, s.n_used
             nslot = T * k
             cap = nslot + 128
-            wg_s = [None if direct else self._get(f"wg{i}", (E, I_, H), bf) for i in range(nset)]
-            wu_s = [None if direct else self._get(f"wu{i}", (E, I_, H), bf) for i in range(nset)]
-            wd_s = [None if direct else self._get(f"wd{i}", (E, H, I_), bf) for i in range(nset)]
+            wg_s = [None if blocks else self._get(f"wg{i}", (E, I_, H), bf) for i in range(nset)]
+            wu_s = [None if blocks else self._get(f"wu{i}", (E, I_, H), bf) for i in range(nset)]
+            wd_s = [None if blocks else self._get(f"wd{i}", (E, H, I_), bf) for i in range(nset)]
             logits = self._get("rl", (T, E), f32)
             xn3 = self._get("xn3", (T, 3 * H), bf)
             ids = self._get("ids", (T, k), i32)
@@ -170,7 +179,7 @@ class GemmPrefill:
             Ap = self._get("Ap", (cap, H), bf)
             act = self._get("act", (cap, I_), bf)
             slot_out = self._get("slot_out", (nslot, H), f32)
-            moe_tiles = G.TileTable(nslot, E, dev, 32) if direct else G.TileTable(nslot, E, dev)
+            moe_tiles = G.TileTable(nslot, E, dev, 32 if direct or nslot <= 8 * E else 64) if blocks else G.TileTable(nslot, E, dev)
         if s.dense_inter and (s.first_dense > 0 or not s.is_moe):
             Id = s.dense_inter
             dg_s = [self._get(f"dg{i}", (Id, H), bf) for i in range(nset)]
@@ -180,7 +189,8 @@ class GemmPrefill:
         st = self.status
 
         def expand(il: int, which: str) -> None:
-            """bf16 copies of layer il's weights into buffer set il % nset: 'attn', 'gate_up', 'down' or 'all'."""
+            """bf16 copies of layer il's weights into buffer set il % nset: 'attn', 'gate_up', 'down', 'experts' (both) or 'all'.
+            Routed experts whose blocks are multiplied as they are have none."""
             b = f"blk.{il}."
             i = il % nset
             if which in ("attn", "all"):
@@ -189,14 +199,16 @@ class GemmPrefill:
                 G.dequant_bf16(w.q[b + "attn_v.weight"], wqkv_s[i][s.q_rows + s.kv_rows:])
                 G.dequant_bf16(w.q[b + "attn_output.weight"], wo_s[i])
             if s.layer_is_moe(il):
+                if blocks:
+                    return
                 if self.expert_source is not None:
                     qg, qu, qd = self.expert_source(il)
                 else:
                     qg, qu, qd = (w.q[b + f"ffn_{n}_exps.weight"] for n in ("gate", "up", "down"))
-                if which in ("gate_up", "all"):
+                if which in ("gate_up", "experts", "all"):
                     G.dequant_bf16(qg, wg_s[i])
                     G.dequant_bf16(qu, wu_s[i])
-                if which in ("down", "all"):
+                if which in ("down", "experts", "all"):
                     G.dequant_bf16(qd, wd_s[i])
             else:
                 if which in ("gate_up", "all"):
@@ -227,19 +239,20 @@ class GemmPrefill:
             if s.dense_inter and (s.first_dense > 0 or not s.is_moe):
                 dg, du, dd = dg_s[i], du_s[i], dd_s[i]
             if resident:
-                hit = self._resident.get(il)
-                if hit is None:
-                    # first use of this layer: expand into the shared scratch as always, then keep a copy
-                    expand(il, "all")
-                    hit = {"wqkv": wqkv.clone(), "wo": wo.clone()}
-                    if s.layer_is_moe(il):
-                        hit.update(wg=wg.clone(), wu=wu.clone(), wd=wd.clone())
-                    else:
+                hit = self._resident.setdefault(il, {})
+                moe = s.layer_is_moe(il)
+                if "wqkv" not in hit or (moe and not blocks and "wg" not in hit):
+                    # first use of this layer (of its experts): expand into the shared scratch as always, then keep a copy
+                    expand(il, "all" if "wqkv" not in hit else "experts")
+                    if "wqkv" not in hit:
+                        hit.update(wqkv=wqkv.clone(), wo=wo.clone())
+                    if not moe:
                         hit.update(dg=dg.clone(), du=du.clone(), dd=dd.clone())
-                    self._resident[il] = hit
+                    elif not blocks:
+                        hit.update(wg=wg.clone(), wu=wu.clone(), wd=wd.clone())
                 wqkv, wo = hit["wqkv"], hit["wo"]
-                if s.layer_is_moe(il):
-                    wg, wu, wd = hit["wg"], hit["wu"], hit["wd"]
+                if moe:
+                    wg, wu, wd = hit.get("wg"), hit.get("wu"), hit.get("wd")
                 else:
                     dg, du, dd = hit["dg"], hit["du"], hit["dd"]
             if ahead:
@@ -325,7 +338,7 @@ class GemmPrefill:
                 self.timing.mark(il, "count_scatter")
                 G.gather_rows_bf16(rows_in, dst_row, moe_tiles.offsets[E:E + 1], cap, k, Ap)
                 self.timing.mark(il, "dispatch")
-                if direct:
+                if blocks:
                     qg, qu, qd = (w.q[b + f"ffn_{n}_exps.weight"] for n in ("gate", "up", "down"))
                     G.qgemm(Ap, qg, moe_tiles, out_bf16=act, W2=qu, status=st, **form)
                     self.timing.mark(il, "gemm_gate_up")
@@ -372,12 +385,28 @@ class GemmPrefill:
             return False
         if self._direct_ok is None:
             s, w = self.e.spec, self.e.w
-            names = ("attn_q", "attn_k", "attn_v", "attn_output", "ffn_gate_exps", "ffn_up_exps", "ffn_down_exps")
-            self._direct_ok = all(
-                s.layer_is_moe(il) and all(G.qgemm_supports(w.q[f"blk.{il}.{n}.weight"]) for n in names)
-                and w.q[f"blk.{il}.ffn_gate_exps.weight"].qtype == w.q[f"blk.{il}.ffn_up_exps.weight"].qtype
+            self._direct_ok = all(s.layer_is_moe(il) for il in range(s.n_layer)) and self._blocks_ok() and all(
+                G.qgemm_supports(w.q[f"blk.{il}.{n}.weight"]) for n in ("attn_q", "attn_k", "attn_v", "attn_output")
                 for il in range(s.n_layer))
         return self._direct_ok and (short or not self._use_resident())
+
+    def _blocks_ok(self) -> bool:
+        """Whether every routed layer's stacks have a kernel that multiplies their blocks."""
+        s, w = self.e.spec, self.e.w
+        return all(all(G.qgemm_supports(w.q[f"blk.{il}.{n}.weight"]) for n in ("ffn_gate_exps", "ffn_up_exps", "ffn_down_exps"))
+                   and w.q[f"blk.{il}.ffn_gate_exps.weight"].qtype == w.q[f"blk.{il}.ffn_up_exps.weight"].qtype
+                   for il in range(s.n_layer) if s.layer_is_moe(il))
+
+    def _expert_blocks(self, T: int) -> bool:
+        """Whether a micro-batch of T tokens multiplies the routed experts' blocks as they are (block_rows)."""
+        s = self.e.spec
+        if not s.is_moe or self.expert_source is not None or not self.direct_rows:
+            return False
+        if self._block_limit is None:
+            kinds = {self.e.w.q[f"blk.{il}.ffn_{n}_exps.weight"].qtype for il in range(s.n_layer) if s.layer_is_moe(il)
+                     for n in ("gate", "up")}               # gate+up are two thirds of the products
+            self._block_limit = min((self.block_rows.get(t, 0) for t in kinds), default=0) if self._blocks_ok() else 0
+        return T * s.n_used <= self._block_limit * s.n_expert
 
     def _use_resident(self) -> bool:
         """Whether the layers' bf16 copies stay in HBM between prompts (decided once, before the first copy exists)."""

@@ -208,6 +208,31 @@ def test_short_prompts_over_quantised_blocks_agree_with_the_bf16_copies(n, start
     assert float((out[0] - out[1]).norm() / out[1].norm()) < 2e-2
 
 
+@pytest.mark.parametrize("kept", [False, True])
+@pytest.mark.parametrize("n", [129, 176, 177, 260])
+def test_experts_over_blocks_beside_bf16_projections_agree_with_the_copies(n, kept):
+    """Prompts on either side of the last one whose experts take their blocks (16 experts, 4 of them a row, 44 rows each: 176),
+    with copies that are kept and without, and a longer prompt behind a shorter one, which completes the copies."""
+    from bloomery_b200.models.spec import tiny_qwen3moe
+    from bloomery_b200.models.weights import Weights, synth_tensors
+    from bloomery_b200.runtime.engine import DecodeEngine
+    spec = tiny_qwen3moe()
+    w = Weights.from_items(spec, synth_tensors(spec, "cpu", seed=0), "cpu").to(DEV)
+    g = torch.Generator().manual_seed(n)
+    ids = torch.randint(0, spec.vocab, (n,), generator=g).tolist()
+    out = []
+    for rows in (128, 0):
+        eng = DecodeEngine(w, n_slots=2, slot_ctx=512)
+        pre = eng._gemm_prefill = eng._new_gemm_prefill()
+        pre.direct_rows, pre.resident_bf16 = rows, kept
+        assert pre._expert_blocks(n) == (rows > 0 and n <= 176)
+        eng.prefill(1, ids[:140], gemm=True)
+        eng.prefill(0, ids, gemm=True)
+        out.append(eng.logits[0].double().cpu())
+    # the same bf16 operands, their fp32 sums in another order, four layers deep (as above)
+    assert float((out[0] - out[1]).norm() / out[1].norm()) < 2e-2
+
+
 @pytest.mark.parametrize("n", [32, 33, 63])
 @pytest.mark.parametrize("mix", ["Q4_K_M", "NVFP4"])
 def test_prompts_below_the_gemm_threshold_round_activations_and_nothing_else(n, mix):

@@ -670,6 +670,24 @@ def test_kept_bf16_copies_serve_all_but_the_prompts_below_the_gemm_threshold():
     assert not pre._direct(40, short=True)                       # experts streamed from the host: no stack to multiply
 
 
+def test_experts_take_their_blocks_up_to_some_rows_an_expert():
+    """Gate and up decide; a type without a limit, streamed experts and ``direct_rows`` 0 leave the experts to the copies."""
+    from types import SimpleNamespace as NS
+    from bloomery_b200.runtime.prefill import GemmPrefill
+
+    def limit(t, **kw):
+        pre = object.__new__(GemmPrefill)
+        q = {f"blk.0.ffn_{n}_exps.weight": NS(qtype=t) for n in ("gate", "up")}
+        spec = NS(is_moe=True, n_layer=1, n_used=8, n_expert=128, layer_is_moe=lambda il: True)
+        vars(pre).update({**dict(e=NS(spec=spec, w=NS(q=q)), direct_rows=128, expert_source=None, _block_limit=None,
+                                 block_rows={"Q4_K": 44, "FP8_B128": 32}, _blocks_ok=lambda: True), **kw})
+        return [pre._expert_blocks(n) for n in (1, 512, 513, 704, 705)]
+    assert limit("Q4_K") == [True] * 4 + [False] and limit("FP8_B128") == [True] * 2 + [False] * 3
+    for kw in (dict(expert_source=object()), dict(direct_rows=0), dict(_blocks_ok=lambda: False)):
+        assert not any(limit("Q4_K", **kw))
+    assert not any(limit("NVFP4"))
+
+
 def test_a_prompt_path_keeps_the_engine_it_was_given_and_an_engine_not_itself(monkeypatch):
     import weakref
     from bloomery_b200.runtime.engine import DecodeEngine
