@@ -52,6 +52,20 @@ __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+// Four sums over the warp at once: lane l gets that of v[l >> 3], the bits of warp_sum (every sum runs through the same tree).  Six
+// shuffles instead of twenty: the first two steps hand half of what a lane holds to its partner.
+__device__ __forceinline__ float warp_sum4(float v0, float v1, float v2, float v3) {
+  const int lane = threadIdx.x & 31;
+  const bool up = lane & 16, odd = lane & 8;
+  float a = up ? v2 : v0, b = up ? v3 : v1;
+  a += __shfl_xor_sync(0xffffffffu, up ? v0 : v2, 16);
+  b += __shfl_xor_sync(0xffffffffu, up ? v1 : v3, 16);
+  float c = odd ? b : a;
+  c += __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+  return c;
+}
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));

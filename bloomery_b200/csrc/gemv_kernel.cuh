@@ -47,23 +47,38 @@ __device__ __forceinline__ void rows_q(const GemvArgs& a, const GemvSeg& s, int 
         }
       }
     }
+    if constexpr (MB == 1 && R > 1) {
+      // lane 8 r stores row r
+      const float sum = warp_sum4(acc[0][0], acc[1][0], R > 2 ? acc[R - 1][0] : 0.f, 0.f);
+      const int r = lane >> 3;
+      if ((lane & 7) == 0 && r < R && r0 + r < r_hi) {
+        const int col = out_col0 + r0 + r;
+        float v = sum * s_scale[0];
+        if (a.push.n_ranks > 0) push_store(a.push, push_epoch, col, v);
+        else {
+          if (a.resid) v += a.resid[col];
+          a.out[col] = v;
+        }
+      }
+    } else {
 #pragma unroll
-    for (int r = 0; r < R; ++r)
+      for (int r = 0; r < R; ++r)
 #pragma unroll
-      for (int m = 0; m < MB; ++m) acc[r][m] = warp_sum(acc[r][m]);
-    if (lane == 0) {
+        for (int m = 0; m < MB; ++m) acc[r][m] = warp_sum(acc[r][m]);
+      if (lane == 0) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        if (r0 + r < r_hi) {
-          const int col = out_col0 + r0 + r;
+        for (int r = 0; r < R; ++r) {
+          if (r0 + r < r_hi) {
+            const int col = out_col0 + r0 + r;
 #pragma unroll
-          for (int m = 0; m < MB; ++m)
-            if (m < a.M) {
-              float v = acc[r][m] * s_scale[m];
-              if (a.push.n_ranks > 0) { push_store(a.push, push_epoch, (long)m * a.out_stride + col, v); continue; }
-              if (a.resid) v += a.resid[(long)m * a.resid_stride + col];
-              a.out[(long)m * a.out_stride + col] = v;
-            }
+            for (int m = 0; m < MB; ++m)
+              if (m < a.M) {
+                float v = acc[r][m] * s_scale[m];
+                if (a.push.n_ranks > 0) { push_store(a.push, push_epoch, (long)m * a.out_stride + col, v); continue; }
+                if (a.resid) v += a.resid[(long)m * a.resid_stride + col];
+                a.out[(long)m * a.out_stride + col] = v;
+              }
+          }
         }
       }
     }
@@ -73,7 +88,7 @@ __device__ __forceinline__ void rows_q(const GemvArgs& a, const GemvSeg& s, int 
 
 // The same for passes of several rows whose weight rows are at most 32 C units long: the weights of R rows stay in registers
 // and the pass's rows walk past them one by one, so nothing is kept per (weight row, row of the pass) and the loop runs
-// over live rows only.  Sums are those of rows_q.  Lane m keeps the results of row m and stores them at the end.
+// over live rows only.  Sums are those of rows_q.  Lane 8 r + m keeps the result of weight row r and row m and stores it at the end.
 // (Accumulators of 2 x 8 instead spilled 1 KB a thread; five rows in a bucket of eight computed eight.)
 template <class T, int R, int C, class Between>
 __device__ __forceinline__ void rows_multi(const GemvArgs& a, const GemvSeg& s, int r_lo, int r_hi, int out_col0, unsigned live,
@@ -81,7 +96,8 @@ __device__ __forceinline__ void rows_multi(const GemvArgs& a, const GemvSeg& s, 
   using U = Unit<T>;
   const int K = a.K, lane = threadIdx.x & 31;
   const int nunits = K / 64;
-  const bool mine = lane < kMaxRows && (live >> lane & 1);
+  const int my_m = lane & 7, my_r = lane >> 3;
+  static_assert(R <= 4 && kMaxRows == 8, "a result a lane");
   const unsigned push_epoch = a.push.n_ranks > 0 ? site_epoch(a.push.step, a.push.sites_per_step, a.push.site_index) : 0u;
   for (int r0 = r_lo; r0 < r_hi || r0 == r_lo; r0 += R) {
     typename U::Regs regs[R][C];
@@ -91,12 +107,10 @@ __device__ __forceinline__ void rows_multi(const GemvArgs& a, const GemvSeg& s, 
       for (int c = 0; c < C; ++c)
         if (c * 32 + lane < nunits && r0 + r < r_hi) U::loadu(s.w + (long)(r0 + r) * s.row_bytes, c * 32 + lane, K, regs[r][c]);
     between();
-    float res[R], old[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      res[r] = old[r] = 0.f;
-      if (a.resid && a.push.n_ranks == 0 && mine && r0 + r < r_hi) old[r] = a.resid[(long)lane * a.resid_stride + out_col0 + r0 + r];
-    }
+    const bool mine = my_r < R && r0 + my_r < r_hi && (live >> my_m & 1);
+    const int col = out_col0 + r0 + my_r;
+    float res = 0.f, old = 0.f;
+    if (a.resid && a.push.n_ranks == 0 && mine) old = a.resid[(long)my_m * a.resid_stride + col];
 #pragma unroll 1
     for (unsigned left = live; left; left &= left - 1) {
       const int m = __ffs(left) - 1;
@@ -114,22 +128,19 @@ __device__ __forceinline__ void rows_multi(const GemvArgs& a, const GemvSeg& s, 
             if (r0 + r < r_hi) acc[r] += ActOf<T>::dot(regs[r][c], u, act);
         }
       }
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const float v = warp_sum(acc[r]);
-        if (lane == m) res[r] = v;
-      }
+      float sum;
+      if constexpr (R == 1) sum = warp_sum(acc[0]);
+      else sum = warp_sum4(acc[0], acc[1], R > 2 ? acc[R - 1] : 0.f, 0.f);
+      if (my_m == m) res = sum;
     }
     if (mine) {
-#pragma unroll
-      for (int r = 0; r < R; ++r)
-        if (r0 + r < r_hi) {
-          const long at = (long)lane * a.out_stride + out_col0 + r0 + r;
-          float v = res[r] * s_scale[lane];
-          if (a.push.n_ranks > 0) { push_store(a.push, push_epoch, at, v); continue; }
-          if (a.resid) v += old[r];
-          a.out[at] = v;
-        }
+      float v = res * s_scale[my_m];
+      if (a.push.n_ranks > 0) {
+        push_store(a.push, push_epoch, (long)my_m * a.out_stride + col, v);
+      } else {
+        if (a.resid) v += old;
+        a.out[(long)my_m * a.out_stride + col] = v;
+      }
     }
     if (r0 + R >= r_hi) break;
   }

@@ -301,40 +301,44 @@ struct GateUpArgs {
   const int* row_seq;
 };
 
-// two activation outputs (2 gate rows + 2 up rows) of one warp, the activations in shared memory (in the chunk layout of T)
-template <class T>
+// R activation outputs (R gate rows + R up rows) of one warp, the activations in shared memory (in the chunk layout of T): lane
+// 8 r gets the gate's and the up product's sum of row r.
+template <class T, int R>
 __device__ __forceinline__ void gate_up_rows(const uint8_t* g0, const uint8_t* u0, long rb, int K, int lane,
-                                             const int8_t* sq, const float2* sds, float (&gacc)[2], float (&uacc)[2]) {
+                                             const int8_t* sq, const float2* sds, float& g, float& u_sum) {
   using U = Unit<T>;
   const int nunits = K / 64;
+  float gacc[R], uacc[R];
 #pragma unroll
-  for (int r = 0; r < 2; ++r) { gacc[r] = 0.f; uacc[r] = 0.f; }
+  for (int r = 0; r < R; ++r) gacc[r] = uacc[r] = 0.f;
   for (int u = lane; u < nunits; u += 32) {
-    typename U::Regs rg[2], ru[2];
+    typename U::Regs rg[R], ru[R];
 #pragma unroll
-    for (int r = 0; r < 2; ++r) { U::loadu(g0 + r * rb, u, K, rg[r]); U::loadu(u0 + r * rb, u, K, ru[r]); }
+    for (int r = 0; r < R; ++r) { U::loadu(g0 + r * rb, u, K, rg[r]); U::loadu(u0 + r * rb, u, K, ru[r]); }
     ActRegs act;
     StagedAct<T>::load(sq, sds, u, nunits, act);
 #pragma unroll
-    for (int r = 0; r < 2; ++r) { gacc[r] += ActOf<T>::dot(rg[r], u, act); uacc[r] += ActOf<T>::dot(ru[r], u, act); }
+    for (int r = 0; r < R; ++r) { gacc[r] += ActOf<T>::dot(rg[r], u, act); uacc[r] += ActOf<T>::dot(ru[r], u, act); }
   }
-#pragma unroll
-  for (int r = 0; r < 2; ++r) { gacc[r] = warp_sum(gacc[r]); uacc[r] = warp_sum(uacc[r]); }
+  g = warp_sum4(gacc[0], gacc[R - 1], uacc[0], uacc[R - 1]);
+  u_sum = __shfl_down_sync(0xffffffffu, g, 16);
 }
 
-// grid (I/32, n_used, M), 256 threads: warp w computes activation rows 2w, 2w+1, 16+2w and 17+2w of the chunk.
+// grid (I/32, n_used, M), 256 threads: in turns of 8 R rows of the chunk, warp w computes activation rows R w .. R w + R - 1.
 // When route.logits is set the grid is one wider in x: every block routes row m itself (redundantly, from the router
 // launch's logits) so no block waits on a completion counter, and the block behind the chunks publishes ids / weights /
 // heat for the launches that follow, which takes the weights' arithmetic off the path of those that multiply.
 // One row is a chain of latencies (logits, picks, weights, sums), so what can overlap does: the activations come in under the
-// picks, which one warp takes where route_pick serves, and the rows of the second half are asked into L2 while the first half
-// is in flight.  30 B shape, one row, us behind the launch in front: 10.2 before and 9.9 now alone in the layer, of which 2
-// go to the picks, 3 to 5 to the first half (1 of them to HBM), 1.8 to the second; what bounds the halves is the issue of
-// some 100 instructions a weight row and lane, two blocks on a third of the processors.  Five rows 36 -> 34.
+// picks, which one warp takes where route_pick serves, and the rows of later turns are asked into L2 while the first turn's
+// are in flight.  30 B shape, one row, us behind the launch in front: 9.3 (10.3 with activations from L2 and picks by the block), of
+// which 2 go to the picks, 3 to 5 to the first turn (1 of them to HBM), 1.5 to the second; what bounds the turns is the issue of
+// some 90 instructions a weight row and lane, two blocks on a third of the processors.  Several rows are bound by their blocks'
+// latencies in turns of the processors: five 30 us (36 before, 34 with R = 2).
 // FAM 0 = ggml integer-dot types, FAM 2 = block-scaled float planes (one kernel per family keeps
 // the plane decoders out of the K-quant bodies' register budget)
-template <int FAM>
-__global__ void __launch_bounds__(256, 2) gate_up_sel_kernel(const GateUpArgs a) {
+// R = 2, two blocks a processor, for one row; R = 1, three blocks, for several, which queue for the processors
+template <int FAM, int R>
+__global__ void __launch_bounds__(256, R == 2 ? 2 : 3) gate_up_sel_kernel(const GateUpArgs a) {
   extern __shared__ __align__(16) uint8_t s_in[];
   const int K = a.K;
   int8_t* sq = reinterpret_cast<int8_t*>(s_in);
@@ -411,10 +415,11 @@ __global__ void __launch_bounds__(256, 2) gate_up_sel_kernel(const GateUpArgs a)
   }
   const long rb = resident_row_bytes(a.gtype, K), first = (long)e * a.I + chunk * 32;
   if (tid == 0 || tid == 128) {
-    // rows 16 .. 31 of the chunk, which the second half reads
-    const uint8_t* p = (tid == 0 ? a.gate : a.up) + (first + 16) * rb;
-    for (long o = 0; o < 16 * rb; o += 32768) {
-      const unsigned nb = (unsigned)((16 * rb - o) < 32768 ? (16 * rb - o) : 32768);
+    // the rows of the chunk behind the first turn's
+    const uint8_t* p = (tid == 0 ? a.gate : a.up) + (first + 8 * R) * rb;
+    const long bytes = (32 - 8 * R) * rb;
+    for (long o = 0; o < bytes; o += 32768) {
+      const unsigned nb = (unsigned)((bytes - o) < 32768 ? (bytes - o) : 32768);
       asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p + o), "r"(nb) : "memory");
     }
   }
@@ -431,12 +436,12 @@ __global__ void __launch_bounds__(256, 2) gate_up_sel_kernel(const GateUpArgs a)
     __syncthreads();
   }
 #pragma unroll 1
-  for (int half = 0; half < 2; ++half) {
-    const long row0 = first + half * 16 + warp * 2;
+  for (int turn = 0; turn < 4 / R; ++turn) {
+    const long row0 = first + turn * 8 * R + warp * R;
     const uint8_t* g0 = a.gate + row0 * rb;
     const uint8_t* u0 = a.up + row0 * rb;
-    float gacc[2], uacc[2];
-    auto rows = [&](auto t) { gate_up_rows<decltype(t)>(g0, u0, rb, K, lane, sq, sds, gacc, uacc); };
+    float g = 0.f, u = 0.f;
+    auto rows = [&](auto t) { gate_up_rows<decltype(t), R>(g0, u0, rb, K, lane, sq, sds, g, u); };
     if constexpr (FAM == 2) {
       switch (a.gtype) {
         case WT_NVFP4: rows(NvFp4{}); break;
@@ -447,7 +452,7 @@ __global__ void __launch_bounds__(256, 2) gate_up_sel_kernel(const GateUpArgs a)
         case WT_Q4_1: rows(Q41{}); break;
         case WT_Q5_0: rows(Q50{}); break;
         case WT_Q5_1: rows(Q51{}); break;
-        default: gacc[0] = gacc[1] = __int_as_float(0x7fc00000); uacc[0] = uacc[1] = 0.f;
+        default: g = __int_as_float(0x7fc00000);
       }
     } else {
       switch (a.gtype) {
@@ -456,16 +461,10 @@ __global__ void __launch_bounds__(256, 2) gate_up_sel_kernel(const GateUpArgs a)
         case WT_Q6_K: rows(Q6K{}); break;
         case WT_Q8_0: rows(Q80{}); break;
         case WT_Q8_F32: rows(Q8F{}); break;
-        default: gacc[0] = gacc[1] = __int_as_float(0x7fc00000); uacc[0] = uacc[1] = 0.f;
+        default: g = __int_as_float(0x7fc00000);
       }
     }
-    if (lane == 0) {
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        float g = gacc[r];
-        s_act[half * 16 + warp * 2 + r] = (g / (1.0f + expf(-g))) * uacc[r];
-      }
-    }
+    if (lane == 0 || (R == 2 && lane == 8)) s_act[turn * 8 * R + warp * R + (lane >> 3)] = (g / (1.0f + expf(-g))) * u;
   }
   __syncthreads();
   if (warp == 0) {
@@ -775,12 +774,15 @@ int bl_gate_up_sel(const int8_t* xq, const float* xds, const float* route_logits
   BL_REQUIRE(smem <= kMaxInput, BL_ERR_LIMIT);
   static PerDevice limit;
   if (limit.due()) {
-    cudaFuncSetAttribute(gate_up_sel_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxInput);
-    cudaFuncSetAttribute(gate_up_sel_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxInput);
+    cudaFuncSetAttribute(gate_up_sel_kernel<0, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxInput);
+    cudaFuncSetAttribute(gate_up_sel_kernel<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxInput);
+    cudaFuncSetAttribute(gate_up_sel_kernel<0, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxInput);
+    cudaFuncSetAttribute(gate_up_sel_kernel<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxInput);
     limit.mark();
   }
   const dim3 grid(I / 32 + (route_logits ? 1 : 0), n_used, M);
-  return (int)launch(is_plane_family(gtype) ? gate_up_sel_kernel<2> : gate_up_sel_kernel<0>, grid, dim3(256), smem, st, a);
+  if (M == 1) return (int)launch(is_plane_family(gtype) ? gate_up_sel_kernel<2, 2> : gate_up_sel_kernel<0, 2>, grid, dim3(256), smem, st, a);
+  return (int)launch(is_plane_family(gtype) ? gate_up_sel_kernel<2, 1> : gate_up_sel_kernel<0, 1>, grid, dim3(256), smem, st, a);
 }
 
 int bl_down_combine(const int8_t* actq, const float* actds, const int* ids, const float* wts, const int* slot_map,

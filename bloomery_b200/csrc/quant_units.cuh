@@ -94,6 +94,15 @@ BL_HD float sum_float(int bits) {
   return f - 12582912.0f;
 }
 
+// byte b of w (0..255) times f, a power of two; exact
+BL_HD float byte_fma(uint32_t w, int b, float f) {
+#if defined(__CUDA_ARCH__)
+  return __fmaf_rn(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u + b)), f, -8388608.0f * f);
+#else
+  return (float)((w >> (8 * b)) & 0xFF) * f;
+#endif
+}
+
 BL_HD float half_bits_to_float(uint16_t h) {
 #if defined(__CUDA_ARCH__)
   return __half2float(__ushort_as_half(h));
@@ -175,23 +184,32 @@ struct Q4K {
     if (i < 4) { sc = q_lo & 63; mn = q_mid & 63; }
     else { sc = (q_hi & 0xF) | ((q_lo >> 6) << 4); mn = (q_hi >> 4) | ((q_mid >> 6) << 4); }
   }
+  // (scale, min) of the unit's two halves as floats, the second scale times `hi`: packed pairs 2j and 2j + 1 by masks that
+  // depend on the lane alone
+  static BL_HD void scales(uint32_t s0, uint32_t s1, uint32_t s2, int j, float hi, float* sc, float* mn) {
+    const uint32_t top = j < 2 ? 0u : 0x0F0F0F0Fu, low = j < 2 ? 0x3F3F3F3Fu : 0x30303030u;
+    const int sh = j < 2 ? 0 : 2;
+    const uint32_t sw = ((s0 >> sh) & low) | (s2 & top), mw = ((s1 >> sh) & low) | ((s2 >> 4) & top);
+    const int b = 2 * (j & 1);
+    sc[0] = byte_fma(sw, b, 1.0f); sc[1] = byte_fma(sw, b + 1, hi);
+    mn[0] = byte_fma(mw, b, 1.0f); mn[1] = byte_fma(mw, b + 1, 1.0f);
+  }
   static BL_HD float dot(const Regs& r, int u, const ActUnit& a) {
     int j = u & 3;
     const uint32_t w[8] = {r.q0.x, r.q0.y, r.q0.z, r.q0.w, r.q1.x, r.q1.y, r.q1.z, r.q1.w};
-    int lo = kSum0, hi = kSum0;
+    int lo = kSum0, hi = kSum0;                        // the high codes stay where they are: sixteen times their sum, exact
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       lo = dot4_us(w[i] & 0x0F0F0F0Fu, a.q[i], lo);
-      hi = dot4_us((w[i] >> 4) & 0x0F0F0F0Fu, a.q[8 + i], hi);
+      hi = dot4_us(w[i] & 0xF0F0F0F0u, a.q[8 + i], hi);
     }
-    int sc0, mn0, sc1, mn1;
-    scale_min(r, 2 * j, sc0, mn0);
-    scale_min(r, 2 * j + 1, sc1, mn1);
+    float sc[2], mn[2];
+    scales(r.s0, r.s1, r.s2, j, 0.0625f, sc, mn);
     float d = half_bits_to_float((uint16_t)(r.dm & 0xFFFF));
     float dmin = half_bits_to_float((uint16_t)(r.dm >> 16));
     // 63 * 32 * 31 * 127 < 2^24: the products of scales and sums are exact
-    const float pos = fma_rn(a.d0, mul_rn(sum_float(kSum0 + sc0), sum_float(lo)), mul_rn(a.d1, mul_rn(sum_float(kSum0 + sc1), sum_float(hi))));
-    const float neg = fma_rn(a.s0, sum_float(kSum0 + mn0), mul_rn(a.s1, sum_float(kSum0 + mn1)));
+    const float pos = fma_rn(a.d0, mul_rn(sc[0], sum_float(lo)), mul_rn(a.d1, mul_rn(sc[1], sum_float(hi))));
+    const float neg = fma_rn(a.s0, mn[0], mul_rn(a.s1, mn[1]));
     return fma_rn(d, pos, -mul_rn(dmin, neg));
   }
   // decode the unit's 64 values (for the embedding gather and the bf16 expander)
@@ -254,15 +272,13 @@ struct Q5K {
       lo = dot4_us(l5[i], a.q[i], lo);
       hi = dot4_us(h5[i], a.q[8 + i], hi);
     }
-    Q4K::Regs t; t.s0 = r.s0; t.s1 = r.s1; t.s2 = r.s2;
-    int sc0, mn0, sc1, mn1;
-    Q4K::scale_min(t, 2 * j, sc0, mn0);
-    Q4K::scale_min(t, 2 * j + 1, sc1, mn1);
+    float sc[2], mn[2];
+    Q4K::scales(r.s0, r.s1, r.s2, j, 1.0f, sc, mn);
     float d = half_bits_to_float((uint16_t)(r.dm & 0xFFFF));
     float dmin = half_bits_to_float((uint16_t)(r.dm >> 16));
     // 63 * 32 * 31 * 127 < 2^24: the products of scales and sums are exact
-    const float pos = fma_rn(a.d0, mul_rn(sum_float(kSum0 + sc0), sum_float(lo)), mul_rn(a.d1, mul_rn(sum_float(kSum0 + sc1), sum_float(hi))));
-    const float neg = fma_rn(a.s0, sum_float(kSum0 + mn0), mul_rn(a.s1, sum_float(kSum0 + mn1)));
+    const float pos = fma_rn(a.d0, mul_rn(sc[0], sum_float(lo)), mul_rn(a.d1, mul_rn(sc[1], sum_float(hi))));
+    const float neg = fma_rn(a.s0, mn[0], mul_rn(a.s1, mn[1]));
     return fma_rn(d, pos, -mul_rn(dmin, neg));
   }
   static BL_HD void decode(const Regs& r, int u, float* out) {
