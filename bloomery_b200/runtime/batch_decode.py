@@ -51,6 +51,7 @@ class BatchDecode:
         self.params = torch.zeros(3, R, **i32)
         self.params[2].fill_(-1)
         self.params_host = torch.zeros(3, R, dtype=torch.int32, pin_memory=True)
+        self._params_np = self.params_host.numpy()              # same memory: rows are written without tensor indexing
         self.tokens, self.row_pos, self.row_seq = self.params[0], self.params[1], self.params[2]
         self.x = torch.zeros(R, H, **f32)
         self.xn = torch.zeros(R, H, **bf)
@@ -118,6 +119,7 @@ class BatchDecode:
         self.hist_cap = 1024
         self.hist = torch.zeros(self.hist_cap * R, **i32)
         self.status = torch.zeros(1, **i32)
+        self.status_host = torch.zeros(1, dtype=torch.int32, pin_memory=True)
         # dense products take the whole bucket as one token tile where a tile size exists for it
         self.dense_tiles: Dict[int, G.TileTable] = {m: G.TileTable.dense(m, dev, 64 if m == 64 else TILE)
                                                     for m in BUCKETS if m <= R}
@@ -425,8 +427,9 @@ class BatchDecode:
         m = len(rows)
         M = self.bucket(m)
         e = self.e
-        h = self.params_host
-        h[0].zero_(); h[1].zero_(); h[2].fill_(-1)
+        h = self._params_np
+        h[:2] = 0
+        h[2] = -1
         for i, (slot, tok, pos) in enumerate(rows):
             e.kv.ensure(slot, pos + 1)
             e.kv.own(slot, pos)
@@ -434,7 +437,7 @@ class BatchDecode:
             e.slot_len[slot] = max(e.slot_len[slot], pos + 1)
         e.kv.sync_table()
         with torch.cuda.stream(self._stream):
-            self.params.copy_(h, non_blocking=True)
+            self.params.copy_(self.params_host, non_blocking=True)
         return M
 
     def launch(self, M: int, advance: bool = False) -> None:
@@ -458,8 +461,9 @@ class BatchDecode:
         self.launch(M)
         with torch.cuda.stream(self._stream):
             self.tokens_out_host.copy_(self.tokens_out, non_blocking=True)
+            self.status_host.copy_(self.status, non_blocking=True)
         self._stream.synchronize()
-        if int(self.status.item()) != 0:
+        if int(self.status_host) != 0:
             raise RuntimeError("a bounded wait inside the GEMM kernel ran out (status word set)")
         self.e.check_fault()
         return self.tokens_out_host[:len(rows)].tolist()
