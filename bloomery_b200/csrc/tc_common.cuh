@@ -150,6 +150,53 @@ __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.
 // generic-proxy writes to shared memory (st.shared) become visible to the async proxy (tcgen05.mma operands, TMA)
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// ---- storing a tile whose lanes are output columns ------------------------------------------
+struct TokenOut {
+  float* c_f32;               // one of c_f32 / c_bf16
+  __nv_bfloat16* c_bf16;
+  unsigned ldc;
+  const float* row_scale;     // optional per-token factor
+  const float* resid;         // optional addend, indexed like the output
+  unsigned ldr;
+  int N;                      // columns
+};
+// Values of this lane's column n for NT tokens, whose output rows (< 0: none) and factors lanes from .. from + NT - 1 hold.  All rows
+// first and then nothing but predicated stores of one 32 x 32 -> 64-bit product each: with the branches of a token between
+// its shuffle and its store, and 64-bit rows, every token took some 300 clocks of a warp that has its scheduler to itself.
+template <int NT>
+__device__ __forceinline__ void store_tokens(const TokenOut& a, float (&f)[NT], int row_l, float scale_l, int from, int n) {
+  const int none = n < a.N ? 0 : -1;
+  int row[NT];
+#pragma unroll
+  for (int i = 0; i < NT; ++i) row[i] = __shfl_sync(0xFFFFFFFFu, row_l, from + i) | none;
+  if (a.row_scale) {
+#pragma unroll
+    for (int i = 0; i < NT; ++i) f[i] *= __shfl_sync(0xFFFFFFFFu, scale_l, from + i);
+  }
+  if (a.resid) {
+    const char* base = reinterpret_cast<const char*>(a.resid + n);
+    const unsigned pitch = a.ldr * 4u;
+    float add[NT];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) add[i] = row[i] >= 0 ? *reinterpret_cast<const float*>(base + (unsigned long long)(unsigned)row[i] * pitch) : 0.0f;
+#pragma unroll
+    for (int i = 0; i < NT; ++i) f[i] += add[i];
+  }
+  if (a.c_f32) {
+    char* base = reinterpret_cast<char*>(a.c_f32 + n);
+    const unsigned pitch = a.ldc * 4u;
+#pragma unroll
+    for (int i = 0; i < NT; ++i)
+      if (row[i] >= 0) *reinterpret_cast<float*>(base + (unsigned long long)(unsigned)row[i] * pitch) = f[i];
+  } else {
+    char* base = reinterpret_cast<char*>(a.c_bf16 + n);
+    const unsigned pitch = a.ldc * 2u;
+#pragma unroll
+    for (int i = 0; i < NT; ++i)
+      if (row[i] >= 0) *reinterpret_cast<__nv_bfloat16*>(base + (unsigned long long)(unsigned)row[i] * pitch) = __float2bfloat16_rn(f[i]);
+  }
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
