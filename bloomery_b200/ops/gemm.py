@@ -93,6 +93,33 @@ def gemm_bf16(A: torch.Tensor, B: torch.Tensor, tiles: TileTable, *, out_f32: Op
     check(rc, "bl_gemm_bf16")
 
 
+PAIR_ROWS = 256                       # token rows of a tile of gemm_pair
+
+
+def gemm_pair(X: torch.Tensor, W: torch.Tensor, tiles: TileTable, *, out_f32: Optional[torch.Tensor] = None,
+              out_bf16: Optional[torch.Tensor] = None, W2: Optional[torch.Tensor] = None, dst_row=None, row_scale=None,
+              resid=None, status: Optional[torch.Tensor] = None) -> None:
+    """:func:`gemm_bf16` on pairs of CTAs (``csrc/gemm_pair.cu``) over a table of up to 256 rows a tile: for products of many
+    tiles, which the loads of single CTAs bound."""
+    assert X.dtype == torch.bfloat16 and W.dtype == torch.bfloat16 and X.stride(-1) == 1 and W.is_contiguous()
+    assert tiles.tile_rows == PAIR_ROWS and (W2 is None or (W2.shape == W.shape and W2.is_contiguous()))
+    if W.dim() == 2:
+        W = W[None]
+    G, N, Kd = W.shape
+    out = out_f32 if out_f32 is not None else out_bf16
+    rc = cuda().bl_gemm_pair(p(X), L(X.stride(0)), L(X.shape[0]), p(W), p(W2), I(G), I(N), I(Kd), p(tiles.mtiles), p(tiles.n_mtiles),
+                             I(tiles.fixed or tiles.max_mtiles), p(out_f32), p(out_bf16), L(out.stride(0)), p(dst_row),
+                             p(row_scale), p(resid), L(resid.stride(0) if resid is not None else 0), p(status), stream())
+    check(rc, "bl_gemm_pair")
+
+
+def pairs_pay(rows: int, N: int) -> bool:
+    """Whether a dense product of ``rows`` by N columns goes to pairs: where their 256 x 256 tiles give most of them one (us, pairs
+    / single CTAs, or clusters of them where there are few tiles: 1,000 rows 2,048 deep by 5,120 30 / 32, 4,096 71 / 78; 4,096
+    deep by 2,048 1,000 rows 28 / 27, 2,000 31 / 33, 4,096 54 / 60)."""
+    return -(-rows // PAIR_ROWS) * -(-N // 256) >= 3 * sm_count() // 8
+
+
 def _ptr_array(ptrs):
     import ctypes
     return (ctypes.c_void_p * len(ptrs))(*[int(x) for x in ptrs])

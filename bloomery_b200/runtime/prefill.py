@@ -75,9 +75,12 @@ class GemmPrefill:
         # Experts alone take their blocks further, copies or not, up to this many rows an expert on average: the products are then
         # bound by what they read, and the blocks are a quarter of the copies, or half.  Types whose expander keeps up with
         # that; NVFP4 (231 against 221 at 256 ids) and Q8_0 (242) do not.  Gate+up and down of the 30 B shape, us a layer, copies
-        # / Q4_K / Q6_K / FP8: 160 ids 219 / 163 / 182 / 181, 384 ids 224 / 180 / 204 / 209, 512 ids 227 / 192 / 216 / 220, 700
-        # ids 231 / 203 / 230 / 233, 1,000 ids 238 / 262 / 294 / 299.
-        self.block_rows = {"Q4_K": 44, "Q5_K": 32, "Q6_K": 32, "FP8_B128": 32}
+        # / Q4_K / Q6_K / FP8: 160 ids 220 / 159 / 174 / 180, 384 ids 224 / 170 / 195 / 201, 700 ids 230 / 178 / 202 / 208, 1,000
+        # ids 237 / 226 / 258 / 263.
+        self.block_rows = {"Q4_K": 64, "Q5_K": 48, "Q6_K": 52, "FP8_B128": 52}
+        # From this many rows an expert on, products over the copies go to pairs of CTAs with 256-row tiles (gate+up and down, us a
+        # layer, pairs / single CTAs: 1,000 ids 240 / 236, 2,048 ids 270 / 285, 4,096 ids 390 / 410).
+        self.pair_rows = 128
         self._direct_ok = None
         self._block_limit = None
         self._work = None
@@ -153,6 +156,14 @@ class GemmPrefill:
                 self._work = G.QgemmWork(dev, 128)
         else:
             dense_tiles = G.TileTable.dense(T, dev, host=True)
+            pair_tiles = G.TileTable.dense(T, dev, G.PAIR_ROWS, host=True)
+
+        def project(X, W, **out):
+            """A dense product over a bf16 copy."""
+            if G.pairs_pay(T, W.shape[0]):
+                G.gemm_pair(X, W, pair_tiles, status=self.status, **out)
+            else:
+                G.gemm_bf16(X, W, dense_tiles, status=self.status, **out)
         n_keys = p0 + T
         T_pad = (n_keys + 127) // 128 * 128
         if not fine:
@@ -179,7 +190,8 @@ class GemmPrefill:
             Ap = self._get("Ap", (cap, H), bf)
             act = self._get("act", (cap, I_), bf)
             slot_out = self._get("slot_out", (nslot, H), f32)
-            moe_tiles = G.TileTable(nslot, E, dev, 32 if direct or nslot <= 8 * E else 64) if blocks else G.TileTable(nslot, E, dev)
+            pairs = not blocks and nslot >= self.pair_rows * E
+            moe_tiles = G.TileTable(nslot, E, dev, (32 if direct or nslot <= 8 * E else 64) if blocks else G.PAIR_ROWS if pairs else G.BM)
         if s.dense_inter and (s.first_dense > 0 or not s.is_moe):
             Id = s.dense_inter
             dg_s = [self._get(f"dg{i}", (Id, H), bf) for i in range(nset)]
@@ -275,7 +287,7 @@ class GemmPrefill:
             else:
                 if not ahead and not resident:
                     expand(il, "attn")
-                G.gemm_bf16(xn, wqkv, dense_tiles, out_f32=qkv, status=st)
+                project(xn, wqkv, out_f32=qkv)
             self.timing.mark(il, "qkv_gemm")
             if fine:
                 K.qk_norm_rope_append(qkv, w.f.get(b + "attn_q_norm.weight"), w.f.get(b + "attn_k_norm.weight"), e.inv_freq,
@@ -315,7 +327,7 @@ class GemmPrefill:
                 G.qgemm(attn, w.q[b + "attn_output.weight"], dense_tiles, out_f32=x, resid=x, status=st, work=self._work,
                         **form)
             else:
-                G.gemm_bf16(attn, wo, dense_tiles, out_f32=x, resid=x, status=st)
+                project(attn, wo, out_f32=x, resid=x)
             self.timing.mark(il, "o_proj")
             if s.layer_is_moe(il):
                 rw = w.q[b + "ffn_gate_inp.weight"]
@@ -347,12 +359,16 @@ class GemmPrefill:
                     if not ahead and not resident:
                         expand(il, "gate_up")
                     self.timing.mark(il, "expand_gate_up")
-                    G.gemm_bf16(Ap, wg, moe_tiles, out_bf16=act, B2=wu, status=st)
+                    if pairs:
+                        G.gemm_pair(Ap, wg, moe_tiles, out_bf16=act, W2=wu, status=st)
+                    else:
+                        G.gemm_bf16(Ap, wg, moe_tiles, out_bf16=act, B2=wu, status=st)
                     self.timing.mark(il, "gemm_gate_up")
                     if not ahead and not resident:
                         expand(il, "down")
                     self.timing.mark(il, "expand_down")
-                    G.gemm_bf16(act, wd, moe_tiles, out_f32=slot_out, dst_row=dst_row, row_scale=row_scale, status=st)
+                    (G.gemm_pair if pairs else G.gemm_bf16)(act, wd, moe_tiles, out_f32=slot_out, dst_row=dst_row,
+                                                            row_scale=row_scale, status=st)
                 self.timing.mark(il, "gemm_down")
                 if il + 1 < s.n_layer and H <= 8192:
                     G.moe_combine_norm(slot_out, pos_of, T, k, x, x, w.f[f"blk.{il + 1}.attn_norm.weight"], s.rms_eps, xn)

@@ -47,6 +47,65 @@ def test_dense_gemm_bf16_out_resid_and_rerun():
     assert int(st) == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 64, 64), (31, 128, 128), (64, 256, 384), (65, 320, 448), (256, 512, 2048), (257, 2048, 768),
+                                   (700, 5120, 2048), (2100, 96, 4096)])
+def test_pair_gemm_dense(M, N, K):
+    """Products of CTA pairs: one token up to tiles of 256 and their remainders, columns that end inside a CTA's 128, a ring that
+    turns often and one that is not filled, and more tiles than pairs."""
+    from bloomery_b200.ops import gemm as G
+    torch.manual_seed(M)
+    A = (torch.randn(M, K, device=DEV) * 0.5).bfloat16()
+    B = (torch.randn(N, K, device=DEV) * 0.5).bfloat16()
+    R = torch.randn(M, N, device=DEV)
+    tiles, st = G.TileTable.dense(M, DEV, G.PAIR_ROWS, host=True), _status()
+    C, S, Cb = torch.full((M, N), float("nan"), device=DEV), R.clone(), torch.zeros(M, N, dtype=torch.bfloat16, device=DEV)
+    G.gemm_pair(A, B, tiles, out_f32=C, status=st)
+    G.gemm_pair(A, B, tiles, out_f32=S, resid=S, status=st)      # in place, as the output projection uses it
+    G.gemm_pair(A, B, tiles, out_bf16=Cb, status=st)
+    ref = A.double() @ B.double().T
+    bound = K * 2.0 ** -24 * (A.double().abs() @ B.double().abs().T) + 1e-6       # fp32 sums of K exact products, any order
+    assert int(st) == 0
+    assert bool(((C - ref).abs() <= bound).all())
+    assert bool(((S - (ref + R)).abs() <= bound + 2.0 ** -23 * (ref + R).abs()).all())
+    assert torch.equal(Cb, C.bfloat16())
+    again = torch.zeros_like(C)
+    G.gemm_pair(A, B, tiles, out_f32=again, status=st)
+    assert torch.equal(again, C)
+
+
+@pytest.mark.parametrize("T,E,k,H,I_", [(40, 8, 2, 256, 64), (300, 4, 2, 512, 192), (1500, 6, 3, 512, 320)])
+def test_pair_gemm_grouped_gated_and_scattered(T, E, k, H, I_):
+    """Gate and up in one accumulator, groups of a few rows to several tiles, one without rows, dropped slots; against the
+    single-CTA products of the same operands."""
+    from bloomery_b200.ops import gemm as G
+    torch.manual_seed(T)
+    ids = torch.stack([torch.randperm(E - 1)[:k] for _ in range(T)]).to(torch.int32).to(DEV)      # the last group is empty
+    ids[3, 1] = -1
+    wts = torch.rand(T, k, device=DEV)
+    x = (torch.randn(T, H, device=DEV) * 0.5).bfloat16()
+    Wg, Wu = ((torch.randn(E, I_, H, device=DEV) * 0.1).bfloat16() for _ in range(2))
+    Wd = (torch.randn(E, H, I_, device=DEV) * 0.1).bfloat16()
+    n, cap, out, st = T * k, T * k + 128, [], _status()
+    for rows in (G.BM, G.PAIR_ROWS):
+        tiles = G.TileTable(n, E, DEV, rows)
+        pos, dst = torch.zeros(n, dtype=torch.int32, device=DEV), torch.zeros(cap, dtype=torch.int32, device=DEV)
+        scale = torch.zeros(cap, device=DEV)
+        G.moe_plan(ids, wts, E, tiles, pos, dst, scale)
+        Ap = torch.full((cap, H), float("nan"), dtype=torch.bfloat16, device=DEV)
+        G.gather_rows_bf16(x, dst, tiles.offsets[E:E + 1], cap, k, Ap)
+        act, y = torch.full((cap, I_), float("nan"), dtype=torch.bfloat16, device=DEV), torch.zeros(n, H, device=DEV)
+        if rows == G.BM:
+            G.gemm_bf16(Ap, Wg, tiles, out_bf16=act, B2=Wu, status=st)
+            G.gemm_bf16(act, Wd, tiles, out_f32=y, dst_row=dst, row_scale=scale, status=st)
+        else:
+            G.gemm_pair(Ap, Wg, tiles, out_bf16=act, W2=Wu, status=st)
+            G.gemm_pair(act, Wd, tiles, out_f32=y, dst_row=dst, row_scale=scale, status=st)
+        out.append(y)
+    assert int(st) == 0
+    # fp32 sums in another order may round an activation to the neighbouring bf16
+    assert float((out[0] - out[1]).norm() / out[0].norm()) < 1e-3
+
+
 def test_grouped_dual_swiglu_and_scatter():
     """The MoE prompt path: rows grouped by expert, gate/up fused with SwiGLU, down scattered with weights."""
     from bloomery_b200.ops import gemm as G
