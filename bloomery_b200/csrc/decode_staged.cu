@@ -421,7 +421,10 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
   // Nor do the angles of the row and the gains: one row takes them ahead of the wait (several rows take them where they are
   // used; kept in registers over the wait they cost five rows 3 us a layer).
   float row_sn[DPL / 2], row_cs[DPL / 2], q_ahead[DPL], k_ahead[DPL];
+  // So does the page that its new key goes to, a load on which the store would wait.
+  int own_page = -1;
   if constexpr (!DEAL) {
+    if (warp < 2 && pos < t1 * kKeyTile && pos / kPage < a.max_pages) own_page = bt[pos / kPage];
 #pragma unroll
     for (int j = 0; j < DPL / 2; ++j) sincosf((float)pos * a.inv_freq[lane + 32 * j], &row_sn[j], &row_cs[j]);
 #pragma unroll
@@ -442,15 +445,18 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
 #pragma unroll
     for (int j = 0; j < DPL; ++j) x[j] = src[lane + 32 * j];
   };
-  auto norm_rope = [&](float (&x)[DPL], const float* gain, const float (&ahead)[DPL], int at, float (&y)[DPL]) {
+  auto square_sum = [&](const float (&x)[DPL]) {
+    double ss = 0.0;
+#pragma unroll
+    for (int j = 0; j < DPL; ++j) ss += (double)(x[j] * x[j]);
+    return ss;
+  };
+  auto rms_of = [&](double ss) { return (float)(1.0 / sqrt(ss / (double)HEAD + (double)a.eps)); };
+  // rms: the factor of the head's norm (rms_of its square sum over the warp)
+  auto norm_rope = [&](float (&x)[DPL], float rms, const float* gain, const float (&ahead)[DPL], int at, float (&y)[DPL]) {
     if (gain) {
-      double ss = 0.0;
 #pragma unroll
-      for (int j = 0; j < DPL; ++j) ss += (double)(x[j] * x[j]);
-      ss = warp_sum_d(ss);
-      const float scale = (float)(1.0 / sqrt(ss / (double)HEAD + (double)a.eps));
-#pragma unroll
-      for (int j = 0; j < DPL; ++j) x[j] = (scale * (DEAL ? gain[lane + 32 * j] : ahead[j])) * x[j];
+      for (int j = 0; j < DPL; ++j) x[j] = (rms * (DEAL ? gain[lane + 32 * j] : ahead[j])) * x[j];
     }
 #pragma unroll
     for (int j = 0; j < DPL / 2; ++j) {
@@ -464,10 +470,10 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
   };
   // row mm of the pass: its key (or value) of this KV head, to where tiles are patched from and, the block's own row, to the cache
   auto new_head = [&](int mm, bool is_k) { return a.qkv + (long)mm * a.qkv_stride + ((long)a.n_q + (is_k ? 0 : a.n_kv) + kvh) * HEAD; };
-  auto append = [&](int idx, int mm, int pp, bool is_k, float (&x)[DPL]) {
+  auto append = [&](int idx, int mm, int pp, bool is_k, float (&x)[DPL], float rms) {
     float y[DPL];
     if (is_k) {
-      norm_rope(x, a.k_gain, k_ahead, pp, y);
+      norm_rope(x, rms, a.k_gain, k_ahead, pp, y);
     } else {
 #pragma unroll
       for (int j = 0; j < DPL; ++j) y[j] = x[j];
@@ -476,7 +482,7 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
     __half* dst = nullptr;
     if (mm == m) {
       const int pslot = pp / kPage;
-      const int page = (pslot < a.max_pages) ? bt[pslot] : -1;
+      const int page = !DEAL && a.M == 1 ? own_page : pslot < a.max_pages ? bt[pslot] : -1;
       if (page >= 0 && page < a.n_pages) dst = (is_k ? a.k_cache : a.v_cache) + (((long)page * a.n_kv + kvh) * kPage + (pp % kPage)) * HEAD;
       else if (lane == 0 && is_k) raise_fault(a.fault, a.layer, FS_PAGE);
     }
@@ -498,7 +504,8 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
     if (hg < G) {
       float x[DPL], y[DPL];
       fetch_head(row + ((long)kvh * G + hg) * HEAD, x);
-      norm_rope(x, a.q_gain, q_ahead, pos, y);
+      const float rms = a.q_gain ? rms_of(warp_sum_d(square_sum(x))) : 0.0f;
+      norm_rope(x, rms, a.q_gain, q_ahead, pos, y);
 #pragma unroll
       for (int j = 0; j < DPL; ++j) sq[hg * QSTR + lane + 32 * j] = y[j] * a.q_scale;
     }
@@ -512,7 +519,15 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
   if (single) {
     np = newest ? 1 : 0;
     if (tid == 0) s_ppos[0] = pos;
-    if (newest && warp < 2) append(0, 0, pos, warp == 0, x_new);
+    // The new key used to reach the cache 2.2 us behind the queries, in the block that then merges.  Its page comes ahead of the
+    // wait and its norm's factor is worked out in front of the branches on key and value: one row of 100 keys 1.79 -> 1.73 ms a
+    // pass, of 4,000 1.865 -> 1.840, of 12,000 (where other blocks take longer than this one) 2.03 -> 2.04.  Its sum run beside
+    // the query's, in one loop, gave the first no more and took 2.055 at the last; the page alone gave nothing.
+    if (newest && warp < 2) {
+      float new_rms = 0.0f;
+      if (warp == 0 && a.k_gain) new_rms = rms_of(warp_sum_d(square_sum(x_new)));
+      append(0, 0, pos, warp == 0, x_new, new_rms);
+    }
   } else {
     if (tid == 0) {
       s_np = 0;
@@ -533,7 +548,7 @@ __global__ void __launch_bounds__(256, HPW == 1 ? 1 : 2) attn_fused_kernel(const
     for (int it = warp; it < 2 * np; it += 8) {
       float x[DPL];
       fetch_head(new_head(s_pm[it >> 1], (it & 1) == 0), x);
-      append(it >> 1, s_pm[it >> 1], s_ppos[it >> 1], (it & 1) == 0, x);
+      append(it >> 1, s_pm[it >> 1], s_ppos[it >> 1], (it & 1) == 0, x, a.k_gain && (it & 1) == 0 ? rms_of(warp_sum_d(square_sum(x))) : 0.0f);
     }
   }
   int first_new = single ? pos : 0x7fffffff;         // tiles that end in front of this position take nothing from the pass
