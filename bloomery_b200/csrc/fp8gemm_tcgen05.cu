@@ -38,6 +38,7 @@ struct F8Args {
   const uint8_t* w2;
   long row_bytes, group_bytes;
   int N, K, tiles_w, stages;
+  int xs_bufs;                // buffers for the activation scales of a tile: 2, or 1 where K leaves no room
   const F8Tile* tiles;
   const int* n_tiles;
   int max_tiles;
@@ -65,6 +66,12 @@ __device__ __forceinline__ void umma_f8(uint32_t tmem_d, uint64_t adesc, uint64_
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
+// four bytes into shared memory, or zeros (bytes = 0)
+__device__ __forceinline__ void f8_copy4(float* smem, const float* gmem, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(smem)), "l"(gmem), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void f8_copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 template <bool DUAL>
 __global__ void __launch_bounds__(F8_THREADS, 1)
 fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUtensorMap tma_w,
@@ -80,7 +87,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
   __shared__ int s_abort;
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int STAGES = a.stages;
-  float* s_xs = reinterpret_cast<float*>(smem + (size_t)STAGES * STAGE_BYTES);     // [K / 128][32 tokens]
+  float* s_xs = reinterpret_cast<float*>(smem + (size_t)STAGES * STAGE_BYTES);     // [xs_bufs][K / 128][32 tokens]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -159,30 +166,70 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
   } else {
     const int q = warp & 3;                                          // TMEM lane quarter of this warp
     const int et = threadIdx.x - 64;                                 // 0 .. 127 among the epilogue threads
+    const TokenOut out{a.c_f32, a.c_bf16, (unsigned)a.ldc, a.row_scale, a.resid, (unsigned)a.ldr, a.N};
     uint32_t part = 0, pphase = 0;
     bool ok = true;
     int ti = 0;
-    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++ti) {
-      const F8Tile mt = a.tiles[t / a.tiles_w];
-      const int n = (t % a.tiles_w) * F8_BM + q * 32 + lane;         // weight row = output column of this thread
-      const bool n_ok = n < a.N;
-      const long wrow = (long)mt.group * a.group_bytes + (long)(n_ok ? n : a.N - 1) * a.row_bytes + a.K;
-      const float* ws = reinterpret_cast<const float*>(a.w + wrow);
-      const float* ws2 = DUAL ? reinterpret_cast<const float*>(a.w2 + wrow) : nullptr;
-      // the row's scales, four K blocks per 16-byte load, fetched four blocks ahead of their use (the scale strip of a
-      // row is padded to 16 bytes, so the last load stays inside the row)
-      const float4* ws4 = reinterpret_cast<const float4*>(ws);
-      const float4* ws24 = reinterpret_cast<const float4*>(ws2);
-      float4 w_cur = ws4[0], w_nxt = w_cur, w2_cur = DUAL ? ws24[0] : make_float4(0.f, 0.f, 0.f, 0.f), w2_nxt = w2_cur;
-      // the activation scales of this tile's 32 tokens, [kb][token]; rows past the tile scale by zero
-      if (ti > 0 && !mbar_wait_warp(&xs_done, (uint32_t)(ti - 1) & 1u, abort_flag)) break;   // the previous tile's readers are done
+    // Everything a tile needs beside its products is asked for while the tile before is worked on: the activation scales go
+    // to shared memory, the row's first weight scales and the routing to registers, the table's entry another tile earlier.
+    // Asked for at the tile's own start and end, one behind the other, these loads and the branches between the stores had a
+    // pass over the weights wait for the epilogue (32 rows x top 8 of 128 experts: down 67.6 us, 46.7 so, gate+up 72.2, 70.7;
+    // the output projection of attention 27.0, 19.6).
+    auto tile_of = [&](int t) { return t < total_tiles ? a.tiles[t / a.tiles_w] : F8Tile{0, 0, 0, 0}; };
+    auto scales_of = [&](const F8Tile& m, int buf) {                 // [kb][token]; rows past the tile scale by zero
       for (int i = et; i < kblocks * F8_BN; i += 128) {
-        const int kb = i >> 5, tok = i & 31;
-        const int r = mt.row0 + tok;
-        s_xs[i] = r < mt.row_end ? a.xs[(long)r * kblocks + kb] : 0.0f;
+        const int kb = i >> 5, r = m.row0 + (i & 31);
+        const bool in = r < m.row_end;
+        f8_copy4(s_xs + buf * kblocks * F8_BN + i, in ? a.xs + (long)r * kblocks + kb : a.xs, in ? 4 : 0);
       }
-      mbar_arrive(&xs_ready);
+    };
+    // the row's scales, four K blocks per 16-byte load, fetched four blocks ahead of their use (the scale strip of a
+    // row is padded to 16 bytes, so the last load stays inside the row)
+    const float4 *ws4 = nullptr, *ws24 = nullptr;
+    float4 w_first = make_float4(0.f, 0.f, 0.f, 0.f), w2_first = w_first;
+    int orow_l = -1;                                                 // lane i: output row and factor of the tile's token i
+    float sc_l = 1.0f;
+    auto open = [&](int t, const F8Tile& m) {
+      const int n = (t % a.tiles_w) * F8_BM + q * 32 + lane;
+      const long wrow = (long)m.group * a.group_bytes + (long)(n < a.N ? n : a.N - 1) * a.row_bytes + a.K;
+      ws4 = reinterpret_cast<const float4*>(a.w + wrow);
+      w_first = ws4[0];
+      if (DUAL) { ws24 = reinterpret_cast<const float4*>(a.w2 + wrow); w2_first = ws24[0]; }
+      const int r = m.row0 + lane;
+      orow_l = -1;
+      sc_l = 1.0f;
+      if (r < m.row_end) {
+        orow_l = a.dst_row ? a.dst_row[r] : r;
+        if (a.row_scale) sc_l = a.row_scale[r];
+      }
+    };
+    F8Tile mt = tile_of(blockIdx.x), mt_next = tile_of(blockIdx.x + gridDim.x);
+    if ((int)blockIdx.x < total_tiles) {
+      open(blockIdx.x, mt);
+      scales_of(mt, 0);
+    }
+    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++ti) {
+      const int n = (t % a.tiles_w) * F8_BM + q * 32 + lane;         // weight row = output column of this thread
+      const int nt = min(F8_BN, mt.row_end - mt.row0);
+      if (a.xs_bufs == 1 && ti > 0) {                                // the only buffer: once the tile before is done with it
+        mbar_arrive(&xs_done);
+        if (!mbar_wait_warp(&xs_done, (uint32_t)(ti - 1) & 1u, abort_flag)) break;
+        scales_of(mt, 0);
+      }
+      f8_copies_done();
+      mbar_arrive(&xs_ready);                                        // all four warps: copies landed, the tile before read
       if (!mbar_wait_warp(&xs_ready, (uint32_t)ti & 1u, abort_flag)) break;
+      const float* xs_t = s_xs + (a.xs_bufs == 1 ? 0 : (ti & 1) * kblocks * F8_BN);
+      const float4 *cur4 = ws4, *cur24 = ws24;
+      float4 w_cur = w_first, w2_cur = w2_first, w_nxt = w_cur, w2_nxt = w2_cur;
+      const int orow = orow_l;
+      const float sc = sc_l;
+      mt = mt_next;
+      if (t + (int)gridDim.x < total_tiles) {
+        open(t + gridDim.x, mt);
+        if (a.xs_bufs > 1) scales_of(mt, (ti + 1) & 1);
+        mt_next = tile_of(t + 2 * (int)gridDim.x);
+      }
       float acc[F8_BN], acc2[DUAL ? F8_BN : 1];
 #pragma unroll
       for (int i = 0; i < F8_BN; ++i) { acc[i] = 0.0f; if (DUAL) acc2[i] = 0.0f; }
@@ -190,7 +237,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
         const int j = kb & 3;
         if (j == 0) {
           if (kb > 0) { w_cur = w_nxt; if (DUAL) w2_cur = w2_nxt; }
-          if (kb + 4 < kblocks) { w_nxt = ws4[(kb >> 2) + 1]; if (DUAL) w2_nxt = ws24[(kb >> 2) + 1]; }
+          if (kb + 4 < kblocks) { w_nxt = cur4[(kb >> 2) + 1]; if (DUAL) w2_nxt = cur24[(kb >> 2) + 1]; }
         }
         const float wsc = j == 0 ? w_cur.x : j == 1 ? w_cur.y : j == 2 ? w_cur.z : w_cur.w;
         const float wsc2 = j == 0 ? w2_cur.x : j == 1 ? w2_cur.y : j == 2 ? w2_cur.z : w2_cur.w;
@@ -205,42 +252,39 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
         __syncwarp();
         if (lane == 0) mbar_arrive(&part_empty[part]);
         if (++part == F8_PARTS) { part = 0; pphase ^= 1; }
-        const float4* xs4 = reinterpret_cast<const float4*>(s_xs + kb * F8_BN);
+        const float4* xs4 = reinterpret_cast<const float4*>(xs_t + kb * F8_BN);
 #pragma unroll
-        for (int i4 = 0; i4 < F8_BN / 4; ++i4) {
-          const float4 x = xs4[i4];
-          const float xv[4] = {x.x, x.y, x.z, x.w};
+        for (int g = 0; g < F8_BN / 8; ++g) {
+          if (8 * g < nt) {                                          // a tile of a decode round has a few tokens
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int i = 4 * i4 + j;
-            acc[i] = fmaf(__uint_as_float(v[i]) * wsc, xv[j], acc[i]);
-            if (DUAL) acc2[i] = fmaf(__uint_as_float(u[i]) * wsc2, xv[j], acc2[i]);
+            for (int i4 = 2 * g; i4 < 2 * g + 2; ++i4) {
+              const float4 x = xs4[i4];
+              const float xv[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const int i = 4 * i4 + j;
+                acc[i] = fmaf(__uint_as_float(v[i]) * wsc, xv[j], acc[i]);
+                if (DUAL) acc2[i] = fmaf(__uint_as_float(u[i]) * wsc2, xv[j], acc2[i]);
+              }
+            }
           }
         }
       }
       if (!ok) break;
-      mbar_arrive(&xs_done);
-      // lane i fetches the routing of token row i of this tile; the store loop broadcasts it
-      const int r_l = mt.row0 + lane;
-      int orow_l = -1;
-      float sc_l = 1.0f;
-      if (r_l < mt.row_end) {
-        orow_l = a.dst_row ? a.dst_row[r_l] : r_l;
-        if (a.row_scale) sc_l = a.row_scale[r_l];
-      }
 #pragma unroll
-      for (int i = 0; i < F8_BN; ++i) {
-        const int orow = __shfl_sync(0xFFFFFFFFu, orow_l, i);
-        const float sc = __shfl_sync(0xFFFFFFFFu, sc_l, i);
-        if (orow < 0 || !n_ok) continue;
-        float f = acc[i];
-        if (DUAL) f = (f / (1.0f + __expf(-f))) * acc2[i];
-        f *= sc;
-        if (a.resid) f += a.resid[(long)orow * a.ldr + n];
-        if (a.c_f32) a.c_f32[(long)orow * a.ldc + n] = f;
-        else a.c_bf16[(long)orow * a.ldc + n] = __float2bfloat16_rn(f);
+      for (int g = 0; g < F8_BN / 4; ++g) {
+        if (4 * g < nt) {
+          float f[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            f[i] = acc[4 * g + i];
+            if constexpr (DUAL) f[i] = (f[i] / (1.0f + __expf(-f[i]))) * acc2[4 * g + i];
+          }
+          store_tokens<4>(out, f, orow, sc, 4 * g, n);
+        }
       }
     }
+    f8_copies_done();                                                // none may land after the CTA is gone
   }
 
   tc_fence_before();
@@ -315,8 +359,10 @@ template <bool DUAL>
 static int fp8_gemm_go(const CUtensorMap& mx, const F8Args& a0, int n_groups, int grid, cudaStream_t st) {
   constexpr int STAGE_BYTES = (DUAL ? 2 : 1) * F8_A_BYTES + F8_B_BYTES;
   F8Args a = a0;
-  const int xs_bytes = (a.K / F8_BK) * F8_BN * 4;
-  int stages = (220 * 1024 - xs_bytes) / STAGE_BYTES;
+  int xs_bytes = (a.K / F8_BK) * F8_BN * 4;
+  a.xs_bufs = 2 * xs_bytes + 4 * STAGE_BYTES <= 220 * 1024 ? 2 : 1;      // a second buffer does not cost the ring its depth
+  xs_bytes *= a.xs_bufs;
+  const int stages = (220 * 1024 - xs_bytes) / STAGE_BYTES;
   a.stages = stages > F8_MAX_STAGES ? F8_MAX_STAGES : stages;
   if (a.stages < 2) return BL_ERR_SHAPE;
   const size_t smem = (size_t)a.stages * STAGE_BYTES + xs_bytes + 1024;
@@ -363,7 +409,7 @@ int bl_fp8_gemm(const void* Xq, long ldx, long rows_x, const float* xs, const vo
   BL_REQUIRE(K >= 128 && K % 128 == 0 && N >= 1 && rows_x >= 1 && n_groups >= 1 && max_tiles >= 1, BL_ERR_SHAPE);
   BL_REQUIRE(tile_rows == F8_BN, BL_ERR_SHAPE);
   BL_REQUIRE(ldx % 16 == 0 && ((uintptr_t)Xq & 15) == 0 && ((uintptr_t)W & 15) == 0 && ((uintptr_t)W2 & 15) == 0, BL_ERR_ALIGN);
-  BL_REQUIRE((c_f32 != nullptr) != (c_bf16 != nullptr), BL_ERR_SHAPE);
+  BL_REQUIRE((c_f32 != nullptr) != (c_bf16 != nullptr) && ldc < 1L << 30 && ldr < 1L << 30, BL_ERR_SHAPE);
   const long rb = resident_row_bytes(WT_FP8_B128, K);
   BL_REQUIRE(rb > 0, BL_ERR_TYPE);
   CUtensorMap mx;

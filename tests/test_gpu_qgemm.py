@@ -206,6 +206,39 @@ def test_fp8_block_scaled_dense_gemm(rows):
     assert float((C - plain).abs().max()) < 0.05 * float(plain.abs().max())
 
 
+@pytest.mark.parametrize("rows,N,K,dual", [(1, 200, 128, False), (5, 38400, 256, False), (9, 38400, 128, True),
+                                           (33, 19200, 640, False), (29, 38400, 256, True), (4768, 128, 73728, False)])
+def test_fp8_tiles_of_one_block_follow_each_other(rows, N, K, dual):
+    """More tiles than blocks, so scales and routing come in a tile ahead: few, ragged and full token groups, a row of
+    scales that ends inside a load, and a K whose scales fit shared memory only once."""
+    from bloomery_b200.ops import gemm as G
+    qw, ref_w = _weight("FP8_B128", (N,), K, 1)
+    qw2, ref_w2 = _weight("FP8_B128", (N,), K, 2) if dual else (None, None)
+    torch.manual_seed(3)
+    X = (torch.randn(rows, K, device=DEV) * 0.5).bfloat16()
+    codes, scales, xv = _fp8_acts(X)
+    dst = torch.randperm(rows, device=DEV).to(torch.int32)
+    factor = torch.rand(rows, device=DEV) + 0.5
+    C = torch.full((rows + 1, N), float("nan"), device=DEV)
+    st = _status()
+    G.fp8_gemm(codes, scales, qw, G.TileTable.dense(rows, DEV, 32), out_f32=C, W2=qw2, dst_row=dst, row_scale=factor, status=st)
+    torch.cuda.synchronize()
+    assert int(st) == 0 and bool(C[rows].isnan().all())
+    pick = torch.arange(rows, device=DEV) if rows < 64 else torch.cat([torch.arange(0, rows, 97, device=DEV), torch.tensor([rows - 1], device=DEV)])
+    # an instruction of 32 values rounds (or cuts) once, the promotion of a block twice, each at most 2^-23 of the terms' sum
+    step = (K / 32 + 2 * K / 128 + 2) * 2.0 ** -23
+    x = xv[pick].double()
+    ref, tol = x @ ref_w.double().T, step * (x.abs() @ ref_w.double().abs().T)
+    if dual:
+        up, tol_up = x @ ref_w2.double().T, step * (x.abs() @ ref_w2.double().abs().T)
+        gate = torch.nn.functional.silu(ref)                     # slope at most 1.1; the exponential and the division a few units
+        tol = 1.1 * tol * (up.abs() + tol_up) + gate.abs() * tol_up + 2.0 ** -18 * (gate * up).abs()
+        ref = gate * up
+    f = factor[pick].double()[:, None]
+    err = (C[dst[pick].long()].double() - ref * f).abs()
+    assert bool((err <= (tol * f + 2.0 ** -22 * (ref * f).abs() + 1e-30)).all()), (err - tol * f).max()
+
+
 def test_fp8_block_scaled_grouped_dual_and_scatter():
     from bloomery_b200.ops import gemm as G
     torch.manual_seed(3)
