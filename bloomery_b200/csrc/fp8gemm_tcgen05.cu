@@ -9,8 +9,8 @@
 // tcgen05.mma kind::f8f6f4 (M 128, N 32, K 32) per stage into one of four partial accumulators in TMEM, and four
 // epilogue warps (lane = weight row) read each partial back with tcgen05.ld and add it into fp32 registers with the
 // block's two scales -- the promotion every 128 values that block-scaled FP8 needs for accuracy.  A pass over the
-// weights is therefore bound by HBM, not by expander warps (gate+up of 64 tokens x top-8 of 128 experts, 403 MB: 87 us
-// here, 118 us with csrc/qgemm_tcgen05.cu, which expands FP8 to bf16 in sixteen producer warps).
+// weights is therefore bound by HBM, not by expander warps (gate+up of 64 tokens x top-8 of 128 experts, 403 MB: 81 us
+// here, 116 us with csrc/qgemm_tcgen05.cu, which expands FP8 to bf16 in sixteen producer warps).
 //   * "dual" mode runs gate and up in one main loop; the epilogue writes silu(gate) * up;
 //   * the epilogue scatters and scales like the other GEMMs (dst_row / row_scale / resid).
 // Every mbarrier wait is bounded by the global timer; on expiry the CTA raises status word 1, leaves its loops, frees

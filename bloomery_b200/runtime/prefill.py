@@ -67,9 +67,9 @@ class GemmPrefill:
         # Micro-batches of at most this many tokens multiply the block-quantised weights as they are (csrc/qgemm_tcgen05.cu)
         # where every prompt would have to expand them to bf16 first: a layer of the 30 B shape is 0.35 GB of blocks and 1.2 GB
         # of copies that are written and read.  Eight layers, 64 / 128 tokens, milliseconds: Q4_K_M 3.1 / 4.1 over the blocks,
-        # 6.0 / 5.8 with the expansion; FP8 3.3 / 4.3 and 9.9 / 10.1; NVFP4 3.6 / 4.6 and 6.2 / 6.5.  Copies that are kept
-        # are the faster ones from about 64 tokens on (3.2 to 3.6 / 3.5 in all three), so there the blocks are left to the
-        # prompts below it, which need their bits (run).
+        # 6.0 / 5.8 with the expansion; FP8 3.3 / 4.3 and 9.9 / 10.1; NVFP4 3.6 / 4.6 and 6.2 / 6.5.  With copies that
+        # are kept, the blocks serve every product of the prompts below GEMM_THRESHOLD, which need their bits (run); above it only
+        # the experts' (block_rows), the projections read their copies (3.2 to 3.6 / 3.5 with copies alone in all three).
         # (0: no micro-batch multiplies blocks.)
         self.direct_rows = 128
         # Experts alone take their blocks further, copies or not, up to this many rows an expert on average: the products are then
