@@ -8,6 +8,9 @@
 // (crates/gpu/src/elem.rs argmax_rows_fault).
 #include "common.cuh"
 
+#include <chrono>
+#include <thread>
+
 namespace bl {
 
 struct EmbedArgs {
@@ -233,6 +236,23 @@ int bl_mtp_prep(const float* e, long e_stride, const float* h, long h_stride, co
   BL_REQUIRE(H % 32 == 0 && M >= 1 && enorm && hnorm, BL_ERR_SHAPE);
   return (int)launch(mtp_prep_kernel, dim3(M), dim3(256), 0, st, e, e_stride, h, h_stride, src, enorm, hnorm, eps, H, xq,
                      (float2*)xds);
+}
+
+// Asks query(arg) until it answers something else than `pending`, for at most `limit_us` microseconds; returns the last answer.
+int bl_poll(int (*query)(void*), void* arg, int pending, long limit_us) {
+  const auto end = std::chrono::steady_clock::now() + std::chrono::microseconds(limit_us);
+  for (;;) {
+    const int rc = query(arg);
+    if (rc != pending || std::chrono::steady_clock::now() >= end) return rc;
+    std::this_thread::yield();
+  }
+}
+
+// 0: the event has come; cudaErrorNotReady: not within `limit_us`; anything else: the context's error.
+int bl_event_wait(cudaEvent_t event, long limit_us) {
+  const int rc = bl_poll([](void* e) { return (int)cudaEventQuery((cudaEvent_t)e); }, event, cudaErrorNotReady, limit_us);
+  if (rc == cudaErrorNotReady) cudaGetLastError();         // no error of a later launch
+  return rc;
 }
 
 const char* bl_error_string(int code) {

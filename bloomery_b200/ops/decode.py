@@ -414,6 +414,18 @@ def fill_u32(t: torch.Tensor, value: int) -> None:
     check(cuda().bl_fill_u32(p(t), ctypes.c_uint(value), I(t.numel()), stream()), "bl_fill_u32")
 
 
+NOT_READY = 600                       # cudaErrorNotReady
+
+
+def event_wait(event: torch.cuda.Event, limit_us: int) -> bool:
+    """Whether ``event``, recorded before, comes within ``limit_us``.  The queries run in native code, so the interpreter's lock is
+    free meanwhile (``event.query()`` keeps it)."""
+    rc = cuda().bl_event_wait(ctypes.c_void_p(event.cuda_event), L(limit_us))
+    if rc != NOT_READY:
+        check(rc, "bl_event_wait")
+    return rc == 0
+
+
 def advance_rows(tokens, row_pos, row_seq, chosen, M: int, hist=None, hist_cap: int = 0, hist_count=None) -> None:
     check(cuda().bl_advance_rows(p(tokens), p(row_pos), p(row_seq), p(chosen), I(M), p(hist), I(hist_cap),
                                  p(hist_count), stream()), "bl_advance_rows")

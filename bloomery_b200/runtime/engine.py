@@ -109,7 +109,6 @@ class DecodeEngine:
         self._stage = [torch.zeros(4, R, dtype=torch.int32, pin_memory=True) for _ in range(self._stage_n)]
         self._stage_np = [t.numpy() for t in self._stage]          # same memory: rows are written without tensor indexing
         self._stage_ev = [None] * self._stage_n
-        self._last_wait: Dict[int, float] = {}       # rows of a pass -> seconds the host last waited for one
         self._stage_i = 0
         self.params_host = self._stage[0]
         self.tokens, self.row_pos, self.row_seq = self.params[0], self.params[1], self.params[2]
@@ -559,18 +558,13 @@ class DecodeEngine:
         self.tokens_out_host.copy_(self.tokens_out, non_blocking=True)
         self._done.record()
         t0 = time.monotonic()
-        # The kernel rounds a nap of any length up to some 50 us, a quarter of a small model's round: naps for three quarters of
-        # the last such wait, and from there on the queries (which let other threads run) follow each other.
-        nap = 0.75 * self._last_wait.get(m, 0.0)
         tok = self.watchdog.enter("step readback") if self.watchdog is not None else None
         try:
-            while not self._done.query():
-                waited = time.monotonic() - t0
-                if waited > self.bound_s:
+            # Naps would be rounded up to some 50 us by the kernel, a quarter of a small model's round, and queries from here would
+            # hold the interpreter's lock against the threads of the server.
+            while not K.event_wait(self._done, 2000):
+                if time.monotonic() - t0 > self.bound_s:
                     raise EngineStalled(f"no answer from the device within {self.bound_s:.0f} s")
-                if waited < nap:
-                    time.sleep(0)
-            self._last_wait[m] = time.monotonic() - t0
         finally:
             if tok is not None:
                 self.watchdog.leave(tok)

@@ -688,6 +688,55 @@ def test_experts_take_their_blocks_up_to_some_rows_an_expert():
     assert not any(limit("NVFP4"))
 
 
+def test_other_threads_run_while_a_pass_is_awaited(monkeypatch):
+    """A pass of 50 ms: a thread that naps and needs the interpreter between its naps gets it each time, not once in the 5 ms
+    after which a thread that keeps it is made to give it up."""
+    import ctypes
+    from types import SimpleNamespace as NS
+    from bloomery_b200.ops import _lib
+    from bloomery_b200.ops import decode as K
+    from bloomery_b200.runtime.engine import DecodeEngine, EngineStalled
+    never = ctypes.cast(ctypes.CDLL(None).abs, ctypes.c_void_p)           # answers what it is asked: always "not yet"
+
+    class Event:
+        def record(self):
+            self.end = time.monotonic() + 0.05
+
+        def query(self):
+            return time.monotonic() >= self.end
+
+    def event_wait(event, limit_us):
+        left = max(0, int(1e6 * (event.end - time.monotonic())))
+        _lib.cuda().bl_poll(never, ctypes.c_void_p(K.NOT_READY), _lib.I(K.NOT_READY), _lib.L(min(limit_us, left)))
+        return event.query()
+
+    monkeypatch.setattr(K, "event_wait", event_wait, raising=False)
+    eng = object.__new__(DecodeEngine)
+    out = NS(copy_=lambda *a, **kw: None)
+    vars(eng).update(tokens_out=out, tokens_out_host=out, _tokens_out_np=NS(tolist=lambda: [7]), _done=Event(), bound_s=10.0,
+                     watchdog=None, waits=Waits())
+    turns, on = [0], [True]
+
+    def other():
+        while on[0]:
+            time.sleep(1e-4)
+            turns[0] += 1
+
+    th = threading.Thread(target=other)
+    th.start()
+    try:
+        time.sleep(0.01)
+        before = turns[0]
+        assert eng.read_tokens(1) == [7]
+        assert turns[0] - before > 40, turns[0] - before
+        eng.bound_s = 0.01
+        with pytest.raises(EngineStalled):
+            eng.read_tokens(1)
+    finally:
+        on[0] = False
+        th.join()
+
+
 def test_a_prompt_path_keeps_the_engine_it_was_given_and_an_engine_not_itself(monkeypatch):
     import weakref
     from bloomery_b200.runtime.engine import DecodeEngine
