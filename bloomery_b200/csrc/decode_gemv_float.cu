@@ -2,5 +2,5 @@
 #include "gemv_kernel.cuh"
 
 namespace bl {
-template cudaError_t gemv_family<true, 1>(const GemvArgs&, int, int, int, cudaStream_t);
+template cudaError_t gemv_family<true, 1>(const GemvArgs&, const GemvPlan&, cudaStream_t);
 }  // namespace bl

@@ -2,6 +2,6 @@
 #include "gemv_kernel.cuh"
 
 namespace bl {
-template cudaError_t gemv_family<true, 2>(const GemvArgs&, int, int, int, cudaStream_t);
-template cudaError_t gemv_family<false, 2>(const GemvArgs&, int, int, int, cudaStream_t);
+template cudaError_t gemv_family<true, 2>(const GemvArgs&, const GemvPlan&, cudaStream_t);
+template cudaError_t gemv_family<false, 2>(const GemvArgs&, const GemvPlan&, cudaStream_t);
 }  // namespace bl

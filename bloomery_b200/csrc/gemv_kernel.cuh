@@ -28,13 +28,16 @@ __device__ __forceinline__ void rows_q(const GemvArgs& a, const GemvSeg& s, int 
 #pragma unroll
         for (int c = 0; c < C; ++c) {
           const int u = base + c * 32 + lane;
-          if (u < nunits && r0 + r < r_hi) U::loadu(s.w + (long)(r0 + r) * s.row_bytes, u, K, regs[r][c]);
+          // a weight row past the end is the segment's last one again; its result is dropped (see the dots below)
+          if (u < nunits) U::loadu(s.w + (long)min(r0 + r, s.rows - 1) * s.row_bytes, u, K, regs[r][c]);
         }
       between();
 #pragma unroll
       for (int c = 0; c < C; ++c) {
         const int u = base + c * 32 + lane;
         if (u < nunits) {
+          // No branch on the weight row: behind one, its codes and scales are taken apart again for every row m (eight rows of a 2,048
+          // deep head: 351 us, 252 without).
 #pragma unroll
           for (int m = 0; m < MB; ++m) {
             // the block's activation rows sit in the conflict-free chunk layout of its weight type
@@ -42,7 +45,7 @@ __device__ __forceinline__ void rows_q(const GemvArgs& a, const GemvSeg& s, int 
             StagedAct<T>::load(sq + (long)m * K, sds + (long)m * (K / 32), u, nunits, act);
 #pragma unroll
             for (int r = 0; r < R; ++r)
-              if (r0 + r < r_hi) acc[r][m] += ActOf<T>::dot(regs[r][c], u, act);
+              acc[r][m] += ActOf<T>::dot(regs[r][c], u, act);
           }
         }
       }
@@ -307,41 +310,58 @@ static inline size_t gemv_smem(int M, int K, bool values) {
   return b;
 }
 
+// How a call of several segments is launched.
+struct GemvPlan {
+  int grid, R, C;       // blocks; weight rows a warp takes at a time; units of a row a lane takes at a time
+  bool multi;           // rows_multi: two rows and more whose weight rows a warp's registers hold, and that are not sums over ranks
+  int MB;               // otherwise: the rows of the kernel
+  size_t smem;
+};
+
 template <int MB, int R, int C, bool NORM, int FAM, bool MULTI>
-static cudaError_t gemv_launch(const GemvArgs& a, int grid, cudaStream_t st) {
-  const size_t smem = gemv_smem(MULTI ? a.M : MB, a.K, FAM == 1 || (MULTI && NORM));
+static cudaError_t gemv_launch(const GemvArgs& a, const GemvPlan& p, cudaStream_t st) {
   static PerDevice limit;
   if (limit.due()) {
     cudaFuncSetAttribute(gemv_kernel<MB, R, C, NORM, FAM, MULTI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     limit.mark();
   }
-  return launch(gemv_kernel<MB, R, C, NORM, FAM, MULTI>, dim3(grid), dim3(256), smem, st, a);
+  return launch(gemv_kernel<MB, R, C, NORM, FAM, MULTI>, dim3(p.grid), dim3(256), p.smem, st, a);
 }
 
 template <bool NORM, int FAM, int MB, bool MULTI>
-static cudaError_t gemv_dispatch_shape(const GemvArgs& a, int R, int C, int grid, cudaStream_t st) {
-  if (C == 2) return gemv_launch<MB, 1, 2, NORM, FAM, MULTI>(a, grid, st);
-  // several rows keep the decoded weights of float planes in registers from one row to the next, which leaves room for one
-  if constexpr (!MULTI || FAM == 0) {
-    if (R >= 3) return gemv_launch<MB, 3, 1, NORM, FAM, MULTI>(a, grid, st);
+static cudaError_t gemv_dispatch_shape(const GemvArgs& a, const GemvPlan& p, cudaStream_t st) {
+  if (p.C == 2) return gemv_launch<MB, 1, 2, NORM, FAM, MULTI>(a, p, st);
+  // several rows keep the decoded weights of float planes in registers from one row to the next, which leaves room for one;
+  // a kernel that takes eight rows as a whole has no room for a third weight row's sums
+  if constexpr (MULTI ? FAM == 0 : MB < kMaxRows) {
+    if (p.R >= 3) return gemv_launch<MB, 3, 1, NORM, FAM, MULTI>(a, p, st);
   }
   if constexpr (!MULTI || FAM != 2) {
-    if (R >= 2) return gemv_launch<MB, 2, 1, NORM, FAM, MULTI>(a, grid, st);
+    if (p.R >= 2) return gemv_launch<MB, 2, 1, NORM, FAM, MULTI>(a, p, st);
   }
-  return gemv_launch<MB, 1, 1, NORM, FAM, MULTI>(a, grid, st);
+  return gemv_launch<MB, 1, 1, NORM, FAM, MULTI>(a, p, st);
+}
+
+template <bool NORM, int FAM, int MB>
+static cudaError_t gemv_dispatch_whole(const GemvArgs& a, const GemvPlan& p, cudaStream_t st) {
+  // Only a reduction in front brings rows here whose units one column a lane holds, and there up to three weight rows are in
+  // flight (two of the half empty columns instead, two ranks: QKV of 2,048 for two rows 19.5 us, 18.5 so; a head 124, 105; four rows
+  // of the head 193, 158).
+  if constexpr (NORM) return gemv_dispatch_shape<NORM, FAM, MB, false>(a, p, st);
+  else return gemv_launch<MB, 1, 2, NORM, FAM, false>(a, p, st);
 }
 
 // One row; several rows; several rows whose weight rows do not fit the registers of a warp (two columns of units a lane), or that
 // are sums over ranks.
 template <bool NORM, int FAM>
-cudaError_t gemv_family(const GemvArgs& a, int R, int C, int grid, cudaStream_t st) {
-  if (a.M == 1) return gemv_dispatch_shape<NORM, FAM, 1, false>(a, R, C, grid, st);
-  if (a.K / 64 > 32 * C || a.red.n_ranks > 0) {
-    if (a.M <= 2) return gemv_launch<2, 1, 2, NORM, FAM, false>(a, grid, st);
-    if (a.M <= 4) return gemv_launch<4, 1, 2, NORM, FAM, false>(a, grid, st);
-    return gemv_launch<kMaxRows, 1, 2, NORM, FAM, false>(a, grid, st);
+cudaError_t gemv_family(const GemvArgs& a, const GemvPlan& p, cudaStream_t st) {
+  if (p.multi) return gemv_dispatch_shape<NORM, FAM, kMaxRows, true>(a, p, st);
+  switch (p.MB) {
+    case 1: return gemv_dispatch_shape<NORM, FAM, 1, false>(a, p, st);
+    case 2: return gemv_dispatch_whole<NORM, FAM, 2>(a, p, st);
+    case 4: return gemv_dispatch_whole<NORM, FAM, 4>(a, p, st);
+    default: return gemv_dispatch_whole<NORM, FAM, kMaxRows>(a, p, st);
   }
-  return gemv_dispatch_shape<NORM, FAM, kMaxRows, true>(a, R, C, grid, st);
 }
 
 }  // namespace bl

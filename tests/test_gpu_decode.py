@@ -82,6 +82,35 @@ def test_gemv_rows_of_a_pass_equal_single_rows(t, Kd, rows):
             assert torch.equal(out[live], one_r[live])
 
 
+@pytest.mark.parametrize("t", ["Q4_K", "Q6_K", "NVFP4", "F32"])
+@pytest.mark.parametrize("Kd,rows", [(256, 40), (2048, 5123), (4096, 301)])
+def test_gemv_behind_a_reduction_equals_the_rows_it_adds_up(t, Kd, rows):
+    """x + the partial rows of two ranks, added in rank order, has the bits of the same sum taken in front of the launch.  The
+    partial rows carry their epoch already, so nothing waits."""
+    from bloomery_b200.ops import decode as K
+    torch.manual_seed(12)
+    if t == "F32":
+        qw = K.QWeight((torch.randn(rows, Kd, device=DEV) * 0.02).view(torch.uint8).reshape(rows, -1), t, Kd)
+    else:
+        qw, _ = _qw(torch.randn(rows, Kd) * 0.02, t)
+    x, gain = torch.randn(8, Kd, device=DEV), 1 + 0.1 * torch.randn(Kd, device=DEV)
+    part = torch.randn(2, 8, Kd, device=DEV)
+    recv = torch.ones(2, 8, Kd, 2, dtype=torch.int32, device=DEV)
+    recv[..., 0] = part.view(torch.int32)
+    step, x_out = torch.zeros(1, dtype=torch.int32, device=DEV), torch.zeros(8, Kd, device=DEV)
+    fault = torch.full((1,), -1, dtype=torch.int32, device=DEV)
+    red = K.ReduceIn(recv.data_ptr(), step.data_ptr(), 1, 0, x_out.data_ptr(), Kd, 2, Kd, fault.data_ptr(), 0)
+    want_x = (x + part[0]) + part[1]
+    want, out = torch.zeros(8, rows, device=DEV), torch.zeros(8, rows, device=DEV)
+    for m in range(8):
+        K.gemv([qw], 1, want[m:m + 1], x=want_x[m:m + 1], gain=gain, eps=1e-6)
+    for M in (1, 2, 3, 8):
+        out.zero_()
+        K.gemv([qw], M, out, x=x, gain=gain, eps=1e-6, red=red, fault=fault)
+        assert torch.equal(out[:M], want[:M]) and torch.equal(x_out[:M], want_x[:M])
+    assert int(fault) == -1
+
+
 def test_gemv_q8in_resid_multiseg():
     from bloomery_b200.ops import decode as K
     torch.manual_seed(1)

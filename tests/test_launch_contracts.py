@@ -96,3 +96,19 @@ def test_a_tile_table_that_a_launch_writes_is_no_longer_fixed(monkeypatch):
         assert t.fixed == 3
         again(t)
         assert t.fixed == 0
+
+
+def _gemv_plan(M, K, reduce=0, norm=1, rows=(4096, 512, 512), types=(12, 12, 14)):
+    """Blocks, weight rows and units a lane takes at a time, rows as a whole, bytes of shared memory on 148 processors."""
+    out = (ctypes.c_long * 5)()
+    n = len(rows)
+    assert cuda().bl_gemv_plan(I(n), (I * n)(*rows), (I * n)(*types), I(K), I(M), I(norm), I(reduce), I(148), out) == 0
+    return list(out)
+
+
+def test_rows_behind_a_reduction_keep_several_weight_rows_in_flight():
+    """A head of 151,936 rows gives a warp more of them than it takes at a time: three, or two beside eight rows' sums."""
+    for M, R in ((1, 3), (2, 3), (3, 3), (4, 3), (5, 2), (8, 2)):
+        assert _gemv_plan(M, 2048, reduce=1, rows=(151936,), types=(14,))[1:3] == [R, 1]
+    assert _gemv_plan(8, 4096, reduce=1)[1:3] == [1, 2]                    # two columns of units a lane are needed there
+    assert cuda().bl_gemv_plan(I(1), (I * 1)(64), (I * 1)(0), I(2048), I(1), I(0), I(0), I(148), (L * 5)()) == TYPE
