@@ -67,10 +67,11 @@ static int gemv_plan(int nseg, const int* rows, const int* wtypes, int K, int M,
     rpw_max = rpw > rpw_max ? rpw : rpw_max;
   }
   p.MB = M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : kMaxRows;
-  p.multi = M > 1 && K / 64 <= 32 * p.C && !reduce;
+  const size_t one_by_one = gemv_smem(M, K, floatw || norm);
+  p.multi = M > 1 && !reduce && (p.C == 1 || (K / 64 <= 64 && (fam != 2 || (!norm && M > 2)) && 2 * (one_by_one + 1024) <= kSmemOfProcessor));
   const int most = p.multi ? (fam == 0 ? 3 : fam == 1 ? 2 : 1) : p.MB == kMaxRows ? 2 : 3;
   p.R = p.C == 2 ? 1 : rpw_max < most ? rpw_max : most;
-  p.smem = gemv_smem(p.multi ? M : p.MB, K, floatw || (p.multi && norm));
+  p.smem = p.multi ? one_by_one : gemv_smem(p.MB, K, floatw);
   return 0;
 }
 

@@ -14,6 +14,7 @@ __device__ __forceinline__ void rows_q(const GemvArgs& a, const GemvSeg& s, int 
   using U = Unit<T>;
   const int K = a.K, lane = threadIdx.x & 31;
   const int nunits = K / 64;
+  constexpr bool PLANE_ROW = MB == 1 && (T::kType == WT_NVFP4 || T::kType == WT_FP8_B128);
   const unsigned push_epoch = a.push.n_ranks > 0 ? site_epoch(a.push.step, a.push.sites_per_step, a.push.site_index) : 0u;
   for (int r0 = r_lo; r0 < r_hi || r0 == r_lo; r0 += R) {
     float acc[R][MB];
@@ -28,8 +29,8 @@ __device__ __forceinline__ void rows_q(const GemvArgs& a, const GemvSeg& s, int 
 #pragma unroll
         for (int c = 0; c < C; ++c) {
           const int u = base + c * 32 + lane;
-          // a weight row past the end is the segment's last one again; its result is dropped (see the dots below)
-          if (u < nunits) U::loadu(s.w + (long)min(r0 + r, s.rows - 1) * s.row_bytes, u, K, regs[r][c]);
+          // a weight row past the end is the segment's last one again; its result is dropped
+          if (u < nunits && (!PLANE_ROW || r0 + r < r_hi)) U::loadu(s.w + (long)min(r0 + r, s.rows - 1) * s.row_bytes, u, K, regs[r][c]);
         }
       between();
 #pragma unroll
@@ -37,7 +38,7 @@ __device__ __forceinline__ void rows_q(const GemvArgs& a, const GemvSeg& s, int 
         const int u = base + c * 32 + lane;
         if (u < nunits) {
           // No branch on the weight row: behind one, its codes and scales are taken apart again for every row m (eight rows of a 2,048
-          // deep head: 351 us, 252 without).
+          // deep head: 351 us, 252 without).  One row of float planes has one, since their dots cost more than it saves.
 #pragma unroll
           for (int m = 0; m < MB; ++m) {
             // the block's activation rows sit in the conflict-free chunk layout of its weight type
@@ -45,7 +46,7 @@ __device__ __forceinline__ void rows_q(const GemvArgs& a, const GemvSeg& s, int 
             StagedAct<T>::load(sq + (long)m * K, sds + (long)m * (K / 32), u, nunits, act);
 #pragma unroll
             for (int r = 0; r < R; ++r)
-              acc[r][m] += ActOf<T>::dot(regs[r][c], u, act);
+              if (!PLANE_ROW || r0 + r < r_hi) acc[r][m] += ActOf<T>::dot(regs[r][c], u, act);
           }
         }
       }
@@ -92,7 +93,10 @@ __device__ __forceinline__ void rows_q(const GemvArgs& a, const GemvSeg& s, int 
 // The same for passes of several rows whose weight rows are at most 32 C units long: the weights of R rows stay in registers
 // and the pass's rows walk past them one by one, so nothing is kept per (weight row, row of the pass) and the loop runs
 // over live rows only.  Sums are those of rows_q.  Lane 8 r + m keeps the result of weight row r and row m and stores it at the end.
-// (Accumulators of 2 x 8 instead spilled 1 KB a thread; five rows in a bucket of eight computed eight.)
+// (Accumulators of 2 x 8 instead spilled 1 KB a thread; five rows in a bucket of eight computed eight.)  The dots have no branch
+// on the weight row, behind which its codes and scales would be taken apart once a row of the pass (head of 151,936 x 2,048, eight
+// rows 230 us, 204 so); two units a lane are too many to be kept taken apart, so there two rows of the pass share that work
+// (8,192 x 4,096 Q6_K, eight rows 33 us, 29 so).
 template <class T, int R, int C, class Between>
 __device__ __forceinline__ void rows_multi(const GemvArgs& a, const GemvSeg& s, int r_lo, int r_hi, int out_col0, unsigned live,
                                            const int8_t* sq, const float2* sds, const float* s_scale, Between&& between) {
@@ -101,6 +105,7 @@ __device__ __forceinline__ void rows_multi(const GemvArgs& a, const GemvSeg& s, 
   const int nunits = K / 64;
   const int my_m = lane & 7, my_r = lane >> 3;
   static_assert(R <= 4 && kMaxRows == 8, "a result a lane");
+  constexpr int P = C == 2 && T::kType != WT_NVFP4 && T::kType != WT_FP8_B128 ? 2 : 1;
   const unsigned push_epoch = a.push.n_ranks > 0 ? site_epoch(a.push.step, a.push.sites_per_step, a.push.site_index) : 0u;
   for (int r0 = r_lo; r0 < r_hi || r0 == r_lo; r0 += R) {
     typename U::Regs regs[R][C];
@@ -108,33 +113,46 @@ __device__ __forceinline__ void rows_multi(const GemvArgs& a, const GemvSeg& s, 
     for (int r = 0; r < R; ++r)
 #pragma unroll
       for (int c = 0; c < C; ++c)
-        if (c * 32 + lane < nunits && r0 + r < r_hi) U::loadu(s.w + (long)(r0 + r) * s.row_bytes, c * 32 + lane, K, regs[r][c]);
+        if (c * 32 + lane < nunits) U::loadu(s.w + (long)min(r0 + r, s.rows - 1) * s.row_bytes, c * 32 + lane, K, regs[r][c]);
     between();
     const bool mine = my_r < R && r0 + my_r < r_hi && (live >> my_m & 1);
     const int col = out_col0 + r0 + my_r;
     float res = 0.f, old = 0.f;
     if (a.resid && a.push.n_ranks == 0 && mine) old = a.resid[(long)my_m * a.resid_stride + col];
 #pragma unroll 1
-    for (unsigned left = live; left; left &= left - 1) {
-      const int m = __ffs(left) - 1;
-      float acc[R];
+    for (unsigned left = live; left;) {
+      int ms[P];                     // the next rows; -1: there is none
 #pragma unroll
-      for (int r = 0; r < R; ++r) acc[r] = 0.f;
+      for (int i = 0; i < P; ++i) {
+        ms[i] = __ffs(left) - 1;
+        left &= left - 1;
+      }
+      float acc[P][R];
+#pragma unroll
+      for (int i = 0; i < P; ++i)
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[i][r] = 0.f;
 #pragma unroll
       for (int c = 0; c < C; ++c) {
         const int u = c * 32 + lane;
         if (u < nunits) {
-          ActRegs act;
-          StagedAct<T>::load(sq + (long)m * K, sds + (long)m * (K / 32), u, nunits, act);
 #pragma unroll
-          for (int r = 0; r < R; ++r)
-            if (r0 + r < r_hi) acc[r] += ActOf<T>::dot(regs[r][c], u, act);
+          for (int i = 0; i < P; ++i) {
+            if (i > 0 && ms[i] < 0) continue;
+            ActRegs act;
+            StagedAct<T>::load(sq + (long)ms[i] * K, sds + (long)ms[i] * (K / 32), u, nunits, act);
+#pragma unroll
+            for (int r = 0; r < R; ++r) acc[i][r] += ActOf<T>::dot(regs[r][c], u, act);
+          }
         }
       }
-      float sum;
-      if constexpr (R == 1) sum = warp_sum(acc[0]);
-      else sum = warp_sum4(acc[0], acc[1], R > 2 ? acc[R - 1] : 0.f, 0.f);
-      if (my_m == m) res = sum;
+#pragma unroll
+      for (int i = 0; i < P; ++i) {
+        float sum;
+        if constexpr (R == 1) sum = warp_sum(acc[i][0]);
+        else sum = warp_sum4(acc[i][0], acc[i][1], R > 2 ? acc[i][R - 1] : 0.f, 0.f);
+        if (my_m == ms[i]) res = sum;
+      }
     }
     if (mine) {
       float v = res * s_scale[my_m];
@@ -310,10 +328,19 @@ static inline size_t gemv_smem(int M, int K, bool values) {
   return b;
 }
 
+constexpr size_t kSmemOfProcessor = 227 * 1024;      // shared memory of its blocks, each of which takes 1 KB more than it asks for
+
 // How a call of several segments is launched.
 struct GemvPlan {
   int grid, R, C;       // blocks; weight rows a warp takes at a time; units of a row a lane takes at a time
-  bool multi;           // rows_multi: two rows and more whose weight rows a warp's registers hold, and that are not sums over ranks
+  // rows_multi: two rows and more whose weight rows a warp's registers hold, that are not sums over ranks and whose blocks fit a
+  // processor two at a time, as they are counted.  The fp32 rows of its norm, 16 KB each at a width of 4,096, do not from six on:
+  // QKV (8,192 + 512 + 512) of eight rows as a whole 45 us, 53 in two waves of rows_multi, of four 31 / 27; a head of 151,936 412 / 479
+  // and 242 / 225.  Float planes with two units a lane cost more to take apart: behind the norm rows_multi never gains (QKV of NVFP4
+  // for four rows 29 / 33, eight 43 / 64), without it from three rows on (passes of the 30 B shape, ms: NVFP4 two rows 3.19 /
+  // 3.31, four 4.75 / 4.81, five 5.88 / 5.72, eight 6.88 / 6.84; FP8 two 4.55 / 4.64, three 6.07 / 5.75, five 8.61 / 7.76, eight
+  // 10.19 / 9.71).
+  bool multi;
   int MB;               // otherwise: the rows of the kernel
   size_t smem;
 };
@@ -330,7 +357,9 @@ static cudaError_t gemv_launch(const GemvArgs& a, const GemvPlan& p, cudaStream_
 
 template <bool NORM, int FAM, int MB, bool MULTI>
 static cudaError_t gemv_dispatch_shape(const GemvArgs& a, const GemvPlan& p, cudaStream_t st) {
-  if (p.C == 2) return gemv_launch<MB, 1, 2, NORM, FAM, MULTI>(a, p, st);
+  if constexpr (!(MULTI && NORM && FAM == 2)) {
+    if (p.C == 2) return gemv_launch<MB, 1, 2, NORM, FAM, MULTI>(a, p, st);
+  }
   // several rows keep the decoded weights of float planes in registers from one row to the next, which leaves room for one;
   // a kernel that takes eight rows as a whole has no room for a third weight row's sums
   if constexpr (MULTI ? FAM == 0 : MB < kMaxRows) {
@@ -351,8 +380,7 @@ static cudaError_t gemv_dispatch_whole(const GemvArgs& a, const GemvPlan& p, cud
   else return gemv_launch<MB, 1, 2, NORM, FAM, false>(a, p, st);
 }
 
-// One row; several rows; several rows whose weight rows do not fit the registers of a warp (two columns of units a lane), or that
-// are sums over ranks.
+// Several rows one by one; one row, and rows as a whole.
 template <bool NORM, int FAM>
 cudaError_t gemv_family(const GemvArgs& a, const GemvPlan& p, cudaStream_t st) {
   if (p.multi) return gemv_dispatch_shape<NORM, FAM, kMaxRows, true>(a, p, st);

@@ -112,3 +112,13 @@ def test_rows_behind_a_reduction_keep_several_weight_rows_in_flight():
         assert _gemv_plan(M, 2048, reduce=1, rows=(151936,), types=(14,))[1:3] == [R, 1]
     assert _gemv_plan(8, 4096, reduce=1)[1:3] == [1, 2]                    # two columns of units a lane are needed there
     assert cuda().bl_gemv_plan(I(1), (I * 1)(64), (I * 1)(0), I(2048), I(1), I(0), I(0), I(148), (L * 5)()) == TYPE
+
+
+def test_the_blocks_of_a_gemv_fit_a_processor_two_at_a_time():
+    """They are counted as one wave of two a processor, whose blocks share 227 KB less 1 KB each: at any width of quantised rows, with
+    or without the norm's fp32 rows, alone or behind a reduction."""
+    for types in ((12, 12, 14), (40, 40, 40)):
+        for K in range(256, 8193, 256):
+            for M in range(1, 9):
+                for kw in (dict(), dict(norm=0), dict(reduce=1)):
+                    assert 2 * (_gemv_plan(M, K, types=types, **kw)[4] + 1024) <= 227 * 1024, (types, K, M, kw)
