@@ -55,13 +55,13 @@ class GemmPrefill:
         self.expand_ahead = True                # bf16 expansion of layer l + 1's weights on a side stream during layer l
         self._side = None
         self.flash = True                       # head size 128: fused attention on tensor memory (csrc/flash_tcgen05.cu)
-        # Resident bf16 copy of every layer's matrices, built by the first prompt that runs (58 GB for a 30 B-parameter
-        # mixture beside its 17 GB of Q4_K_M blocks): later prompts skip the expansion launches altogether.  None = only
-        # when the copy leaves a quarter of the card free; True / False force it.
+        # Resident bf16 copy of every layer's matrices, built by the first prompt that multiplies them (58 GB for a 30 B-parameter
+        # mixture beside its 17 GB of Q4_K_M blocks, 56 of them the routed experts'): later prompts skip the expansion launches
+        # altogether.  None = only when the copy leaves a quarter of the card free; True / False force it.
         from ..utils import levers
         self.resident_bf16 = {"1": True, "0": False}.get(str(levers.get("BLOOMERY_PREFILL_BF16")), None)
         self._resident = {}
-        self._resident_ok = None
+        self._resident_ok = self._resident_experts_ok = None
         from .timing import PromptTiming
         self.timing = PromptTiming()            # arm() it to get per-unit milliseconds of the next micro-batch
         # Micro-batches of at most this many tokens multiply the block-quantised weights as they are (csrc/qgemm_tcgen05.cu)
@@ -135,7 +135,7 @@ class GemmPrefill:
         # by HBM traffic, the products by the tensor cores, so the two overlap.  Two sets of bf16 buffers alternate.
         direct = fine or self._direct(T)
         blocks = direct or self._expert_blocks(T)           # the routed experts' weights are multiplied as they are
-        resident = not direct and self._use_resident()
+        resident = not direct and self._use_resident(experts=not blocks)
         ahead = self.expert_source is None and self.expand_ahead and not resident and not direct
         nset = 2 if ahead else 1
         wqkv_s = [None if direct else self._get(f"wqkv{i}", (qkv_w, H), bf) for i in range(nset)]
@@ -424,23 +424,29 @@ class GemmPrefill:
             self._block_limit = min((self.block_rows.get(t, 0) for t in kinds), default=0) if self._blocks_ok() else 0
         return T * s.n_used <= self._block_limit * s.n_expert
 
-    def _use_resident(self) -> bool:
-        """Whether the layers' bf16 copies stay in HBM between prompts (decided once, before the first copy exists)."""
+    def _use_resident(self, experts: bool = False) -> bool:
+        """Whether the layers' bf16 copies stay in HBM between prompts; ``experts``: whether those of the routed experts do, which
+        the first prompt that needs them makes.  Each is decided once, by the memory that is free right before its first copy."""
         if self.expert_source is not None or self.resident_bf16 is False:
             return False
         if any(q.qtype == "BF16" and q.data.dim() == 3 for q in self.e.w.q.values()):     # bf16 stacks: a copy would only double them
             return False
+        s = self.e.spec
+        of_experts = 2 * 3 * s.n_expert * s.moe_inter * s.hidden * s.n_layer if s.is_moe else 0
         if self._resident_ok is None:
-            if self.resident_bf16:
-                self._resident_ok = True
-            else:
-                s = self.e.spec
-                per_layer = (s.q_rows + 2 * s.kv_rows) * s.hidden + s.hidden * s.q_rows
-                per_layer += 3 * s.n_expert * s.moe_inter * s.hidden if s.is_moe else 3 * (s.dense_inter or 0) * s.hidden
-                need = 2 * per_layer * s.n_layer
-                free, total = torch.cuda.mem_get_info(self.e.device)
-                self._resident_ok = free - need >= total // 4
-        return self._resident_ok
+            per_layer = (s.q_rows + 2 * s.kv_rows) * s.hidden + s.hidden * s.q_rows
+            per_layer += 0 if s.is_moe else 3 * (s.dense_inter or 0) * s.hidden
+            self._resident_ok = bool(self.resident_bf16) or self._room_for(2 * per_layer * s.n_layer + of_experts)
+        if not experts or not of_experts or not self._resident_ok:
+            return self._resident_ok
+        if self._resident_experts_ok is None:
+            self._resident_experts_ok = bool(self.resident_bf16) or self._room_for(of_experts)
+        return self._resident_experts_ok
+
+    def _room_for(self, need: int) -> bool:
+        """Whether ``need`` more bytes leave a quarter of the card free."""
+        free, total = torch.cuda.mem_get_info(self.e.device)
+        return free - need >= total // 4
 
     def _attn_tables(self, T: int, Tq: int, c0: int, n_q: int, Gq: int, pos0: int = 0):
         key = ("attn", T, Tq, c0, n_q, pos0)

@@ -235,6 +235,27 @@ def test_experts_over_blocks_beside_bf16_projections_agree_with_the_copies(n, ke
     assert float((out[0] - out[1]).norm() / out[1].norm()) < 2e-2
 
 
+def test_prompts_run_where_only_the_projections_copies_found_room():
+    """A prompt over the experts' blocks that keeps the projections' copies, then one that needs the experts' and is refused them: the
+    bits of prompts that keep nothing."""
+    from bloomery_b200.models.spec import tiny_qwen3moe
+    from bloomery_b200.models.weights import Weights, synth_tensors
+    from bloomery_b200.runtime.engine import DecodeEngine
+    spec = tiny_qwen3moe()
+    w = Weights.from_items(spec, synth_tensors(spec, "cpu", seed=0), "cpu").to(DEV)
+    ids = torch.randint(0, spec.vocab, (600,), generator=torch.Generator().manual_seed(7)).tolist()
+    out = []
+    for room in (True, False):
+        eng = DecodeEngine(w, n_slots=2, slot_ctx=768)
+        pre = eng._gemm_prefill = eng._new_gemm_prefill()
+        pre._resident_ok, pre._resident_experts_ok = room, False
+        for slot, n in ((0, 140), (1, 600), (0, 200)):
+            eng.prefill(slot, ids[:n], gemm=True)
+            out.append(eng.logits[0].clone())
+        assert ("wqkv" in pre._resident.get(0, {})) == room and "wg" not in pre._resident.get(0, {})
+    assert all(torch.equal(a, b) for a, b in zip(out[:3], out[3:]))
+
+
 @pytest.mark.parametrize("n", [32, 33, 63])
 @pytest.mark.parametrize("mix", ["Q4_K_M", "NVFP4"])
 def test_prompts_below_the_gemm_threshold_round_activations_and_nothing_else(n, mix):

@@ -670,6 +670,37 @@ def test_kept_bf16_copies_serve_all_but_the_prompts_below_the_gemm_threshold():
     assert not pre._direct(40, short=True)                       # experts streamed from the host: no stack to multiply
 
 
+def test_room_for_the_experts_copies_is_looked_for_when_they_are_made(monkeypatch):
+    """Short prompts keep the projections' copies only; by the first one that needs the experts', the memory may be gone."""
+    from types import SimpleNamespace as NS
+    from bloomery_b200.runtime.prefill import GemmPrefill
+    spec = NS(is_moe=True, n_layer=4, n_expert=8, moe_inter=256, hidden=512, q_rows=512, kv_rows=128, dense_inter=0)
+    experts, rest = 2 * 3 * 8 * 256 * 512 * 4, 2 * (512 + 256 + 512) * 512 * 4
+    total = 100 * experts
+    free = [0]
+    monkeypatch.setattr("torch.cuda.mem_get_info", lambda dev=None: (free[0], total))
+
+    def prefill(resident=None):
+        pre = object.__new__(GemmPrefill)
+        vars(pre).update(e=NS(spec=spec, device="cpu", w=NS(q={})), expert_source=None, resident_bf16=resident,
+                         _resident_ok=None, _resident_experts_ok=None)
+        return pre
+    free[0] = total // 4 + experts + rest
+    pre = prefill()
+    assert pre._use_resident()
+    free[0] = total // 4 + experts - 1                       # another pool took some of it in between
+    assert not pre._use_resident(experts=True) and pre._use_resident()
+    free[0] = total
+    assert not pre._use_resident(experts=True)               # decided once
+    free[0] = total // 4 + experts + rest
+    pre = prefill()
+    assert pre._use_resident(experts=True) and pre._use_resident()
+    free[0] = total // 4 + experts + rest - 1
+    pre = prefill()
+    assert not pre._use_resident() and not pre._use_resident(experts=True)
+    assert prefill(True)._use_resident(experts=True) and not prefill(False)._use_resident(experts=True)
+
+
 def test_experts_take_their_blocks_up_to_some_rows_an_expert():
     """Gate and up decide; a type without a limit, streamed experts and ``direct_rows`` 0 leave the experts to the copies."""
     from types import SimpleNamespace as NS
