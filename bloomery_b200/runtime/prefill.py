@@ -156,11 +156,12 @@ class GemmPrefill:
                 self._work = G.QgemmWork(dev, 128)
         else:
             dense_tiles = G.TileTable.dense(T, dev, host=True)
-            pair_tiles = G.TileTable.dense(T, dev, G.PAIR_ROWS, host=True)
+            on_pairs = {n for n in (qkv_w, H) if G.pairs_pay(T, n)}       # widths of the projections that go to pairs of CTAs
+            pair_tiles = G.TileTable.dense(T, dev, G.PAIR_ROWS, host=True) if on_pairs else None
 
         def project(X, W, **out):
             """A dense product over a bf16 copy."""
-            if G.pairs_pay(T, W.shape[0]):
+            if W.shape[0] in on_pairs:
                 G.gemm_pair(X, W, pair_tiles, status=self.status, **out)
             else:
                 G.gemm_bf16(X, W, dense_tiles, status=self.status, **out)

@@ -235,6 +235,26 @@ def test_experts_over_blocks_beside_bf16_projections_agree_with_the_copies(n, ke
     assert float((out[0] - out[1]).norm() / out[1].norm()) < 2e-2
 
 
+@pytest.mark.parametrize("rows", [1 << 30, 200, 1])
+def test_a_prompt_has_a_table_for_pairs_where_a_projection_goes_to_them(monkeypatch, rows):
+    """The 256-row table is written by the host, two blocking copies in front of the first layer: prompts below the products that
+    pairs pay for do without it."""
+    from bloomery_b200.models.spec import tiny_qwen3moe
+    from bloomery_b200.models.weights import Weights, synth_tensors
+    from bloomery_b200.ops import gemm as G
+    from bloomery_b200.runtime.engine import DecodeEngine
+    spec = tiny_qwen3moe()
+    w = Weights.from_items(spec, synth_tensors(spec, "cpu", seed=0), "cpu").to(DEV)
+    made, dense = [], G.TileTable.dense
+    monkeypatch.setattr(G.TileTable, "dense", lambda n, dev, tile_rows=128, host=False: made.append(tile_rows) or dense(n, dev, tile_rows, host))
+    monkeypatch.setattr(G, "pairs_pay", lambda n, width: n >= rows)
+    eng = DecodeEngine(w, n_slots=1, slot_ctx=512)
+    for n in (140, 300):
+        made.clear()
+        eng.prefill(0, list(range(n)), gemm=True)
+        assert (G.PAIR_ROWS in made) == (n >= rows), (n, rows, made)
+
+
 def test_prompts_run_where_only_the_projections_copies_found_room():
     """A prompt over the experts' blocks that keeps the projections' copies, then one that needs the experts' and is refused them: the
     bits of prompts that keep nothing."""
