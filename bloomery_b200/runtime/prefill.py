@@ -73,11 +73,17 @@ class GemmPrefill:
         # (0: no micro-batch multiplies blocks.)
         self.direct_rows = 128
         # Experts alone take their blocks further, copies or not, up to this many rows an expert on average: the products are then
-        # bound by what they read, and the blocks are a quarter of the copies, or half.  Types whose expander keeps up with
-        # that; NVFP4 (231 against 221 at 256 ids) and Q8_0 (242) do not.  Gate+up and down of the 30 B shape, us a layer, copies
-        # / Q4_K / Q6_K / FP8: 160 ids 220 / 159 / 174 / 180, 384 ids 224 / 170 / 195 / 201, 700 ids 230 / 178 / 202 / 208, 1,000
-        # ids 237 / 226 / 258 / 263.
-        self.block_rows = {"Q4_K": 64, "Q5_K": 48, "Q6_K": 52, "FP8_B128": 52}
+        # bound by what they read, and the blocks are a quarter of the copies, or half.  Types of gate and up whose expander
+        # keeps up with that; NVFP4 and Q8_0 do not.  Gate+up and down of the 30 B shape, us a layer:
+        #            copies     Q4_K       Q5_K       Q6_K       FP8        Q8_0       NVFP4
+        #   160 ids  154 + 66   109 + 57   122 + 61   128 + 61   129 + 65   177 + 76   151 + 83
+        #   700      157 + 73   117 + 61   130 + 65   136 + 66   136 + 71   185 + 79   158 + 87
+        #   832      159 + 75   117 + 65   131 + 70   136 + 69   136 + 75   186 + 83   158 + 92
+        #   1,000    159 + 77   149 + 83   168 + 90   174 + 89   173 + 93   235 + 104  201 + 116
+        # (whole prompts in Q4_K_M, blocks / copies: 900 ids 20.3 / 21.3 ms, 960 21.2 / 21.5, 1,000 22.3 / 21.6).  A down stack of any
+        # type costs less than gate and up save up to 52 rows an expert, beyond them only one that is in the table.
+        self.block_rows = {"Q4_K": 60, "Q5_K": 52, "Q6_K": 52, "FP8_B128": 52}
+        self.block_rows_any_down = 52
         # From this many rows an expert on, products over the copies go to pairs of CTAs with 256-row tiles (gate+up and down, us a
         # layer, pairs / single CTAs: 1,000 ids 240 / 236, 2,048 ids 270 / 285, 4,096 ids 390 / 410).
         self.pair_rows = 128
@@ -420,9 +426,12 @@ class GemmPrefill:
         if not s.is_moe or self.expert_source is not None or not self.direct_rows:
             return False
         if self._block_limit is None:
-            kinds = {self.e.w.q[f"blk.{il}.ffn_{n}_exps.weight"].qtype for il in range(s.n_layer) if s.layer_is_moe(il)
-                     for n in ("gate", "up")}               # gate+up are two thirds of the products
-            self._block_limit = min((self.block_rows.get(t, 0) for t in kinds), default=0) if self._blocks_ok() else 0
+            kinds = {n: {self.e.w.q[f"blk.{il}.ffn_{n}_exps.weight"].qtype for il in range(s.n_layer) if s.layer_is_moe(il)}
+                     for n in ("gate", "up", "down")}
+            limits = [self.block_rows.get(t, 0) for t in kinds["gate"] | kinds["up"]]
+            if not all(t in self.block_rows for t in kinds["down"]):
+                limits.append(self.block_rows_any_down)
+            self._block_limit = min(limits, default=0) if self._blocks_ok() else 0
         return T * s.n_used <= self._block_limit * s.n_expert
 
     def _use_resident(self, experts: bool = False) -> bool:

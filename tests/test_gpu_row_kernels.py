@@ -226,7 +226,7 @@ def test_experts_over_blocks_beside_bf16_projections_agree_with_the_copies(n, ke
         eng = DecodeEngine(w, n_slots=2, slot_ctx=768)
         pre = eng._gemm_prefill = eng._new_gemm_prefill()
         pre.direct_rows, pre.resident_bf16 = rows, kept
-        pre.pair_rows = 128 if rows else 1 << 20
+        pre.pair_rows, pre.block_rows = 128 if rows else 1 << 20, dict.fromkeys(pre.block_rows, 64)
         assert pre._expert_blocks(n) == (rows > 0 and n <= 256)
         eng.prefill(1, ids[:140], gemm=True)
         eng.prefill(0, ids, gemm=True)
