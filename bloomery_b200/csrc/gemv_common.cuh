@@ -121,9 +121,11 @@ __device__ __forceinline__ void copy_q8_row(const int8_t* xq, const float2* xds,
   cp_async_commit();
 }
 
-// Sum of eight squares, rounded the same way in every kernel that takes a row's.
+// Sum of eight squares, rounded the same way in every kernel of a family (FLOATW: with float rows among the weights) that takes a
+// row's.  The families round another one of the first two squares by itself.
+template <bool FLOATW>
 __device__ __forceinline__ float sum_sq8(const float4& a, const float4& b) {
-  float s = fma_rn(a.x, a.x, mul_rn(a.y, a.y));
+  float s = FLOATW ? fma_rn(a.x, a.x, mul_rn(a.y, a.y)) : fma_rn(a.y, a.y, mul_rn(a.x, a.x));
   s = fma_rn(a.z, a.z, s); s = fma_rn(a.w, a.w, s);
   s = fma_rn(b.x, b.x, s); s = fma_rn(b.y, b.y, s); s = fma_rn(b.z, b.z, s);
   return fma_rn(b.w, b.w, s);
@@ -164,7 +166,7 @@ __device__ __forceinline__ void prologue_norm(const GemvArgs& a, int8_t* sq, flo
       }
       float4 g0 = __ldg(reinterpret_cast<const float4*>(a.gain + i0)), g1 = __ldg(reinterpret_cast<const float4*>(a.gain + i0 + 4));
       float v[8] = {x0.x * g0.x, x0.y * g0.y, x0.z * g0.z, x0.w * g0.w, x1.x * g1.x, x1.y * g1.y, x1.z * g1.z, x1.w * g1.w};
-      ss += sum_sq8(x0, x1);
+      ss += sum_sq8<FLOATW>(x0, x1);
       float amax = 0.f;
 #pragma unroll
       for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
@@ -241,7 +243,7 @@ __device__ __forceinline__ void prologue_norm_rows(const GemvArgs& a, unsigned l
       const float4 x0 = *reinterpret_cast<const float4*>(x + i0), x1 = *reinterpret_cast<const float4*>(x + i0 + 4);
       const float4 g0 = __ldg(reinterpret_cast<const float4*>(a.gain + i0)), g1 = __ldg(reinterpret_cast<const float4*>(a.gain + i0 + 4));
       const float v[8] = {x0.x * g0.x, x0.y * g0.y, x0.z * g0.z, x0.w * g0.w, x1.x * g1.x, x1.y * g1.y, x1.z * g1.z, x1.w * g1.w};
-      ss += sum_sq8(x0, x1);
+      ss += sum_sq8<FLOATW>(x0, x1);
       float amax = 0.f;
 #pragma unroll
       for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));

@@ -82,6 +82,45 @@ def test_gemv_rows_of_a_pass_equal_single_rows(t, Kd, rows):
             assert torch.equal(out[live], one_r[live])
 
 
+def _fma32(a, b, c):
+    """fp32 a * b + c with one rounding: the product and nearly every sum fit the 64 bits of an x87 number."""
+    import numpy as np
+    return (a.astype(np.longdouble) * b.astype(np.longdouble) + np.asarray(c, np.float32).astype(np.longdouble)).astype(np.float32)
+
+
+@pytest.mark.parametrize("t", ["Q8_0", "F32"])
+@pytest.mark.parametrize("M", [1, 8])
+def test_gemv_norm_sums_squares_in_its_stated_order(t, M):
+    """The factor of the norm, read off a row with one weight, is that of eight squares a thread added up as written in the
+    kernel: one product rounded (the second with float rows, else the first), the others joined to the additions."""
+    import numpy as np
+    from bloomery_b200.ops import decode as K
+    Kd, n = 2048, 2000
+    g = torch.Generator().manual_seed(5)
+    x = torch.randn(n, Kd, generator=g)
+    w = torch.zeros(1, Kd)
+    w[0, 0] = 127 / 128
+    qw = K.QWeight(w.to(DEV).view(torch.uint8), t, Kd) if t == "F32" else _qw(w, t)[0]
+    gain = torch.ones(Kd, device=DEV)
+    xd, out = x.to(DEV), torch.zeros(n, 1, device=DEV)
+    for i in range(0, n, M):
+        K.gemv([qw], M, out[i:i + M], x=xd[i:i + M], gain=gain, eps=1e-6)
+    v = x.numpy().reshape(n, Kd // 8, 8)
+    one, two = (0, 1) if t == "F32" else (1, 0)
+    ss = _fma32(v[..., one], v[..., one], v[..., two] * v[..., two])
+    for j in range(2, 8):
+        ss = _fma32(v[..., j], v[..., j], ss)
+    s = np.float32(1) / np.sqrt((ss.astype(np.float64).sum(1) / Kd).astype(np.float32) + np.float32(1e-6))
+    if t == "F32":
+        acc = x[:, 0].numpy() * np.float32(127 / 128)
+    else:
+        c, ds = Q.quantize_act_q8(x)
+        acc = (np.float32(1 / 128) * ds[:, 0, 0].numpy()) * (127 * c[:, 0].int()).float().numpy()
+    want = acc * s
+    # the sum over the threads is in fp64 in another order, which can turn a rounding once in some 1e8 rows
+    assert np.array_equal(out[:, 0].cpu().numpy(), want), (out[:, 0].cpu().numpy() != want).sum()
+
+
 @pytest.mark.parametrize("t", ["Q4_K", "Q6_K", "NVFP4", "F32"])
 @pytest.mark.parametrize("Kd,rows", [(256, 40), (2048, 5123), (4096, 301)])
 def test_gemv_behind_a_reduction_equals_the_rows_it_adds_up(t, Kd, rows):
