@@ -51,8 +51,8 @@ __device__ __forceinline__ void rows_staged(const GemvArgs& a, const uint8_t* sw
       for (int m = 0; m < MB; ++m) {
         ActRegs act;
         StagedAct<T>::load(sq + (long)m * K, sds + (long)m * (K / 32), u, nunits, act);
-        acc0[m] += ActOf<T>::dot(g0, u, act);
-        if constexpr (kPair) acc1[m] += ActOf<T>::dot(g1, u, act);
+        acc0[m] = ActOf<T>::dot(g0, u, act, acc0[m]);
+        if constexpr (kPair) acc1[m] = ActOf<T>::dot(g1, u, act, acc1[m]);
       }
     }
 #pragma unroll
@@ -1338,7 +1338,7 @@ __device__ __forceinline__ float down_row_staged(const DownStagedArgs& a, const 
         ActRegs act;
         const long ab = (long)j * a.I;
         StagedAct<T>::load(sact + ab, sads + ab / 32, u, upe, act);
-        const float v = ActOf<T>::dot(regs, u, act);
+        const float v = ActOf<T>::dot(regs, u, act, 0.f);
 #pragma unroll
         for (int q = 0; q < kMaxTopK; ++q) if (q == j) part[q] += v;
       }

@@ -46,7 +46,7 @@ __device__ __forceinline__ void rows_q(const GemvArgs& a, const GemvSeg& s, int 
             StagedAct<T>::load(sq + (long)m * K, sds + (long)m * (K / 32), u, nunits, act);
 #pragma unroll
             for (int r = 0; r < R; ++r)
-              if (!PLANE_ROW || r0 + r < r_hi) acc[r][m] += ActOf<T>::dot(regs[r][c], u, act);
+              if (!PLANE_ROW || r0 + r < r_hi) acc[r][m] = ActOf<T>::dot(regs[r][c], u, act, acc[r][m]);
           }
         }
       }
@@ -142,7 +142,7 @@ __device__ __forceinline__ void rows_multi(const GemvArgs& a, const GemvSeg& s, 
             ActRegs act;
             StagedAct<T>::load(sq + (long)ms[i] * K, sds + (long)ms[i] * (K / 32), u, nunits, act);
 #pragma unroll
-            for (int r = 0; r < R; ++r) acc[i][r] += ActOf<T>::dot(regs[r][c], u, act);
+            for (int r = 0; r < R; ++r) acc[i][r] = ActOf<T>::dot(regs[r][c], u, act, acc[i][r]);
           }
         }
       }

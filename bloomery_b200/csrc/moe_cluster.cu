@@ -89,7 +89,7 @@ __device__ __forceinline__ void down_rows_cluster(const uint8_t* sw, long rb, in
         U::loadu(sw + (long)r * rb, hl, I, regs);
         ActRegs act;
         StagedAct<T>::load(actq, ads, hl, upe, act);
-        acc = ActOf<T>::dot(regs, hl, act);
+        acc = ActOf<T>::dot(regs, hl, act, 0.f);
       }
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
@@ -103,7 +103,7 @@ __device__ __forceinline__ void down_rows_cluster(const uint8_t* sw, long rb, in
         U::loadu(sw + (long)r * rb, u, I, regs);
         ActRegs act;
         StagedAct<T>::load(actq, ads, u, upe, act);
-        acc += ActOf<T>::dot(regs, u, act);
+        acc = ActOf<T>::dot(regs, u, act, acc);
       }
       acc = warp_sum(acc);
       if (lane == 0) s_p[r] = acc;

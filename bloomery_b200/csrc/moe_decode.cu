@@ -318,7 +318,7 @@ __device__ __forceinline__ void gate_up_rows(const uint8_t* g0, const uint8_t* u
     ActRegs act;
     StagedAct<T>::load(sq, sds, u, nunits, act);
 #pragma unroll
-    for (int r = 0; r < R; ++r) { gacc[r] += ActOf<T>::dot(rg[r], u, act); uacc[r] += ActOf<T>::dot(ru[r], u, act); }
+    for (int r = 0; r < R; ++r) { gacc[r] = ActOf<T>::dot(rg[r], u, act, gacc[r]); uacc[r] = ActOf<T>::dot(ru[r], u, act, uacc[r]); }
   }
   g = warp_sum4(gacc[0], gacc[R - 1], uacc[0], uacc[R - 1]);
   u_sum = __shfl_down_sync(0xffffffffu, g, 16);
@@ -520,7 +520,7 @@ __device__ __forceinline__ float down_row(const DownArgs& a, int d, int lane, co
     if (use[c]) {
       ActRegs act;
       StagedAct<T>::load(sq, sds, lane + 32 * c, total, act);
-      part += ActOf<T>::dot(regs[c], unit[c], act);
+      part += ActOf<T>::dot(regs[c], unit[c], act, 0.f);
       if (c + 1 == UPL || lane + 32 * (c + 1) >= total || slot[c + 1 < UPL ? c + 1 : c] != slot[c]) { y = fmaf(w, part, y); part = 0.f; }
     }
   }

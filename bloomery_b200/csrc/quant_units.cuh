@@ -547,7 +547,7 @@ struct Q3K {
     r.sc = ld32(p + 96 + 8 * n + 4 * jp);
     r.d = ld32(p + 112) & 0xFFFF;
   }
-  static BL_HD float dot(const Regs& r, int u, const ActUnit& a) {
+  static BL_HD float dot(const Regs& r, int u, const ActUnit& a, float add = 0.f) {
     const int n = (u >> 1) & 1, jp = u & 1;
     float acc = 0.f;
 #pragma unroll
@@ -566,7 +566,7 @@ struct Q3K {
       const int sc = (int)(int8_t)((r.sc >> (8 * g)) & 0xFF);
       acc = fma_rn((g >> 1) ? a.d1 : a.d0, (float)(sc * (s + 4 * sh - 4 * sx)), acc);
     }
-    return mul_rn(half_bits_to_float((uint16_t)r.d), acc);
+    return fma_rn(half_bits_to_float((uint16_t)r.d), acc, add);
   }
   static BL_HD void decode(const Regs& r, int u, float* out) {
     const int n = (u >> 1) & 1, jp = u & 1;
@@ -785,7 +785,7 @@ struct Fp8B128 {
     return (float)(int8_t)((w >> (8 * b)) & 0xFF);
 #endif
   }
-  static BL_HD float dot(const Regs& r, const uint32_t* aq, const float* ad) {
+  static BL_HD float dot(const Regs& r, const uint32_t* aq, const float* ad, float add = 0.f) {
     float acc0 = 0.f, acc1 = 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -802,7 +802,7 @@ struct Fp8B128 {
         }
       }
     }
-    return mul_rn(r.sc, fma_rn(ad[0], acc0, mul_rn(ad[1], acc1)));
+    return fma_rn(r.sc, fma_rn(ad[0], acc0, mul_rn(ad[1], acc1)), add);
   }
   static BL_HD void decode(const Regs& r, float* out) {
 #pragma unroll
@@ -935,7 +935,9 @@ template <> struct Unit<Fp8B128> {
 // ---------------------------------------------------------------------------------
 // Activation registers of one unit: 16 code words and up to four {d, s} pairs, fetched
 // once (from shared or global memory) and reused against several weight rows.
-//   ActOf<T>::load(xq_row_words, xds_row, u, regs);  ActOf<T>::dot(wregs, u, regs)
+//   ActOf<T>::load(xq_row_words, xds_row, u, regs);  ActOf<T>::dot(wregs, u, regs, sum)
+// dot adds the unit's products to `sum`; a type whose last step is a product with a scale joins that to the addition (Q3_K, Q6_K,
+// FP8), which saves a rounding where a lane has several units of a row.
 // ---------------------------------------------------------------------------------
 struct ActRegs { uint32_t q[16]; float d[4]; float s[4]; };
 
@@ -955,11 +957,12 @@ template <class T> struct ActOf {
     for (int i = 0; i < 4; ++i) ld_act128(xq + 16 * u + 4 * i, a.q + 4 * i);
     a.d[0] = xds[2 * u].x; a.s[0] = xds[2 * u].y; a.d[1] = xds[2 * u + 1].x; a.s[1] = xds[2 * u + 1].y;
   }
-  static BL_HD float dot(const typename Unit<T>::Regs& r, int u, const ActRegs& a) {
+  static BL_HD float dot(const typename Unit<T>::Regs& r, int u, const ActRegs& a, float sum) {
     ActUnit au{a.q, a.d[0], a.s[0], a.d[1], a.s[1]};
-    if constexpr (T::kType == WT_Q8_0 || T::kType == WT_Q8_F32 || T::kType == WT_Q4_0 || T::kType == WT_Q4_1 || T::kType == WT_Q5_0 ||
-                  T::kType == WT_Q5_1) return T::dot(r, au);
-    else return T::dot(r, u, au);
+    if constexpr (T::kType == WT_Q3_K) return T::dot(r, u, au, sum);
+    else if constexpr (T::kType == WT_Q8_0 || T::kType == WT_Q8_F32 || T::kType == WT_Q4_0 || T::kType == WT_Q4_1 || T::kType == WT_Q5_0 ||
+                  T::kType == WT_Q5_1) return sum + T::dot(r, au);
+    else return sum + T::dot(r, u, au);
   }
 };
 
@@ -972,7 +975,7 @@ template <> struct ActOf<Q6K> {
       a.d[g] = xds[8 * sb + 4 * n + g].x;
     }
   }
-  static BL_HD float dot(const Q6K::Regs& r, int u, const ActRegs& a) {
+  static BL_HD float dot(const Q6K::Regs& r, int u, const ActRegs& a, float sum) {
     const int n = (u >> 1) & 1, h = u & 1;
     uint32_t c[4][4];
     Q6K::codes(r, c);
@@ -988,7 +991,7 @@ template <> struct ActOf<Q6K> {
       s -= 32 * sx;                       // 128 * 16 * 63 * 127 < 2^24: the product with the scale is exact
       acc = fma_rn(a.d[g], mul_rn(sum_float(kSum0 + Q6K::scale(r, 8 * n + 2 * g + h)), sum_float(s)), acc);
     }
-    return mul_rn(half_bits_to_float((uint16_t)r.d), acc);
+    return fma_rn(half_bits_to_float((uint16_t)r.d), acc, sum);
   }
 };
 
@@ -998,7 +1001,7 @@ template <> struct ActOf<NvFp4> {
     for (int i = 0; i < 4; ++i) ld_act128(xq + 16 * u + 4 * i, a.q + 4 * i);
     a.d[0] = xds[2 * u].x; a.d[1] = xds[2 * u + 1].x;
   }
-  static BL_HD float dot(const NvFp4::Regs& r, int, const ActRegs& a) { return NvFp4::dot(r, a.q, a.d); }
+  static BL_HD float dot(const NvFp4::Regs& r, int, const ActRegs& a, float sum) { return sum + NvFp4::dot(r, a.q, a.d); }
 };
 template <> struct ActOf<Fp8B128> {
   static BL_HD void load(const uint32_t* xq, const F2* xds, int u, ActRegs& a) {
@@ -1006,7 +1009,7 @@ template <> struct ActOf<Fp8B128> {
     for (int i = 0; i < 4; ++i) ld_act128(xq + 16 * u + 4 * i, a.q + 4 * i);
     a.d[0] = xds[2 * u].x; a.d[1] = xds[2 * u + 1].x;
   }
-  static BL_HD float dot(const Fp8B128::Regs& r, int, const ActRegs& a) { return Fp8B128::dot(r, a.q, a.d); }
+  static BL_HD float dot(const Fp8B128::Regs& r, int, const ActRegs& a, float sum) { return Fp8B128::dot(r, a.q, a.d, sum); }
 };
 
 // Resident row size for a weight type and row length.

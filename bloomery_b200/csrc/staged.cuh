@@ -74,7 +74,7 @@ __device__ __forceinline__ void gate_up_rows_staged(const uint8_t* g0, const uin
     ActRegs act;
     StagedAct<T>::load(xq, xds, u, nunits, act);
 #pragma unroll
-    for (int r = 0; r < 2; ++r) { gacc[r] += ActOf<T>::dot(rg[r], u, act); uacc[r] += ActOf<T>::dot(ru[r], u, act); }
+    for (int r = 0; r < 2; ++r) { gacc[r] = ActOf<T>::dot(rg[r], u, act, gacc[r]); uacc[r] = ActOf<T>::dot(ru[r], u, act, uacc[r]); }
   }
 #pragma unroll
   for (int r = 0; r < 2; ++r) { gacc[r] = warp_sum(gacc[r]); uacc[r] = warp_sum(uacc[r]); }

@@ -121,6 +121,33 @@ def test_gemv_norm_sums_squares_in_its_stated_order(t, M):
     assert np.array_equal(out[:, 0].cpu().numpy(), want), (out[:, 0].cpu().numpy() != want).sum()
 
 
+@pytest.mark.parametrize("M", [1, 3, 8])
+def test_gemv_joins_a_scale_to_the_sum_of_a_lanes_units(M):
+    """Two weights that one lane meets in its first and second unit, FP8: the second unit's product with its scale is not rounded
+    before it is added."""
+    import numpy as np
+    from bloomery_b200.ops import decode as K
+    Kd, n = 4096, 64
+    g = torch.Generator().manual_seed(6)
+    w = torch.zeros(n, Kd)
+    w[:, 0], w[:, 2048] = torch.rand(n, generator=g) + 0.1, -torch.rand(n, generator=g) - 0.1
+    qw, _ = _qw(w, "FP8_B128")
+    codes = torch.zeros(M, Kd, dtype=torch.int8)
+    codes[:, 0], codes[:, 2048] = torch.randint(1, 128, (2, M), generator=g).to(torch.int8)
+    d = torch.rand(M, Kd // 32, generator=g) * 0.01
+    ds = torch.stack([d, torch.zeros_like(d)], -1).contiguous()
+    out = torch.zeros(M, n, device=DEV)
+    K.gemv([qw], M, out, xq=codes.to(DEV), xds=ds.to(DEV))
+    row = qw.data.cpu()
+    scale = row[:, Kd:Kd + 4 * (Kd // 128)].contiguous().view(torch.float32).numpy()
+    value = row[:, :Kd].contiguous().view(torch.float8_e4m3fn).float().numpy()
+    want = np.zeros((M, n), np.float32)
+    for u in (0, 2048):
+        dots = (value[None, :, u] * codes[:, u, None].float().numpy()) * d[:, u // 32, None].numpy()
+        want = _fma32(np.broadcast_to(scale[None, :, u // 128], dots.shape), dots, want)
+    assert np.array_equal(out.cpu().numpy(), want)
+
+
 @pytest.mark.parametrize("t", ["Q4_K", "Q6_K", "NVFP4", "F32"])
 @pytest.mark.parametrize("Kd,rows", [(256, 40), (2048, 5123), (4096, 301)])
 def test_gemv_behind_a_reduction_equals_the_rows_it_adds_up(t, Kd, rows):
