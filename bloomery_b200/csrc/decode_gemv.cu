@@ -85,7 +85,8 @@ void bl_set_pdl(int on) { g_use_pdl = on ? 1 : 0; }
 
 // out[m, :] = (resid[m, :] +) W_seg * act(m), for up to four weight segments.
 //   norm != 0: act = q8(RMSNorm(x[m]) * gain); else act = (xq, xds) given.
-// row_seq (optional, M > 1): rows with a negative entry fill a bucket and nothing else; they need not be computed.
+// row_seq (optional, M > 1): rows with a negative entry fill a bucket and nothing else; they need not be computed.  Not with push_desc:
+// the ranks that add the pushed rows up wait for every one of them.
 // Returns 0, a negative contract code, or a positive cudaError_t.
 int bl_gemv(int nseg, const void* const* w, const int* rows, const int* wtypes, int K, int M,
             int norm, const float* x, long x_stride, const float* gain, float eps,
@@ -121,6 +122,7 @@ int bl_gemv(int nseg, const void* const* w, const int* rows, const int* wtypes, 
   a.out = out; a.out_stride = out_stride; a.resid = resid; a.resid_stride = resid_stride;
   a.fault = fault; a.layer = layer;
   if (red_desc) { BL_REQUIRE(norm && a.red.n_ranks <= kMaxRanks && a.red.H == K, BL_ERR_SHAPE); }
+  BL_REQUIRE(!(push_desc && row_seq), BL_ERR_SHAPE);
   if (push_desc) { a.push = *(const PushOut*)push_desc; BL_REQUIRE(a.push.n_ranks <= kMaxRanks, BL_ERR_SHAPE); }
   BL_REQUIRE(plan.smem <= 200 * 1024, BL_ERR_LIMIT);
   cudaError_t e;

@@ -126,7 +126,7 @@ def gemv(segs: Sequence[QWeight], M: int, out: torch.Tensor, *, x: Optional[torc
          row_seq: Optional[torch.Tensor] = None) -> None:
     """``prefetch``: up to six tensors a later launch will stream (the next layer's projections); the launch asks L2
     for them before it waits for its predecessor.  ``row_seq``: rows with a negative entry only fill the pass's bucket;
-    their results may be left out."""
+    their results may be left out; refused with ``push``, whose receivers wait for every row."""
     fams = [_family(sg.qtype) for sg in segs]
     if len(set(fams) - {1}) > 1 or (2 in fams and 1 in fams):
         # segments of different kernel families (e.g. a Q5_0 fallback tensor beside K-quants): one call per run

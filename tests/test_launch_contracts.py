@@ -122,3 +122,11 @@ def test_the_blocks_of_a_gemv_fit_a_processor_two_at_a_time():
             for M in range(1, 9):
                 for kw in (dict(), dict(norm=0), dict(reduce=1)):
                     assert 2 * (_gemv_plan(M, K, types=types, **kw)[4] + 1024) <= 227 * 1024, (types, K, M, kw)
+
+
+def test_rows_that_other_ranks_wait_for_are_not_left_out():
+    from bloomery_b200.ops.decode import PushOut
+    push = PushOut()
+    push.n_ranks = 2
+    assert cuda().bl_gemv(I(1), (P * 1)(A), (I * 1)(64), (I * 1)(WT_Q4_K), I(2048), I(4), I(0), P(0), L(0), P(0), F(1e-6), P(A), P(A),
+                          P(A), L(64), P(0), L(0), P(0), ctypes.byref(push), P(0), I(0), I(148), I(0), P(0), P(0), P(A), P(0)) == SHAPE
