@@ -5,7 +5,7 @@ CUDA events.
     python -m bloomery_b200.ops.kernel_bench NAME [replays] [context] [--no-staged] [--rows M]
 
 NAME: chain (the six launches of a layer in order) | qkv | attn | o | router | gateup | down | rope | flash |
-flash_mma | gemm | gemmdist | pflash | prope | mplan | qgu | qdown | qo | qq | bgu | bdown | mla | sampler | sampler_split | gap.  ``--no-staged`` runs the register-streaming kernels
+flash_mma | gemm | gemmpair | gemmdist | pflash | prope | mplan | qgu | qdown | qo | qq | bgu | bdown | pgu | pdown | mla | sampler | sampler_split | gap.  ``--no-staged`` runs the register-streaming kernels
 instead of the shared-memory staged ones; ``--form exact`` / ``--form fine`` picks how the weights of qgu / qdown are expanded.
 It is also the small workload the ncu summaries under ``profiles/``
 were captured on.
@@ -116,6 +116,12 @@ def main(argv=None) -> int:
         extra = dict(G=G, A=(torch.randn(4096, 2048, device=dev) * 0.1).bfloat16(), B=(torch.randn(5120, 2048, device=dev) * 0.1).bfloat16(),
                      C=torch.zeros(4096, 5120, device=dev, dtype=torch.bfloat16), tt=G.TileTable.dense(4096, dev),
                      gst=torch.zeros(1, dtype=torch.int32, device=dev))
+    if which == "gemmpair":
+        # QKV of `ctx` rows on pairs of CTAs
+        from bloomery_b200.ops import gemm as G
+        extra = dict(G=G, A=(torch.randn(ctx, H, device=dev) * 0.1).bfloat16(), B=(torch.randn(QR + 2 * n_kv * hd, H, device=dev) * 0.1).bfloat16(),
+                     C=torch.zeros(ctx, QR + 2 * n_kv * hd, device=dev), tt=G.TileTable.dense(ctx, dev, G.PAIR_ROWS, host=True),
+                     gst=torch.zeros(1, dtype=torch.int32, device=dev))
     if which == "pflash":
         # prompt flash attention of `ctx` tokens (32 query heads over 4 key/value heads of 128)
         from bloomery_b200.ops import gemm as G
@@ -135,14 +141,14 @@ def main(argv=None) -> int:
         extra = dict(G=G, mids=torch.stack([torch.randperm(E, device=dev)[:TOPK] for _ in range(ctx)]).to(torch.int32).contiguous(),
                      mwts=torch.rand(ctx, TOPK, device=dev), mtt=G.TileTable(n, E, dev), mpos_of=torch.zeros(n, dtype=torch.int32, device=dev),
                      mdst=torch.zeros(n + 128, dtype=torch.int32, device=dev), mscale=torch.zeros(n + 128, device=dev))
-    if which in ("qgu", "qdown", "bgu", "bdown", "fgu", "fdown"):
+    if which in ("qgu", "qdown", "bgu", "bdown", "fgu", "fdown", "pgu", "pdown"):
         # expert products of `ctx` tokens x 8 experts of 128: q* = quantised weights expanded inside the GEMM,
-        # b* = expansion launch + bf16 GEMM; --rows picks the token tile (32 or 128) of the q* forms
+        # b* = expansion launch + bf16 GEMM, p* = bf16 copies on pairs of CTAs; --rows picks the token tile (32, 64 or 128) of the q* forms
         from bloomery_b200.ops import gemm as G
         n = ctx * TOPK
-        tr = 32 if rows == 32 or which[0] == "f" else 128
+        tr = 32 if rows == 32 or which[0] == "f" else 64 if rows == 64 else 128
         mids = torch.stack([torch.randperm(E, device=dev)[:TOPK] for _ in range(ctx)]).to(torch.int32).contiguous()
-        tt = G.TileTable(n, E, dev, tr if which[0] in "qf" else 128)
+        tt = G.TileTable(n, E, dev, tr if which[0] in "qf" else G.PAIR_ROWS if which[0] == "p" else 128)
         dst = torch.zeros(n + 128, dtype=torch.int32, device=dev)
         scale = torch.zeros(n + 128, device=dev)
         G.moe_plan(mids, torch.rand(ctx, TOPK, device=dev), E, tt, torch.zeros(n, dtype=torch.int32, device=dev), dst, scale)
@@ -150,6 +156,9 @@ def main(argv=None) -> int:
                      xa=(torch.randn(n + 128, H, device=dev) * 0.3).bfloat16(), act=torch.zeros(n + 128, I, device=dev, dtype=torch.bfloat16),
                      so=torch.zeros(n, H, device=dev), wg=torch.zeros(E, I, H, device=dev, dtype=torch.bfloat16),
                      wu=torch.zeros(E, I, H, device=dev, dtype=torch.bfloat16), wd=torch.zeros(E, H, I, device=dev, dtype=torch.bfloat16))
+        if which[0] == "p":
+            for wb in ("wg", "wu", "wd"):
+                extra[wb].normal_(std=0.03)
         if which[0] == "f":
             extra.update(xa8=torch.randint(0, 120, (n + 128, H), dtype=torch.uint8, device=dev), xas=torch.rand(n + 128, H // 128, device=dev),
                          act8=torch.randint(0, 120, (n + 128, I), dtype=torch.uint8, device=dev), acts=torch.rand(n + 128, I // 128, device=dev))
@@ -246,6 +255,9 @@ def main(argv=None) -> int:
             if which == "qdown": X["G"].qgemm(X["act"], l["d"], X["tt"], out_f32=X["so"], dst_row=X["dst"], row_scale=X["scale"], status=X["gst"], **form)
             if which == "fgu": X["G"].fp8_gemm(X["xa8"], X["xas"], l["g"], X["tt"], out_bf16=X["act"], W2=l["u"], status=X["gst"])
             if which == "fdown": X["G"].fp8_gemm(X["act8"], X["acts"], l["d"], X["tt"], out_f32=X["so"], dst_row=X["dst"], row_scale=X["scale"], status=X["gst"])
+            if which == "gemmpair": X["G"].gemm_pair(X["A"], X["B"], X["tt"], out_f32=X["C"], status=X["gst"])
+            if which == "pgu": X["G"].gemm_pair(X["xa"], X["wg"], X["tt"], out_bf16=X["act"], W2=X["wu"], status=X["gst"])
+            if which == "pdown": X["G"].gemm_pair(X["act"], X["wd"], X["tt"], out_f32=X["so"], dst_row=X["dst"], row_scale=X["scale"], status=X["gst"])
             if which == "bgu":
                 X["G"].dequant_bf16(l["g"], X["wg"]); X["G"].dequant_bf16(l["u"], X["wu"])
                 X["G"].gemm_bf16(X["xa"], X["wg"], X["tt"], out_bf16=X["act"], B2=X["wu"], status=X["gst"])

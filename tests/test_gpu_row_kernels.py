@@ -212,8 +212,8 @@ def test_short_prompts_over_quantised_blocks_agree_with_the_bf16_copies(n, start
 @pytest.mark.parametrize("n", [129, 256, 257, 600])
 def test_experts_over_blocks_beside_bf16_projections_agree_with_the_copies(n, kept):
     """Prompts on either side of the last one whose experts take their blocks (16 experts, 4 of them a row, 64 rows each: 256),
-    with copies that are kept and without, and a longer prompt behind a shorter one, which completes the copies; 600 ids
-    are products of CTA pairs."""
+    with copies that are kept and without, and a longer prompt behind a shorter one, which completes the copies; the experts of
+    600 ids are products of CTA pairs."""
     from bloomery_b200.models.spec import tiny_qwen3moe
     from bloomery_b200.models.weights import Weights, synth_tensors
     from bloomery_b200.runtime.engine import DecodeEngine
@@ -253,6 +253,33 @@ def test_a_prompt_has_a_table_for_pairs_where_a_projection_goes_to_them(monkeypa
         made.clear()
         eng.prefill(0, list(range(n)), gemm=True)
         assert (G.PAIR_ROWS in made) == (n >= rows), (n, rows, made)
+
+
+@pytest.mark.parametrize("n", [257, 600])
+def test_projections_on_pairs_of_ctas_agree_with_single_ones(monkeypatch, n):
+    """QKV and the output projection, which adds to the residual rows in place, of a prompt of two and of three tiles of 256 rows."""
+    from bloomery_b200.models.spec import tiny_qwen3moe
+    from bloomery_b200.models.weights import Weights, synth_tensors
+    from bloomery_b200.ops import gemm as G
+    from bloomery_b200.runtime.engine import DecodeEngine
+    spec = tiny_qwen3moe()
+    w = Weights.from_items(spec, synth_tensors(spec, "cpu", seed=0), "cpu").to(DEV)
+    ids = torch.randint(0, spec.vocab, (n,), generator=torch.Generator().manual_seed(n)).tolist()
+    calls, pair = [], G.gemm_pair
+    monkeypatch.setattr(G, "gemm_pair", lambda X, W, tiles, **kw: calls.append((W.shape[0], kw.get("resid") is not None)) or pair(X, W, tiles, **kw))
+    out = []
+    for pays in (True, False):
+        monkeypatch.setattr(G, "pairs_pay", lambda rows, width: pays)
+        eng = DecodeEngine(w, n_slots=1, slot_ctx=768)
+        pre = eng._gemm_prefill = eng._new_gemm_prefill()
+        pre.pair_rows = 1 << 20                                  # experts on single CTAs in both
+        calls.clear()
+        eng.prefill(0, ids, gemm=True)
+        widths = [(spec.q_rows + 2 * spec.kv_rows, False), (spec.hidden, True)]
+        assert calls == (widths * spec.n_layer if pays else [])
+        out.append(eng.logits[0].double().cpu())
+    # the same bf16 operands, their fp32 sums in another order, four layers deep (as above)
+    assert float((out[0] - out[1]).norm() / out[1].norm()) < 2e-2
 
 
 def test_prompts_run_where_only_the_projections_copies_found_room():
