@@ -2,8 +2,10 @@
 //   C[t, n] = sum_k X[t, k] * W[g][n, k]        fp32 accumulate in tensor memory
 //
 // A CTA that multiplies 128 x 256 on its own fetches 48 KB for a 64-deep step of 512 tensor-core clocks, and 148 of them ask L2
-// for 12 TB/s, which is what bounds them (QKV of 4,096 ids, 2,048 x 5,120: 80 us, 1.07 PFLOP/s).  A pair shares one 256 x 256
-// product: each CTA fetches half of either operand, 32 KB a step, and the tensor cores of both read the other's half.
+// for 13 TB/s, which is what bounds them (QKV of 4,096 ids, 2,048 x 5,120: 77 us, 1.11 PFLOP/s).  A pair shares one 256 x 256
+// product: each CTA fetches half of either operand, 32 KB a step, and the tensor cores of both read the other's half (70.5 us,
+// 1.22 PFLOP/s; 671 MB from L2, 9.2 TB/s, tensor pipe 73 % busy).  What is left is the last wave: 320 tiles on at most 74 pairs are
+// 4.3 waves of five.
 //
 // The weights are the M side (256 rows of a pair, 128 of each CTA) and the tokens the N side, 64 to 256 of a tile, so a group of a
 // hundred rows pays for 128, not for 256, and a group's weights are read once.  The gated form (gate and up) gives each CTA 64 rows

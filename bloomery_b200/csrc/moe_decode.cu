@@ -331,8 +331,8 @@ __device__ __forceinline__ void gate_up_rows(const uint8_t* g0, const uint8_t* u
 // One row is a chain of latencies (logits, picks, weights, sums), so what can overlap does: the activations come in under the
 // picks, which one warp takes where route_pick serves, and the rows of later turns are asked into L2 while the first turn's
 // are in flight.  30 B shape, one row, us behind the launch in front: 9.3 (10.3 with activations from L2 and picks by the block), of
-// which 2 go to the picks, 3 to 5 to the first turn (1 of them to HBM), 1.5 to the second; what bounds the turns is the issue of
-// some 90 instructions a weight row and lane, two blocks on a third of the processors.  Several rows are bound by their blocks'
+// which 2 go to the picks, 3 to 5 to the first turn (1 of them to HBM), 1.5 to the second; its schedulers issue in 14 % of the
+// cycles, and a warp waits for loads and for the picks.  Several rows are bound by their blocks'
 // latencies in turns of the processors: five 30 us (36 before, 34 with R = 2).
 // FAM 0 = ggml integer-dot types, FAM 2 = block-scaled float planes (one kernel per family keeps
 // the plane decoders out of the K-quant bodies' register budget)
@@ -529,8 +529,8 @@ __device__ __forceinline__ float down_row(const DownArgs& a, int d, int lane, co
 
 // OCC = blocks a processor.  One row has 256 blocks for 148 processors and wants its registers; several rows queue for the
 // processors (five rows: 34 us with two, 29 with three, before the activations were staged; FP8 rows 36 us either way).
-// The launch in front asked L2 for the weights, so a row is bound by latencies and by the load unit: activations read from L2
-// sixteen bytes in every 64 took half of a warp's 380 wavefronts.  With them in shared memory, one request for a super-block's
+// The launch in front asked L2 for the weights, so a row is bound by latencies (its schedulers issue in 38 % of the cycles), of which
+// activations read from L2, sixteen bytes in every 64, were a large part.  With them in shared memory, one request for a super-block's
 // head and the residual asked for in front, one row takes 6.5 us a layer of the 30 B shape (9.0 before), five 23 (28).
 template <int UPL, int FAM, int OCC>
 __global__ void __launch_bounds__(256, OCC) down_combine_kernel(const DownArgs a) {

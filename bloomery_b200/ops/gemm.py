@@ -115,8 +115,8 @@ def gemm_pair(X: torch.Tensor, W: torch.Tensor, tiles: TileTable, *, out_f32: Op
 
 def pairs_pay(rows: int, N: int) -> bool:
     """Whether a dense product of ``rows`` by N columns goes to pairs: where their 256 x 256 tiles give most of them one (us, pairs
-    / single CTAs, or clusters of them where there are few tiles: 1,000 rows 2,048 deep by 5,120 30 / 32, 4,096 71 / 78; 4,096
-    deep by 2,048 1,000 rows 28 / 27, 2,000 31 / 33, 4,096 54 / 60)."""
+    / single CTAs, or clusters of them where there are few tiles: 2,048 deep by 5,120 1,000 rows 31 / 33, 2,000 43 / 47, 4,096 71 / 77;
+    4,096 deep by 2,048 1,000 rows 31 / 33, too few to matter, 2,000 33 / 37, 4,096 58 / 66)."""
     return -(-rows // PAIR_ROWS) * -(-N // 256) >= 3 * sm_count() // 8
 
 

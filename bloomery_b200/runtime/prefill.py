@@ -5,13 +5,14 @@ Counterpart of the reference's GEMM ubatches (``crates/gpu/src/arch/qwen3moe/uba
 per layer norm -> QKV GEMM -> norm/RoPE/append -> prefill flash -> o GEMM -> router logits +
 route -> grouped gate/up GEMM with SwiGLU -> grouped down GEMM -> combine).  Here:
 
-  * block-quantised weights of the layer are expanded to bf16 scratch right before use
-    (one expander kernel per matrix; the scratch is shared by all layers);
-  * every matmul is the persistent TMA + tcgen05 kernel; gate and up run in one main loop
-    with SwiGLU in the epilogue; the down GEMM's epilogue scatters router-weighted rows to
+  * short micro-batches multiply the quantised blocks as they are, the routed experts of longer ones too up to some rows an
+    expert (``direct_rows``, ``block_rows``); other products read bf16 copies of the weights, which are kept between prompts
+    where memory allows, else expanded a layer ahead on a side stream (one expander kernel per matrix);
+  * products over copies are persistent TMA + tcgen05 kernels, on single CTAs or pairs of them; gate and up run in one main
+    loop with SwiGLU in the epilogue; the down GEMM's epilogue scatters router-weighted rows to
     their (token, slot) cell and a fixed-order combine adds slots in ascending order;
-  * attention is three launches per query chunk: Q K^T (grouped over heads, KV head shared
-    by its query heads), causal softmax, P V (epilogue writes token-major rows).
+  * attention is one launch (``csrc/flash_tcgen05.cu``) for heads of 128; other head sizes take three per query chunk: Q K^T
+    (grouped over heads, KV head shared by its query heads), causal softmax, P V (epilogue writes token-major rows).
 
 Token bits are not equal to the 8-row pass path (bf16 operands, different sum order); a
 band test covers it, as the reference does (``ubatch.rs:19-30``).
@@ -85,7 +86,9 @@ class GemmPrefill:
         self.block_rows = {"Q4_K": 60, "Q5_K": 52, "Q6_K": 52, "FP8_B128": 52}
         self.block_rows_any_down = 52
         # From this many rows an expert on, products over the copies go to pairs of CTAs with 256-row tiles (gate+up and down, us a
-        # layer, pairs / single CTAs: 1,000 ids 240 / 236, 2,048 ids 270 / 285, 4,096 ids 390 / 410).
+        # layer, pairs / single CTAs: 1,000 ids 263 / 246, 2,048 ids 287 / 288, 4,096 ids 433 / 440; whole prompts with the projections on
+        # single CTAs in both, ms: 2,000 ids 27.6 / 27.6, 2,700 33.9 / 34.9, 4,096 47.0 / 47.5, and with them on pairs too 27.4,
+        # 33.5, 46.4).
         self.pair_rows = 128
         self._direct_ok = None
         self._block_limit = None
