@@ -31,6 +31,7 @@ from ..ops import gemm as G
 from .engine import GEMM_THRESHOLD
 from .kv import PAGE
 
+PROCESSORS = 148       # of a B200
 
 POISON = None          # None: follow the BLOOMERY_POISON lever; tests set True / False
 
@@ -82,7 +83,11 @@ class GemmPrefill:
         #   832      159 + 75   117 + 65   131 + 70   136 + 69   136 + 75   186 + 83   158 + 92
         #   1,000    159 + 77   149 + 83   168 + 90   174 + 89   173 + 93   235 + 104  201 + 116
         # (whole prompts in Q4_K_M, blocks / copies: 900 ids 20.3 / 21.3 ms, 960 21.2 / 21.5, 1,000 22.3 / 21.6).  A down stack of any
-        # type costs less than gate and up save up to 52 rows an expert, beyond them only one that is in the table.
+        # type costs less than gate and up save up to 52 rows an expert, beyond them only one that is in the table.  What ends
+        # the blocks' lead is a second 64-row tile of many experts, for which their weights are expanded again.  Where two tiles of every
+        # expert find a processor at once that takes no longer, so stacks that small go up to 64 rows in every type of the table
+        # (16 experts of 256 x 512, 256 ids, whole prompts, us, blocks / copies: Q4_K 1,565 / 1,671, kept copies 1,265 / 1,252; FP8 1,557 /
+        # 1,677 and 1,262 / 1,261).
         self.block_rows = {"Q4_K": 60, "Q5_K": 52, "Q6_K": 52, "FP8_B128": 52}
         self.block_rows_any_down = 52
         # From this many rows an expert on, products over the copies go to pairs of CTAs with 256-row tiles (gate+up and down, us a
@@ -429,12 +434,17 @@ class GemmPrefill:
         if not s.is_moe or self.expert_source is not None or not self.direct_rows:
             return False
         if self._block_limit is None:
-            kinds = {n: {self.e.w.q[f"blk.{il}.ffn_{n}_exps.weight"].qtype for il in range(s.n_layer) if s.layer_is_moe(il)}
+            q = self.e.w.q
+            kinds = {n: {q[k].qtype for k in (f"blk.{il}.ffn_{n}_exps.weight" for il in range(s.n_layer) if s.layer_is_moe(il)) if k in q}
                      for n in ("gate", "up", "down")}
             limits = [self.block_rows.get(t, 0) for t in kinds["gate"] | kinds["up"]]
-            if not all(t in self.block_rows for t in kinds["down"]):
+            listed = kinds["down"] <= self.block_rows.keys()
+            if not listed:
                 limits.append(self.block_rows_any_down)
             self._block_limit = min(limits, default=0) if self._blocks_ok() else 0
+            tiles = 2 * s.n_expert
+            if self._block_limit and listed and tiles <= PROCESSORS and tiles * -(-max(s.hidden, s.moe_inter) // 128) <= PROCESSORS:
+                self._block_limit = max(self._block_limit, 64)
         return T * s.n_used <= self._block_limit * s.n_expert
 
     def _use_resident(self, experts: bool = False) -> bool:

@@ -212,8 +212,8 @@ def test_short_prompts_over_quantised_blocks_agree_with_the_bf16_copies(n, start
 @pytest.mark.parametrize("n", [129, 256, 257, 600])
 def test_experts_over_blocks_beside_bf16_projections_agree_with_the_copies(n, kept):
     """Prompts on either side of the last one whose experts take their blocks (16 experts, 4 of them a row, 64 rows each: 256),
-    with copies that are kept and without, and a longer prompt behind a shorter one, which completes the copies; the experts of
-    600 ids are products of CTA pairs."""
+    with copies that are kept and without, and a longer prompt behind a shorter one, which completes the copies; 600 ids
+    are products of CTA pairs."""
     from bloomery_b200.models.spec import tiny_qwen3moe
     from bloomery_b200.models.weights import Weights, synth_tensors
     from bloomery_b200.runtime.engine import DecodeEngine
@@ -226,7 +226,7 @@ def test_experts_over_blocks_beside_bf16_projections_agree_with_the_copies(n, ke
         eng = DecodeEngine(w, n_slots=2, slot_ctx=768)
         pre = eng._gemm_prefill = eng._new_gemm_prefill()
         pre.direct_rows, pre.resident_bf16 = rows, kept
-        pre.pair_rows, pre.block_rows = 128 if rows else 1 << 20, dict.fromkeys(pre.block_rows, 64)
+        pre.pair_rows = 128 if rows else 1 << 20
         assert pre._expert_blocks(n) == (rows > 0 and n <= 256)
         eng.prefill(1, ids[:140], gemm=True)
         eng.prefill(0, ids, gemm=True)

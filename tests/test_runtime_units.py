@@ -702,25 +702,52 @@ def test_room_for_the_experts_copies_is_looked_for_when_they_are_made(monkeypatc
 
 
 def test_experts_take_their_blocks_up_to_some_rows_an_expert():
-    """Gate and up decide, and a down stack whose expander does not keep up; a type without a limit, streamed experts and
-    ``direct_rows`` 0 leave the experts to the copies."""
+    """Gate and up decide; a type without a limit, streamed experts and ``direct_rows`` 0 leave the experts to the copies."""
     from types import SimpleNamespace as NS
     from bloomery_b200.runtime.prefill import GemmPrefill
 
-    def limit(t, down=None, **kw):
+    def limit(t, **kw):
         pre = object.__new__(GemmPrefill)
         q = {f"blk.0.ffn_{n}_exps.weight": NS(qtype=t) for n in ("gate", "up")}
-        q["blk.0.ffn_down_exps.weight"] = NS(qtype=down or t)
         spec = NS(is_moe=True, n_layer=1, n_used=8, n_expert=128, layer_is_moe=lambda il: True)
         vars(pre).update({**dict(e=NS(spec=spec, w=NS(q=q)), direct_rows=128, expert_source=None, _block_limit=None,
-                                 block_rows={"Q4_K": 44, "FP8_B128": 32}, block_rows_any_down=36, _blocks_ok=lambda: True), **kw})
-        return [pre._expert_blocks(n) for n in (1, 512, 513, 576, 577, 704, 705)]
-    assert limit("Q4_K") == [True] * 6 + [False] and limit("FP8_B128") == [True] * 2 + [False] * 5
-    assert limit("Q4_K", "FP8_B128") == limit("Q4_K") and limit("Q4_K", "NVFP4") == [True] * 4 + [False] * 3
-    assert limit("FP8_B128", "Q8_0") == limit("FP8_B128")
+                                 block_rows={"Q4_K": 44, "FP8_B128": 32}, _blocks_ok=lambda: True), **kw})
+        return [pre._expert_blocks(n) for n in (1, 512, 513, 704, 705)]
+    assert limit("Q4_K") == [True] * 4 + [False] and limit("FP8_B128") == [True] * 2 + [False] * 3
     for kw in (dict(expert_source=object()), dict(direct_rows=0), dict(_blocks_ok=lambda: False)):
         assert not any(limit("Q4_K", **kw))
-    assert not any(limit("NVFP4")) and not any(limit("NVFP4", "Q4_K"))
+    assert not any(limit("NVFP4"))
+
+def test_a_down_stack_that_does_not_keep_up_ends_the_blocks_sooner():
+    """Gate and up have their limit; a down stack of a type without one is taken to a limit of its own, if that is the lower one."""
+    from types import SimpleNamespace as NS
+    from bloomery_b200.runtime.prefill import GemmPrefill
+
+    def limit(t, down):
+        pre = object.__new__(GemmPrefill)
+        q = {f"blk.0.ffn_{n}_exps.weight": NS(qtype=t) for n in ("gate", "up")}
+        q["blk.0.ffn_down_exps.weight"] = NS(qtype=down)
+        spec = NS(is_moe=True, n_layer=1, n_used=8, n_expert=128, layer_is_moe=lambda il: True)
+        vars(pre).update(e=NS(spec=spec, w=NS(q=q)), direct_rows=128, expert_source=None, _block_limit=None,
+                         block_rows={"Q4_K": 44, "FP8_B128": 32}, block_rows_any_down=36, _blocks_ok=lambda: True)
+        return [pre._expert_blocks(n) for n in (1, 512, 513, 576, 577, 704, 705)]
+    assert limit("Q4_K", "Q4_K") == limit("Q4_K", "FP8_B128") == [True] * 6 + [False]
+    assert limit("Q4_K", "NVFP4") == [True] * 4 + [False] * 3
+    assert limit("FP8_B128", "FP8_B128") == limit("FP8_B128", "Q8_0") == [True] * 2 + [False] * 5
+    assert not any(limit("NVFP4", "Q4_K"))
+
+
+@pytest.mark.parametrize("experts,hidden,most", [(16, 512, 64), (16, 640, 44), (18, 512, 64), (19, 512, 44), (74, 128, 64), (75, 128, 44)])
+def test_experts_whose_second_tiles_find_idle_processors_take_their_blocks_to_the_end_of_the_first(experts, hidden, most):
+    """Two tiles of every expert by 128 weight rows, on 148 processors."""
+    from types import SimpleNamespace as NS
+    from bloomery_b200.runtime.prefill import GemmPrefill
+    pre = object.__new__(GemmPrefill)
+    q = {f"blk.0.ffn_{n}_exps.weight": NS(qtype="Q4_K") for n in ("gate", "up", "down")}
+    spec = NS(is_moe=True, n_layer=1, n_used=1, n_expert=experts, hidden=hidden, moe_inter=128, layer_is_moe=lambda il: True)
+    vars(pre).update(e=NS(spec=spec, w=NS(q=q)), direct_rows=128, expert_source=None, _block_limit=None,
+                     block_rows={"Q4_K": 44}, block_rows_any_down=36, _blocks_ok=lambda: True)
+    assert pre._expert_blocks(most * experts) and not pre._expert_blocks(most * experts + 1)
 
 
 def test_other_threads_run_while_a_pass_is_awaited(monkeypatch):
